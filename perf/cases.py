@@ -3,13 +3,15 @@
 Each case is a dict of plain values; ``kind`` selects the path.  ``listed()`` names one representative of each use,
 ``draw(rng)`` gives another size of the same ranges, ``prepare`` builds what a program holds before the call, ``run`` is
 one pass, ``work`` its unavoidable bytes and operations, ``tolerance`` how far another correct implementation of the
-same precision may be.
+same precision may be, ``exact`` what the pass gives in 64 bits.
 """
 from __future__ import annotations
 
 import math
 
 import torch
+import torch.nn.functional as F
+from torch.utils.checkpoint import checkpoint
 
 import spiraltorch_b200 as st
 from spiraltorch_b200 import vision
@@ -304,3 +306,195 @@ def tolerance(case):
     if kind == "topk":
         return "exact"
     return {"rel": 1e-6, "max": 1e-5}           # measured: 8e-8, single values 4.4e-7
+
+
+# ---- 64-bit references ------------------------------------------------------------------------------------------------
+# The inputs and initial weights are those of ``prepare``; everything after that is plain torch in 64 bits.
+
+def _leaf(t):
+    return t.detach().double().requires_grad_(True)
+
+
+def _lm_exact(c, s):
+    model = s["trainer"].model if c["kind"] == "lm_train" else s["model"]
+    cfg, heads, dim = model.cfg, c["heads"], c["d"] // c["heads"]
+    w = {n: _leaf(p) for n, p in model.p.items()}
+    tokens = s["tokens"].to(DEV)
+    b, length = tokens.shape
+
+    def norm(x, name):
+        if cfg.norm == "rms":
+            return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + cfg.norm_eps) * w[name + ".gamma"]
+        return F.layer_norm(x, (c["d"],), w[name + ".gamma"], w[name + ".beta"], cfg.norm_eps)
+
+    half = torch.arange(0, dim, 2, dtype=torch.float64, device=DEV) / dim
+    angle = torch.arange(length, dtype=torch.float64, device=DEV)[:, None] / cfg.rope_base ** half
+    cos, sin = angle.cos(), angle.sin()
+
+    def turn(x):
+        if cfg.positional != "rope":
+            return x
+        u, v = x.chunk(2, -1)
+        return torch.cat([u * cos - v * sin, v * cos + u * sin], -1)
+
+    keys = torch.arange(length, device=DEV)
+    dead = keys[None, :] > keys[:, None]
+
+    def block(x, n):
+        qkv = (norm(x, f"h{n}.norm1") @ w[f"h{n}.qkv.weight"].t()).view(b, length, 3, heads, dim).permute(2, 0, 3, 1, 4)
+        q, k, v = turn(qkv[0]), turn(qkv[1]), qkv[2]
+        o = []
+        for i in range(b):
+            p = torch.softmax((q[i] @ k[i].transpose(-1, -2) / math.sqrt(dim)).masked_fill(dead, float("-inf")), -1)
+            o.append(p @ v[i])
+        o = torch.stack(o).transpose(1, 2).reshape(b, length, c["d"])
+        x = x + o @ w[f"h{n}.proj.weight"].t()
+        return x + F.gelu(norm(x, f"h{n}.norm2") @ w[f"h{n}.fc1.weight"].t(), approximate="tanh") @ w[f"h{n}.fc2.weight"].t()
+
+    x = w["embed.weight"][tokens]
+    if cfg.positional == "learned":
+        x = x + w["pos.weight"][:length]
+    for n in range(c["layers"]):
+        x = checkpoint(block, x, n, use_reentrant=False)
+    logits = norm(x, "norm_f").reshape(b * length, -1) @ w["embed.weight"].t()
+    if c["kind"] == "lm_logits":
+        return logits.detach()
+    loss = F.cross_entropy(logits, s["targets"].to(DEV).reshape(-1))
+    loss.backward()
+    opt = s["trainer"].optimizer
+    total = math.sqrt(sum(float(t.grad.pow(2).sum()) for t in w.values()))
+    clip = min(1.0, opt.max_grad_norm / (total + 1e-6)) if opt.max_grad_norm > 0 else 1.0
+    weights, moments = torch.zeros_like(opt.master, dtype=torch.float64), torch.zeros_like(opt.m, dtype=torch.float64)
+    for name, at, n, _ in model.named_flat_views():
+        g = w[name].grad.reshape(-1) * clip
+        old = w[name].detach().reshape(-1)
+        decay = opt.weight_decay if at < opt.decay_elems else 0.0
+        weights[at:at + n] = old - opt.lr * (g / (g.abs() + opt.eps) + decay * old)
+        moments[at:at + n] = (1 - opt.betas[0]) * g
+    return {"loss": loss.item(), "weights": weights, "moments": moments}
+
+
+def _conv_exact(c, s):
+    model = s["model"]
+    w = {n: _leaf(p) for n, p in model.p.items()}
+    x, ic = s["images"].double(), 3
+    for stage, oc in enumerate(STAGES):
+        for i in range(2):
+            k = w[f"conv{stage}_{i}.weight"].view(oc, 3, 3, ic).permute(0, 3, 1, 2)
+            x = torch.relu(F.conv2d(x, k, w[f"conv{stage}_{i}.bias"], padding=1))
+            ic = oc
+        x = F.max_pool2d(x, 2)
+    logits = (x.mean((2, 3)) @ w["head.weight"].t() + w["head.bias"])[:, :c["classes"]]
+    if c["kind"] == "conv_logits":
+        return logits.detach()
+    loss = F.cross_entropy(logits, s["labels"])
+    loss.backward()
+    weights, momentum = s["opt"].master.double(), torch.zeros_like(s["opt"].buf, dtype=torch.float64)
+    for name, (at, n, _) in model._offsets.items():
+        g = w[name].grad.reshape(-1)
+        momentum[at:at + n] = g
+        weights[at:at + n] -= s["opt"].lr * g
+    return {"loss": loss.item(), "weights": weights, "momentum": momentum}
+
+
+def _contrastive_exact(c, s):
+    p = [_leaf(t) for t in s["encoder"].parameters()]
+    weight, bias, gamma, beta = p[0:3], p[3:6], p[6:8], p[8:10]
+    g = torch.Generator(device=DEV).manual_seed(s["seed"])
+    noise = [torch.randn(s["base"].shape, generator=g, device=DEV) for _ in range(2)]
+
+    def embed(x):
+        for i in range(3):
+            x = x @ weight[i].t() + bias[i]
+            if i < 2:
+                x = F.gelu(F.layer_norm(x, (x.shape[-1],), gamma[i], beta[i], 1e-5), approximate="tanh")
+        return F.normalize(x, dim=-1)
+
+    a, b = (embed(s["base"].double() + 0.1 * n.double()) for n in noise)
+    loss = F.cross_entropy(a @ b.t() / 0.1, torch.arange(c["batch"], device=DEV))
+    loss.backward()
+    return [loss.item()] + [t.grad for t in p]
+
+
+def _attention_exact(c, s):
+    q, k, v = (_leaf(s[n]) for n in "qkv")
+    o, keys = [], torch.arange(c["seq"], device=DEV)
+    grads = [torch.empty_like(q) for _ in range(3)]
+    for i in range(c["contexts"]):
+        n = int(s["lengths"][i]) if c["lengths"] else c["seq"]
+        score = q[i, :n] @ k[i, :n].t() / math.sqrt(c["dim"])
+        if c["z_bias"]:
+            score = score + s["z_bias"][i, :n].double()
+        if c["causal"]:
+            score = score.masked_fill(keys[None, :n] > keys[:n, None], float("-inf"))
+        y = F.pad(torch.softmax(score, -1) @ v[i, :n], (0, 0, 0, c["seq"] - n))
+        for g, t in zip(grads, torch.autograd.grad(y, (q, k, v), s["grad"][i].double())):
+            g[i] = t[i]
+        o.append(y.detach())
+    return (torch.stack(o), *grads)
+
+
+def _mlp_exact(c, s):
+    p = [t.value.double() for t in s["net"].parameters()]     # fc1 weight and bias, gain, offset, head weight and bias
+    total = 0.0
+    for x, y in s["batches"]:
+        leaf = [_leaf(t) for t in p]
+        h = torch.relu(F.layer_norm(x.torch().double() @ leaf[0] + leaf[1], (c["hidden"],), leaf[2].reshape(-1), leaf[3].reshape(-1), 1e-5))
+        loss = F.mse_loss(h @ leaf[4] + leaf[5], y.torch().double())
+        p = [t.detach() - 1e-2 / c["batch"] * g for t, g in zip(leaf, torch.autograd.grad(loss, leaf))]
+        total += loss.item()
+    return [total / c["batches"]] + p
+
+
+def _rnn_exact(c, s):
+    leaf = [_leaf(t.value) for t in s["net"].parameters()]    # input weights, recurrent weights, bias, head weight and bias
+    x, hidden = _leaf(s["x"].torch()), c["hidden"]
+    h = cell = torch.zeros(c["batch"], hidden, dtype=torch.float64, device=DEV)
+    past = []
+    for t in range(c["steps"]):
+        into = h + past[t - 2] if c["cell"] == "wave" and t >= 2 else h
+        z = x[:, t * c["in"]:(t + 1) * c["in"]] @ leaf[0] + into @ leaf[1] + leaf[2]
+        if c["cell"] == "tanh":
+            h = torch.tanh(z)
+        elif c["cell"] == "wave":
+            h = torch.tanh(z[:, :hidden]) * torch.sigmoid(z[:, hidden:])
+        else:
+            i, f, g, o = z.chunk(4, 1)
+            cell = torch.sigmoid(f) * cell + torch.sigmoid(i) * torch.tanh(g)
+            h = torch.sigmoid(o) * torch.tanh(cell)
+        past.append(h)
+    loss = F.mse_loss(h @ leaf[3] + leaf[4], s["y"].torch().double())
+    dx, *grads = torch.autograd.grad(loss, [x] + leaf)
+    return [loss.detach().reshape(1, 1), dx] + [t.detach() - 1e-2 / c["batch"] * g for t, g in zip(leaf, grads)]
+
+
+def _image_exact(c, s):
+    x, r = s["photo"].to(DEV).double(), c["resize_to"]
+    means = (x * 1.1).mean((0, 2, 3)).view(1, 3, 1, 1)
+    x = F.interpolate(x, (r, r), mode="bilinear", align_corners=False)
+    at = (r - c["size"]) // 2
+    x = x[:, :, at:at + c["size"], at:at + c["size"]] * 1.1
+    x = (x - means) * 1.1 + means
+    gray = (x * torch.tensor([0.29899597, 0.587096, 0.11390703], dtype=torch.float64, device=DEV).view(1, 3, 1, 1)).sum(1, keepdim=True)
+    red, green, blue = ((x - gray) * 1.1 + gray).unbind(1)
+    y = 0.299 * red + 0.587 * green + 0.114 * blue
+    u, v = -0.14713 * red - 0.28886 * green + 0.436 * blue, 0.615 * red - 0.51499 * green - 0.10001 * blue
+    u, v = u * math.cos(0.05) - v * math.sin(0.05), u * math.sin(0.05) + v * math.cos(0.05)
+    return torch.stack([y + 1.13983 * v, y - 0.39465 * u - 0.5806 * v, y + 2.03211 * u], 1).flip(-1).cpu()
+
+
+def exact(case, seed):
+    """The outputs of ``run`` in 64 bits; ``None`` for a selection, whose values are inputs, and for work of over 4e14
+    operations."""
+    c, kind = case, case["kind"]
+    if kind == "topk" or work(case)["flops"] > 4e14:
+        return None
+    s = prepare(case, seed)
+    if kind == "fft":
+        z = torch.fft.fft(s["x"].to(torch.complex128))
+        return z, torch.fft.ifft(z)
+    form = {"lm_train": _lm_exact, "lm_logits": _lm_exact, "conv_train": _conv_exact, "conv_logits": _conv_exact,
+            "contrastive": _contrastive_exact, "attention": _attention_exact, "mlp": _mlp_exact, "rnn": _rnn_exact,
+            "image": _image_exact}[kind]
+    with torch.set_grad_enabled(kind not in ("lm_logits", "conv_logits", "image")):
+        return form(c, s)
