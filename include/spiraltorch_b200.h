@@ -281,6 +281,8 @@ int st_norm_fwd(int rms, const void* x, const void* residual, const void* gamma,
 int st_poincare_project(const float* x, float* y, int rows, int cols, float curvature, void* stream_v);   /* csrc/optim/optim.cu */
 int st_preprocess(const float* in, float* out, const StPreprocessArgs* a, void* stream_v);   /* csrc/vision/vision.cu */
 int st_rank_select(const float* in, float* out_v, int* out_i, int rows, int cols, int k, int mode, void* stream_v);   /* csrc/rank/rank.cu */
+int st_rank_topk(const float* in, float* out_v, int* out_i, int rows, int cols, int k, int mode, void* workspace, void* stream_v);   /* csrc/rank/rank.cu */
+long long st_rank_topk_workspace(int rows, int cols, int k);   /* csrc/rank/rank.cu */
 int st_read_error_word(unsigned* out, int clear);   /* csrc/runtime/runtime.cu */
 int st_rnn_scan(const StRnnScanArgs* a, void* stream_v);   /* csrc/recurrent/scan.cu */
 int st_rnn_scan_supported(int H, int cell);   /* csrc/recurrent/scan.cu */

@@ -3,10 +3,12 @@
 CUDA tensors run ``csrc/rank/rank.cu``; CPU tensors run a PyTorch restatement of the
 reference's CPU mirror (crates/st-core/src/backend/rankk_software.rs:38-110): non-finite
 entries are ignored, ties go to the lower column index, unused slots are ``NaN`` / ``-1``.
+Top / bottom with ``k <= 128`` stream rows of any length past candidate lists in registers; mid and larger ``k`` select
+inside one CTA's shared memory.
 
 ``plan_rank`` returns a small plan object in the spirit of ``plan_rank`` /
-``RankPlan`` (crates/st-core/src/ops/rank_entry.rs): on sm_100a the choices are fixed (one CTA
-per row, shared-memory bitonic network, block arg-max for k = 1), so the plan only records them.
+``RankPlan`` (crates/st-core/src/ops/rank_entry.rs).  It names the reference's families (bitonic network, two stages,
+arg-max) and their sizes; which kernel form runs follows from the sizes alone.
 
 ``distributed_topk`` is the three-stage scheme of crates/st-core/src/distributed/topk3_stage.rs:
 local select → all-gather of the ``(value, index)`` candidates → exact merge
@@ -92,8 +94,6 @@ def rank_select(x: torch.Tensor, k: int, kind: str = "topk", choice=None):
     global launch_count
     mode = MODES[kind]
     rows, cols = x.shape
-    if choice is None and mode != 2 and k > 1 and 1024 <= cols <= MAX_KERNEL_COLS and native.use_native(x):
-        choice = _tuned_choice(rows, cols, k, kind)
     if choice is not None and choice.use_2ce and mode != 2 and 0 < k and native.use_native(x) and cols <= MAX_KERNEL_COLS \
             and 0 < choice.tile < cols and -(-cols // choice.tile) * min(k, choice.tile) < cols:
         return _rank_select_two_stage(x, k, kind, chunk=choice.tile)
@@ -101,44 +101,36 @@ def rank_select(x: torch.Tensor, k: int, kind: str = "topk", choice=None):
         raise ValueError(f"k={k} exceeds cols={cols}")
     if not native.use_native(x):
         return rank_select_reference(x, k, mode)
-    if cols > MAX_KERNEL_COLS:
+    wide = cols > MAX_KERNEL_COLS
+    if wide and not (mode != 2 and 0 < k <= MAX_LIST_K):
         if mode == 2 or k == 0:
             return rank_select_reference(x, k, mode)     # mid-k needs the global order statistics
         return _rank_select_two_stage(x, k, kind)
     xf = x.float().contiguous()
     out_v = torch.empty((rows, k), dtype=torch.float32, device=x.device)
     out_i = torch.empty((rows, k), dtype=torch.int32, device=x.device)
-    st = native.lib().st_rank_select(native.ptr(xf), native.ptr(out_v), native.ptr(out_i), ctypes.c_int(rows),
-                                     ctypes.c_int(cols), ctypes.c_int(k), ctypes.c_int(mode),
-                                     native.stream_ptr(x.device))
-    native.check(st, "st_rank_select")
-    launch_count += 1
+    dims = (ctypes.c_int(rows), ctypes.c_int(cols), ctypes.c_int(k))
+    lib = native.lib()
+    if wide:
+        lib.st_rank_topk_workspace.restype = ctypes.c_longlong
+        words = lib.st_rank_topk_workspace(*dims)
+        lists = torch.empty(words, dtype=torch.int64, device=x.device) if words else None
+        native.check(lib.st_rank_topk(native.ptr(xf), native.ptr(out_v), native.ptr(out_i), *dims, ctypes.c_int(mode),
+                                      native.ptr(lists), native.stream_ptr(x.device)), "st_rank_topk")
+        launch_count += 2 if words else 1
+    else:
+        native.check(lib.st_rank_select(native.ptr(xf), native.ptr(out_v), native.ptr(out_i), *dims, ctypes.c_int(mode),
+                                        native.stream_ptr(x.device)), "st_rank_select")
+        launch_count += 1
     return out_v, out_i
 
 
-_choice_cache: dict = {}
-
-
-def _tuned_choice(rows: int, cols: int, k: int, kind: str):
-    """The three-voice chooser's pick for this shape (cached per power-of-two row bucket): on rows of 1024 to 8192
-    columns the tuned table often prefers per-chunk candidates + merge over one full-width sort."""
-    key = (1 << max(rows - 1, 0).bit_length(), cols, k, MODES[kind])
-    hit = _choice_cache.get(key)
-    if hit is None:
-        from .. import unison
-        from ..device_caps import DeviceCaps
-        hit = unison.choose_unified_rank(rows, cols, k, DeviceCaps.cuda(), "topk" if MODES[kind] == 0 else "bottomk").choice
-        if len(_choice_cache) > 4096:
-            _choice_cache.clear()
-        _choice_cache[key] = hit
-    return hit
-
-
-MAX_KERNEL_COLS = 8192      # one CTA sorts a row of at most this many (value, index) keys in shared memory
+MAX_KERNEL_COLS = 8192      # one CTA holds a row of at most this many values in shared memory
+MAX_LIST_K = 128            # top / bottom of at most this many: warps stream a row of any length past lists in registers
 
 
 def _rank_select_two_stage(x: torch.Tensor, k: int, kind: str, chunk: int = 0):
-    """Rows wider than one CTA's shared-memory sort: select per column chunk, then select among the candidates
+    """Rows wider than one CTA's shared-memory sort with k above the warp lists: select per column chunk, then among the candidates
     (the reference's two-stage path: rankk_exact_2ce.wgsl, crates/st-core/src/distributed/topk3_stage.rs:56).
     Exact, including the tie rule: candidates keep chunk order and, inside a chunk, the kernel's own order, so
     equal values still resolve to the lower column."""

@@ -68,6 +68,31 @@ def test_rank_two_stage_for_wide_rows_matches_cpu(rows, cols, k):
     assert R.plan_rank("topk", rows, cols, k, backend="cuda").kernel.startswith("two_stage")
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,k", [(1, 33, 1), (3, 64, 31), (9, 127, 32), (2600, 130, 33), (5, 511, 64), (5, 513, 65), (2, 2048, 128),
+                                         (70, 8192, 128), (6, 8190, 129), (2, 8193, 32), (80, 8196, 7), (1, 50001, 128), (3, 30000, 2)])
+def test_rank_forms_at_their_edges(rows, cols, k):
+    """List lengths 32 / 64 / 128 and the step past them, odd and unaligned rows, one to 32 warps per row and rows split
+    over CTAs; ties, infinities and NaN included.  Selections are exact."""
+    torch.manual_seed(rows + cols)
+    x = torch.randn(rows * cols + 1)
+    x = (x * 4).round() / 4 if cols % 2 else x                  # many ties in the odd cases
+    x[torch.randint(0, x.numel(), (rows * cols // 50 + 1,))] = float("inf")
+    x[torch.randint(0, x.numel(), (rows * cols // 50 + 1,))] = -float("inf")
+    x[torch.randint(0, x.numel(), (rows * cols // 50 + 1,))] = float("nan")
+    x = x + 0.0                                                 # one zero: the CPU form does not order -0 and +0
+    for at in (0, 1):                                           # rows at 16-byte boundaries, and off them
+        h = x[at:at + rows * cols].view(rows, cols).clone()
+        d = x.cuda()[at:at + rows * cols].view(rows, cols)
+        h[0], d[0] = 1.5, 1.5                                   # a row of equal values
+        h[-1, k // 2:], d[-1, k // 2:] = float("nan"), float("nan")    # a row with fewer values than k
+        for kind in ("topk", "bottomk") + (("midk",) if cols <= 8192 else ()):
+            cv, ci = R.rank_select(h, k, kind)
+            gv, gi = R.rank_select(d, k, kind)
+            assert torch.equal(ci, gi.cpu()), (kind, at)
+            assert torch.equal(torch.nan_to_num(cv, nan=-7.0), torch.nan_to_num(gv.cpu(), nan=-7.0))
+
+
 @pytest.mark.parametrize("dev", _dev_params())
 def test_compaction(dev):
     x = torch.tensor([[0.1, 5.0, 0.3, NAN, 0.2, -1.0], [9.0, 9.0, 9.0, 9.0, 9.0, 9.0]], device=dev)
