@@ -66,24 +66,70 @@ bool nhwc_map(CUtensorMap* out, const void* base, int N, int H, int W, int C, in
   return encode_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-__global__ void im2col3x3_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col,
-                                       int N, int H, int W, int C, int Kpad) {
-  const long long total = (long long)N * H * W * Kpad;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int k = i % Kpad;
-    const long long pix = i / Kpad;
-    const int w = pix % W;
-    const int h = (pix / W) % H;
-    const int n = pix / ((long long)W * H);
-    __nv_bfloat16 v = __float2bfloat16(0.0f);
-    if (k < 9 * C) {
-      const int tap = k / C, c = k - tap * C;
-      const int hh = h + tap / 3 - 1, ww = w + tap % 3 - 1;
-      if (hh >= 0 && hh < H && ww >= 0 && ww < W) v = x[(((long long)n * H + hh) * W + ww) * C + c];
+// One thread writes eight neighbouring entries of a pixel's row of the column matrix with one 16-byte store: the bound is
+// that store (67 MB and 230 us before for 256 images of 64 x 64 x 3, one 2-byte store and four divisions per entry).
+// The index is 32-bit where the matrix allows it: 64-bit divisions took 61 us here.
+template <typename Index>
+__global__ void __launch_bounds__(256)
+im2col3x3_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col,
+                       int N, int H, int W, int C, int Kpad, int aligned) {
+  const int K8 = Kpad / 8;
+  const Index total = (Index)N * H * W * K8;
+  for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (Index)gridDim.x * blockDim.x) {
+    const int k0 = (int)(i % K8) * 8;
+    const Index pix = i / K8;
+    const int w = (int)(pix % W);
+    const int h = (int)((pix / W) % H);
+    int tap = k0 / C, c = k0 - tap * C;
+    __nv_bfloat16 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = __float2bfloat16(0.0f);
+      const int dh = tap / 3 - 1, dw = tap % 3 - 1;
+      if (tap < 9 && h + dh >= 0 && h + dh < H && w + dw >= 0 && w + dw < W) v[j] = x[((long long)pix + dh * W + dw) * C + c];
+      if (++c == C) { c = 0; ++tap; }
     }
+    if (aligned) {
+      uint4 u;
+      u.x = __bfloat16_as_ushort(v[0]) | (uint32_t)__bfloat16_as_ushort(v[1]) << 16;
+      u.y = __bfloat16_as_ushort(v[2]) | (uint32_t)__bfloat16_as_ushort(v[3]) << 16;
+      u.z = __bfloat16_as_ushort(v[4]) | (uint32_t)__bfloat16_as_ushort(v[5]) << 16;
+      u.w = __bfloat16_as_ushort(v[6]) | (uint32_t)__bfloat16_as_ushort(v[7]) << 16;
+      *reinterpret_cast<uint4*>(col + (long long)i * 8) = u;
+    } else {
+      for (int j = 0; j < 8; ++j) col[(long long)i * 8 + j] = v[j];
+    }
+  }
+}
+
+// The same with C % 8 == 0 and 16-byte aligned input: eight channels of one tap are one load and one store.
+template <typename Index>
+__global__ void __launch_bounds__(256)
+im2col3x3_c8_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, int N, int H, int W, int C8, int K8) {
+  const Index total = (Index)N * H * W * K8;
+  for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (Index)gridDim.x * blockDim.x) {
+    const int k = (int)(i % K8);
+    const Index pix = i / K8;
+    const int w = (int)(pix % W);
+    const int h = (int)((pix / W) % H);
+    const int tap = k / C8, c = k - tap * C8;
+    const int dh = tap / 3 - 1, dw = tap % 3 - 1;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (tap < 9 && h + dh >= 0 && h + dh < H && w + dw >= 0 && w + dw < W) v = x[((long long)pix + dh * W + dw) * C8 + c];
     col[i] = v;
   }
+}
+
+// Weights of the data-gradient convolution: out[ic][8 - tap][oc] = in[oc][tap][ic], 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256)
+dgrad_weights_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int OC, int IC) {
+  __shared__ __nv_bfloat16 tile[32][33];
+  const int tap = blockIdx.z, ic0 = blockIdx.x * 32, oc0 = blockIdx.y * 32;
+  for (int r = threadIdx.y; r < 32; r += 8)
+    if (oc0 + r < OC && ic0 + threadIdx.x < IC) tile[r][threadIdx.x] = in[((long long)(oc0 + r) * 9 + tap) * IC + ic0 + threadIdx.x];
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += 8)
+    if (ic0 + r < IC && oc0 + threadIdx.x < OC) out[((long long)(ic0 + r) * 9 + 8 - tap) * OC + oc0 + threadIdx.x] = tile[threadIdx.x][r];
 }
 
 // Eight channels per thread (16-byte loads, one 16-byte store of y and one 8-byte store of idx); C % 8 == 0.
@@ -157,6 +203,69 @@ __global__ void maxpool2_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bf
   }
 }
 
+// Eight channels per thread; C % 8 == 0 and 16-byte aligned tensors.  With `pooled` (the forward's output) the gradient
+// is also masked where the pooled value is not positive, which is the ReLU in front of the pool: only the arg-max of a
+// window receives a gradient, and its value is the pooled one.  With `dbias` the masked gradient's channel sums are added
+// to it: each thread keeps to one group of eight channels (C / 8 divides the block), so the sums stay in registers.
+// Bound by its bytes: 134 MB written and 84 MB read for 256 x 64 x 64 x 64; the scalar kernel, the mask and the column
+// sums took 318 us in five launches.
+__global__ void __launch_bounds__(256)
+maxpool2_bwd8_kernel(const uint4* __restrict__ dy, const uint2* __restrict__ idx, const uint4* __restrict__ pooled,
+                     uint4* __restrict__ dx, float* __restrict__ dbias, int N, int H, int W, int C8) {
+  const int OH = H / 2, OW = W / 2;
+  const long long total = (long long)N * OH * OW * C8;
+  float sum[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sum[j] = 0.0f;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)(i % C8);
+    const long long p = i / C8;
+    const int ow = (int)(p % OW);
+    const long long nh = p / OW;                     // image * OH + row: the window's first row is 2 nh of N * H
+    const uint4 gv = dy[i];
+    const uint2 av = idx[i];
+    uint32_t g[4] = {gv.x, gv.y, gv.z, gv.w};
+    if (pooled) {
+      const uint4 yv = pooled[i];
+      const uint32_t y[4] = {yv.x, yv.y, yv.z, yv.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 f = unpack_bf16x2(y[q]);
+        g[q] &= (f.x > 0.0f ? 0x0000FFFFu : 0u) | (f.y > 0.0f ? 0xFFFF0000u : 0u);
+      }
+    }
+    if (dbias) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 f = unpack_bf16x2(g[q]);
+        sum[2 * q] += f.x;
+        sum[2 * q + 1] += f.y;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      uint32_t o[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t a = (q < 2 ? av.x : av.y) >> ((q & 1) * 16);     // arg-max of channels 2 q and 2 q + 1
+        o[q] = g[q] & (((a & 0xFFu) == t ? 0x0000FFFFu : 0u) | (((a >> 8) & 0xFFu) == t ? 0xFFFF0000u : 0u));
+      }
+      dx[((2 * nh + (t >> 1)) * W + 2 * ow + (t & 1)) * C8 + c] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  if (!dbias) return;
+  __shared__ float sh[256 * 8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sh[threadIdx.x * 8 + j] = sum[j];
+  __syncthreads();
+  for (int ch = threadIdx.x; ch < C8 * 8; ch += 256) {                  // thread t owns channels of group t % C8
+    float s = 0.0f;
+    for (int t = ch >> 3; t < 256; t += C8) s += sh[t * 8 + (ch & 7)];
+    atomicAdd(dbias + ch, s);
+  }
+}
+
 __global__ void maxpool2_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const unsigned char* __restrict__ idx,
                                     __nv_bfloat16* __restrict__ dx, int N, int H, int W, int C) {
   const int OH = H / 2, OW = W / 2;
@@ -227,11 +336,11 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   const int P = a->N * a->H * a->W;
   CUtensorMap tmA, tmB;
   if (!nhwc_map(&tmA, a->x, a->N, a->H, a->W, a->C, a->W, Hb, Nb)) return ST_ERR_CUDA;
-  const bool small = a->OC <= 128;
+  const int BN = a->OC <= 64 ? 64 : (a->OC <= 128 ? 128 : 256);
   {
     uint64_t dims[3] = {(uint64_t)9 * a->C, (uint64_t)a->OC, 1};
     uint64_t strides[2] = {(uint64_t)9 * a->C * 2, (uint64_t)9 * a->C * 2 * a->OC};
-    uint32_t box[3] = {BK, (uint32_t)(small ? 128 : 256), 1};
+    uint32_t box[3] = {BK, (uint32_t)BN, 1};
     if (!encode_tmap(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
   }
@@ -257,7 +366,8 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   p.use_tma_store = 1;
   p.err = st::error_word();
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (small) return launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s);
+  if (BN == 64) return launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s);
+  if (BN == 128) return launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, false, false>(tmA, tmB, tmC, p, s);
 }
 
@@ -277,8 +387,7 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "conv3x3_wgrad: image width must divide 64 and the batch must fill whole pixel blocks");
   const int P = a->N * a->H * a->W;
   const int kblocks_total = P / BK;
-  const bool small = a->C <= 128;
-  const int BNv = small ? 128 : 256;
+  const int BNv = a->C <= 64 ? 64 : (a->C <= 128 ? 128 : 256);
   const int tiles = ((a->OC + BM - 1) / BM) * ((a->C + BNv - 1) / BNv) * 9;
   int splits = a->splits;
   if (splits <= 0) {
@@ -307,15 +416,25 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
   p.out_fp32 = 1; p.accumulate = 2;
   p.err = st::error_word();
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (small) return launch_gemm<128, 6, true, true>(tmA, tmB, tmC, p, s);
+  if (BNv == 64) return launch_gemm<64, 8, true, true>(tmA, tmB, tmC, p, s);
+  if (BNv == 128) return launch_gemm<128, 6, true, true>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, true, true>(tmA, tmB, tmC, p, s);
 }
 
 ST_API int st_im2col3x3_small(const void* x, void* col, int N, int H, int W, int C, int Kpad, void* stream_v) {
   if (9 * C > Kpad || (Kpad & 7)) return st::fail(ST_ERR_INVALID, "im2col: Kpad must be a multiple of 8 and >= 9*C");
-  const long long total = (long long)N * H * W * Kpad;
-  im2col3x3_small_kernel<<<grid_for(total, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), N, H, W, C, Kpad);
+  const bool aligned = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
+  const long long total = (long long)N * H * W * (Kpad / 8);
+  const int grid = grid_for(total, 256);
+  const bool narrow = total + (long long)grid * 256 < (1ll << 31);     // the last step's index must not wrap either
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  if (aligned && (C & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    auto kern = narrow ? im2col3x3_c8_kernel<unsigned> : im2col3x3_c8_kernel<long long>;
+    kern<<<grid, 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<uint4*>(col), N, H, W, C / 8, Kpad / 8);
+  } else {
+    auto kern = narrow ? im2col3x3_small_kernel<unsigned> : im2col3x3_small_kernel<long long>;
+    kern<<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), N, H, W, C, Kpad, aligned);
+  }
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -336,7 +455,40 @@ ST_API int st_maxpool2_fwd(const void* x, void* y, void* idx, int N, int H, int 
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
+// Weights [OC][9][IC] (tap-major) to those of the data gradient, [IC][9][OC] with the taps reversed.
+ST_API int st_conv3x3_dgrad_weights(const void* w, void* wt, int OC, int IC, void* stream_v) {
+  if (!w || !wt || OC <= 0 || IC <= 0) return st::fail(ST_ERR_INVALID, "conv3x3_dgrad_weights: bad arguments");
+  dgrad_weights_kernel<<<dim3((IC + 31) / 32, (OC + 31) / 32, 9), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(wt), OC, IC);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+// Backward of ReLU followed by the pool: dx, and the channel sums of dx added to dbias (fp32 [C], may be null).  Needs
+// C / 8 to divide 256 and 16-byte aligned tensors.
+ST_API int st_maxpool2_relu_bwd(const void* dy, const void* idx, const void* pooled, void* dx, float* dbias, int N, int H,
+                                int W, int C, void* stream_v) {
+  if (!dy || !idx || !pooled || !dx || N <= 0) return st::fail(ST_ERR_INVALID, "maxpool2_relu_bwd: bad arguments");
+  if ((H & 1) || (W & 1) || (C & 7) || C <= 0 || 256 % (C / 8) != 0)
+    return st::fail(ST_ERR_INVALID, "maxpool2_relu_bwd: H and W must be even and C / 8 must divide 256");
+  if (((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(pooled) | reinterpret_cast<uintptr_t>(dx)) & 15) ||
+      (reinterpret_cast<uintptr_t>(idx) & 7))
+    return st::fail(ST_ERR_INVALID, "maxpool2_relu_bwd: tensors must be 16-byte aligned");
+  maxpool2_bwd8_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+      static_cast<const uint4*>(dy), static_cast<const uint2*>(idx), static_cast<const uint4*>(pooled),
+      static_cast<uint4*>(dx), dbias, N, H, W, C / 8);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
 ST_API int st_maxpool2_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, void* stream_v) {
+  if ((H & 1) == 0 && (W & 1) == 0 && (C & 7) == 0 &&
+      ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0 && (reinterpret_cast<uintptr_t>(idx) & 7) == 0) {
+    maxpool2_bwd8_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+        static_cast<const uint4*>(dy), static_cast<const uint2*>(idx), nullptr, static_cast<uint4*>(dx), nullptr, N, H, W, C / 8);
+    ST_CUDA_CHECK(cudaGetLastError());
+    return ST_OK;
+  }
   maxpool2_bwd_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0,
                         reinterpret_cast<cudaStream_t>(stream_v)>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const unsigned char*>(idx), static_cast<__nv_bfloat16*>(dx),

@@ -107,12 +107,15 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __rest
   if (threadIdx.x == 0 && cc < cols) atomicAdd(out + cc, t);
 }
 
-// Vectorised variant: each thread owns 8 adjacent columns (one 16-byte load per row) and block.y = 8
-// row lanes; four rows are in flight per thread.  Needs cols % 8 == 0 and 16-byte aligned rows.
+// Vectorised variant: each thread owns 8 adjacent columns (one 16-byte load per row); blockDim.x threads cover the
+// columns of the block and the rest of the 256 are row lanes, so narrow matrices (64 channels: 8 of 32 threads had
+// columns, 47 us for 134 MB) keep every thread loading.  Four rows are in flight per thread.  Needs cols % 8 == 0 and
+// 16-byte aligned rows.
 __global__ void __launch_bounds__(256)
 colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long rows, int cols, long long ld) {
-  __shared__ float sh[8][32 * 8 + 1];
-  const int c0 = (blockIdx.x * 32 + threadIdx.x) * 8;
+  __shared__ float sh[256 * 8 + 32];
+  const int lanes = blockDim.y, width = blockDim.x * 8;
+  const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   const long long rows_per = (rows + gridDim.y - 1) / gridDim.y;
   const long long r0 = blockIdx.y * rows_per;
   const long long r1 = min(rows, r0 + rows_per);
@@ -121,10 +124,10 @@ colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, lon
   for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
   if (c0 < cols) {
     long long r = r0 + threadIdx.y;
-    for (; r + 24 < r1; r += 32) {
+    for (; r + 3 * lanes < r1; r += 4 * lanes) {
       uint4 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (r + 8 * u) * ld + c0);
+      for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (r + lanes * u) * ld + c0);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
@@ -136,7 +139,7 @@ colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, lon
         }
       }
     }
-    for (; r < r1; r += 8) {
+    for (; r < r1; r += lanes) {
       const uint4 v = *reinterpret_cast<const uint4*>(x + r * ld + c0);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -148,13 +151,13 @@ colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, lon
     }
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) sh[threadIdx.y][threadIdx.x * 8 + j] = acc[j];
+  for (int j = 0; j < 8; ++j) sh[threadIdx.y * (width + 1) + threadIdx.x * 8 + j] = acc[j];
   __syncthreads();
-  const int t = threadIdx.y * 32 + threadIdx.x;   // 256 threads, one column each
+  const int t = threadIdx.y * blockDim.x + threadIdx.x;
+  if (t >= width) return;
   float s = 0.0f;
-#pragma unroll
-  for (int y = 0; y < 8; ++y) s += sh[y][t];
-  const int c = blockIdx.x * 256 + t;
+  for (int y = 0; y < lanes; ++y) s += sh[y * (width + 1) + t];
+  const int c = blockIdx.x * width + t;
   if (c < cols) atomicAdd(out + c, s);
 }
 
@@ -555,7 +558,9 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
     int chunks = (int)((rows + 255) / 256);
     if (chunks < 1) chunks = 1;
     if (chunks > 512) chunks = 512;
-    colsum8_kernel<<<dim3((cols + 255) / 256, chunks), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+    int bx = 8;
+    while (bx < 32 && bx * 8 < cols) bx <<= 1;
+    colsum8_kernel<<<dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
         static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;

@@ -316,125 +316,181 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = gemm_bid; t < total_tiles && ok; t += grid_stride) {
-        int b, tm, tn;
-        map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
-        const int m0 = tm * BM, n0 = tn * BN;
-        const CUtensorMap* mapA = &tmA;
-        int m_coord = m0;
-        if constexpr (COMM == COMM_AG) {
-          const int src = m0 / cm.rows_per_chunk;
-          const int sub = (m0 - src * cm.rows_per_chunk) / (cm.rows_per_chunk / cm.sub_per_chunk);
-          if (src == cm.g.rank) {
-            // the local rows are read from the shard itself; nothing to wait for
-            mapA = &tmA_local;
-            m_coord = m0 - src * cm.rows_per_chunk;
-          } else if (!wait_flag_ge(cm.g.signals[cm.g.rank] + cm.slot_arrive + src * kMaxSubChunks + sub,
-                                   cm.arrive_target)) {
-            *abort_flag = 1;
-            report_error(p.err, ERR_FLAG_TIMEOUT, 0xA601u);
-            break;
+    // The whole warp walks the schedule and one lane issues.  With warp-uniform control flow the loop's addresses and
+    // coordinates sit in uniform registers, which TMA and tcgen05 instructions read; issued from inside a one-lane
+    // branch, with descriptors rebuilt per instruction, these two loops set the pace of short or narrow K blocks: the weight
+    // gradient of a 64-channel 3x3 convolution over a million pixels took 315 us and takes 240, a training step of the
+    // conv classifier (256 x 64 x 64) 2.55 ms and takes 2.27.  Wide products of the language models did not change.
+    const bool leader = COMM == COMM_AG ? lane == 0 : elect_one();
+    const uint32_t smem0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+    const uint32_t full0 = __shfl_sync(0xffffffffu, smem_u32(full_bar), 0);
+    const uint32_t empty0 = full0 + STAGES * 8;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = gemm_bid; t < total_tiles && ok; t += grid_stride) {
+      int b, tm, tn;
+      map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
+      const int m0 = tm * BM, n0 = tn * BN;
+      const CUtensorMap* mapA = &tmA;
+      int m_coord = m0;
+      if constexpr (COMM == COMM_AG) {
+        const int src = m0 / cm.rows_per_chunk;
+        const int sub = (m0 - src * cm.rows_per_chunk) / (cm.rows_per_chunk / cm.sub_per_chunk);
+        if (src == cm.g.rank) {
+          // the local rows are read from the shard itself; nothing to wait for
+          mapA = &tmA_local;
+          m_coord = m0 - src * cm.rows_per_chunk;
+        } else {
+          bool landed = true;
+          if (leader) {
+            landed = wait_flag_ge(cm.g.signals[cm.g.rank] + cm.slot_arrive + src * kMaxSubChunks + sub, cm.arrive_target);
+            if (!landed) {
+              *abort_flag = 1;
+              report_error(p.err, ERR_FLAG_TIMEOUT, 0xA601u);
+            }
           }
-          fence_proxy_async_global();
+          if (!__all_sync(0xffffffffu, landed)) break;
         }
+        if (leader) fence_proxy_async_global();
+      }
+      // one K block per ring stage: wait until its MMAs have read it, then hand the copies to the TMA unit
+      auto k_loop = [&](uint32_t bytes, auto&& copies) {
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          const uint32_t fb = smem_u32(&full_bar[stage]);
-          mbar_arrive_expect_tx(fb, L::STAGE_BYTES);
-          const uint32_t sa = smem_u32(smem + stage * L::STAGE_BYTES);
-          const uint32_t sb = sa + L::A_BYTES;
-          const int k0 = kb * BK;
-          if (p.conv.mode == 1) {
-            // A: 128 output pixels (Nb images x Hb rows x W) shifted by the tap, 64 channels
-            const int tap = kb / p.conv.c_chunks, cc = kb - tap * p.conv.c_chunks;
-            const int hblocks = p.conv.H / p.conv.Hb;
-            const int img0 = (tm / hblocks) * p.conv.Nb, h0 = (tm % hblocks) * p.conv.Hb;
-            tma_load_4d(sa, mapA, fb, cc * 64, tap % 3 - 1, h0 + tap / 3 - 1, img0);
-            tma_load_3d(sb, &tmB, fb, k0, n0, 0);
-          } else if (p.conv.mode == 2) {
-            // batch index = tap + taps * split; K block = 64 consecutive pixels
-            const int tap = b % p.conv.taps, split = b / p.conv.taps;
-            const int kg = split * k_blocks + kb;                  // global pixel block
-            const int hblocks = p.conv.H / p.conv.Hb;
-            const int img0 = (kg / hblocks) * p.conv.Nb, h0 = (kg % hblocks) * p.conv.Hb;
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kg * BK, 0);
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_4d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, tap % 3 - 1, h0 + tap / 3 - 1, img0);
-          } else {
-            if constexpr (!A_MN) {
-              tma_load_3d(sa, mapA, fb, k0, m_coord, b);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BM / 64; ++j)
-                tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, k0, b);
-            }
-            if constexpr (!B_MN) {
-              tma_load_3d(sb, &tmB, fb, k0, n0, b);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_3d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, k0, b);
-            }
-          }
+          if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u, abort_flag)) return false;
+          const uint32_t fb = full0 + stage * 8;
+          const uint32_t sa = smem0 + stage * L::STAGE_BYTES;
+          if (leader) mbar_arrive_expect_tx(fb, bytes);
+          copies(kb, fb, sa, sa + L::A_BYTES);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
+        return true;
+      };
+      // MN-major operands arrive as 64-wide boxes: a box wholly outside the matrix is not fetched (what the shared
+      // memory holds in its place only reaches rows or columns of the accumulator that are never stored)
+      const int boxes_a = (A_MN && COMM == COMM_NONE) ? min(BM / 64, (p.M - m0 + 63) / 64) : BM / 64;
+      const int boxes_b = (B_MN && COMM == COMM_NONE) ? min(BN / 64, (p.N - n0 + 63) / 64) : BN / 64;
+      const bool whole = boxes_a == BM / 64 && boxes_b == BN / 64;
+      const uint32_t stage_bytes = (boxes_a + boxes_b) * (64 * BK * 2);
+      // Convolution coordinates advance by additions: six divisions per K block took about 950 SM cycles, twice the
+      // tensor work of the largest tile.
+      if (!A_MN && !B_MN && p.conv.mode == 1) {
+        // A: 128 output pixels (Nb images x Hb rows x W) shifted by the tap, 64 channels
+        const int hblocks = p.conv.H / p.conv.Hb;
+        const int img = (tm / hblocks) * p.conv.Nb, h0 = (tm % hblocks) * p.conv.Hb;
+        int tap_w = -1, tap_h = -1, chunk = 0;
+        ok = k_loop(stage_bytes, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
+          if (leader) {
+            tma_load_4d(sa, mapA, fb, chunk * 64, tap_w, h0 + tap_h, img);
+            tma_load_3d(sb, &tmB, fb, kb * BK, n0, 0);
+          }
+          if (++chunk == p.conv.c_chunks) {
+            chunk = 0;
+            if (++tap_w == 2) { tap_w = -1; ++tap_h; }
+          }
+        });
+      } else if (A_MN && B_MN && p.conv.mode == 2) {
+        // batch index = tap + taps * split; K block = 64 consecutive pixels
+        const int tap = b % p.conv.taps, hblocks = p.conv.H / p.conv.Hb;
+        int pix_block = (b / p.conv.taps) * k_blocks;
+        int img = (pix_block / hblocks) * p.conv.Nb, h0 = (pix_block % hblocks) * p.conv.Hb;
+        const int tap_w = tap % 3 - 1, tap_h = tap / 3 - 1;
+        ok = k_loop(stage_bytes, [&](int, uint32_t fb, uint32_t sa, uint32_t sb) {
+          if (leader) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j)
+              if (j < boxes_a) tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, pix_block * BK, 0);
+#pragma unroll
+            for (int j = 0; j < BN / 64; ++j)
+              if (j < boxes_b) tma_load_4d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, tap_w, h0 + tap_h, img);
+          }
+          ++pix_block;
+          h0 += p.conv.Hb;
+          if (h0 == p.conv.H) { h0 = 0; img += p.conv.Nb; }
+        });
+      } else if (whole) {
+        ok = k_loop(L::STAGE_BYTES, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
+          if (!leader) return;
+          if constexpr (!A_MN) {
+            tma_load_3d(sa, mapA, fb, kb * BK, m_coord, b);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j)
+              tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kb * BK, b);
+          }
+          if constexpr (!B_MN) {
+            tma_load_3d(sb, &tmB, fb, kb * BK, n0, b);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BN / 64; ++j)
+              tma_load_3d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, kb * BK, b);
+          }
+        });
+      } else {
+        ok = k_loop(stage_bytes, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
+          if (!leader) return;
+          if constexpr (!A_MN) {
+            tma_load_3d(sa, mapA, fb, kb * BK, m_coord, b);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j)
+              if (j < boxes_a) tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kb * BK, b);
+          }
+          if constexpr (!B_MN) {
+            tma_load_3d(sb, &tmB, fb, kb * BK, n0, b);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BN / 64; ++j)
+              if (j < boxes_b) tma_load_3d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, kb * BK, b);
+          }
+        });
       }
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer ---------------------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int iter = 0;
-      bool ok = true;
-      for (int t = gemm_bid; t < total_tiles && ok; t += grid_stride, ++iter) {
-        const int acc = iter & 1;
-        const uint32_t acc_phase = (iter >> 1) & 1;
-        if (!mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1u, abort_flag)) break;
-        tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait(smem_u32(&full_bar[stage]), phase, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * L::STAGE_BYTES);
-          const uint32_t sb = sa + L::A_BYTES;
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            uint64_t da, db;
-            if constexpr (!A_MN)
-              da = make_smem_desc_sw128(sa + k * (UMMA_K * 2), 16, 1024);
-            else
-              da = make_smem_desc_sw128(sa + k * (UMMA_K * 128), 64 * BK * 2, 1024);
-            if constexpr (!B_MN)
-              db = make_smem_desc_sw128(sb + k * (UMMA_K * 2), 16, 1024);
-            else
-              db = make_smem_desc_sw128(sb + k * (UMMA_K * 128), 64 * BK * 2, 1024);
-            umma_bf16_ss(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(smem_u32(&empty_bar[stage]));  // frees the smem stage when MMAs finish
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+    const bool leader = elect_one();
+    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+    // descriptor words are formed once: the high word is common, the low word advances by constants
+    constexpr uint32_t desc_hi = smem_desc_hi(1024);
+    constexpr uint32_t a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4, b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+    const uint32_t smem0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+    const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint32_t full0 = __shfl_sync(0xffffffffu, smem_u32(full_bar), 0);
+    const uint32_t empty0 = full0 + STAGES * 8, tfull0 = full0 + 2 * STAGES * 8, tempty0 = tfull0 + 16;
+    const uint32_t a_lo0 = smem_desc_lo(smem0, A_MN ? 64 * BK * 2 : 16);
+    const uint32_t b_lo0 = smem_desc_lo(smem0 + L::A_BYTES, B_MN ? 64 * BK * 2 : 16);
+    int stage = 0;
+    uint32_t phase = 0;
+    int iter = 0;
+    bool ok = true;
+    for (int t = gemm_bid; t < total_tiles && ok; t += grid_stride, ++iter) {
+      const int acc = iter & 1;
+      const uint32_t acc_phase = (iter >> 1) & 1;
+      if (!mbar_wait_warp(tempty0 + acc * 8, acc_phase ^ 1u, abort_flag)) break;
+      tc_fence_after();
+      const uint32_t tmem_d = tmem0 + acc * BN;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_warp(full0 + stage * 8, phase, abort_flag)) {
+          ok = false;
+          break;
         }
-        if (ok) umma_commit(smem_u32(&tfull_bar[acc]));
+        tc_fence_after();
+        const uint32_t a_lo = a_lo0 + stage * (L::STAGE_BYTES >> 4), b_lo = b_lo0 + stage * (L::STAGE_BYTES >> 4);
+        if (leader) {
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_ss_split(tmem_d, a_lo + k * a_step, desc_hi, b_lo + k * b_step, desc_hi, idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit(empty0 + stage * 8);  // frees the smem stage when MMAs finish
+          if (kb + 1 == k_blocks) umma_commit(tfull0 + acc * 8);
+        }
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
     }
   } else if (warp < 6) {
@@ -598,9 +654,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
         if (p.bias) {
+          if (full && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (full || col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+            for (int q = 0; q < 4; ++q) {
+              const uint4 u = __ldg(reinterpret_cast<const uint4*>(p.bias + col0) + q);
+              const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
+              v[q * 8 + 0] += f0.x; v[q * 8 + 1] += f0.y; v[q * 8 + 2] += f1.x; v[q * 8 + 3] += f1.y;
+              v[q * 8 + 4] += f2.x; v[q * 8 + 5] += f2.y; v[q * 8 + 6] += f3.x; v[q * 8 + 7] += f3.y;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (full || col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+          }
         }
         if (p.aux_out) {
           __nv_bfloat16* a = p.aux_out + (long long)row * p.ld_aux_out + col0;

@@ -88,8 +88,8 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "gemm: backward activation needs aux_in");
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
 
-  const bool small_n = a->N <= 128;
-  const int BN = small_n ? 128 : 256;
+  // the narrowest tile that covers N: a wider one multiplies and fetches columns that are not there
+  const int BN = a->N <= 64 ? 64 : (a->N <= 128 ? 128 : 256);
 
   CUtensorMap tmA, tmB;
   {
@@ -151,7 +151,9 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
       return ST_ERR_CUDA;
   }
 
-  if (small_n)
+  if (BN == 64)
+    return dispatch_major<64, 8>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
+  if (BN == 128)
     return dispatch_major<128, 6>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
   return dispatch_major<256, 4>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
 }

@@ -315,6 +315,14 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   return ST_OK;
 }
 
+// out[i] (+)= sum over p of partial[p * n + i], in a fixed order.
+ST_API int st_reduce_partials(const float* partial, float* out, int parts, int n, int accumulate, void* stream_v) {
+  if (!partial || !out || parts <= 0 || n <= 0) return st::fail(ST_ERR_INVALID, "reduce_partials: bad arguments");
+  reduce_partials_kernel<<<(n + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, parts, n, accumulate);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
 // dgamma / dbeta are fp32 [d]; with accumulate != 0 the kernel adds to them.
 ST_API int st_norm_bwd(int rms, const void* dy, const void* x, const void* gamma,
                        const float* mean, const float* rstd, const void* dres, void* dx,

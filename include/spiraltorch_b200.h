@@ -246,6 +246,7 @@ int st_ce_stats(const void* logits, const long long* target, float* row_max, flo
 int st_clip_coef(const float* sumsq, float norm_scale, float max_norm, float* coef, float* norm_out, void* stream_v);   /* csrc/optim/optim.cu */
 int st_colsum(const void* x, float* out, long long rows, int cols, long long ld, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_compact_rows(const float* in, float* out_v, int* out_i, int* counts, int rows, int cols, float low, float high, void* stream_v);   /* csrc/rank/rank.cu */
+int st_conv3x3_dgrad_weights(const void* w, void* wt, int OC, int IC, void* stream_v);   /* csrc/conv/conv.cu */
 int st_conv3x3_fwd(const StConvArgs* a, void* stream_v);   /* csrc/conv/conv.cu */
 int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v);   /* csrc/conv/conv.cu */
 int st_dft_max_len();   /* csrc/spectral/spectral.cu */
@@ -270,6 +271,7 @@ int st_lstm_gate_bwd(const float* act, const float* c_prev, const float* c, cons
 int st_lstm_gate_fwd(const float* z, const float* c_prev, float* c_out, float* h_out, float* act, int B, int H, void* stream);   /* csrc/recurrent/recurrent.cu */
 int st_maxpool2_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, void* stream_v);   /* csrc/conv/conv.cu */
 int st_maxpool2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream_v);   /* csrc/conv/conv.cu */
+int st_maxpool2_relu_bwd(const void* dy, const void* idx, const void* pooled, void* dx, float* dbias, int N, int H, int W, int C, void* stream_v);   /* csrc/conv/conv.cu */
 int st_nd_indexer(const unsigned* positions, unsigned* out_index, unsigned* out_segment, long long n, const unsigned* dims4, const unsigned* strides4, unsigned segments, unsigned segment_stride, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_nerf_composite_bwd(const float* sigma, const float* rad, const float* deltas, const float* accum, const float* d_accum, float* d_sigma, float* d_rad, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */
 int st_nerf_composite_fwd(const float* sigma, const float* rad, const float* deltas, float* accum, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */
@@ -284,6 +286,7 @@ int st_rank_select(const float* in, float* out_v, int* out_i, int rows, int cols
 int st_rank_topk(const float* in, float* out_v, int* out_i, int rows, int cols, int k, int mode, void* workspace, void* stream_v);   /* csrc/rank/rank.cu */
 long long st_rank_topk_workspace(int rows, int cols, int k);   /* csrc/rank/rank.cu */
 int st_read_error_word(unsigned* out, int clear);   /* csrc/runtime/runtime.cu */
+int st_reduce_partials(const float* partial, float* out, int parts, int n, int accumulate, void* stream_v);   /* csrc/norm/norm.cu */
 int st_rnn_scan(const StRnnScanArgs* a, void* stream_v);   /* csrc/recurrent/scan.cu */
 int st_rnn_scan_supported(int H, int cell);   /* csrc/recurrent/scan.cu */
 int st_rope(void* x, const float* cos_t, const float* sin_t, long long T, int heads, int D, long long ld, int seq_len, int pos_offset, int backward, void* stream_v);   /* csrc/elementwise/elementwise.cu */

@@ -112,17 +112,16 @@ class ConvClassifier(nn.Module):
         k = len(acts) - 1                           # index of the pooled output of the last stage
         for s in reversed(range(4)):
             idx, ph, pw = pools[s]
-            d = C.maxpool2_backward(d, idx, ph, pw)         # gradient w.r.t. the (post-ReLU) conv output
+            # gradient with respect to the convolution output in front of ReLU and pool, and its bias gradient
+            d = C.maxpool2_relu_backward(d, idx, acts[k], ph, pw, P[f"conv{s}_1.bias"].main_grad)
             k -= 1                                          # acts[k] = output of conv s_1
             for i in (1, 0):
-                y, xin = acts[k], acts[k - 1]
-                if i == 1:
-                    # the pooled gradient is already zero where the ReLU was inactive only by chance: mask it
-                    d = torch.where(y > 0, d, torch.zeros_like(d))
+                xin = acts[k - 1]
                 w = P[f"conv{s}_{i}.weight"]
                 ic = xin.shape[-1]
                 C.conv3x3_wgrad(d, xin, w.main_grad)
-                ew.colsum(d.reshape(-1, d.shape[-1]), P[f"conv{s}_{i}.bias"].main_grad, accumulate=True)
+                if i == 0:
+                    ew.colsum(d.reshape(-1, d.shape[-1]), P[f"conv{s}_0.bias"].main_grad, accumulate=True)
                 if k - 1 > 0:
                     d = C.conv3x3(d, C.dgrad_weights(w, ic), relu_mask_of=xin)
                 if layer_done:

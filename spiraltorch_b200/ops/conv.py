@@ -15,6 +15,7 @@ import torch
 import torch.nn.functional as F
 
 from . import native
+from .elementwise import colsum
 from .gemm import gemm
 
 launch_count = 0
@@ -43,7 +44,14 @@ def from_tap_major(w_tap: torch.Tensor, ic: int) -> torch.Tensor:
 
 def dgrad_weights(w_tap: torch.Tensor, ic: int) -> torch.Tensor:
     """Weights of the data-gradient convolution: ``Wt[ic][kh'][kw'][oc] = W[oc][2-kh'][2-kw'][ic]``."""
+    global launch_count
     oc = w_tap.shape[0]
+    if native.use_native(w_tap) and w_tap.dtype == torch.bfloat16 and w_tap.is_contiguous() and w_tap.shape[1] == 9 * ic:
+        out = torch.empty((ic, 9 * oc), dtype=torch.bfloat16, device=w_tap.device)
+        native.check(native.lib().st_conv3x3_dgrad_weights(native.ptr(w_tap), native.ptr(out), ctypes.c_int(oc), ctypes.c_int(ic),
+                                                           native.stream_ptr(w_tap.device)), "st_conv3x3_dgrad_weights")
+        launch_count += 1
+        return out
     return w_tap.reshape(oc, 3, 3, ic).flip(1, 2).permute(3, 1, 2, 0).reshape(ic, 9 * oc).contiguous()
 
 
@@ -178,6 +186,34 @@ def maxpool2_backward(dy: torch.Tensor, idx: torch.Tensor, H: int, W: int) -> to
     native.check(st, "st_maxpool2_bwd")
     launch_count += 1
     return dx
+
+
+def maxpool2_relu_backward(dy: torch.Tensor, idx: torch.Tensor, pooled: torch.Tensor, H: int, W: int,
+                           bias_grad: torch.Tensor) -> torch.Tensor:
+    """Gradient before ``maxpool2(relu(z))`` with respect to ``z``, and its channel sums added to ``bias_grad`` (fp32
+    ``[C]``).  ``pooled`` is the pool's output: the arg-max of a window carries its value, so the ReLU's mask is the
+    pooled value's sign."""
+    global launch_count
+    N, OH, OW, C = dy.shape
+    if native.use_native(dy) and dy.dtype == torch.bfloat16 and C % 8 == 0 and 256 % (C // 8) == 0 and pooled.is_contiguous() \
+            and idx.is_contiguous() and bias_grad.is_contiguous() and not native.deterministic_reduction() \
+            and (H, W) == (2 * OH, 2 * OW):
+        native.require_cuda("maxpool2_relu_backward", dy, idx, pooled, bias_grad)
+        assert pooled.shape == dy.shape and idx.shape == dy.shape and pooled.dtype == torch.bfloat16 and idx.dtype == torch.uint8
+        assert bias_grad.dtype == torch.float32 and bias_grad.numel() == C
+        d = dy.contiguous()
+        if not (d.data_ptr() | pooled.data_ptr()) % 16 and not idx.data_ptr() % 8:
+            dx = torch.empty((N, H, W, C), dtype=dy.dtype, device=dy.device)
+            native.check(native.lib().st_maxpool2_relu_bwd(native.ptr(d), native.ptr(idx), native.ptr(pooled), native.ptr(dx),
+                                                           native.ptr(bias_grad), ctypes.c_int(N), ctypes.c_int(H),
+                                                           ctypes.c_int(W), ctypes.c_int(C), native.stream_ptr(dy.device)),
+                         "st_maxpool2_relu_bwd")
+            launch_count += 1
+            return dx
+    # the channel sums of the masked gradient are those of its pooled form: every window has one receiver
+    g = torch.where(pooled > 0, dy, torch.zeros_like(dy))
+    colsum(g.reshape(-1, C), bias_grad, accumulate=True)
+    return maxpool2_backward(g, idx, H, W)
 
 
 def global_avgpool(x: torch.Tensor) -> torch.Tensor:

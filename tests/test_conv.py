@@ -96,3 +96,55 @@ def test_classifier_cuda_tracks_cpu():
     assert abs(lg.item() - lc.item()) < 5e-2
     cos = torch.nn.functional.cosine_similarity(gpu.flat_grad.cpu(), cpu.flat_grad, dim=0).item()
     assert cos > 0.98, cos
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,H,W,Cin,OC", [(2, 6, 10, 3, 64), (1, 4, 4, 5, 72), (3, 12, 6, 8, 40), (2, 24, 24, 64, 64), (2, 64, 64, 64, 8)])
+def test_conv_steps_off_the_main_sizes(N, H, W, Cin, OC):
+    """Column matrices with odd and vectorised channel counts, output tiles 64 columns wide, the data gradient's weights,
+    and the fused pool / ReLU / bias backward."""
+    torch.manual_seed(N * H + OC)
+    x = torch.randn(N, H, W, Cin, device="cuda").bfloat16()
+    w = (torch.randn(OC, 9 * Cin, device="cuda") * (2.0 / (9 * Cin)) ** 0.5).bfloat16()
+    wt = C.dgrad_weights(w, Cin)
+    assert torch.equal(wt.cpu(), C.dgrad_weights(w.cpu(), Cin))
+    y = C.conv3x3(x, w, None, relu=True)
+    assert _rel(y.cpu(), C._conv_ref(x.cpu().float(), w.cpu().float(), None, 1, None)) < 2e-2      # bf16 output: 2^-8
+    dy = torch.randn(N, H, W, OC, device="cuda").bfloat16()
+    dw, rdw = torch.zeros(OC, 9 * Cin, device="cuda"), torch.zeros(OC, 9 * Cin)
+    C.conv3x3_wgrad(dy, x, dw)
+    C.conv3x3_wgrad(dy.cpu().float(), x.cpu().float(), rdw)
+    assert _rel(dw.cpu(), rdw) < 1e-4                                                               # fp32 sums
+    pooled, idx = C.maxpool2(y)
+    g = torch.randn_like(pooled)
+    db, rdb = torch.full((OC,), 0.5, device="cuda"), torch.full((OC,), 0.5)
+    dx = C.maxpool2_relu_backward(g, idx, pooled, H, W, db)
+    ref = C.maxpool2_relu_backward(g.cpu().float(), idx.cpu(), pooled.cpu().float(), H, W, rdb)
+    assert torch.equal(dx.cpu().float(), ref) and torch.allclose(db.cpu(), rdb, rtol=1e-4, atol=1e-4)
+    masked = torch.where(y > 0, C.maxpool2_backward(g, idx, H, W), torch.zeros_like(y))
+    assert torch.equal(dx, masked)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,accumulate", [(64, 32, 65536, False), (72, 40, 1536, True), (128, 64, 1024, False), (8, 200, 3 * 521, True),
+                                              (200, 72, 4096, True)])
+def test_weight_gradient_in_parts(M, N, K, accumulate):
+    """Few output tiles over a long sum: the parts' fixed-order sum, odd divisors of K, and boxes outside the matrix."""
+    from spiraltorch_b200.ops import gemm as G
+    torch.manual_seed(M + N)
+    a, b = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    out = torch.full((M, N), 0.5, device="cuda")
+    ref = a.double().t() @ b.double() + (0.5 if accumulate else 0.0)
+    G.gemm(a, b, a_mn=True, b_mn=True, out=out, accumulate=accumulate)
+    assert ((out - ref).norm() / ref.norm()).item() < 1e-5
+    again = torch.full((M, N), 0.5, device="cuda")
+    G.gemm(a, b, a_mn=True, b_mn=True, out=again, accumulate=accumulate)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 8), (1000, 64), (257, 104), (3000, 256), (100, 264)])
+def test_column_sums_of_narrow_matrices(rows, cols):
+    from spiraltorch_b200.ops import elementwise as E
+    x = torch.randn(rows, cols, device="cuda").bfloat16()
+    assert torch.allclose(E.colsum(x).double(), x.double().sum(0), rtol=1e-5, atol=1e-3)
