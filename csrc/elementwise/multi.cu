@@ -1,0 +1,173 @@
+// Small-tensor work of the layer protocol in one launch each: finite checks, scaled copies and plain updates over a list
+// of fp32 tensors, and the mean-squared-error loss.
+//
+// A training step of a small model through the layer API is bound by launches and host reads, not by bytes (a step of a
+// 64-128-8 perceptron moves 0.3 MB in 170 launches and ten host reads, 2.3 ms): one check of one tensor was five launches
+// and a host read.  Here a list of tensors is one grid, blockIdx.y the tensor, and what the host has to know (did every
+// block see finite values) is written by the blocks straight into pinned host memory, so that a stream synchronisation
+// is all that the check costs on top of its launch.
+#include "../common/host.h"
+#include "../common/ptx.cuh"
+
+namespace {
+
+constexpr int kMultiMax = 48;        // tensors per launch: the table travels as a kernel argument
+constexpr int kMultiThreads = 256;
+constexpr int kMultiBlocks = 32;     // blocks per tensor at most; 32 x 256 threads read 4 MB in about 3 us
+
+struct MultiTable {
+  const float* src[kMultiMax];
+  float* dst[kMultiMax];
+  long long n[kMultiMax];
+};
+
+enum MultiOp : int { MULTI_CHECK = 0, MULTI_DIV = 1, MULTI_STEP = 2 };
+
+// CHECK: bad[block] = some src element is not finite.  DIV: the same, and dst = src / value.  STEP: dst -= value * src,
+// the product rounded before the difference.
+template <int OP>
+__global__ void __launch_bounds__(kMultiThreads)
+multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict__ bad) {
+  const float* __restrict__ src = t.src[blockIdx.y];
+  float* dst = t.dst[blockIdx.y];
+  const long long n = t.n[blockIdx.y], stride = (long long)gridDim.x * kMultiThreads;
+  bool odd = false;
+  for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n; i += 4 * stride) {
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = i + u * stride < n ? src[i + u * stride] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long at = i + u * stride;
+      if (OP != MULTI_STEP) odd |= !isfinite(v[u]);
+      if (at < n) {
+        if (OP == MULTI_DIV) dst[at] = __fdiv_rn(v[u], value);
+        if (OP == MULTI_STEP) dst[at] = __fsub_rn(dst[at], __fmul_rn(value, v[u]));
+      }
+    }
+  }
+  if (OP != MULTI_STEP) {
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) bad[blockIdx.y * gridDim.x + blockIdx.x] = odd;
+  }
+}
+
+__device__ __forceinline__ float block_sum_256(float v, float* sh) {
+  v = st::warp_sum(v);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float s = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kMultiThreads / 32; ++i) s += sh[i];
+  return s;
+}
+
+// value = mean((p - t)^2).  Blocks leave their sums in `part` and the last one to finish adds them in block order, so the
+// result does not depend on scheduling.  bad[block]: a prediction or a target is not finite.
+__global__ void __launch_bounds__(kMultiThreads)
+mse_forward_kernel(const float* __restrict__ p, const float* __restrict__ t, long long n, float* __restrict__ value,
+                   float* __restrict__ part, unsigned* __restrict__ arrived, int* __restrict__ bad) {
+  __shared__ float sh[kMultiThreads / 32];
+  __shared__ bool last;
+  float s = 0.0f;
+  bool odd = false;
+  for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kMultiThreads) {
+    const float a = p[i], b = t[i], d = a - b;
+    odd |= !isfinite(a) || !isfinite(b);
+    s += d * d;
+  }
+  odd = __syncthreads_or(odd);
+  s = block_sum_256(s, sh);
+  if (threadIdx.x == 0) {
+    bad[blockIdx.x] = odd;
+    last = false;
+    if (gridDim.x == 1) {
+      *value = s / (float)n;
+    } else {
+      part[blockIdx.x] = s;
+      __threadfence();
+      last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __syncthreads();
+  float total = threadIdx.x < gridDim.x ? *reinterpret_cast<volatile float*>(part + threadIdx.x) : 0.0f;
+  total = block_sum_256(total, sh);
+  if (threadIdx.x == 0) *value = total / (float)n;
+}
+
+// g = (1 / n) * 2 (p - t)
+__global__ void __launch_bounds__(kMultiThreads)
+mse_backward_kernel(const float* __restrict__ p, const float* __restrict__ t, long long n, float inv_n, float* __restrict__ g,
+                    int* __restrict__ bad) {
+  bool odd = false;
+  for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kMultiThreads) {
+    const float a = p[i], b = t[i];
+    odd |= !isfinite(a) || !isfinite(b);
+    g[i] = inv_n * (2.0f * (a - b));
+  }
+  odd = __syncthreads_or(odd);
+  if (threadIdx.x == 0) bad[blockIdx.x] = odd;
+}
+
+int blocks_for(long long n, int most) {
+  const long long b = (n + 4 * kMultiThreads - 1) / (4 * kMultiThreads);
+  return (int)(b < 1 ? 1 : (b > most ? most : b));
+}
+
+}  // namespace
+
+// Tensors per st_multi call, and ints of result a call over tensors of at most `most` elements writes per tensor.
+ST_API int st_multi_max() { return kMultiMax; }
+ST_API int st_multi_blocks(long long most) { return blocks_for(most, kMultiBlocks); }
+
+// op 0: finite check of src; 1: dst = src / value and finite check of src; 2: dst -= value * src.  `bad` (op 0 and 1):
+// count * st_multi_blocks(largest n) ints, tensor by tensor, in memory that the device can write (pinned host memory).
+ST_API int st_multi(int op, int count, const void* const* src, void* const* dst, const long long* n, float value, int* bad,
+                    void* stream_v) {
+  if (count <= 0) return ST_OK;
+  if (count > kMultiMax) return st::fail(ST_ERR_TOO_LARGE, "multi: too many tensors for one launch");
+  if (op < MULTI_CHECK || op > MULTI_STEP || !src || !n || (op != MULTI_CHECK && !dst) || (op != MULTI_STEP && !bad))
+    return st::fail(ST_ERR_INVALID, "multi: bad arguments");
+  MultiTable t;
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    t.src[i] = static_cast<const float*>(src[i]);
+    t.dst[i] = dst ? static_cast<float*>(dst[i]) : nullptr;
+    t.n[i] = n[i];
+    most = n[i] > most ? n[i] : most;
+  }
+  const dim3 grid(blocks_for(most, kMultiBlocks), count);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  if (op == MULTI_CHECK) multi_kernel<MULTI_CHECK><<<grid, kMultiThreads, 0, s>>>(t, value, bad);
+  else if (op == MULTI_DIV) multi_kernel<MULTI_DIV><<<grid, kMultiThreads, 0, s>>>(t, value, bad);
+  else multi_kernel<MULTI_STEP><<<grid, kMultiThreads, 0, s>>>(t, value, bad);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+// 32-bit words of workspace st_mse_forward wants, and blocks (ints of `bad`) that both directions write.
+ST_API int st_mse_workspace() { return kMultiThreads + 1; }
+ST_API int st_mse_blocks(long long n) { return blocks_for(n, kMultiThreads); }
+
+ST_API int st_mse_forward(const float* p, const float* t, long long n, float* value, void* workspace, int* bad, void* stream_v) {
+  if (!p || !t || !value || !workspace || !bad || n <= 0) return st::fail(ST_ERR_INVALID, "mse: bad arguments");
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  float* part = static_cast<float*>(workspace);
+  unsigned* arrived = reinterpret_cast<unsigned*>(part + kMultiThreads);
+  const int blocks = blocks_for(n, kMultiThreads);
+  if (blocks > 1) ST_CUDA_CHECK(cudaMemsetAsync(arrived, 0, sizeof(unsigned), s));
+  mse_forward_kernel<<<blocks, kMultiThreads, 0, s>>>(p, t, n, value, part, arrived, bad);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+ST_API int st_mse_backward(const float* p, const float* t, long long n, float* g, int* bad, void* stream_v) {
+  if (!p || !t || !g || !bad || n <= 0) return st::fail(ST_ERR_INVALID, "mse: bad arguments");
+  mse_backward_kernel<<<blocks_for(n, kMultiThreads), kMultiThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+      p, t, n, 1.0f / (float)n, g, bad);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}

@@ -272,6 +272,13 @@ int st_lstm_gate_fwd(const float* z, const float* c_prev, float* c_out, float* h
 int st_maxpool2_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, void* stream_v);   /* csrc/conv/conv.cu */
 int st_maxpool2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream_v);   /* csrc/conv/conv.cu */
 int st_maxpool2_relu_bwd(const void* dy, const void* idx, const void* pooled, void* dx, float* dbias, int N, int H, int W, int C, void* stream_v);   /* csrc/conv/conv.cu */
+int st_mse_backward(const float* p, const float* t, long long n, float* g, int* bad, void* stream_v);   /* csrc/elementwise/multi.cu */
+int st_mse_blocks(long long n);   /* csrc/elementwise/multi.cu */
+int st_mse_forward(const float* p, const float* t, long long n, float* value, void* workspace, int* bad, void* stream_v);   /* csrc/elementwise/multi.cu */
+int st_mse_workspace();   /* csrc/elementwise/multi.cu */
+int st_multi(int op, int count, const void* const* src, void* const* dst, const long long* n, float value, int* bad, void* stream_v);   /* csrc/elementwise/multi.cu */
+int st_multi_blocks(long long most);   /* csrc/elementwise/multi.cu */
+int st_multi_max();   /* csrc/elementwise/multi.cu */
 int st_nd_indexer(const unsigned* positions, unsigned* out_index, unsigned* out_segment, long long n, const unsigned* dims4, const unsigned* strides4, unsigned segments, unsigned segment_stride, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_nerf_composite_bwd(const float* sigma, const float* rad, const float* deltas, const float* accum, const float* d_accum, float* d_sigma, float* d_rad, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */
 int st_nerf_composite_fwd(const float* sigma, const float* rad, const float* deltas, float* accum, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */

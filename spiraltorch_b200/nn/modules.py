@@ -29,6 +29,7 @@ from ..optim.amegagrad import AmegaHypergrad, AmegaRealgrad
 from ..tensor import Tensor, TensorError
 
 
+from ..ops import multi as _multi  # noqa: E402
 from ..ops import recurrent as _rec  # noqa: E402
 from . import functional as _fn  # noqa: E402
 
@@ -46,6 +47,11 @@ def assert_finite(tensors, describe) -> None:
     (no host read possible) the flag is OR-ed into the capturing step's error word instead, which its owner polls."""
     tensors = [t for t in tensors if t is not None]
     if not tensors:
+        return
+    if _multi.takes(tensors):
+        bad = _multi.first_nonfinite(tensors)
+        if bad is not None:
+            raise TensorError(describe(bad))
         return
     oks = [torch.isfinite(t).all() for t in tensors]
     ok = oks[0] if len(oks) == 1 else torch.stack(oks).all()
@@ -176,9 +182,19 @@ class Module:
             grads = torch.autograd.grad(y, [xt] + [leaves[p.name] for p in plist], g, allow_unused=True)
         batch = max(1, xt.shape[0])
         live = [(p, gp) for p, gp in zip(plist, grads[1:]) if gp is not None]
-        assert_finite([gp for _, gp in live], lambda i: f"non-finite gradient for parameter {live[i][0].name}")
-        for p, gp in live:
-            p.accumulate(gp / batch)
+        found = [gp for _, gp in live]
+        if _multi.takes(found):
+            means, bad = _multi.divided(found, float(batch))        # check and division in one launch
+            if bad is not None:
+                raise TensorError(f"non-finite gradient for parameter {live[bad][0].name}")
+        else:
+            assert_finite(found, lambda i: f"non-finite gradient for parameter {live[i][0].name}")
+            means = [gp / batch for gp in found]
+        for (p, _), mean in zip(live, means):
+            if p.gradient is None and p.hypergrad is None and p.realgrad is None and type(p) is Parameter:
+                p.gradient = mean.reshape(p.value.shape)            # a fresh tensor: nothing to clone
+            else:
+                p.accumulate(mean)
         gx = grads[0] if grads[0] is not None else torch.zeros_like(xt)
         return Tensor._wrap(gx.detach())
 
@@ -199,6 +215,13 @@ class Module:
             p.zero()
 
     def apply_step(self, fallback_lr: float = 1e-2) -> None:
+        plain = [p for p in self.parameters() if type(p) is Parameter and p.trainable and p.hypergrad is None
+                 and p.realgrad is None and p.gradient is not None]
+        if plain and len({id(p) for p in plain}) == len(plain) and _multi.takes([t for p in plain for t in (p.value, p.gradient)]) \
+                and not any(p.value.requires_grad for p in plain):
+            _multi.descend_([p.value for p in plain], [p.gradient for p in plain], fallback_lr)
+            for p in plain:
+                p.gradient = None
         for p in self.parameters():
             p.apply_step(fallback_lr)
 

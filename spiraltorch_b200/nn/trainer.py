@@ -28,7 +28,7 @@ import torch
 from .. import plugin
 from ..ops import native
 from ..tensor import Tensor, TensorError
-from .modules import Module
+from .modules import Module, assert_finite
 
 
 @dataclass
@@ -434,11 +434,13 @@ class ModuleTrainer:
                     module.backward(x, Tensor._wrap(bands[0].torch() + bands[1].torch() + bands[2].torch()))
             else:
                 module.backward(x, grad)
-            for p in module.parameters():
-                for a in p.accumulators():
-                    if not torch.isfinite(a).all():
-                        module.zero_accumulators()
-                        raise TensorError(f"non-finite gradient in '{p.name}'; accumulators were cleared")
+            held = [(p, a) for p in module.parameters() for a in p.accumulators()]
+            try:
+                assert_finite([a for _, a in held],
+                              lambda i: f"non-finite gradient in '{held[i][0].name}'; accumulators were cleared")
+            except TensorError:
+                module.zero_accumulators()
+                raise
             gnorm = 0.0
             if getattr(self, "psi_meter", None) is not None:
                 gnorm = math.sqrt(sum(float(a.pow(2).sum()) for p in module.parameters() for a in p.accumulators()))

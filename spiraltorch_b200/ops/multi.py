@@ -1,0 +1,99 @@
+"""Finite checks, scaled copies and plain updates over lists of small fp32 tensors, and the mean-squared-error loss
+(``csrc/elementwise/multi.cu``): one launch per list, and no device-to-host copy for what the host has to know - the
+kernels write it into pinned memory, so a check is a launch and a stream synchronisation.
+
+The callers (:mod:`spiraltorch_b200.nn`) keep their PyTorch statement for tensors that :func:`takes` refuses.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import Optional, Sequence
+
+import torch
+
+from . import native
+
+launch_count = 0
+_MAX = 48
+_CHECK, _DIV, _STEP = 0, 1, 2
+
+
+def takes(tensors: Sequence[torch.Tensor]) -> bool:
+    """Whether the kernels take these tensors: dense non-empty fp32 on the current CUDA device, outside a graph capture
+    (a captured stream cannot be waited for)."""
+    if not tensors or not tensors[0].is_cuda or torch.cuda.is_current_stream_capturing():
+        return False
+    dev = tensors[0].device
+    return dev.index == torch.cuda.current_device() and all(
+        type(t) in (torch.Tensor, torch.nn.Parameter) and t.device == dev and t.dtype == torch.float32 and t.is_contiguous()
+        and t.numel() > 0 for t in tensors)
+
+
+def _run(op: int, src, dst, value: float) -> Optional[int]:
+    """Index of the first tensor of ``src`` with a value that is not finite, or None (always None for an update)."""
+    global launch_count
+    lib, stream = native.lib(), torch.cuda.current_stream()
+    first = None
+    for at in range(0, len(src), _MAX):
+        s = src[at:at + _MAX]
+        n = len(s)
+        counts = [t.numel() for t in s]
+        blocks = lib.st_multi_blocks(ctypes.c_longlong(max(counts)))
+        bad = None if op == _STEP else torch.empty(n * blocks, dtype=torch.int32, pin_memory=True)
+        ptrs = (ctypes.c_void_p * n)(*[t.data_ptr() for t in s])
+        outs = None if dst is None else (ctypes.c_void_p * n)(*[t.data_ptr() for t in dst[at:at + _MAX]])
+        native.check(lib.st_multi(ctypes.c_int(op), ctypes.c_int(n), ptrs, outs, (ctypes.c_longlong * n)(*counts),
+                                  ctypes.c_float(value), None if bad is None else ctypes.c_void_p(bad.data_ptr()),
+                                  ctypes.c_void_p(stream.cuda_stream)), "st_multi")
+        launch_count += 1
+        if bad is not None:
+            stream.synchronize()
+            hits = bad.nonzero()
+            if first is None and hits.numel():
+                first = at + int(hits[0]) // blocks
+    return first
+
+
+def first_nonfinite(tensors: Sequence[torch.Tensor]) -> Optional[int]:
+    """Index of the first tensor that holds an infinity or a NaN, or None."""
+    return _run(_CHECK, tensors, None, 0.0)
+
+
+def divided(tensors: Sequence[torch.Tensor], value: float):
+    """``([t / value for t in tensors], index of the first tensor that is not finite or None)``."""
+    out = [torch.empty_like(t) for t in tensors]
+    return out, _run(_DIV, tensors, out, value)
+
+
+def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: float) -> None:
+    """``v -= lr * g`` for every pair, in place."""
+    _run(_STEP, grads, values, lr)
+    for v in values:
+        torch.autograd.graph.increment_version(v)      # copies of the values are cached by version
+
+
+def mse_forward(p: torch.Tensor, t: torch.Tensor):
+    """``(mean((p - t)^2) of shape (1, 1), all inputs are finite)``."""
+    global launch_count
+    lib, stream, n = native.lib(), torch.cuda.current_stream(), p.numel()
+    value = torch.empty((1, 1), dtype=torch.float32, device=p.device)
+    work = torch.empty(lib.st_mse_workspace(), dtype=torch.float32, device=p.device)
+    bad = torch.empty(lib.st_mse_blocks(ctypes.c_longlong(n)), dtype=torch.int32, pin_memory=True)
+    native.check(lib.st_mse_forward(native.ptr(p), native.ptr(t), ctypes.c_longlong(n), native.ptr(value), native.ptr(work),
+                                    ctypes.c_void_p(bad.data_ptr()), ctypes.c_void_p(stream.cuda_stream)), "st_mse_forward")
+    launch_count += 1
+    stream.synchronize()
+    return value, not bool(bad.any())
+
+
+def mse_backward(p: torch.Tensor, t: torch.Tensor):
+    """``(2 (p - t) / n, all inputs are finite)``."""
+    global launch_count
+    lib, stream, n = native.lib(), torch.cuda.current_stream(), p.numel()
+    g = torch.empty_like(p)
+    bad = torch.empty(lib.st_mse_blocks(ctypes.c_longlong(n)), dtype=torch.int32, pin_memory=True)
+    native.check(lib.st_mse_backward(native.ptr(p), native.ptr(t), ctypes.c_longlong(n), native.ptr(g),
+                                     ctypes.c_void_p(bad.data_ptr()), ctypes.c_void_p(stream.cuda_stream)), "st_mse_backward")
+    launch_count += 1
+    stream.synchronize()
+    return g, not bool(bad.any())

@@ -306,3 +306,41 @@ def test_graphed_train_step_matches_eager_steps_and_reports_non_finite_inputs():
     step(xe, st.Tensor._wrap(bad))
     with pytest.raises(st.TensorError):
         step.check()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[1], [5, 0, 1024], [4097, 33, 70000, 2], [7] * 100, [3_000_001, 1]])
+def test_tensor_lists_in_one_launch(sizes):
+    """Checks, divisions and updates of lists: single elements, block edges, more tensors than one launch holds."""
+    from spiraltorch_b200.ops import multi
+    g = torch.Generator(device="cuda").manual_seed(1)
+    ts = [torch.randn(n, generator=g, device="cuda") for n in sizes if n]
+    assert multi.takes(ts) and not multi.takes(ts + [torch.empty(0, device="cuda")]) and not multi.takes([ts[0].cpu()])
+    assert not multi.takes([torch.randn(4, 6, device="cuda").t()]) and not multi.takes([ts[0].double()])
+    assert multi.first_nonfinite(ts) is None
+    out, bad = multi.divided(ts, 3.0)
+    # correctly rounded, as on the CPU
+    assert bad is None and all(torch.equal(o.cpu(), t.cpu() / 3.0) for o, t in zip(out, ts))
+    values = [torch.randn(t.shape, generator=g, device="cuda") for t in ts]
+    want, versions = [v - 0.01 * t for v, t in zip(values, ts)], [v._version for v in values]
+    multi.descend_(values, ts, 0.01)
+    assert all(torch.equal(v, w) and v._version > n for v, w, n in zip(values, want, versions))
+    for k, odd in ((len(ts) - 1, float("nan")), (len(ts) // 2, float("-inf"))):
+        ts[k][-1] = odd
+        assert multi.first_nonfinite(ts) == k and multi.divided(ts, 2.0)[1] == k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 341), (32, 32), (33, 32), (4096, 100)])
+def test_mean_squared_error_in_one_launch(rows, cols):
+    import spiraltorch as st
+    p, t = torch.randn(rows, cols, device="cuda"), torch.randn(rows, cols, device="cuda")
+    loss = st.nn.MeanSquaredError()
+    ref = (p.double() - t.double()).pow(2).mean().item()
+    assert abs(loss.forward(st.Tensor(p), st.Tensor(t)).torch().item() - ref) <= 1e-6 * ref
+    want = torch.autograd.functional.jacobian(lambda x: (x - t).pow(2).mean(), p) if p.numel() < 2000 else 2 * (p - t) / p.numel()
+    assert torch.allclose(loss.backward(st.Tensor(p), st.Tensor(t)).torch(), want, rtol=3e-7, atol=0)     # two roundings
+    t[-1, -1] = float("inf")
+    for call in (loss.forward, loss.backward):
+        with pytest.raises(Exception, match="non-finite"):
+            call(st.Tensor(p), st.Tensor(t))
