@@ -31,6 +31,13 @@ from ..tensor import Tensor, TensorError
 from .modules import Module, assert_finite
 
 
+def _peak_memory_mb() -> float:
+    """``torch.cuda.max_memory_allocated()`` in MiB, read from the nested statistics: flattening all of them, as that call
+    does, takes longer than a small model's launches."""
+    stats = torch.cuda.memory.memory_stats_as_nested_dict()
+    return stats["allocated_bytes"]["all"]["peak"] / 2 ** 20 if "allocated_bytes" in stats else 0.0
+
+
 @dataclass
 class RoundtableConfig:
     top_k: int = 8
@@ -451,7 +458,7 @@ class ModuleTrainer:
             stats.total_loss += lv
             stats.tensor_backend["ops_total"] += 1
             metrics = StepMetrics(step_time_ms=(time.perf_counter() - t0) * 1e3,
-                                  mem_peak_mb=(torch.cuda.max_memory_allocated() / 2 ** 20) if self.device.type == "cuda" else 0.0,
+                                  mem_peak_mb=_peak_memory_mb() if self.device.type == "cuda" else 0.0,
                                   extra={"loss": lv, **({f"band_{k}": v for k, v in (self.last_band_energy or {}).items()})})
             if self.monitor is not None:
                 self.monitor.observe(metrics)

@@ -12,6 +12,7 @@ Reference parity: ``Tensor::matmul``, ``matmul_bias_relu/gelu``, ``matmul_bias_a
 from __future__ import annotations
 
 import ctypes
+import struct
 from typing import Optional
 
 import torch
@@ -25,20 +26,10 @@ _ACT_NAMES = {None: 0, "none": 0, "relu": 1, "gelu": 2, "gelu_bwd": 3, "relu_bwd
 launch_count = 0
 
 
-class _GemmArgs(ctypes.Structure):
-    _fields_ = [
-        ("A", ctypes.c_void_p), ("B", ctypes.c_void_p), ("C", ctypes.c_void_p),
-        ("bias", ctypes.c_void_p), ("residual", ctypes.c_void_p),
-        ("aux_out", ctypes.c_void_p), ("aux_in", ctypes.c_void_p),
-        ("lda", ctypes.c_longlong), ("ldb", ctypes.c_longlong), ("ldc", ctypes.c_longlong),
-        ("ldr", ctypes.c_longlong), ("ld_aux_out", ctypes.c_longlong), ("ld_aux_in", ctypes.c_longlong),
-        ("batch_stride_a", ctypes.c_longlong), ("batch_stride_b", ctypes.c_longlong),
-        ("batch_stride_c", ctypes.c_longlong),
-        ("M", ctypes.c_int), ("N", ctypes.c_int), ("K", ctypes.c_int), ("batch", ctypes.c_int),
-        ("a_mn_major", ctypes.c_int), ("b_mn_major", ctypes.c_int),
-        ("out_fp32", ctypes.c_int), ("accumulate", ctypes.c_int), ("act", ctypes.c_int),
-        ("alpha", ctypes.c_float), ("max_ctas", ctypes.c_int),
-    ]
+# StGemmArgs of csrc/gemm/gemm_sm100.cu: A, B, C, bias, residual, aux_out, aux_in; lda, ldb, ldc, ldr, ld_aux_out,
+# ld_aux_in and the batch strides of A, B, C; M, N, K, batch, a_mn_major, b_mn_major, out_fp32, accumulate, act; alpha;
+# max_ctas.  Packed in one call: filling the 27 fields of a ctypes structure costs as much as the launch itself.
+_pack_args = struct.Struct("@7P9q9ifi").pack
 
 
 #: split the K loop of weight-gradient GEMMs whose tile count fills the SMs badly (the partial
@@ -165,6 +156,16 @@ def _pad_to(t: torch.Tensor, rows: int, cols: int) -> torch.Tensor:
     return out
 
 
+def _tma_ready(t: torch.Tensor) -> torch.Tensor:
+    """``t``, or a padded copy: TMA needs 16-byte aligned rows, so the contiguous dimension is padded to a multiple of 8."""
+    stride = t.stride()
+    c = t.shape[-1]
+    if stride[-1] == 1 and stride[-2] % 8 == 0 and c % 8 == 0 and (len(stride) < 3 or stride[0] % 8 == 0) \
+            and t.data_ptr() % 16 == 0:
+        return t
+    return _pad_to(t.contiguous() if stride[-1] != 1 else t, t.shape[-2], (c + 7) // 8 * 8)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          bias: Optional[torch.Tensor] = None, act=None, residual: Optional[torch.Tensor] = None,
@@ -201,16 +202,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         a = a.to(torch.bfloat16)
     if b.dtype != torch.bfloat16:
         b = b.to(torch.bfloat16)
-    # TMA needs 16-byte aligned rows: pad the contiguous dimension to a multiple of 8.
-    def _fix(t):
-        r, c = t.shape[-2], t.shape[-1]
-        c8 = (c + 7) // 8 * 8
-        if t.stride(-1) != 1 or t.stride(-2) % 8 != 0 or t.data_ptr() % 16 != 0 or c8 != c or \
-                (t.dim() == 3 and t.stride(0) % 8 != 0):
-            return _pad_to(t.contiguous() if t.stride(-1) != 1 else t, r, c8)
-        return t
-    a = _fix(a)
-    b = _fix(b)
+    a, b = _tma_ready(a), _tma_ready(b)
     batch = a.shape[0] if batched else 1
     if out is None:
         shape = (batch, M, N) if batched else (M, N)
@@ -221,54 +213,37 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     for t in (bias, residual, aux_out, aux_in):
         if t is not None:
             assert t.dtype == torch.bfloat16 and t.stride(-1) == 1, "epilogue operands must be bf16"
-    args = _GemmArgs()
-    args.A, args.B, args.C = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.bias = 0 if bias is None else bias.data_ptr()
-    args.residual = 0 if residual is None else residual.data_ptr()
-    args.aux_out = 0 if aux_out is None else aux_out.data_ptr()
-    args.aux_in = 0 if aux_in is None else aux_in.data_ptr()
-    args.lda, args.ldb, args.ldc = a.stride(-2), b.stride(-2), out.stride(-2)
-    args.ldr = 0 if residual is None else residual.stride(-2)
-    args.ld_aux_out = 0 if aux_out is None else aux_out.stride(-2)
-    args.ld_aux_in = 0 if aux_in is None else aux_in.stride(-2)
-    args.batch_stride_a = a.stride(0) if batched else 0
-    args.batch_stride_b = b.stride(0) if batched else 0
-    args.batch_stride_c = out.stride(0) if batched else 0
-    args.M, args.N, args.K, args.batch = M, N, K, batch
-    args.a_mn_major, args.b_mn_major = int(a_mn), int(b_mn)
-    args.out_fp32 = int(out.dtype == torch.float32)
-    args.accumulate = int(accumulate)
-    plain_wgrad = a_mn and b_mn and not batched and out.dtype == torch.float32 and bias is None and residual is None \
-        and aux_out is None and act_id == 0
-    parts = _partial_splits(M, N, K) if SPLIT_K and plain_wgrad and max_ctas == 0 and out.is_contiguous() else 1
-    if parts > 1:
-        kc = K // parts
-        part = torch.empty((parts, M, N), dtype=torch.float32, device=a.device)
-        args.C, args.ldc, args.K, args.batch, args.accumulate = part.data_ptr(), N, kc, parts, 0
-        args.batch_stride_a, args.batch_stride_b, args.batch_stride_c = kc * a.stride(0), kc * b.stride(0), M * N
-        args.act, args.alpha, args.max_ctas = 0, float(alpha), 0
-        stream = native.stream_ptr(a.device)
-        native.check(native.lib().st_gemm_bf16(ctypes.byref(args), stream), "st_gemm_bf16")
-        native.check(native.lib().st_reduce_partials(native.ptr(part), native.ptr(out), ctypes.c_int(parts), ctypes.c_int(M * N),
-                                                     ctypes.c_int(int(accumulate)), stream), "st_reduce_partials")
-        launch_count += 2
-        return out
-    split = _split_k(M, N, K) if (SPLIT_K and not native.deterministic_reduction() and accumulate and a_mn and b_mn and not batched and
-                                  out.dtype == torch.float32 and N % 32 == 0 and out.stride(0) % 4 == 0
-                                  and bias is None and residual is None and act_id == 0) else 1
-    if split > 1:
-        # weight-gradient shape with a poor tile count: split the long reduction over `split`
-        # CTAs per tile (expressed as a batch over K) and add the partials with fp32 atomics
-        kc = K // split
-        args.K, args.batch = kc, split
-        args.batch_stride_a, args.batch_stride_b, args.batch_stride_c = kc * a.stride(0), kc * b.stride(0), 0
-        args.accumulate = 2
-    args.act = act_id
-    args.alpha = float(alpha)
-    args.max_ctas = int(max_ctas)
-    st = native.lib().st_gemm_bf16(ctypes.byref(args), native.stream_ptr(a.device))
-    native.check(st, "st_gemm_bf16")
+    lib, stream = native.lib(), native.stream_ptr(a.device)
+    fp32 = out.dtype == torch.float32
+    target, ldc, k_part, parts, acc, max_ctas = out, out.stride(-2), K, batch, int(accumulate), int(max_ctas)
+    strides = (a.stride(0), b.stride(0), out.stride(0)) if batched else (0, 0, 0)
+    in_parts = False
+    if SPLIT_K and a_mn and b_mn and fp32 and not batched and bias is None and residual is None and act_id == 0:
+        n = _partial_splits(M, N, K) if aux_out is None and max_ctas == 0 and out.is_contiguous() else 1
+        if n > 1:
+            in_parts = True
+            target, ldc, acc = torch.empty((n, M, N), dtype=torch.float32, device=a.device), N, 0
+        elif accumulate and N % 32 == 0 and out.stride(0) % 4 == 0 and not native.deterministic_reduction():
+            # weight-gradient shape with a poor tile count: split the long reduction over CTAs of the same tile
+            # (expressed as a batch over K) and add the partials with fp32 atomics
+            n = _split_k(M, N, K)
+            acc = 2 if n > 1 else acc
+        if n > 1:
+            k_part, parts = K // n, n
+            strides = (k_part * a.stride(0), k_part * b.stride(0), M * N if in_parts else 0)
+    args = _pack_args(
+        a.data_ptr(), b.data_ptr(), target.data_ptr(), 0 if bias is None else bias.data_ptr(),
+        0 if residual is None else residual.data_ptr(), 0 if aux_out is None else aux_out.data_ptr(),
+        0 if aux_in is None else aux_in.data_ptr(), a.stride(-2), b.stride(-2), ldc,
+        0 if residual is None else residual.stride(-2), 0 if aux_out is None else aux_out.stride(-2),
+        0 if aux_in is None else aux_in.stride(-2), *strides, M, N, k_part, parts, int(a_mn), int(b_mn), int(fp32), acc,
+        act_id, float(alpha), max_ctas)
+    native.check(lib.st_gemm_bf16(args, stream), "st_gemm_bf16")
     launch_count += 1
+    if in_parts:
+        native.check(lib.st_reduce_partials(native.ptr(target), native.ptr(out), ctypes.c_int(n), ctypes.c_int(M * N),
+                                            ctypes.c_int(int(accumulate)), stream), "st_reduce_partials")
+        launch_count += 1
     return out
 
 

@@ -117,8 +117,14 @@ def set_wait_timeout(seconds: Optional[float]) -> None:
     check(lib().st_set_wait_timeout_ns(ctypes.c_ulonglong(ns)), "st_set_wait_timeout_ns")
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)      # the handle without a Stream object around it
+
+
 def stream_ptr(device: Optional[torch.device] = None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    index = getattr(device, "index", None)
+    if _raw_stream is None or index is None:
+        return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(_raw_stream(index))
 
 
 def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
