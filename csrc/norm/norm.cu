@@ -210,10 +210,195 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
 }
 
-// out[c] (+)= sum_p partial[p, c].  A CTA owns 32 columns; its 8 thread rows sum every 8th partial
-// (each a coalesced 128-byte read) and are combined through shared memory.
+// ---- rows of up to 1024 features: one warp per row --------------------------------------------------------------------
+// A block per row leaves most of its 256 threads without a vector below 2048 features (96 busy at 768) and passes two to
+// four block barriers per row; a warp keeps a row of up to 1024 in registers and needs shuffles only.
+// T is bf16, or float for the layer protocol, whose tensors then need no conversion passes around the call.
+constexpr int WARP_ROWS = NT / 32;      // rows in flight per CTA
+
+__device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+__device__ __forceinline__ void store8(float* p, const float (&f)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+__device__ __forceinline__ float as_stored(float v, const __nv_bfloat16*) { return __bfloat162float(__float2bfloat16(v)); }
+__device__ __forceinline__ float as_stored(float v, const float*) { return v; }
+
+template <typename T, bool RMS, int MV>
+__global__ void __launch_bounds__(NT)
+norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ gamma,
+                     const T* __restrict__ beta, T* __restrict__ y, T* __restrict__ sum_out, float* __restrict__ mean_out,
+                     float* __restrict__ rstd_out, int rows, int d, float eps) {
+  const int row = blockIdx.x * WARP_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int nvec = d >> 3;
+  const size_t base = (size_t)row * d;
+  float v[MV][8];
+  float s = 0.0f;
+#pragma unroll
+  for (int i = 0; i < MV; ++i) {
+    const int vi = lane + i * 32;
+    if (vi < nvec) load8(x + base + vi * 8, v[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < MV; ++i) {
+    const int vi = lane + i * 32;
+    if (vi < nvec) {
+      if (residual) {
+        float r[8];
+        load8(residual + base + vi * 8, r);
+        // normalise what is stored (rounded to T) so forward and backward agree
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[i][j] = sum_out ? as_stored(v[i][j] + r[j], x) : v[i][j] + r[j];
+      }
+      if (sum_out) store8(sum_out + base + vi * 8, v[i]);      // without a residual: a copy of x
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += RMS ? v[i][j] * v[i][j] : v[i][j];
+    }
+  }
+  s = warp_sum(s) / d;
+  float mean = 0.0f, rstd;
+  if (RMS) {
+    rstd = rsqrtf(s + eps);
+  } else {
+    mean = s;
+    float q = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MV; ++i) {
+      if (lane + i * 32 < nvec) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float c = v[i][j] - mean;
+          q += c * c;
+        }
+      }
+    }
+    rstd = rsqrtf(warp_sum(q) / d + eps);
+  }
+  if (lane == 0) {
+    if (mean_out) mean_out[row] = mean;
+    rstd_out[row] = rstd;
+  }
+#pragma unroll
+  for (int i = 0; i < MV; ++i) {
+    const int vi = lane + i * 32;
+    if (vi < nvec) {
+      float g[8], o[8];
+      load8(gamma + vi * 8, g);
+      if (!RMS && beta) {
+        float b[8];
+        load8(beta + vi * 8, b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = (v[i][j] - mean) * rstd * g[j] + b[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = (v[i][j] - mean) * rstd * g[j];
+      }
+      store8(y + base + vi * 8, o);
+    }
+  }
+}
+
+// Persistent: a warp walks rows and keeps its lanes' share of dgamma / dbeta in registers; the CTA's warps add theirs in
+// warp order through shared memory and leave one partial per CTA.
+template <typename T, bool RMS, int MV>
+__global__ void __launch_bounds__(NT, 2)
+norm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
+                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
+                     T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta, int rows, int d) {
+  __shared__ float sh[(RMS ? 1 : 2) * MV * 256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = d >> 3;
+  float dg[MV][8], db[RMS ? 1 : MV][8];
+#pragma unroll
+  for (int i = 0; i < MV; ++i) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      dg[i][j] = 0.0f;
+      if (!RMS) db[i][j] = 0.0f;
+    }
+  }
+  for (int row = blockIdx.x * WARP_ROWS + warp; row < rows; row += gridDim.x * WARP_ROWS) {
+    const size_t base = (size_t)row * d;
+    const float mean = RMS ? 0.0f : mean_in[row], rstd = rstd_in[row];
+    float xh[MV][8], gy[MV][8];
+    float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MV; ++i) {
+      const int vi = lane + i * 32;
+      if (vi < nvec) {
+        load8(x + base + vi * 8, xh[i]);
+        load8(dy + base + vi * 8, gy[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < MV; ++i) {
+      if (lane + i * 32 < nvec) {
+        float g[8];                      // from L1: kept across rows it cost a second resident CTA
+        load8(gamma + (lane + i * 32) * 8, g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float dv = gy[i][j];
+          xh[i][j] = (xh[i][j] - mean) * rstd;
+          gy[i][j] = dv * g[j];
+          dg[i][j] += dv * xh[i][j];
+          if (!RMS) db[i][j] += dv;
+          s1 += gy[i][j] * xh[i][j];
+          s2 += gy[i][j];
+        }
+      }
+    }
+    const float m1 = warp_sum(s1) / d, m2 = RMS ? 0.0f : warp_sum(s2) / d;
+#pragma unroll
+    for (int i = 0; i < MV; ++i) {
+      const int vi = lane + i * 32;
+      if (vi < nvec) {
+        float o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = rstd * (gy[i][j] - m2 - xh[i][j] * m1);
+        if (dres) {  // gradient arriving through the residual branch
+          float r[8];
+          load8(dres + base + vi * 8, r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += r[j];
+        }
+        store8(dx + base + vi * 8, o);
+      }
+    }
+  }
+  for (int w = 0; w < WARP_ROWS; ++w) {
+    if (warp == w) {
+#pragma unroll
+      for (int i = 0; i < MV; ++i)
+        if (lane + i * 32 < nvec) {
+          float* p = sh + (lane + i * 32) * 8;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            p[j] = w == 0 ? dg[i][j] : p[j] + dg[i][j];
+            if (!RMS) p[MV * 256 + j] = w == 0 ? db[i][j] : p[MV * 256 + j] + db[i][j];
+          }
+        }
+    }
+    __syncthreads();
+  }
+  for (int c = threadIdx.x; c < d; c += NT) {
+    partial_dgamma[(size_t)blockIdx.x * d + c] = sh[c];
+    if (!RMS && partial_dbeta) partial_dbeta[(size_t)blockIdx.x * d + c] = sh[MV * 256 + c];
+  }
+}
+
+// out[c] (+)= sum_p partial[p, c]; with out2, blockIdx.y = 1 does the same for the second set of partials.  A CTA owns
+// 32 columns; its 8 thread rows sum every 8th partial (each a coalesced 128-byte read) and are combined through shared
+// memory.
 __global__ void __launch_bounds__(256)
-reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, int parts, int d, int accumulate) {
+reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, const float* __restrict__ partial2,
+                       float* __restrict__ out2, int parts, int d, int accumulate) {
+  if (blockIdx.y) {
+    partial = partial2;
+    out = out2;
+  }
   __shared__ float sh[8][33];
   const int cx = threadIdx.x & 31, k = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -236,6 +421,51 @@ reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ ou
   }
 }
 
+constexpr int kWarpRowFeatures = 1024;
+
+template <typename T>
+int fwd_warp(int rms, const T* x, const T* r, const T* g, const T* b, T* y, T* s, float* mean, float* rstd, int rows, int d,
+             float eps, cudaStream_t stream) {
+  const int grid = (rows + WARP_ROWS - 1) / WARP_ROWS;
+#define ST_FWD_WARP(MVV) \
+  if (rms) norm_fwd_warp_kernel<T, true, MVV><<<grid, NT, 0, stream>>>(x, r, g, b, y, s, mean, rstd, rows, d, eps); \
+  else norm_fwd_warp_kernel<T, false, MVV><<<grid, NT, 0, stream>>>(x, r, g, b, y, s, mean, rstd, rows, d, eps)
+  switch ((d + 255) / 256) {
+    case 1: ST_FWD_WARP(1); break;
+    case 2: ST_FWD_WARP(2); break;
+    case 3: ST_FWD_WARP(3); break;
+    default: ST_FWD_WARP(4); break;
+  }
+#undef ST_FWD_WARP
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+template <typename T>
+int bwd_warp(int rms, const T* dy, const T* x, const T* g, const float* mean, const float* rstd, const T* dres, T* dx,
+             float* pg, float* pb, int rows, int d, int grid, cudaStream_t stream) {
+#define ST_BWD_WARP(MVV) \
+  if (rms) norm_bwd_warp_kernel<T, true, MVV><<<grid, NT, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, nullptr, rows, d); \
+  else norm_bwd_warp_kernel<T, false, MVV><<<grid, NT, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, pb, rows, d)
+  switch ((d + 255) / 256) {
+    case 1: ST_BWD_WARP(1); break;
+    case 2: ST_BWD_WARP(2); break;
+    case 3: ST_BWD_WARP(3); break;
+    default: ST_BWD_WARP(4); break;
+  }
+#undef ST_BWD_WARP
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+int reduce_param_grads(int rms, const float* pg, const float* pb, float* dgamma, float* dbeta, int grid, int d, int accumulate,
+                       cudaStream_t stream) {
+  const bool both = !rms && dbeta;
+  reduce_partials_kernel<<<dim3((d + 31) / 32, both ? 2 : 1), 256, 0, stream>>>(pg, dgamma, pb, dbeta, grid, d, accumulate);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
 }  // namespace
 
 namespace st {
@@ -243,8 +473,13 @@ int norm_bwd_grid(int rows) {
   int g = sm_count() * 2;
   return rows < g ? rows : g;
 }
-// CTAs for the regular entry: as many as stay resident (register footprint grows with d)
+// CTAs for the regular entry: as many as stay resident (register footprint grows with d); one warp per row up to
+// kWarpRowFeatures
 int norm_bwd_grid_for(int rows, int d) {
+  if (d <= kWarpRowFeatures) {
+    const int need = (rows + WARP_ROWS - 1) / WARP_ROWS, most = sm_count() * 2;
+    return need < most ? need : most;
+  }
   const int per_sm = d <= 2048 ? 4 : 2;
   int g = sm_count() * per_sm;
   return rows < g ? rows : g;
@@ -269,6 +504,7 @@ ST_API int st_norm_fwd(int rms, const void* x, const void* residual, const void*
   auto B = static_cast<const __nv_bfloat16*>(beta);
   auto Y = static_cast<__nv_bfloat16*>(y);
   auto S = static_cast<__nv_bfloat16*>(sum_out);
+  if (d <= kWarpRowFeatures) return fwd_warp<__nv_bfloat16>(rms, X, R, G, B, Y, S, mean, rstd, rows, d, eps, s);
 #define ST_NORM_FWD(RMSV, MVV) norm_fwd_kernel<RMSV, MVV><<<rows, NT, 0, s>>>(X, R, G, B, Y, S, mean, rstd, rows, d, eps)
   const int mv = d <= NT * 8 ? 1 : (d <= NT * 16 ? 2 : 4);
   if (rms) {
@@ -299,6 +535,10 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   auto G = static_cast<const __nv_bfloat16*>(gamma);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
+  if (d <= kWarpRowFeatures) {
+    if (int e = bwd_warp<__nv_bfloat16>(rms, DY, X, G, mean, rstd, DR, DX, pg, rms ? nullptr : pb, rows, d, grid, s)) return e;
+    return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
+  }
 #define ST_NORM_BWD(RMSV, MVV, PB) norm_bwd_kernel<RMSV, MVV><<<grid, NT, 0, s>>>(DY, X, G, mean, rstd, DR, DX, pg, PB, rows, d)
   const int mv = d <= NT * 8 ? 1 : (d <= NT * 16 ? 2 : 4);
   if (rms) {
@@ -308,19 +548,37 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   }
 #undef ST_NORM_BWD
   ST_CUDA_CHECK(cudaGetLastError());
-  reduce_partials_kernel<<<(d + 31) / 32, 256, 0, s>>>(pg, dgamma, grid, d, accumulate);
-  if (!rms && dbeta)
-    reduce_partials_kernel<<<(d + 31) / 32, 256, 0, s>>>(pb, dbeta, grid, d, accumulate);
-  ST_CUDA_CHECK(cudaGetLastError());
-  return ST_OK;
+  return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
 }
 
 // out[i] (+)= sum over p of partial[p * n + i], in a fixed order.
 ST_API int st_reduce_partials(const float* partial, float* out, int parts, int n, int accumulate, void* stream_v) {
   if (!partial || !out || parts <= 0 || n <= 0) return st::fail(ST_ERR_INVALID, "reduce_partials: bad arguments");
-  reduce_partials_kernel<<<(n + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, parts, n, accumulate);
+  reduce_partials_kernel<<<(n + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, nullptr, nullptr, parts, n, accumulate);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
+}
+
+// fp32 tensors throughout, rows of at most 1024 features, 16-byte aligned: the layer protocol's LayerNorm without
+// conversion passes.  scratch: st_norm_bwd_scratch_elems floats.
+ST_API int st_norm_f32_max_features() { return kWarpRowFeatures; }
+ST_API int st_norm_fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y,
+                           float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v) {
+  if (int e = check_dims(rows, d)) return e;
+  if (d > kWarpRowFeatures) return st::fail(ST_ERR_TOO_LARGE, "norm_f32: feature dimension above 1024");
+  return fwd_warp<float>(rms, x, residual, gamma, beta, y, sum_out, mean, rstd, rows, d, eps, reinterpret_cast<cudaStream_t>(stream_v));
+}
+ST_API int st_norm_bwd_f32(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd,
+                           const float* dres, float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows,
+                           int d, void* stream_v) {
+  if (int e = check_dims(rows, d)) return e;
+  if (d > kWarpRowFeatures) return st::fail(ST_ERR_TOO_LARGE, "norm_f32: feature dimension above 1024");
+  if (!scratch) return st::fail(ST_ERR_INVALID, "norm_f32: scratch buffer is required");
+  const int grid = st::norm_bwd_grid_for(rows, d);
+  float* pb = scratch + (size_t)grid * d;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  if (int e = bwd_warp<float>(rms, dy, x, gamma, mean, rstd, dres, dx, scratch, rms ? nullptr : pb, rows, d, grid, s)) return e;
+  return reduce_param_grads(rms, scratch, pb, dgamma, dbeta, grid, d, accumulate, s);
 }
 
 // dgamma / dbeta are fp32 [d]; with accumulate != 0 the kernel adds to them.

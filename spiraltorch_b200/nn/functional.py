@@ -104,25 +104,38 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 # layer norm (optionally with a residual added first)
 # ------------------------------------------------------------------------------------------------------
 class _LayerNormFn(torch.autograd.Function):
+    """The tensors stay fp32 where the kernels take them so (rows of up to 1024 features); wider rows pass through bf16."""
+
     @staticmethod
     def forward(ctx, x, gamma, beta, eps, residual):
-        xb = x.detach().to(torch.bfloat16).contiguous()
-        rb = None if residual is None else residual.detach().to(torch.bfloat16).contiguous()
-        gb, bb = bf16_of(gamma).reshape(-1), bf16_of(beta).reshape(-1)
-        y, summed, mean, rstd = _norm.norm_forward(xb, gb, bb, float(eps), False, rb)
-        ctx.save_for_backward(xb if summed is None else summed, gb, mean, rstd)
-        ctx.has_residual = residual is not None
-        ctx.pshape = gamma.shape
+        ctx.has_residual, ctx.pshape = residual is not None, gamma.shape
         launch_counts["layer_norm"] += 1
-        return y.float()
+        xd, rd = x.detach(), None if residual is None else residual.detach()
+        ctx.fp32 = x.dim() == 2 and _norm.takes_f32(x.shape[-1], xd, gamma, beta, rd)
+        if ctx.fp32:
+            g, b = gamma.detach().reshape(-1), beta.detach().reshape(-1)
+        else:
+            xd = xd.to(torch.bfloat16).contiguous()
+            rd = None if rd is None else rd.to(torch.bfloat16).contiguous()
+            g, b = bf16_of(gamma).reshape(-1), bf16_of(beta).reshape(-1)
+        # the backward reads copies, as with the bf16 operands: the caller may go on to change x or the gain in place
+        keep = ctx.fp32 and any(ctx.needs_input_grad)
+        y, summed, mean, rstd = _norm.norm_forward(xd, g, b, float(eps), False, rd, copy_input=keep)
+        ctx.save_for_backward(xd if summed is None else summed, g.clone() if keep else g, mean, rstd)
+        return y if ctx.fp32 else y.float()
 
     @staticmethod
     def backward(ctx, dy):
-        xin, gb, mean, rstd = ctx.saved_tensors
-        dyb = dy.to(torch.bfloat16).contiguous()
+        xin, g, mean, rstd = ctx.saved_tensors
+        if ctx.fp32:
+            d = dy.contiguous()
+            if not _norm.takes_f32(d.shape[-1], d):
+                d = d.float().clone(memory_format=torch.contiguous_format)
+        else:
+            d = dy.to(torch.bfloat16).contiguous()
         dg = torch.empty(xin.shape[1], dtype=torch.float32, device=xin.device)
         db = torch.empty_like(dg)
-        dx = _norm.norm_backward(dyb, xin, gb, mean, rstd, False, dg, db, False).float()
+        dx = _norm.norm_backward(d, xin, g, mean, rstd, False, dg, db, False).float()
         return dx, dg.reshape(ctx.pshape), db.reshape(ctx.pshape), None, (dx if ctx.has_residual else None)
 
 

@@ -29,6 +29,12 @@ def _get_scratch(device, elems: int) -> torch.Tensor:
     return buf
 
 
+def takes_f32(d: int, *tensors: Optional[torch.Tensor]) -> bool:
+    """Whether the fp32 form of the kernels takes these tensors (``None`` entries are skipped)."""
+    return d % 8 == 0 and 0 < d <= 1024 and all(
+        t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in tensors)
+
+
 def norm_reference(x, gamma, beta, eps, rms, residual=None):
     xf = x.float()
     if residual is not None:
@@ -47,9 +53,9 @@ def norm_reference(x, gamma, beta, eps, rms, residual=None):
     return y, xf, mean.squeeze(-1), rstd.squeeze(-1)
 
 
-def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=None, out=None):
-    """x2: [rows, d] bf16.  Returns (y, summed_input_or_None, mean, rstd); ``out`` (contiguous, same shape and
-    dtype) receives y when given."""
+def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=None, out=None, copy_input: bool = False):
+    """x2: [rows, d] bf16, or fp32 throughout where :func:`takes_f32`.  Returns (y, summed_input_or_None, mean, rstd); ``out`` (contiguous, same shape and
+    dtype) receives y when given.  ``copy_input`` (fp32 form): without a residual the second result is a copy of x2."""
     global launch_count
     rows, d = x2.shape
     if out is not None:
@@ -61,10 +67,11 @@ def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=
             y = out.copy_(y)
         return y, (xs.to(x2.dtype) if residual is not None else None), mean, rstd
     y = torch.empty_like(x2) if out is None else out
-    s = torch.empty_like(x2) if residual is not None else None
+    s = torch.empty_like(x2) if residual is not None or (copy_input and x2.dtype == torch.float32) else None
     mean = torch.empty(rows, dtype=torch.float32, device=x2.device)
     rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
-    st = native.lib().st_norm_fwd(
+    entry = native.lib().st_norm_fwd_f32 if x2.dtype == torch.float32 else native.lib().st_norm_fwd
+    st = entry(
         ctypes.c_int(int(rms)), native.ptr(x2), native.ptr(residual), native.ptr(gamma), native.ptr(beta),
         native.ptr(y), native.ptr(s), native.ptr(mean), native.ptr(rstd), ctypes.c_int(rows),
         ctypes.c_int(d), ctypes.c_float(eps), native.stream_ptr(x2.device))
@@ -101,13 +108,13 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
     lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
     need = lib.st_norm_bwd_scratch_elems(ctypes.c_int(rows), ctypes.c_int(d))
     scratch = _get_scratch(x2.device, int(need))
-    st = lib.st_norm_bwd(
+    st = (lib.st_norm_bwd_f32 if x2.dtype == torch.float32 else lib.st_norm_bwd)(
         ctypes.c_int(int(rms)), native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(mean),
         native.ptr(rstd), native.ptr(dres), native.ptr(dx), native.ptr(dgamma), native.ptr(dbeta),
         ctypes.c_int(int(accumulate)), native.ptr(scratch), ctypes.c_int(rows), ctypes.c_int(d),
         native.stream_ptr(x2.device))
     native.check(st, "st_norm_bwd")
-    launch_count += 2 if rms or dbeta is None else 3
+    launch_count += 2
     return dx
 
 

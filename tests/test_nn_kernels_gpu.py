@@ -344,3 +344,45 @@ def test_mean_squared_error_in_one_launch(rows, cols):
     for call in (loss.forward, loss.backward):
         with pytest.raises(Exception, match="non-finite"):
             call(st.Tensor(p), st.Tensor(t))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,d", [(1, 8), (7, 256), (9, 264), (2400, 768), (5000, 1024), (3, 1032)])
+def test_norm_with_a_warp_per_row(rows, d, rms, dtype):
+    """Vector counts 1 to 4 per lane, partial ones, more rows than a grid holds, the first width past the warp form (bf16
+    only), residual and gradient sums; bounds: one rounding of the output type, fp32 sums over the rows."""
+    if dtype == torch.float32 and d > 1024:
+        assert not N.takes_f32(d)
+        return
+    torch.manual_seed(rows + d)
+    x, r, dy, dres = (torch.randn(rows, d, device=DEV).to(dtype) for _ in range(4))
+    g, b = torch.randn(d, device=DEV).to(dtype), (None if rms else torch.randn(d, device=DEV).to(dtype))
+    tol = 2 ** -8 if dtype == torch.bfloat16 else 2e-6
+    y, s, mean, rstd = N.norm_forward(x, g, b, 1e-5, rms, r)
+    assert torch.equal(s, x + r)
+    sd = s.double()
+    mu = 0 if rms else sd.mean(-1, keepdim=True)
+    rs = torch.rsqrt((sd - mu).pow(2).mean(-1, keepdim=True) + 1e-5)
+    want = (sd - mu) * rs * g.double() + (0 if rms else b.double())
+    assert ((y.double() - want).abs() <= tol * want.abs() + 1e-5).all()
+    dg, db = torch.full((d,), 0.5, device=DEV), (None if rms else torch.full((d,), 0.25, device=DEV))
+    dx = N.norm_backward(dy, s, g, mean, rstd, rms, dg, db, True, dres)
+    xh, gy = (sd - mu) * rs, dy.double() * g.double()
+    m2 = 0 if rms else gy.mean(-1, keepdim=True)
+    want = rs * (gy - m2 - xh * (gy * xh).mean(-1, keepdim=True)) + dres.double()
+    assert ((dx.double() - want).abs() <= tol * want.abs() + 2e-5).all()
+    assert torch.allclose(dg.double(), 0.5 + (dy.double() * xh).sum(0), rtol=1e-5, atol=1e-3)
+    if not rms:
+        assert torch.allclose(db.double(), 0.25 + dy.double().sum(0), rtol=1e-5, atol=1e-3)
+
+
+def test_layer_norm_backward_reads_the_values_of_the_forward():
+    x, g, b = (torch.randn(s, device=DEV, requires_grad=True) for s in ((6, 64), (1, 64), (1, 64)))
+    want = torch.autograd.grad(Fn.layer_norm(x, g, b).sum(), (x, g, b))
+    h = x * 1.0
+    y = Fn.layer_norm(h, g, b).sum()
+    with torch.no_grad():
+        h.mul_(3.0)
+        g.add_(1.0)
+    assert all(torch.equal(p, q) for p, q in zip(torch.autograd.grad(y, (x, g, b)), want))
