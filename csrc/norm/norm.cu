@@ -212,7 +212,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 
 // ---- rows of up to 1024 features: one warp per row --------------------------------------------------------------------
 // A block per row leaves most of its 256 threads without a vector below 2048 features (96 busy at 768) and passes two to
-// four block barriers per row; a warp keeps a row of up to 1024 in registers and needs shuffles only.
+// four block barriers per row; a warp keeps a row of up to 1024 in registers and needs shuffles only.  Forward of 16384 rows
+// of 768 features: 36 us with a block per row, 19 now, 15 of bytes.
 // T is bf16, or float for the layer protocol, whose tensors then need no conversion passes around the call.
 constexpr int WARP_ROWS = NT / 32;      // rows in flight per CTA
 
@@ -226,6 +227,30 @@ __device__ __forceinline__ void store8(float* p, const float (&f)[8]) {
 }
 __device__ __forceinline__ float as_stored(float v, const __nv_bfloat16*) { return __bfloat162float(__float2bfloat16(v)); }
 __device__ __forceinline__ float as_stored(float v, const float*) { return v; }
+
+// Eight elements as they lie in memory
+template <typename T>
+struct Raw8;
+template <>
+struct Raw8<__nv_bfloat16> {
+  uint4 u;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+  }
+};
+template <>
+struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) {
+    a = reinterpret_cast<const float4*>(p)[0];
+    b = reinterpret_cast<const float4*>(p)[1];
+  }
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+  }
+};
 
 template <typename T, bool RMS, int MV>
 __global__ void __launch_bounds__(NT)
@@ -302,126 +327,132 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, co
   }
 }
 
-// Persistent: a warp walks rows and keeps its lanes' share of dgamma / dbeta in registers; the CTA's warps add theirs in
-// warp order through shared memory and leave one partial per CTA.
-template <typename T, bool RMS, int MV>
-__global__ void __launch_bounds__(NT, 2)
-norm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
+// Backward for up to 2048 features: thread t owns the 8 columns from 8 t, a persistent CTA of d / 8 threads takes ROWS rows
+// per step.  The gradient sums of a column then need 16 registers, not 16 per vector of a whole row (a warp per row spilled
+// at 1024 features and kept 16 rows in flight per SM), all loads of a step are issued together, and its row sums cost one
+// barrier: two to four per row with a block per row.
+template <typename T, bool RMS, int ROWS>
+__global__ void __launch_bounds__(NT)
+norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
                      T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta, int rows, int d) {
-  __shared__ float sh[(RMS ? 1 : 2) * MV * 256];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = d >> 3;
-  float dg[MV][8], db[RMS ? 1 : MV][8];
+  __shared__ float sh[2][NT / 32][2 * ROWS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int c0 = threadIdx.x * 8;
+  const bool live = c0 < d;
+  float g[8], dg[8], db[8];
 #pragma unroll
-  for (int i = 0; i < MV; ++i) {
+  for (int j = 0; j < 8; ++j) g[j] = dg[j] = db[j] = 0.0f;
+  if (live) load8(gamma + c0, g);
+  int buf = 0;
+  for (long long row0 = (long long)blockIdx.x * ROWS; row0 < rows; row0 += (long long)gridDim.x * ROWS, buf ^= 1) {
+    Raw8<T> xr[ROWS], yr[ROWS], rr[ROWS];
+    float mean[ROWS], rstd[ROWS], sums[2 * ROWS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      dg[i][j] = 0.0f;
-      if (!RMS) db[i][j] = 0.0f;
-    }
-  }
-  for (int row = blockIdx.x * WARP_ROWS + warp; row < rows; row += gridDim.x * WARP_ROWS) {
-    const size_t base = (size_t)row * d;
-    const float mean = RMS ? 0.0f : mean_in[row], rstd = rstd_in[row];
-    float xh[MV][8], gy[MV][8];
-    float s1 = 0.0f, s2 = 0.0f;
-#pragma unroll
-    for (int i = 0; i < MV; ++i) {
-      const int vi = lane + i * 32;
-      if (vi < nvec) {
-        load8(x + base + vi * 8, xh[i]);
-        load8(dy + base + vi * 8, gy[i]);
+    for (int r = 0; r < ROWS; ++r) {
+      if (row0 + r < rows && live) {
+        const size_t at = (size_t)(row0 + r) * d + c0;
+        xr[r].load(x + at);
+        yr[r].load(dy + at);
+        if (dres) rr[r].load(dres + at);
       }
     }
 #pragma unroll
-    for (int i = 0; i < MV; ++i) {
-      if (lane + i * 32 < nvec) {
-        float g[8];                      // from L1: kept across rows it cost a second resident CTA
-        load8(gamma + (lane + i * 32) * 8, g);
+    for (int r = 0; r < ROWS; ++r) {
+      const bool in = row0 + r < rows;
+      mean[r] = !RMS && in ? mean_in[row0 + r] : 0.0f;
+      rstd[r] = in ? rstd_in[row0 + r] : 0.0f;
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      float s1 = 0.0f, s2 = 0.0f;
+      if (row0 + r < rows && live) {
+        float xv[8], dv[8];
+        xr[r].get(xv);
+        yr[r].get(dv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float dv = gy[i][j];
-          xh[i][j] = (xh[i][j] - mean) * rstd;
-          gy[i][j] = dv * g[j];
-          dg[i][j] += dv * xh[i][j];
-          if (!RMS) db[i][j] += dv;
-          s1 += gy[i][j] * xh[i][j];
-          s2 += gy[i][j];
+          const float xh = (xv[j] - mean[r]) * rstd[r], gy = dv[j] * g[j];
+          dg[j] += dv[j] * xh;
+          if (!RMS) db[j] += dv[j];
+          s1 += gy * xh;
+          s2 += gy;
         }
       }
+      sums[2 * r] = warp_sum(s1);
+      sums[2 * r + 1] = RMS ? 0.0f : warp_sum(s2);
     }
-    const float m1 = warp_sum(s1) / d, m2 = RMS ? 0.0f : warp_sum(s2) / d;
+    if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < MV; ++i) {
-      const int vi = lane + i * 32;
-      if (vi < nvec) {
-        float o[8];
+      for (int i = 0; i < 2 * ROWS; ++i) sh[buf][warp][i] = sums[i];
+    }
+    __syncthreads();      // the other buffer's readers are past it: they arrive here only after reading
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd * (gy[i][j] - m2 - xh[i][j] * m1);
-        if (dres) {  // gradient arriving through the residual branch
-          float r[8];
-          load8(dres + base + vi * 8, r);
+    for (int i = 0; i < 2 * ROWS; ++i) {
+      float t = 0.0f;
+      for (int w = 0; w < warps; ++w) t += sh[buf][w][i];
+      sums[i] = t / d;
+    }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += r[j];
-        }
-        store8(dx + base + vi * 8, o);
+    for (int r = 0; r < ROWS; ++r) {
+      if (row0 + r >= rows || !live) continue;
+      float xv[8], dv[8], o[8];
+      xr[r].get(xv);
+      yr[r].get(dv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        o[j] = rstd[r] * (dv[j] * g[j] - sums[2 * r + 1] - (xv[j] - mean[r]) * rstd[r] * sums[2 * r]);
+      if (dres) {  // gradient arriving through the residual branch
+        float q[8];
+        rr[r].get(q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += q[j];
       }
+      store8(dx + (size_t)(row0 + r) * d + c0, o);
     }
   }
-  for (int w = 0; w < WARP_ROWS; ++w) {
-    if (warp == w) {
-#pragma unroll
-      for (int i = 0; i < MV; ++i)
-        if (lane + i * 32 < nvec) {
-          float* p = sh + (lane + i * 32) * 8;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            p[j] = w == 0 ? dg[i][j] : p[j] + dg[i][j];
-            if (!RMS) p[MV * 256 + j] = w == 0 ? db[i][j] : p[MV * 256 + j] + db[i][j];
-          }
-        }
-    }
-    __syncthreads();
-  }
-  for (int c = threadIdx.x; c < d; c += NT) {
-    partial_dgamma[(size_t)blockIdx.x * d + c] = sh[c];
-    if (!RMS && partial_dbeta) partial_dbeta[(size_t)blockIdx.x * d + c] = sh[MV * 256 + c];
-  }
+  if (!live) return;
+  store8(partial_dgamma + (size_t)blockIdx.x * d + c0, dg);
+  if (!RMS && partial_dbeta) store8(partial_dbeta + (size_t)blockIdx.x * d + c0, db);
 }
 
 // out[c] (+)= sum_p partial[p, c]; with out2, blockIdx.y = 1 does the same for the second set of partials.  A CTA owns
-// 32 columns; its 8 thread rows sum every 8th partial (each a coalesced 128-byte read) and are combined through shared
+// 32 columns; its 32 thread rows sum every 32nd partial (each a coalesced 128-byte read) and are combined through shared
 // memory.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, const float* __restrict__ partial2,
                        float* __restrict__ out2, int parts, int d, int accumulate) {
   if (blockIdx.y) {
     partial = partial2;
     out = out2;
   }
-  __shared__ float sh[8][33];
+  __shared__ float sh[32][33];
   const int cx = threadIdx.x & 31, k = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
   float s0 = 0.0f, s1 = 0.0f;
   if (c < d) {
     int p = k;
-    for (; p + 8 < parts; p += 16) {
+    for (; p + 32 < parts; p += 64) {
       s0 += partial[(size_t)p * d + c];
-      s1 += partial[(size_t)(p + 8) * d + c];
+      s1 += partial[(size_t)(p + 32) * d + c];
     }
     if (p < parts) s0 += partial[(size_t)p * d + c];
   }
   sh[k][cx] = s0 + s1;
   __syncthreads();
-  if (k == 0 && c < d) {
-    float t = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t += sh[i][cx];
-    out[c] = accumulate ? out[c] + t : t;
-  }
+  const float t = warp_sum(sh[cx][k]);       // thread row k now holds column k's 32 sums
+  const int cc = blockIdx.x * 32 + k;
+  if (cx == 0 && cc < d) out[cc] = accumulate ? out[cc] + t : t;
 }
 
-constexpr int kWarpRowFeatures = 1024;
+constexpr int kWarpRowFeatures = 1024;   // forward, fp32 form
+// Backward with a thread per 8 columns: 16384 rows of 768 / 1024 features in 31 / 38 us where a block per row took 62 / 67
+// (15 / 21 of bytes); with 2048 features LayerNorm takes 73 instead of 88 us, but RMSNorm 73 instead of 63, because the
+// block kernel keeps four CTAs resident without the offset's sums.  Two rows per step and 768 threads per SM are the best
+// of {1, 2, 4} x {512, 768, 1024}.
+constexpr int kRowsThreads = 768;
+inline bool rows_kernel(int rms, int d) { return d <= kWarpRowFeatures || (!rms && d <= NT * 8); }
+inline int bwd_threads(int d) { return (d + 255) / 256 * 32; }
 
 template <typename T>
 int fwd_warp(int rms, const T* x, const T* r, const T* g, const T* b, T* y, T* s, float* mean, float* rstd, int rows, int d,
@@ -442,18 +473,12 @@ int fwd_warp(int rms, const T* x, const T* r, const T* g, const T* b, T* y, T* s
 }
 
 template <typename T>
-int bwd_warp(int rms, const T* dy, const T* x, const T* g, const float* mean, const float* rstd, const T* dres, T* dx,
+int bwd_rows(int rms, const T* dy, const T* x, const T* g, const float* mean, const float* rstd, const T* dres, T* dx,
              float* pg, float* pb, int rows, int d, int grid, cudaStream_t stream) {
-#define ST_BWD_WARP(MVV) \
-  if (rms) norm_bwd_warp_kernel<T, true, MVV><<<grid, NT, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, nullptr, rows, d); \
-  else norm_bwd_warp_kernel<T, false, MVV><<<grid, NT, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, pb, rows, d)
-  switch ((d + 255) / 256) {
-    case 1: ST_BWD_WARP(1); break;
-    case 2: ST_BWD_WARP(2); break;
-    case 3: ST_BWD_WARP(3); break;
-    default: ST_BWD_WARP(4); break;
-  }
-#undef ST_BWD_WARP
+  constexpr int ROWS = 2;
+  const int threads = bwd_threads(d);
+  if (rms) norm_bwd_rows_kernel<T, true, ROWS><<<grid, threads, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, nullptr, rows, d);
+  else norm_bwd_rows_kernel<T, false, ROWS><<<grid, threads, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, pb, rows, d);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -461,7 +486,7 @@ int bwd_warp(int rms, const T* dy, const T* x, const T* g, const float* mean, co
 int reduce_param_grads(int rms, const float* pg, const float* pb, float* dgamma, float* dbeta, int grid, int d, int accumulate,
                        cudaStream_t stream) {
   const bool both = !rms && dbeta;
-  reduce_partials_kernel<<<dim3((d + 31) / 32, both ? 2 : 1), 256, 0, stream>>>(pg, dgamma, pb, dbeta, grid, d, accumulate);
+  reduce_partials_kernel<<<dim3((d + 31) / 32, both ? 2 : 1), 1024, 0, stream>>>(pg, dgamma, pb, dbeta, grid, d, accumulate);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -473,11 +498,11 @@ int norm_bwd_grid(int rows) {
   int g = sm_count() * 2;
   return rows < g ? rows : g;
 }
-// CTAs for the regular entry: as many as stay resident (register footprint grows with d); one warp per row up to
-// kWarpRowFeatures
+// CTAs for the regular entry: as many as stay resident (register footprint grows with d)
 int norm_bwd_grid_for(int rows, int d) {
   if (d <= kWarpRowFeatures) {
-    const int need = (rows + WARP_ROWS - 1) / WARP_ROWS, most = sm_count() * 2;
+    const int resident = kRowsThreads / bwd_threads(d);
+    const int need = (rows + 1) / 2, most = sm_count() * (resident < 16 ? resident : 16);
     return need < most ? need : most;
   }
   const int per_sm = d <= 2048 ? 4 : 2;
@@ -529,14 +554,15 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   if (int e = check_dims(rows, d)) return e;
   if (grid < 1) return st::fail(ST_ERR_INVALID, "norm_bwd: grid must be positive");
   float* pg = scratch;
-  float* pb = scratch + (size_t)grid * d;
+  float* pb = scratch + (size_t)grid * d;      // (a smaller grid below leaves the space between unused)
   auto DY = static_cast<const __nv_bfloat16*>(dy);
   auto X = static_cast<const __nv_bfloat16*>(x);
   auto G = static_cast<const __nv_bfloat16*>(gamma);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
-  if (d <= kWarpRowFeatures) {
-    if (int e = bwd_warp<__nv_bfloat16>(rms, DY, X, G, mean, rstd, DR, DX, pg, rms ? nullptr : pb, rows, d, grid, s)) return e;
+  if (rows_kernel(rms, d)) {
+    if (d > kWarpRowFeatures && grid > st::sm_count() * 3) grid = st::sm_count() * 3;      // 768 of 256 threads
+    if (int e = bwd_rows<__nv_bfloat16>(rms, DY, X, G, mean, rstd, DR, DX, pg, rms ? nullptr : pb, rows, d, grid, s)) return e;
     return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
   }
 #define ST_NORM_BWD(RMSV, MVV, PB) norm_bwd_kernel<RMSV, MVV><<<grid, NT, 0, s>>>(DY, X, G, mean, rstd, DR, DX, pg, PB, rows, d)
@@ -544,7 +570,7 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   if (rms) {
     if (mv == 1) ST_NORM_BWD(true, 1, nullptr); else if (mv == 2) ST_NORM_BWD(true, 2, nullptr); else ST_NORM_BWD(true, 4, nullptr);
   } else {
-    if (mv == 1) ST_NORM_BWD(false, 1, pb); else if (mv == 2) ST_NORM_BWD(false, 2, pb); else ST_NORM_BWD(false, 4, pb);
+    if (mv == 2) ST_NORM_BWD(false, 2, pb); else ST_NORM_BWD(false, 4, pb);
   }
 #undef ST_NORM_BWD
   ST_CUDA_CHECK(cudaGetLastError());
@@ -554,7 +580,7 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
 // out[i] (+)= sum over p of partial[p * n + i], in a fixed order.
 ST_API int st_reduce_partials(const float* partial, float* out, int parts, int n, int accumulate, void* stream_v) {
   if (!partial || !out || parts <= 0 || n <= 0) return st::fail(ST_ERR_INVALID, "reduce_partials: bad arguments");
-  reduce_partials_kernel<<<(n + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, nullptr, nullptr, parts, n, accumulate);
+  reduce_partials_kernel<<<(n + 31) / 32, 1024, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, nullptr, nullptr, parts, n, accumulate);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -577,7 +603,7 @@ ST_API int st_norm_bwd_f32(int rms, const float* dy, const float* x, const float
   const int grid = st::norm_bwd_grid_for(rows, d);
   float* pb = scratch + (size_t)grid * d;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (int e = bwd_warp<float>(rms, dy, x, gamma, mean, rstd, dres, dx, scratch, rms ? nullptr : pb, rows, d, grid, s)) return e;
+  if (int e = bwd_rows<float>(rms, dy, x, gamma, mean, rstd, dres, dx, scratch, rms ? nullptr : pb, rows, d, grid, s)) return e;
   return reduce_param_grads(rms, scratch, pb, dgamma, dbeta, grid, d, accumulate, s);
 }
 

@@ -348,7 +348,7 @@ def test_mean_squared_error_in_one_launch(rows, cols):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("rows,d", [(1, 8), (7, 256), (9, 264), (2400, 768), (5000, 1024), (3, 1032)])
+@pytest.mark.parametrize("rows,d", [(1, 8), (7, 256), (9, 264), (2400, 768), (5000, 1024), (3, 1032), (2500, 2048)])
 def test_norm_with_a_warp_per_row(rows, d, rms, dtype):
     """Vector counts 1 to 4 per lane, partial ones, more rows than a grid holds, the first width past the warp form (bf16
     only), residual and gradient sums; bounds: one rounding of the output type, fp32 sums over the rows."""
