@@ -31,6 +31,8 @@
 namespace st {
 bool encode_bshd_tmap(CUtensorMap* out, const void* base, int B, int S, int H, int D,
                       long long sb, long long ss, long long sh, int box_rows);
+int attn_key_bias(const float* kb, long long kb_sb, long long kb_sh, const int* lengths, float* ws, int B, int H, int Sk,
+                  long long* out_sb, long long* out_sh, cudaStream_t stream);
 }
 
 namespace {
@@ -41,6 +43,9 @@ constexpr int EW_WARPS = 16;                       // element-wise warps: four t
 constexpr int EW_THREADS = EW_WARPS * 32;
 constexpr int NUM_THREADS = EW_THREADS + 64;       // + TMA producer warp + MMA warp
 constexpr int MODE_KV = 0, MODE_Q = 1;
+// Biases: none; a bias per (query, key) among them, read and compared per element; key bias and length only, as padded rows
+// in the log2 domain (minus infinity where masked): 16-byte loads, no comparisons.
+constexpr int BIAS_NONE = 0, BIAS_FULL = 1, BIAS_KEYS = 2;
 
 struct AttnBwdParams {
   const float* lse;
@@ -58,7 +63,36 @@ struct AttnBwdParams {
   const float* attn_bias;
   const int* lengths;
   long long kb_sb, kb_sh, ab_sb, ab_sh, ab_sq;
+  const float* kb_pad;          // BIAS_KEYS
+  long long kp_sb, kp_sh;
+  int grad_f32;                 // dQ, dK and dV are fp32
 };
+
+// 32 accumulator columns of a row, scaled, as bf16 or fp32; `row` is an element offset
+__device__ __forceinline__ void store_grad(__nv_bfloat16* base, int f32, long long row, const uint32_t (&t)[32], float scale) {
+  if (f32) {
+    float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + row);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      o[q] = make_float4(__uint_as_float(t[4 * q]) * scale, __uint_as_float(t[4 * q + 1]) * scale,
+                         __uint_as_float(t[4 * q + 2]) * scale, __uint_as_float(t[4 * q + 3]) * scale);
+    return;
+  }
+  uint4* o = reinterpret_cast<uint4*>(base + row);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 u;
+    u.x = pack_bf16x2(__uint_as_float(t[q * 8 + 0]) * scale, __uint_as_float(t[q * 8 + 1]) * scale);
+    u.y = pack_bf16x2(__uint_as_float(t[q * 8 + 2]) * scale, __uint_as_float(t[q * 8 + 3]) * scale);
+    u.z = pack_bf16x2(__uint_as_float(t[q * 8 + 4]) * scale, __uint_as_float(t[q * 8 + 5]) * scale);
+    u.w = pack_bf16x2(__uint_as_float(t[q * 8 + 6]) * scale, __uint_as_float(t[q * 8 + 7]) * scale);
+    o[q] = u;
+  }
+}
+__device__ __forceinline__ void zero_grad_row(__nv_bfloat16* base, int f32, long long row, int d) {
+  uint4* o = f32 ? reinterpret_cast<uint4*>(reinterpret_cast<float*>(base) + row) : reinterpret_cast<uint4*>(base + row);
+  for (int q = 0; q < (f32 ? d / 4 : d / 8); ++q) o[q] = make_uint4(0, 0, 0, 0);
+}
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -95,7 +129,7 @@ __device__ __forceinline__ void store8_bf16(uint8_t* tile, int r, int c16, const
   *reinterpret_cast<uint4*>(tile + sw128_offset(r, c16)) = u;
 }
 
-template <int D, int MODE, bool BIAS>
+template <int D, int MODE, int BIAS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -149,7 +183,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     I.h = rem % p.H;
     I.b = rem / p.H;
     I.t_begin = MODE == MODE_KV ? (p.causal ? I.own : 0) : 0;
-    const int t_end = MODE == MODE_KV ? n_q : (p.causal ? min(I.own + 1, n_kv) : n_kv);
+    int t_end = MODE == MODE_KV ? n_q : (p.causal ? min(I.own + 1, n_kv) : n_kv);
+    if (BIAS != BIAS_NONE && p.lengths) {      // keys and queries from the valid length on contribute nothing
+      const int live = (max(0, min(p.Sk, p.lengths[I.b])) + BLK - 1) / BLK;
+      t_end = I.own < live ? min(t_end, live) : 0;
+    }
     I.n_iter = max(t_end - I.t_begin, 0);
     return I;
   };
@@ -369,6 +407,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float lse2 = 0.0f, dlt = 0.0f;
     int row_g = own * BLK + r;
     bool row_ok = row_g < p.Sq;
+    int q_live = p.Sq;                          // queries from here on are masked
+    if (BIAS == BIAS_KEYS && p.lengths) q_live = min(p.Sq, max(0, min(p.Sk, p.lengths[b])));
     if (MODE == MODE_Q && row_ok) {
       const long long stat_idx = ((long long)b * p.H + h) * p.Sq + row_g;
       lse2 = p.lse[stat_idx] * LOG2E;
@@ -403,7 +443,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const int kv0 = kv_tile * BLK;
       // tiles that need no masking: every row and column valid and strictly below the diagonal
-      constexpr bool biased = BIAS;   // additive biases / valid lengths: a separate instantiation, the plain one is unchanged
+      constexpr bool biased = BIAS != BIAS_NONE;   // additive biases / valid lengths: instantiations of their own
       const bool plain = (q_tile + 1) * BLK <= p.Sq && (kv_tile + 1) * BLK <= p.Sk &&
                          !(p.causal && kv_tile >= q_tile) && !biased;
       float pv[32];
@@ -418,7 +458,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         uint32_t s_r[32];
         tmem_ld_32x32(tmem_base + lane_off + S_COL + part * 32, s_r);
         tmem_ld_wait();
-        if (plain) {
+        if constexpr (BIAS == BIAS_KEYS) {
+          // exp2(S c + bias - lse): masked keys carry -inf in the bias, masked rows +inf in the subtrahend (a fully masked
+          // row has lse = -inf and contributes nothing)
+          const float sub = row_g < q_live && lse2 > -INFINITY ? lse2 : INFINITY;
+          const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), ns2 = make_float2(-sub, -sub);
+          const float4* bias = reinterpret_cast<const float4*>(p.kb_pad + b * p.kp_sb + h * p.kp_sh + kv0 + part * 32);
+#pragma unroll
+          for (int q = 0; q < 32; q += 4) {
+            const float4 v = __ldg(bias + q / 4);
+            const float2 x = fma2(make_float2(__uint_as_float(s_r[q]), __uint_as_float(s_r[q + 1])), sc2, add2(make_float2(v.x, v.y), ns2));
+            const float2 y = fma2(make_float2(__uint_as_float(s_r[q + 2]), __uint_as_float(s_r[q + 3])), sc2, add2(make_float2(v.z, v.w), ns2));
+            pv[q] = fast_exp2(x.x); pv[q + 1] = fast_exp2(x.y);
+            pv[q + 2] = fast_exp2(y.x); pv[q + 3] = fast_exp2(y.y);
+          }
+          if (p.causal && kv_tile >= q_tile) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q)
+              if (kv0 + part * 32 + q > row_g) pv[q] = 0.0f;
+          }
+        } else if (plain) {
 #pragma unroll
           for (int q = 0; q < 32; ++q) pv[q] = fast_exp2(__uint_as_float(s_r[q]) * p.scale_log2 - lse2);
         } else if constexpr (!biased) {
@@ -495,48 +554,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // 32 accumulator columns per thread: chunk `part` (and, for D > 128, every fourth one after it)
       const int own_row = own * BLK + r;
       for (int ch = part; ch < D / 32; ch += EW_WARPS / 4) {
+        // TMEM loads are warp-collective: every lane issues them, only the stores are predicated
         if (MODE == MODE_KV) {
-          const bool kv_ok = own_row < p.Sk;
-          __nv_bfloat16* dvp = p.dV + (long long)b * p.dv_sb + (long long)own_row * p.dv_ss + (long long)h * p.dv_sh + ch * 32;
-          __nv_bfloat16* dkp = p.dK + (long long)b * p.dk_sb + (long long)own_row * p.dk_ss + (long long)h * p.dk_sh + ch * 32;
-          // TMEM loads are warp-collective: every lane issues them, only the stores are predicated
           uint32_t tv[32], tk[32];
           tmem_ld_32x32(tmem_base + lane_off + ACC0_COL + ch * 32, tv);
           tmem_ld_32x32(tmem_base + lane_off + ACC1_COL + ch * 32, tk);
           tmem_ld_wait();
-          if (kv_ok) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 uv, uk;
-              uv.x = pack_bf16x2(__uint_as_float(tv[q * 8 + 0]), __uint_as_float(tv[q * 8 + 1]));
-              uv.y = pack_bf16x2(__uint_as_float(tv[q * 8 + 2]), __uint_as_float(tv[q * 8 + 3]));
-              uv.z = pack_bf16x2(__uint_as_float(tv[q * 8 + 4]), __uint_as_float(tv[q * 8 + 5]));
-              uv.w = pack_bf16x2(__uint_as_float(tv[q * 8 + 6]), __uint_as_float(tv[q * 8 + 7]));
-              uk.x = pack_bf16x2(__uint_as_float(tk[q * 8 + 0]) * p.scale, __uint_as_float(tk[q * 8 + 1]) * p.scale);
-              uk.y = pack_bf16x2(__uint_as_float(tk[q * 8 + 2]) * p.scale, __uint_as_float(tk[q * 8 + 3]) * p.scale);
-              uk.z = pack_bf16x2(__uint_as_float(tk[q * 8 + 4]) * p.scale, __uint_as_float(tk[q * 8 + 5]) * p.scale);
-              uk.w = pack_bf16x2(__uint_as_float(tk[q * 8 + 6]) * p.scale, __uint_as_float(tk[q * 8 + 7]) * p.scale);
-              reinterpret_cast<uint4*>(dvp)[q] = uv;
-              reinterpret_cast<uint4*>(dkp)[q] = uk;
-            }
+          if (own_row < p.Sk) {
+            store_grad(p.dV, p.grad_f32, (long long)b * p.dv_sb + (long long)own_row * p.dv_ss + (long long)h * p.dv_sh + ch * 32, tv, 1.0f);
+            store_grad(p.dK, p.grad_f32, (long long)b * p.dk_sb + (long long)own_row * p.dk_ss + (long long)h * p.dk_sh + ch * 32, tk, p.scale);
           }
         } else {
-          const bool q_ok = own_row < p.Sq;
-          __nv_bfloat16* dqp = p.dQ + (long long)b * p.dq_sb + (long long)own_row * p.dq_ss + (long long)h * p.dq_sh + ch * 32;
           uint32_t tq[32];
           tmem_ld_32x32(tmem_base + lane_off + ACC0_COL + ch * 32, tq);
           tmem_ld_wait();
-          if (q_ok) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 u;
-              u.x = pack_bf16x2(__uint_as_float(tq[q * 8 + 0]) * p.scale, __uint_as_float(tq[q * 8 + 1]) * p.scale);
-              u.y = pack_bf16x2(__uint_as_float(tq[q * 8 + 2]) * p.scale, __uint_as_float(tq[q * 8 + 3]) * p.scale);
-              u.z = pack_bf16x2(__uint_as_float(tq[q * 8 + 4]) * p.scale, __uint_as_float(tq[q * 8 + 5]) * p.scale);
-              u.w = pack_bf16x2(__uint_as_float(tq[q * 8 + 6]) * p.scale, __uint_as_float(tq[q * 8 + 7]) * p.scale);
-              reinterpret_cast<uint4*>(dqp)[q] = u;
-            }
-          }
+          if (own_row < p.Sq)
+            store_grad(p.dQ, p.grad_f32, (long long)b * p.dq_sb + (long long)own_row * p.dq_ss + (long long)h * p.dq_sh + ch * 32, tq, p.scale);
         }
       }
     }
@@ -548,20 +581,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     if (n_iter == 0 && part == 0) {
       // nothing attends to / from this tile: its gradient rows are zero
-      const uint4 z = make_uint4(0, 0, 0, 0);
       const int own_row = own * BLK + r;
       if (MODE == MODE_KV) {
         if (own_row < p.Sk) {
-          __nv_bfloat16* dvp = p.dV + (long long)b * p.dv_sb + (long long)own_row * p.dv_ss + (long long)h * p.dv_sh;
-          __nv_bfloat16* dkp = p.dK + (long long)b * p.dk_sb + (long long)own_row * p.dk_ss + (long long)h * p.dk_sh;
-          for (int q = 0; q < D / 8; ++q) {
-            reinterpret_cast<uint4*>(dvp)[q] = z;
-            reinterpret_cast<uint4*>(dkp)[q] = z;
-          }
+          zero_grad_row(p.dV, p.grad_f32, (long long)b * p.dv_sb + (long long)own_row * p.dv_ss + (long long)h * p.dv_sh, D);
+          zero_grad_row(p.dK, p.grad_f32, (long long)b * p.dk_sb + (long long)own_row * p.dk_ss + (long long)h * p.dk_sh, D);
         }
       } else if (own_row < p.Sq) {
-        __nv_bfloat16* dqp = p.dQ + (long long)b * p.dq_sb + (long long)own_row * p.dq_ss + (long long)h * p.dq_sh;
-        for (int q = 0; q < D / 8; ++q) reinterpret_cast<uint4*>(dqp)[q] = z;
+        zero_grad_row(p.dQ, p.grad_f32, (long long)b * p.dq_sb + (long long)own_row * p.dq_ss + (long long)h * p.dq_sh, D);
       }
     }
     }   // work items
@@ -582,9 +609,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // delta[b,h,s] = sum_d O[b,s,h,d] * dO[b,s,h,d].  D / 8 lanes share one (b,s,h) row, each with one
 // 16-byte load of O and of dO (a warp covers 2 rows at D = 128, 4 at D = 64): one row per warp with 4-byte
 // loads left this bandwidth-bound pass at a quarter of the copy rate.
-template <int D>
+// With F32 the gradient arrives in fp32: this pass also writes the bf16 form that the tensor cores read (strides do_*) and
+// takes the products with it.
+template <int D, bool F32>
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
+attn_delta_kernel(const __nv_bfloat16* __restrict__ O, __nv_bfloat16* __restrict__ dO, const float* __restrict__ dO32,
                   float* __restrict__ delta, int B, int S, int H, long long o_sb, long long o_ss, long long o_sh,
                   long long do_sb, long long do_ss, long long do_sh) {
   constexpr int LPR = D / 8;                       // lanes per row
@@ -603,7 +632,16 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __re
       s = (int)(bs % S);
       bb = (int)(bs / S);
       const uint4 a = *reinterpret_cast<const uint4*>(O + bb * o_sb + s * o_ss + hh * o_sh + sub * 8);
-      const uint4 g = *reinterpret_cast<const uint4*>(dO + bb * do_sb + s * do_ss + hh * do_sh + sub * 8);
+      __nv_bfloat16* gp = dO + bb * do_sb + s * do_ss + hh * do_sh + sub * 8;
+      uint4 g;
+      if constexpr (F32) {
+        const float4* src = reinterpret_cast<const float4*>(dO32 + w * D + sub * 8);
+        const float4 u = src[0], v = src[1];
+        g = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+        *reinterpret_cast<uint4*>(gp) = g;
+      } else {
+        g = *reinterpret_cast<const uint4*>(gp);
+      }
       const uint32_t av[4] = {a.x, a.y, a.z, a.w}, gv[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -634,8 +672,8 @@ struct StAttnBwdArgs {
   const int* lengths;
 };
 
-// delta: fp32 [B,H,Sq] workspace.  dQ_acc is unused (kept in the argument block for ABI stability).
-ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) {
+namespace {
+int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_ws, void* stream_v) {
   if (!a || !a->Q || !a->K || !a->V || !a->O || !a->dO || !a->lse || !a->delta ||
       !a->dQ || !a->dK || !a->dV)
     return st::fail(ST_ERR_INVALID, "attn_bwd: null pointer");
@@ -658,13 +696,13 @@ ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) {
     long long blocks = (rows + rows_per_block - 1) / rows_per_block;
     if (blocks > 148 * 16) blocks = 148 * 16;
     auto Op = static_cast<const __nv_bfloat16*>(a->O);
-    auto dOp = static_cast<const __nv_bfloat16*>(a->dO);
-    if (a->D == 128)
-      attn_delta_kernel<128><<<(unsigned)blocks, 256, 0, s>>>(Op, dOp, a->delta, a->B, a->Sq, a->H, a->o_sb, a->o_ss,
-                                                            a->o_sh, a->do_sb, a->do_ss, a->do_sh);
-    else
-      attn_delta_kernel<64><<<(unsigned)blocks, 256, 0, s>>>(Op, dOp, a->delta, a->B, a->Sq, a->H, a->o_sb, a->o_ss,
-                                                           a->o_sh, a->do_sb, a->do_ss, a->do_sh);
+    auto dOp = static_cast<__nv_bfloat16*>(const_cast<void*>(a->dO));        // written only from dO32
+    auto delta = [&](auto kernel) {
+      kernel<<<(unsigned)blocks, 256, 0, s>>>(Op, dOp, dO32, a->delta, a->B, a->Sq, a->H, a->o_sb, a->o_ss, a->o_sh, a->do_sb,
+                                              a->do_ss, a->do_sh);
+    };
+    if (a->D == 128) { if (dO32) delta(attn_delta_kernel<128, true>); else delta(attn_delta_kernel<128, false>); }
+    else { if (dO32) delta(attn_delta_kernel<64, true>); else delta(attn_delta_kernel<64, false>); }
     ST_CUDA_CHECK(cudaGetLastError());
   }
 
@@ -690,7 +728,14 @@ ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) {
   p.key_bias = a->key_bias; p.kb_sb = a->kb_sb; p.kb_sh = a->kb_sh;
   p.attn_bias = a->attn_bias; p.ab_sb = a->ab_sb; p.ab_sh = a->ab_sh; p.ab_sq = a->ab_sq;
   p.lengths = a->lengths;
+  p.grad_f32 = grad_f32;
+  p.kb_pad = nullptr; p.kp_sb = p.kp_sh = 0;
   const bool biased = a->key_bias || a->attn_bias || a->lengths;
+  const bool keyb = biased && !a->attn_bias && bias_ws;
+  if (keyb) {
+    if (int e = st::attn_key_bias(a->key_bias, a->kb_sb, a->kb_sh, a->lengths, bias_ws, a->B, a->H, a->Sk, &p.kp_sb, &p.kp_sh, s)) return e;
+    p.kb_pad = bias_ws;
+  }
   static int num_sms = 0;
   if (num_sms == 0) {
     int dev = 0;
@@ -707,23 +752,25 @@ ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) {
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
   };
-  int rc;
-  if (a->D == 128) {
-    if (biased) {
-      if ((rc = launch(attn_bwd_kernel<128, MODE_KV, true>, BwdSmem<128, MODE_KV>::TOTAL, grid_kv)) != ST_OK) return rc;
-      if ((rc = launch(attn_bwd_kernel<128, MODE_Q, true>, BwdSmem<128, MODE_Q>::TOTAL, grid_q)) != ST_OK) return rc;
-    } else {
-      if ((rc = launch(attn_bwd_kernel<128, MODE_KV, false>, BwdSmem<128, MODE_KV>::TOTAL, grid_kv)) != ST_OK) return rc;
-      if ((rc = launch(attn_bwd_kernel<128, MODE_Q, false>, BwdSmem<128, MODE_Q>::TOTAL, grid_q)) != ST_OK) return rc;
-    }
-  } else {
-    if (biased) {
-      if ((rc = launch(attn_bwd_kernel<64, MODE_KV, true>, BwdSmem<64, MODE_KV>::TOTAL, grid_kv)) != ST_OK) return rc;
-      if ((rc = launch(attn_bwd_kernel<64, MODE_Q, true>, BwdSmem<64, MODE_Q>::TOTAL, grid_q)) != ST_OK) return rc;
-    } else {
-      if ((rc = launch(attn_bwd_kernel<64, MODE_KV, false>, BwdSmem<64, MODE_KV>::TOTAL, grid_kv)) != ST_OK) return rc;
-      if ((rc = launch(attn_bwd_kernel<64, MODE_Q, false>, BwdSmem<64, MODE_Q>::TOTAL, grid_q)) != ST_OK) return rc;
-    }
-  }
-  return ST_OK;
+  // both passes of a bias form: dK / dV per KV tile, then dQ per query tile
+  auto both = [&](auto kv, int kv_smem, auto q, int q_smem) -> int {
+    if (int e = launch(kv, kv_smem, grid_kv)) return e;
+    return launch(q, q_smem, grid_q);
+  };
+#define ST_BWD_BOTH(DV, BV) \
+  both(attn_bwd_kernel<DV, MODE_KV, BV>, BwdSmem<DV, MODE_KV>::TOTAL, attn_bwd_kernel<DV, MODE_Q, BV>, BwdSmem<DV, MODE_Q>::TOTAL)
+  if (a->D == 128) return keyb ? ST_BWD_BOTH(128, BIAS_KEYS) : biased ? ST_BWD_BOTH(128, BIAS_FULL) : ST_BWD_BOTH(128, BIAS_NONE);
+  return keyb ? ST_BWD_BOTH(64, BIAS_KEYS) : biased ? ST_BWD_BOTH(64, BIAS_FULL) : ST_BWD_BOTH(64, BIAS_NONE);
+#undef ST_BWD_BOTH
+}
+}  // namespace
+
+// delta: fp32 [B,H,Sq] workspace.  dQ_acc is unused (kept in the argument block for ABI stability).
+ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) { return attn_bwd_run(a, nullptr, 0, nullptr, stream_v); }
+
+// The same with, all optional: the output's gradient in fp32 (dO32, contiguous [B, Sq, H, D]; a->dO then receives its bf16
+// form), gradients in fp32 (grad_f32: dQ, dK, dV are float*, strides in elements), and a workspace of
+// st_attn_bias_workspace floats for a key bias or lengths.
+ST_API int st_attn_bwd_f32(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, void* stream_v) {
+  return attn_bwd_run(a, dO32, grad_f32, bias_workspace, stream_v);
 }

@@ -47,7 +47,11 @@ struct AttnFwdParams {
   const float* attn_bias;      // [B, (H,) Sq, Sk] or null; element strides ab_sb, ab_sh, ab_sq (keys contiguous)
   const int* lengths;          // [B] valid keys (and queries) per batch entry, or null
   long long kb_sb, kb_sh, ab_sb, ab_sh, ab_sq;
-  // ---- pair kernel only: optional phase clock sums of CTA 0 (null = off) ----
+  // ---- pair kernel only ----
+  const float* kb_pad;         // key bias and length as written by attn_key_bias_kernel, element strides kp_sb, kp_sh
+  long long kp_sb, kp_sh;
+  float* O32;                  // fp32 copy of the output, contiguous [B, Sq, H, D], or null
+  // optional phase clock sums of CTA 0 (null = off)
   unsigned long long* trace;
 };
 
@@ -435,6 +439,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // warp alternates the two tiles (PV_0, QK_0, PV_1, QK_1, ...), so the tensor pipe works on one tile while the other
 // tile's warpgroup is in its softmax.  Shared-memory traffic per query tile and KV tile drops from 224 KB (two
 // operand reads per product, K and V written per tile, P written and read) to 128 KB.
+// With a key bias or valid lengths (KEYB) the logits take them from a padded fp32 row per batch entry (and head), already
+// in the log2 domain and minus infinity wherever a key is masked: 16-byte loads that all lanes share, one packed multiply-
+// add per two logits and no comparisons.  The single-tile kernel loaded and compared per element: 244 us for 96 contexts of
+// up to 1000 keys, D = 64, where this form takes 99.  A bias per (query, key) stays with the single-tile kernel.
 // ------------------------------------------------------------------------------------------------------------------
 // Phase clocks of CTA 0 (SM cycles summed over the launch), written when tracing is switched on:
 //   softmax warp 0:  0 steps, 1 wait for S, 2 S load, 3 maximum / rescale, 4 first half of P, 5 second half of P,
@@ -458,7 +466,22 @@ struct PairSmem {
   static constexpr int TOTAL = BAR_OFF + 256;
 };
 
-template <int D>
+// out[b, (h,) key] = key_bias * log2(e) for the keys below the valid length, minus infinity from there to the padded end
+__global__ void attn_key_bias_kernel(const float* __restrict__ kb, long long kb_sb, long long kb_sh, const int* __restrict__ lengths,
+                                     float* __restrict__ out, int heads, int Sk, int padded, long long total) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int key = (int)(i % padded);
+    const long long row = i / padded;
+    const int b = (int)(row / heads), h = (int)(row % heads);
+    int len = Sk;
+    if (lengths) len = max(0, min(Sk, lengths[b]));
+    float v = -INFINITY;
+    if (key < len) v = kb ? kb[b * kb_sb + h * kb_sh + key] * 1.4426950408889634f : 0.0f;
+    out[i] = v;
+  }
+}
+
+template <int D, bool KEYB>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const AttnFwdParams p) {
@@ -503,8 +526,13 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int rem = w % hb;
     h = rem % p.H;
     b = rem / p.H;
-    n0 = p.causal ? min(n_kv_all, 2 * qp + 1) : n_kv_all;
-    n1 = (2 * qp + 1 < p.n_q) ? (p.causal ? min(n_kv_all, 2 * qp + 2) : n_kv_all) : 0;
+    int n_kv = n_kv_all, q_live = p.Sq;
+    if (KEYB && p.lengths) {
+      q_live = max(0, min(p.Sk, p.lengths[b]));      // queries from there on give zeros
+      n_kv = (q_live + BLK - 1) / BLK;
+    }
+    n0 = 2 * qp * BLK < q_live ? (p.causal ? min(n_kv, 2 * qp + 1) : n_kv) : 0;
+    n1 = (2 * qp + 1 < p.n_q && (2 * qp + 1) * BLK < q_live) ? (p.causal ? min(n_kv, 2 * qp + 2) : n_kv) : 0;
   };
 
   if (threadIdx.x == 0) {
@@ -715,9 +743,22 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       int qp, h, b, n0, n1;
       item_at(w, qp, h, b, n0, n1);
       const int n_kv = t == 0 ? n0 : n1;
-      if (n_kv <= 0) continue;
       const int q_tile = 2 * qp + t;
       const int row_g = q_tile * BLK + r;
+      if (n_kv <= 0) {
+        if (KEYB && row_g < p.Sq) {      // a query tile beyond the valid length, or a context without keys
+          __nv_bfloat16* op = p.O + (long long)b * p.o_sb + (long long)row_g * p.o_ss + (long long)h * p.o_sh;
+          for (int c = 0; c < D / 8; ++c) reinterpret_cast<uint4*>(op)[c] = make_uint4(0, 0, 0, 0);
+          if (p.O32) {
+            float4* o32 = reinterpret_cast<float4*>(p.O32 + (((long long)b * p.Sq + row_g) * p.H + h) * D);
+            for (int c = 0; c < D / 4; ++c) o32[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          }
+          p.lse[((long long)b * p.H + h) * p.Sq + row_g] = -INFINITY;
+        }
+        continue;
+      }
+      const bool row_live = !KEYB || !p.lengths || row_g < min(p.Sk, p.lengths[b]);
+      const float4* bias_row = KEYB ? reinterpret_cast<const float4*>(p.kb_pad + b * p.kp_sb + h * p.kp_sh) : nullptr;
       float m = -INFINITY, l = 0.0f;
       for (int j = 0; j < n_kv; ++j) {
         if (tr) c0 = static_cast<uint32_t>(clock());
@@ -739,7 +780,18 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (tr) { c1 = static_cast<uint32_t>(clock()); tacc[2] += c1 - c0; c0 = c1; }
         const int col0 = j * BLK;
         float mx = -INFINITY;
-        if ((p.causal && j == q_tile) || col0 + BLK > p.Sk) {
+        if constexpr (KEYB) {      // to the log2 domain, bias added; keys that are masked or past the end become -inf
+          const float2 sc2 = make_float2(sc, sc);
+#pragma unroll
+          for (int c = 0; c < BLK; c += 4) {
+            const float4 bias = __ldg(bias_row + (col0 + c) / 4);
+            const float2 x = fma2(make_float2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, make_float2(bias.x, bias.y));
+            const float2 y = fma2(make_float2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, make_float2(bias.z, bias.w));
+            sr[c] = __float_as_uint(x.x); sr[c + 1] = __float_as_uint(x.y);
+            sr[c + 2] = __float_as_uint(y.x); sr[c + 3] = __float_as_uint(y.y);
+          }
+        }
+        if ((p.causal && j == q_tile) || (!KEYB && col0 + BLK > p.Sk)) {
 #pragma unroll
           for (int c = 0; c < BLK; ++c) {
             const int col = col0 + c;
@@ -760,7 +812,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           }
           mx = fmaxf(fmaxf(max3(mc[0], mc[1], mc[2]), max3(mc[3], mc[4], mc[5])), fmaxf(mc[6], mc[7]));
         }
-        const float m_new = fmaxf(m, mx * sc);
+        const float m_new = fmaxf(m, KEYB ? mx : mx * sc);
         bool raise = false;
         float alpha = 1.0f;
         if (j == 0) {
@@ -799,7 +851,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
             const int cc = hlf * 64 + 2 * c;
-            const float2 x = fma2(make_float2(__uint_as_float(sr[cc]), __uint_as_float(sr[cc + 1])), sc2, nm2);
+            const float2 sv = make_float2(__uint_as_float(sr[cc]), __uint_as_float(sr[cc + 1]));
+            const float2 x = KEYB ? add2(sv, nm2) : fma2(sv, sc2, nm2);
             const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
             rs2[c & 1] = add2(rs2[c & 1], e);
             pr[c] = pack_bf16x2(e.x, e.y);
@@ -826,14 +879,21 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (!mbar_wait_warp(smem_u32(&o_full[t]), items & 1, abort_flag)) { ok = false; break; }
       ++items;
       tc_fence_after();
-      const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+      const float inv = l > 0.0f && row_live ? 1.0f / l : 0.0f;
       __nv_bfloat16* op = p.O + (long long)b * p.o_sb + (long long)row_g * p.o_ss + (long long)h * p.o_sh;
+      float4* o32 = p.O32 ? reinterpret_cast<float4*>(p.O32 + (((long long)b * p.Sq + row_g) * p.H + h) * D) : nullptr;
 #pragma unroll
       for (int ch = 0; ch < D / 32; ++ch) {
         uint32_t v[32];
         tmem_ld_32x32(o_addr + ch * 32, v);
         tmem_ld_wait();
         if (row_g < p.Sq) {
+          if (o32) {
+#pragma unroll
+            for (int c4 = 0; c4 < 8; ++c4)
+              o32[ch * 8 + c4] = make_float4(__uint_as_float(v[c4 * 4]) * inv, __uint_as_float(v[c4 * 4 + 1]) * inv,
+                                             __uint_as_float(v[c4 * 4 + 2]) * inv, __uint_as_float(v[c4 * 4 + 3]) * inv);
+          }
 #pragma unroll
           for (int c8 = 0; c8 < 4; ++c8) {
             uint4 u;
@@ -847,7 +907,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       if (row_g < p.Sq)
         p.lse[((long long)b * p.H + h) * p.Sq + row_g] =
-            (l > 0.0f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+            (l > 0.0f && row_live) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
       if (tr) { tacc[6] += static_cast<uint32_t>(clock()) - c0; tacc[7] += 1; }
       // the next item's first PV_t overwrites O_t only after this warpgroup's next p_full arrival, which follows
       // these loads in program order
@@ -881,6 +941,22 @@ bool encode_bshd_tmap(CUtensorMap* out, const void* base, int B, int S, int H, i
   uint32_t box[4] = {64, 1, (uint32_t)box_rows, 1};
   return encode_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box,
                      CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// Padded rows of key bias and length (see attn_key_bias_kernel): one per batch entry, or per head where the bias differs
+// by head.  Rows are whole 128-key tiles.
+int attn_key_bias(const float* kb, long long kb_sb, long long kb_sh, const int* lengths, float* ws, int B, int H, int Sk,
+                  long long* out_sb, long long* out_sh, cudaStream_t stream) {
+  if (reinterpret_cast<uintptr_t>(ws) & 15) return fail(ST_ERR_INVALID, "attention: the bias workspace must be 16-byte aligned");
+  const int heads = kb && kb_sh != 0 ? H : 1, padded = (Sk + BLK - 1) / BLK * BLK;
+  const long long total = (long long)B * heads * padded;
+  *out_sb = (long long)heads * padded;
+  *out_sh = heads > 1 ? padded : 0;
+  long long blocks = (total + 255) / 256;
+  if (blocks > 16ll * sm_count()) blocks = 16ll * sm_count();
+  attn_key_bias_kernel<<<(unsigned)blocks, 256, 0, stream>>>(kb, kb_sb, kb_sh, lengths, ws, heads, Sk, padded, total);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
 }
 }  // namespace st
 
@@ -919,7 +995,8 @@ ST_API int st_attn_fwd_read_trace(unsigned long long* out, int n) {
 ST_API void st_attn_fwd_set_pair_kernel(int on) { g_pair_kernel = on ? 1 : 0; }
 ST_API int st_attn_fwd_get_pair_kernel() { return g_pair_kernel; }
 
-ST_API int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v) {
+namespace {
+int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* stream_v) {
   if (!a || !a->Q || !a->K || !a->V || !a->O || !a->lse) return st::fail(ST_ERR_INVALID, "attn_fwd: null pointer");
   if (a->D != 64 && a->D != 128) return st::fail(ST_ERR_INVALID, "attn_fwd: head_dim must be 64 or 128");
   if (a->causal && a->Sq != a->Sk) return st::fail(ST_ERR_INVALID, "attn_fwd: causal needs seq_q == seq_k");
@@ -949,10 +1026,19 @@ ST_API int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v) {
   p.attn_bias = a->attn_bias; p.ab_sb = a->ab_sb; p.ab_sh = a->ab_sh; p.ab_sq = a->ab_sq;
   p.lengths = a->lengths;
   p.trace = nullptr;
+  p.kb_pad = nullptr; p.kp_sb = p.kp_sh = 0;
+  p.O32 = out32;
   const bool biased = a->key_bias || a->attn_bias || a->lengths;
   if (p.n_items <= 0) return ST_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (!biased && g_pair_kernel) {
+  const bool keyb = biased && !a->attn_bias && bias_ws && g_pair_kernel;
+  if (out32 && !(g_pair_kernel && (!biased || keyb)))
+    return st::fail(ST_ERR_INVALID, "attn_fwd: the fp32 output needs the pair kernel (no bias per query and key)");
+  if (keyb) {
+    if (int e = st::attn_key_bias(a->key_bias, a->kb_sb, a->kb_sh, a->lengths, bias_ws, a->B, a->H, a->Sk, &p.kp_sb, &p.kp_sh, s)) return e;
+    p.kb_pad = bias_ws;
+  }
+  if ((!biased || keyb) && g_pair_kernel) {
     // two query tiles per CTA: the items are (query pair, head, batch)
     if (g_pair_trace_on) ST_CUDA_CHECK(cudaGetSymbolAddress(reinterpret_cast<void**>(&p.trace), g_pair_trace));
     p.n_items = ((p.n_q + 1) / 2) * a->H * a->B;
@@ -966,9 +1052,14 @@ ST_API int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v) {
       kern<<<pgrid, PAIR_THREADS, smem_bytes, s>>>(tq, tk, tv, p);
       return ST_OK;
     };
-    static bool pcfg[2][st::kMaxDevices] = {{false}};
-    const int prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128>, PairSmem<128>::TOTAL, pcfg[0])
-                                : plaunch(attn_fwd_pair_kernel<64>, PairSmem<64>::TOTAL, pcfg[1]);
+    static bool pcfg[4][st::kMaxDevices] = {{false}};
+    int prc;
+    if (keyb)
+      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, true>, PairSmem<128>::TOTAL, pcfg[2])
+                        : plaunch(attn_fwd_pair_kernel<64, true>, PairSmem<64>::TOTAL, pcfg[3]);
+    else
+      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, false>, PairSmem<128>::TOTAL, pcfg[0])
+                        : plaunch(attn_fwd_pair_kernel<64, false>, PairSmem<64>::TOTAL, pcfg[1]);
     if (prc != ST_OK) return prc;
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
@@ -996,4 +1087,16 @@ ST_API int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v) {
   if (rc != ST_OK) return rc;
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
+}
+}  // namespace
+
+ST_API int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v) { return attn_fwd_run(a, nullptr, nullptr, stream_v); }
+
+// Floats of workspace for a key bias or lengths: B * H * (Sk rounded up to 128).
+ST_API long long st_attn_bias_workspace(int B, int H, int Sk) { return (long long)B * H * ((Sk + BLK - 1) / BLK * BLK); }
+
+// The same with an fp32 copy of the output in out32 (contiguous [B, Sq, H, D], may be null) and a workspace with which a key
+// bias or valid lengths run on the pair kernel (null: on the single-tile kernel).
+ST_API int st_attn_fwd_f32(const StAttnFwdArgs* a, float* out32, float* bias_workspace, void* stream_v) {
+  return attn_fwd_run(a, out32, bias_workspace, stream_v);
 }

@@ -52,6 +52,20 @@ multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict_
   }
 }
 
+// dst (bf16) = src (fp32) for a list of tensors, eight elements per thread and step; the tail element by element
+__global__ void __launch_bounds__(kMultiThreads)
+multi_cast_kernel(const __grid_constant__ MultiTable t) {
+  const float* __restrict__ src = t.src[blockIdx.y];
+  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(t.dst[blockIdx.y]);
+  const long long n = t.n[blockIdx.y], n8 = n / 8;
+  for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n8; i += (long long)gridDim.x * kMultiThreads) {
+    const float4 a = reinterpret_cast<const float4*>(src)[2 * i], b = reinterpret_cast<const float4*>(src)[2 * i + 1];
+    reinterpret_cast<uint4*>(dst)[i] = make_uint4(st::pack_bf16x2(a.x, a.y), st::pack_bf16x2(a.z, a.w),
+                                                  st::pack_bf16x2(b.x, b.y), st::pack_bf16x2(b.z, b.w));
+  }
+  if (blockIdx.x == 0 && n8 * 8 + threadIdx.x < n) dst[n8 * 8 + threadIdx.x] = __float2bfloat16(src[n8 * 8 + threadIdx.x]);
+}
+
 __device__ __forceinline__ float block_sum_256(float v, float* sh) {
   v = st::warp_sum(v);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
@@ -144,6 +158,27 @@ ST_API int st_multi(int op, int count, const void* const* src, void* const* dst,
   if (op == MULTI_CHECK) multi_kernel<MULTI_CHECK><<<grid, kMultiThreads, 0, s>>>(t, value, bad);
   else if (op == MULTI_DIV) multi_kernel<MULTI_DIV><<<grid, kMultiThreads, 0, s>>>(t, value, bad);
   else multi_kernel<MULTI_STEP><<<grid, kMultiThreads, 0, s>>>(t, value, bad);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+// bf16 copies of fp32 tensors; every pointer 16-byte aligned.
+ST_API int st_multi_cast_bf16(int count, const void* const* src, void* const* dst, const long long* n, void* stream_v) {
+  if (count <= 0) return ST_OK;
+  if (count > kMultiMax) return st::fail(ST_ERR_TOO_LARGE, "multi_cast: too many tensors for one launch");
+  if (!src || !dst || !n) return st::fail(ST_ERR_INVALID, "multi_cast: bad arguments");
+  MultiTable t;
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    if ((reinterpret_cast<uintptr_t>(src[i]) | reinterpret_cast<uintptr_t>(dst[i])) & 15)
+      return st::fail(ST_ERR_INVALID, "multi_cast: tensors must be 16-byte aligned");
+    t.src[i] = static_cast<const float*>(src[i]);
+    t.dst[i] = static_cast<float*>(dst[i]);
+    t.n[i] = n[i];
+    most = n[i] > most ? n[i] : most;
+  }
+  const dim3 grid(blocks_for(most / 2, 8 * st::sm_count()), count);
+  multi_cast_kernel<<<grid, kMultiThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(t);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }

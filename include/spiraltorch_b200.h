@@ -232,8 +232,11 @@ int st_adamw(void* grad, int grad_is_bf16, float* master, float* m, float* v, vo
 int st_ag_arrivals_for(int max_ctas);   /* csrc/comm/tp_gemm.cu */
 int st_ag_arrivals_per_launch();   /* csrc/comm/tp_gemm.cu */
 int st_ag_gemm(const StAgGemmArgs* a, void* stream_v);   /* csrc/comm/tp_gemm.cu */
+long long st_attn_bias_workspace(int B, int H, int Sk);   /* csrc/attention/attn_fwd.cu */
 int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v);   /* csrc/attention/attn_bwd.cu */
+int st_attn_bwd_f32(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, void* stream_v);   /* csrc/attention/attn_bwd.cu */
 int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v);   /* csrc/attention/attn_fwd.cu */
+int st_attn_fwd_f32(const StAttnFwdArgs* a, float* out32, float* bias_workspace, void* stream_v);   /* csrc/attention/attn_fwd.cu */
 int st_attn_fwd_get_pair_kernel();   /* csrc/attention/attn_fwd.cu */
 int st_attn_fwd_read_trace(unsigned long long* out, int n);   /* csrc/attention/attn_fwd.cu */
 void st_attn_fwd_set_pair_kernel(int on);   /* csrc/attention/attn_fwd.cu */
@@ -278,6 +281,7 @@ int st_mse_forward(const float* p, const float* t, long long n, float* value, vo
 int st_mse_workspace();   /* csrc/elementwise/multi.cu */
 int st_multi(int op, int count, const void* const* src, void* const* dst, const long long* n, float value, int* bad, void* stream_v);   /* csrc/elementwise/multi.cu */
 int st_multi_blocks(long long most);   /* csrc/elementwise/multi.cu */
+int st_multi_cast_bf16(int count, const void* const* src, void* const* dst, const long long* n, void* stream_v);   /* csrc/elementwise/multi.cu */
 int st_multi_max();   /* csrc/elementwise/multi.cu */
 int st_nd_indexer(const unsigned* positions, unsigned* out_index, unsigned* out_segment, long long n, const unsigned* dims4, const unsigned* strides4, unsigned segments, unsigned segment_stride, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_nerf_composite_bwd(const float* sigma, const float* rad, const float* deltas, const float* accum, const float* d_accum, float* d_sigma, float* d_rad, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */

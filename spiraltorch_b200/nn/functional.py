@@ -317,6 +317,8 @@ def scaled_dot_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scal
     scale = 1.0 / math.sqrt(D) if scale is None else scale
     if _on_kernels(q, k, v) and D in (64, 128) and v.shape[-1] == D:
         launch_counts["attention"] += 1
+        if attn_bias is None and _attn.takes_f32(q, k, v):
+            return _attn._AttentionF32Fn.apply(q, k, v, causal, scale, z_bias, lengths)
         o = _attn.attention(q.to(torch.bfloat16).unsqueeze(2), k.to(torch.bfloat16).unsqueeze(2),
                             v.to(torch.bfloat16).unsqueeze(2), causal=causal, scale=scale,
                             key_bias=z_bias, attn_bias=None if attn_bias is None else attn_bias.unsqueeze(1),

@@ -149,11 +149,22 @@ def _check_shapes(q, k, v) -> None:
         raise ValueError(f"attention: k/v {tuple(k.shape)} do not match q {tuple(q.shape)} in batch, heads or head_dim")
 
 
+def _bias_workspace(q, k, key_bias, attn_bias, lengths) -> Optional[torch.Tensor]:
+    """Room for the padded key-bias rows of the kernels that take a key bias or lengths without a bias per (query, key)."""
+    if attn_bias is not None or (key_bias is None and lengths is None):
+        return None
+    lib = native.lib()
+    lib.st_attn_bias_workspace.restype = ctypes.c_longlong
+    n = lib.st_attn_bias_workspace(ctypes.c_int(q.shape[0]), ctypes.c_int(q.shape[2]), ctypes.c_int(k.shape[1]))
+    return torch.empty(n, dtype=torch.float32, device=q.device)
+
+
 def attention_forward(q, k, v, causal: bool = True, scale: Optional[float] = None, *,
                       key_bias: Optional[torch.Tensor] = None, attn_bias: Optional[torch.Tensor] = None,
-                      lengths: Optional[torch.Tensor] = None):
+                      lengths: Optional[torch.Tensor] = None, out32: Optional[torch.Tensor] = None):
     """Returns ``(o, lse)``; ``o`` is contiguous ``[B,S,H,D]`` bf16, ``lse`` fp32 ``[B,H,S]``.
-    Optional additive biases and valid lengths as in :func:`attention_reference`."""
+    Optional additive biases and valid lengths as in :func:`attention_reference`.  ``out32`` (CUDA, contiguous fp32 of
+    ``o``'s shape, pair kernel) also receives the output before it is rounded."""
     global launch_count
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
@@ -178,14 +189,19 @@ def attention_forward(q, k, v, causal: bool = True, scale: Optional[float] = Non
     a.scale, a.causal = float(scale), int(causal)
     keep: list = []
     _bias_args(a, q, k, key_bias, attn_bias, lengths, keep)
-    native.check(native.lib().st_attn_fwd(ctypes.byref(a), native.stream_ptr(q.device)), "st_attn_fwd")
+    work = _bias_workspace(q, k, key_bias, attn_bias, lengths)
+    if out32 is not None:
+        assert out32.shape == o.shape and out32.dtype == torch.float32 and out32.is_contiguous() and out32.device == q.device
+    native.check(native.lib().st_attn_fwd_f32(ctypes.byref(a), native.ptr(out32), native.ptr(work), native.stream_ptr(q.device)),
+                 "st_attn_fwd")
     launch_count += 1
     return o, lse
 
 
 def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional[float] = None,
-                       dq=None, dk=None, dv=None, *, key_bias=None, attn_bias=None, lengths=None):
-    """Returns ``(dq, dk, dv)`` (bf16, ``[B,S,H,D]``); outputs may be preallocated strided views."""
+                       dq=None, dk=None, dv=None, *, key_bias=None, attn_bias=None, lengths=None, do32=None):
+    """Returns ``(dq, dk, dv)`` (bf16, ``[B,S,H,D]``); outputs may be preallocated strided views, all bf16 or all fp32.
+    ``do32`` (CUDA, contiguous fp32): the output's gradient, of which ``do`` then receives the bf16 form."""
     global launch_count
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
@@ -227,7 +243,16 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
     a.scale, a.causal = float(scale), int(causal)
     keep: list = []
     _bias_args(a, q, k, key_bias, attn_bias, lengths, keep)
-    native.check(native.lib().st_attn_bwd(ctypes.byref(a), native.stream_ptr(dev)), "st_attn_bwd")
+    work = _bias_workspace(q, k, key_bias, attn_bias, lengths)
+    f32 = dq.dtype == torch.float32
+    for t, n in ((dq, "dq"), (dk, "dk"), (dv, "dv")):
+        if t.dtype != (torch.float32 if f32 else torch.bfloat16) or t.stride(-1) != 1:
+            raise ValueError(f"attention_backward: {n} must be a view with contiguous D, and all gradients bf16 or all fp32")
+    if do32 is not None:
+        assert do32.shape == do.shape and do32.dtype == torch.float32 and do32.is_contiguous() and do32.device == dev
+        assert do32.data_ptr() % 16 == 0
+    native.check(native.lib().st_attn_bwd_f32(ctypes.byref(a), native.ptr(do32), ctypes.c_int(int(f32)), native.ptr(work),
+                                              native.stream_ptr(dev)), "st_attn_bwd")
     launch_count += 3
     return dq, dk, dv
 
@@ -250,6 +275,44 @@ class _AttentionFn(torch.autograd.Function):
         dq, dk, dv = attention_backward(q, k, v, o, lse, do, ctx.causal, ctx.scale, key_bias=kb, attn_bias=ab,
                                         lengths=ln)
         return dq, dk, dv, None, None, None, None, None
+
+
+class _AttentionF32Fn(torch.autograd.Function):
+    """The same for fp32 ``[B,S,D]`` tensors of one head: one conversion launch brings q, k and v to bf16, the kernels write
+    the output and the gradients in fp32 themselves, and the output's gradient is rounded in the pass that forms the row
+    products with it."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, causal, scale, key_bias, lengths):
+        from . import multi
+        qb, kb, vb = (t.unsqueeze(2) for t in multi.to_bf16((q.detach(), k.detach(), v.detach())))
+        out = torch.empty_like(q, memory_format=torch.contiguous_format)
+        o, lse = attention_forward(qb, kb, vb, causal, scale, key_bias=key_bias, lengths=lengths, out32=out.unsqueeze(2))
+        ctx.save_for_backward(qb, kb, vb, o, lse)
+        ctx.causal, ctx.scale, ctx.extras = causal, scale, (key_bias, lengths)
+        return out
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, o, lse = ctx.saved_tensors
+        d32 = do.to(torch.float32).contiguous()
+        if d32.data_ptr() % 16:
+            d32 = d32.clone()
+        dq, dk, dv = (torch.empty(t.shape, dtype=torch.float32, device=t.device) for t in (q, k, v))
+        attention_backward(q, k, v, o, lse, torch.empty_like(o), ctx.causal, ctx.scale, dq, dk, dv, key_bias=ctx.extras[0],
+                           lengths=ctx.extras[1], do32=d32.unsqueeze(2))
+        return dq.squeeze(2), dk.squeeze(2), dv.squeeze(2), None, None, None, None
+
+
+def takes_f32(q, k, v) -> bool:
+    """Whether :class:`_AttentionF32Fn` takes these ``[B,S,D]`` tensors."""
+    return pair_kernel_on() and all(t.is_cuda and t.dtype == torch.float32 and t.dim() == 3 and t.is_contiguous()
+                                    and t.data_ptr() % 16 == 0 and t.numel() > 0 for t in (q, k, v))
+
+
+def pair_kernel_on() -> bool:
+    _apply_env_once()
+    return pair_kernel_enabled()
 
 
 def attention(q, k, v, causal: bool = True, scale: Optional[float] = None, *,

@@ -72,6 +72,19 @@ def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: 
         torch.autograd.graph.increment_version(v)      # copies of the values are cached by version
 
 
+def to_bf16(tensors: Sequence[torch.Tensor]):
+    """bf16 copies of dense 16-byte aligned fp32 CUDA tensors."""
+    global launch_count
+    out = [torch.empty(t.shape, dtype=torch.bfloat16, device=t.device) for t in tensors]
+    n = len(out)
+    native.require_cuda("to_bf16", *tensors)
+    native.check(native.lib().st_multi_cast_bf16(
+        ctypes.c_int(n), (ctypes.c_void_p * n)(*[t.data_ptr() for t in tensors]), (ctypes.c_void_p * n)(*[t.data_ptr() for t in out]),
+        (ctypes.c_longlong * n)(*[t.numel() for t in out]), native.stream_ptr(out[0].device)), "st_multi_cast_bf16")
+    launch_count += 1
+    return out
+
+
 def mse_forward(p: torch.Tensor, t: torch.Tensor):
     """``(mean((p - t)^2) of shape (1, 1), all inputs are finite)``."""
     global launch_count

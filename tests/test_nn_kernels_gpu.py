@@ -386,3 +386,48 @@ def test_layer_norm_backward_reads_the_values_of_the_forward():
         h.mul_(3.0)
         g.add_(1.0)
     assert all(torch.equal(p, q) for p, q in zip(torch.autograd.grad(y, (x, g, b)), want))
+
+
+@pytest.mark.parametrize("B,Sq,Sk,H,D,causal,heads,lengths", [
+    (3, 130, 130, 2, 64, False, False, [130, 0, 1]), (4, 257, 257, 1, 128, True, True, [128, 129, 127, 257]),
+    (2, 300, 77, 1, 64, False, True, None), (2, 100, 385, 2, 128, False, False, [385, 90]), (1, 1, 1, 1, 64, True, False, None),
+    (2, 200, 200, 3, 64, False, None, [199, 64])])
+def test_attention_with_key_bias_and_lengths_on_the_pair_kernel(B, Sq, Sk, H, D, causal, heads, lengths):
+    """Empty, one-key and tile-edge lengths, query tiles beyond them, unequal sequence lengths, bias per head, masked keys;
+    forward and both backward passes against the general kernels' arithmetic in fp32.  P and dS are bf16: 2^-8 of the
+    largest value."""
+    torch.manual_seed(Sq + Sk + D)
+    q, do = (torch.randn(B, Sq, H, D, device=DEV).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Sk, H, D, device=DEV).bfloat16() for _ in range(2))
+    kb = None
+    if heads is not None:
+        kb = torch.randn(*((B, H, Sk) if heads else (B, Sk)), device=DEV) * 2
+        kb[..., Sk // 3] = float("-inf")
+    ln = None if lengths is None else torch.tensor(lengths, device=DEV, dtype=torch.int32)
+    o32 = torch.empty(B, Sq, H, D, device=DEV)
+    o, lse = A.attention_forward(q, k, v, causal, None, key_bias=kb, lengths=ln, out32=o32)
+    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+    ro, rlse = A.attention_reference(qf, kf, vf, causal, 1 / math.sqrt(D), key_bias=kb, lengths=ln)
+    close = lambda x, y: (x.float() - y).abs().max() <= 2e-2 * y.abs().max().clamp(min=1e-3)  # noqa: E731
+    assert close(o, ro) and close(o32, ro) and torch.equal(o, o32.bfloat16())
+    live = torch.isfinite(rlse)
+    assert torch.equal(live, torch.isfinite(lse)) and (lse[live] - rlse[live]).abs().max() < 1e-2 if live.any() else True
+    grads = torch.autograd.grad(torch.nan_to_num(ro), (qf, kf, vf), do.float(), allow_unused=True)
+    grads = [torch.nan_to_num(g) for g in grads]
+    f32 = [torch.full(t.shape, float("nan"), device=DEV) for t in (q, k, v)]
+    given = torch.empty_like(do)
+    A.attention_backward(q, k, v, o, lse, given, causal, None, *f32, key_bias=kb, lengths=ln, do32=do.float())
+    assert torch.equal(given, do)
+    b16 = A.attention_backward(q, k, v, o, lse, do, causal, None, key_bias=kb, lengths=ln)
+    for g, f, h in zip(grads, f32, b16):
+        assert close(f, g) and torch.equal(f.bfloat16(), h)
+
+
+def test_attention_backward_does_not_read_the_returned_output():
+    q, k, v = (torch.randn(3, 150, 64, device=DEV, requires_grad=True) for _ in range(3))
+    g = torch.randn(3, 150, 64, device=DEV)
+    want = torch.autograd.grad(Fn.scaled_dot_attention(q, k, v), (q, k, v), g)
+    y = Fn.scaled_dot_attention(q, k, v)
+    with torch.no_grad():
+        y.detach().zero_()
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, (q, k, v), g), want))
