@@ -220,78 +220,186 @@ fft_pow2_kernel(const float* __restrict__ in, float* __restrict__ out, const flo
 #undef ST_FFT_PASS
 }
 
-// Streaming form for long batches of contiguous complex rows: a persistent CTA walks rows blockIdx.x, + gridDim.x, ...
-// and, while it works through the passes of one row, a bulk asynchronous copy brings the next row into a staging
-// buffer, so the only exposed global-memory latency is that of the CTA's first row.  The first pass reads the staging
-// buffer; everything else is the kernel above.  n = 8^a * tail with a >= 2.
-__global__ void __launch_bounds__(512, 2)
-fft_pow2_stream_kernel(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ window,
-                       FftLayout L, int n, int log2n, int inverse, int batches, unsigned* err) {
+// ---- long batches of complex rows: radix-16 passes, twiddles in shared memory, next rows prefetched ----------------------
+// A persistent CTA of 256 threads works on 4096 points at a time: one row of 4096 or 4096 / n shorter ones.  Every thread
+// holds 16 points, so a transform is log16(n) passes and a tail of 2, 4 or 8, with one exchange buffer between them; while
+// the passes of one group run, bulk asynchronous copies bring the next group into a staging buffer.  The radix-8 kernel
+// above with such copies was bound by instruction issue (883 per 8 points at n = 4096: four passes, a sincospi and a chain
+// of products for each butterfly's twiddles): 134 us for 8192 rows of 4096, where this one takes 103 and the bytes 82.
+constexpr int F16_POINTS = 4096, F16_THREADS = F16_POINTS / 16;
+
+__device__ __forceinline__ float2 add_c(float2 a, float2 b) { return st::add2(a, b); }                       // one packed add
+__device__ __forceinline__ float2 sub_c(float2 a, float2 b) { return st::fma2(b, make_float2(-1.0f, -1.0f), a); }
+
+__device__ __forceinline__ void dft4_c(float2& x0, float2& x1, float2& x2, float2& x3) {
+  const float2 a = add_c(x0, x2), b = sub_c(x0, x2), c = add_c(x1, x3), d = mul_neg_i(sub_c(x1, x3));
+  x0 = add_c(a, c); x1 = add_c(b, d); x2 = sub_c(a, c); x3 = sub_c(b, d);
+}
+
+// 16-point DFT as 4 x 4: input b + 4 a, output c + 4 d in v[4 c + d]
+__device__ __forceinline__ void dft16(float2 (&v)[16]) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) dft4_c(v[b], v[b + 4], v[b + 8], v[b + 12]);
+  constexpr float h = 0.70710678118654752f, c1 = 0.92387953251128674f, s1 = 0.38268343236508977f;
+  auto rot45 = [](float2 x) { return make_float2(h * (x.x + x.y), h * (x.y - x.x)); };                 // * exp(-i pi / 4)
+  v[5] = cmul(v[5], make_float2(c1, -s1));
+  v[6] = rot45(v[6]);
+  v[7] = cmul(v[7], make_float2(s1, -c1));
+  v[9] = rot45(v[9]);
+  v[10] = mul_neg_i(v[10]);
+  v[11] = mul_neg_i(rot45(v[11]));
+  v[13] = cmul(v[13], make_float2(s1, -c1));
+  v[14] = mul_neg_i(rot45(v[14]));
+  v[15] = cmul(v[15], make_float2(-c1, s1));
+#pragma unroll
+  for (int c = 0; c < 4; ++c) dft4_c(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+__device__ __forceinline__ constexpr int dft16_at(int k) { return 4 * (k & 3) + (k >> 2); }
+
+template <int LOGN>
+struct Fft16 {
+  static constexpr int N = 1 << LOGN, TPR = N / 16, ROWS = F16_POINTS / N;
+  static constexpr int PASSES = LOGN / 4, TAIL = 1 << (LOGN % 4);
+  // twiddle tables, entry (r - 1) ns + k = exp(-2 pi i r k / (radix ns)): pass 1 (ns 16), pass 2 (ns 256), tail (ns N / TAIL)
+  static constexpr int TW1 = PASSES > 1 ? 15 * 16 : 0, TW2 = PASSES > 2 ? 15 * 256 : 0;
+  static constexpr int TWT = TAIL > 1 ? (TAIL - 1) * (N / TAIL) : 0;
+  // one slot of padding per 16: the first pass writes 16 neighbours per thread, every other access is contiguous
+  static constexpr int BUF = F16_POINTS + F16_POINTS / 16;
+  static constexpr int SMEM = (BUF + F16_POINTS + TW1 + TW2 + TWT) * 8 + 32;
+};
+
+template <int LOGN>
+__global__ void __launch_bounds__(F16_THREADS, 3)
+fft16_stream_kernel(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ window, FftLayout L,
+                    int inverse, int batches, unsigned* err) {
+  using F = Fft16<LOGN>;
+  constexpr int N = F::N, TPR = F::TPR;
   extern __shared__ __align__(16) float2 smem[];
-  constexpr bool VEC = true;
-  constexpr int complex_in = 1;
-  const int padded = n + (((n - 1) >> 6) << 3);
-  float2* a = smem;
-  float2* b = smem + padded;
-  float2* stage = smem + 2 * padded;                                  // n complex values, 16-byte aligned (padded is a multiple of 8)
-  uint64_t* bar = reinterpret_cast<uint64_t*>(stage + n);
+  float2* buf = smem;
+  float2* stage = buf + F::BUF;                                       // 16-byte aligned: BUF is even
+  float2* tw1 = stage + F16_POINTS;
+  float2* tw2 = tw1 + F::TW1;
+  float2* twt = tw2 + F::TW2;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(twt + F::TWT + ((F::TW1 + F::TW2 + F::TWT) & 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bar + 1);
-  const uint32_t row_bytes = static_cast<uint32_t>(n) * 8u;
-  auto row_in = [&](int batch) { return in + (batch / L.batch1) * L.in_b0 + (batch % L.batch1) * L.in_b1; };
-  if (threadIdx.x == 0) {
+  const int t = threadIdx.x, g = t / TPR, j = t % TPR;
+  const int groups = (batches + F::ROWS - 1) / F::ROWS;
+  const bool packed = F::ROWS == 1 || (L.batch1 == 1 && L.in_b0 == 2 * N);      // a group's rows are one piece of memory
+  auto table = [&](float2* w, int entries, int ns, int radix) {
+    for (int e = t; e < entries; e += F16_THREADS) {
+      float sn, cs;
+      sincospif(-2.0f * (float)((e / ns + 1) * (e % ns)) / (float)(radix * ns), &sn, &cs);      // exact quotient
+      w[e] = make_float2(cs, sn);
+    }
+  };
+  if (F::TW1) table(tw1, F::TW1, 16, 16);
+  if (F::TW2) table(tw2, F::TW2, 256, 16);
+  if (F::TWT) table(twt, F::TWT, N / F::TAIL, F::TAIL);
+  if (t == 0) {
     st::mbar_init(st::smem_u32(bar), 1);
     *abort_flag = 0;
     st::fence_barrier_init();
   }
   __syncthreads();
-  if (threadIdx.x == 0 && static_cast<int>(blockIdx.x) < batches) {
-    st::mbar_arrive_expect_tx(st::smem_u32(bar), row_bytes);
-    st::bulk_load_g2s(st::smem_u32(stage), row_in(blockIdx.x), row_bytes, st::smem_u32(bar));
-  }
-  const float scale = inverse ? 1.0f / (float)n : 1.0f;
-  const int eights = log2n / 3, tail = 1 << (log2n - 3 * eights);
+  auto fetch = [&](int group) {      // by one thread
+    const int first = group * F::ROWS, rows = min(F::ROWS, batches - first);
+    st::mbar_arrive_expect_tx(st::smem_u32(bar), rows * N * 8);
+    for (int r = 0; r < (packed ? 1 : rows); ++r) {
+      const int b = first + r;
+      st::bulk_load_g2s(st::smem_u32(stage + r * N), in + (b / L.batch1) * L.in_b0 + (b % L.batch1) * L.in_b1,
+                        (packed ? rows : 1) * N * 8, st::smem_u32(bar));
+    }
+  };
+  if (t == 0 && static_cast<int>(blockIdx.x) < groups) fetch(blockIdx.x);
+  const float scale = inverse ? 1.0f / (float)N : 1.0f;
+  // slots of this thread's 16 points g N + j + q TPR (the second term of a slot does not depend on j where TPR < 16)
+  float2* const mine = buf + g * (N + N / 16) + j + (TPR >= 16 ? j / 16 : 0);
+  auto at = [](int q) { return q * TPR + q * TPR / 16; };
   uint32_t phase = 0;
-  for (int batch = blockIdx.x; batch < batches; batch += gridDim.x) {
-    float* gout = out + (batch / L.batch1) * L.out_b0 + (batch % L.batch1) * L.out_b1;
-    const float* gin = reinterpret_cast<const float*>(stage);
+  for (int group = blockIdx.x; group < groups; group += gridDim.x) {
+    const int batch = group * F::ROWS + g;
+    const bool live = batch < batches;
     // bounded wait; the CTA decides together, so nobody is left at a barrier by a thread that gave up
     if (!__syncthreads_and(st::mbar_wait(st::smem_u32(bar), phase, abort_flag) ? 1 : 0)) break;
     phase ^= 1u;
-#define ST_FFT_PASS(R, FIRST, LAST, NSC, SRC, DST, NS) \
-  stockham_pass<R, FIRST, LAST, NSC, VEC>(SRC, DST, gin, gout, window, L.in_i, L.out_i, n, NS, complex_in, inverse, scale)
-    ST_FFT_PASS(8, true, false, 1, nullptr, a, 1);
-    __syncthreads();                       // the staging buffer has been read by everyone: refill it with the next row
-    if (threadIdx.x == 0 && batch + static_cast<int>(gridDim.x) < batches) {
-      st::mbar_arrive_expect_tx(st::smem_u32(bar), row_bytes);
-      st::bulk_load_g2s(st::smem_u32(stage), row_in(batch + gridDim.x), row_bytes, st::smem_u32(bar));
-    }
-    float2* src = a;
-    float2* dst = b;
-    int ns = 8;
-    bool done = false;
-    for (int p = 1; p < eights && !done; ++p) {
-      if (p == eights - 1 && tail == 1) {
-        if (p == 1) ST_FFT_PASS(8, false, true, 8, src, nullptr, 8);
-        else if (p == 2) ST_FFT_PASS(8, false, true, 64, src, nullptr, 64);
-        else ST_FFT_PASS(8, false, true, 0, src, nullptr, ns);
-        done = true;
-        break;
+    float2 v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      float2 x = stage[g * N + j + q * TPR];       // rows past the batch hold an earlier group's points: not stored
+      if (window) {
+        const float w = window[j + q * TPR];
+        x.x *= w; x.y *= w;
       }
-      if (p == 1) ST_FFT_PASS(8, false, false, 8, src, dst, 8);
-      else if (p == 2) ST_FFT_PASS(8, false, false, 64, src, dst, 64);
-      else ST_FFT_PASS(8, false, false, 0, src, dst, ns);
+      v[q] = make_float2(x.x, inverse ? -x.y : x.y);
+    }
+    dft16(v);
+    __syncthreads();                               // the staging buffer and the exchange buffer have been read by everyone
+    if (t == 0 && group + static_cast<int>(gridDim.x) < groups) fetch(group + gridDim.x);
+    {
+      float2* o = buf + g * (N + N / 16) + 17 * j;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) o[k] = v[dft16_at(k)];
+    }
+    __syncthreads();
+    if constexpr (F::PASSES == 3 || (F::PASSES == 2 && F::TAIL > 1)) {
+      const int k = j & 15;
+      v[0] = mine[0];
+#pragma unroll
+      for (int q = 1; q < 16; ++q) v[q] = cmul(mine[at(q)], tw1[(q - 1) * 16 + k]);
+      dft16(v);
       __syncthreads();
-      float2* t = src; src = dst; dst = t;
-      ns *= 8;
+      float2* o = buf + g * (N + N / 16) + (j / 16) * 272 + k;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) o[17 * r] = v[dft16_at(r)];
+      __syncthreads();
     }
-    if (!done) {
-      if (tail == 2) ST_FFT_PASS(2, false, true, 0, src, nullptr, ns);
-      else ST_FFT_PASS(4, false, true, 0, src, nullptr, ns);
+    float2* gout = reinterpret_cast<float2*>(out + (live ? (batch / L.batch1) * L.out_b0 + (batch % L.batch1) * L.out_b1 : 0)) + j;
+    auto put = [&](int q, float2 y) {
+      if (live) gout[q * TPR] = make_float2(y.x * scale, (inverse ? -y.y : y.y) * scale);
+    };
+    if constexpr (F::TAIL == 1) {
+      const float2* w = F::PASSES == 3 ? tw2 : tw1;
+      v[0] = mine[0];
+#pragma unroll
+      for (int q = 1; q < 16; ++q) v[q] = cmul(mine[at(q)], w[(q - 1) * TPR + j]);
+      dft16(v);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) put(q, v[dft16_at(q)]);
+    } else {
+      constexpr int R = F::TAIL, B = 16 / R, NS = N / R;      // B butterflies of radix R: points b + r B of the thread's 16
+#pragma unroll
+      for (int b = 0; b < B; ++b) {
+        float2 x[8];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          x[r] = mine[at(b + r * B)];
+          if (r > 0) x[r] = cmul(x[r], twt[(r - 1) * NS + j + b * TPR]);
+        }
+        dft_regs<R>(x);
+#pragma unroll
+        for (int r = 0; r < R; ++r) put(b + r * B, x[r]);
+      }
     }
-#undef ST_FFT_PASS
-    __syncthreads();                       // the last pass has read its source before the next row's first pass writes `a`
   }
-  if (*abort_flag && threadIdx.x == 0) st::report_error(err, st::ERR_MBAR_TIMEOUT, 0xF7F1u);
+  if (*abort_flag && t == 0) st::report_error(err, st::ERR_MBAR_TIMEOUT, 0xF7F1u);
+}
+
+template <int LOGN>
+int launch_fft16(const float* in, float* out, const float* window, const FftLayout& L, int inverse, int batches, cudaStream_t stream) {
+  using F = Fft16<LOGN>;
+  static int resident[st::kMaxDevices] = {};      // CTAs per SM: 2 or 3, by the size of the twiddle tables
+  const int dev = st::current_device();
+  if (!resident[dev]) {
+    ST_CUDA_CHECK(cudaFuncSetAttribute(fft16_stream_kernel<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+    int n = 0;
+    ST_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fft16_stream_kernel<LOGN>, F16_THREADS, F::SMEM));
+    resident[dev] = n > 0 ? n : 1;
+  }
+  const int groups = (batches + F::ROWS - 1) / F::ROWS, most = resident[dev] * st::sm_count();
+  fft16_stream_kernel<LOGN><<<groups < most ? groups : most, F16_THREADS, F::SMEM, stream>>>(in, out, window, L, inverse, batches,
+                                                                                           st::error_word());
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
 }
 
 // Direct DFT for lengths that are not powers of two: out[k] = sum_i x[i] * w^(k*i mod n), twiddles from a table.
@@ -468,20 +576,20 @@ ST_API int st_fft_1d(const StFftArgs* a, void* stream_v) {
     const bool vec = a->complex_in && a->in_i == 2 && a->out_i == 2 && a->n > 1 &&
                      ((a->in_b0 | a->in_b1 | a->out_b0 | a->out_b1) & 1) == 0 &&
                      ((reinterpret_cast<uintptr_t>(a->in) | reinterpret_cast<uintptr_t>(a->out)) & 7) == 0;
-    // long batches of contiguous, 16-byte aligned rows: persistent CTAs with the next row prefetched asynchronously
-    const size_t stream_smem = smem + (size_t)a->n * sizeof(float2) + 16;
-    const bool streamed = vec && log2n >= 6 && a->n <= 4096 && grid > 4 * st::sm_count() &&
-                          ((a->in_b0 | a->in_b1) & 3) == 0 && (reinterpret_cast<uintptr_t>(a->in) & 15) == 0;
-    if (streamed) {
-      static bool stream_cfg[st::kMaxDevices] = {};
-      if (!stream_cfg[dev]) {
-        ST_CUDA_CHECK(cudaFuncSetAttribute(fft_pow2_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (2 * (4096 + 4096 / 8) + 4096) * (int)sizeof(float2) + 16));
-        stream_cfg[dev] = true;
+    // 16-byte aligned rows, and at least one group of 4096 points per SM (below that, a CTA per row spreads the work wider)
+    if (vec && log2n >= 6 && log2n <= 12 && (long long)grid * a->n >= (long long)F16_POINTS * st::sm_count() &&
+        ((a->in_b0 | a->in_b1) & 3) == 0 && (reinterpret_cast<uintptr_t>(a->in) & 15) == 0) {
+      switch (log2n) {
+        case 6: return launch_fft16<6>(a->in, a->out, a->window, L, a->inverse, grid, stream);
+        case 7: return launch_fft16<7>(a->in, a->out, a->window, L, a->inverse, grid, stream);
+        case 8: return launch_fft16<8>(a->in, a->out, a->window, L, a->inverse, grid, stream);
+        case 9: return launch_fft16<9>(a->in, a->out, a->window, L, a->inverse, grid, stream);
+        case 10: return launch_fft16<10>(a->in, a->out, a->window, L, a->inverse, grid, stream);
+        case 11: return launch_fft16<11>(a->in, a->out, a->window, L, a->inverse, grid, stream);
+        default: return launch_fft16<12>(a->in, a->out, a->window, L, a->inverse, grid, stream);
       }
-      fft_pow2_stream_kernel<<<2 * st::sm_count(), threads, stream_smem, stream>>>(a->in, a->out, a->window, L, a->n, log2n, a->inverse,
-                                                                                    grid, st::error_word());
-    } else if (vec) fft_pow2_kernel<true><<<grid, threads, smem, stream>>>(a->in, a->out, a->window, L, a->n, log2n, a->complex_in, a->inverse);
+    }
+    if (vec) fft_pow2_kernel<true><<<grid, threads, smem, stream>>>(a->in, a->out, a->window, L, a->n, log2n, a->complex_in, a->inverse);
     else fft_pow2_kernel<false><<<grid, threads, smem, stream>>>(a->in, a->out, a->window, L, a->n, log2n, a->complex_in, a->inverse);
   } else {
     if (smem > 48 * 1024 && !configured[dev][1]) {

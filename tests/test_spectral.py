@@ -166,3 +166,33 @@ def test_field_spectra_multipliers_and_renderer_on_gpu():
     vox, harm, decay = _temporal_case("cuda")
     out = vision.TemporalRenderer(frames=7, sample_rate_hz=12.0).render(vox, decay, harm)
     assert out.data.is_cuda and torch.allclose(out.data.cpu(), _temporal_oracle(vox.cpu(), harm.cpu(), decay.cpu(), 7, 12.0), atol=2e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [64, 128, 256, 512, 1024, 2048, 4096])
+def test_fft_of_long_batches(n):
+    """Groups of 4096 points: every pass / tail combination, a last group that is not full, windows, both directions, and
+    rows that are not one piece of memory.  Bound: fp32 rounding over log2(n) stages, against 64 bits."""
+    import ctypes
+    from spiraltorch_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rows = 4096 * 160 // n + 3
+    x = torch.view_as_complex(torch.randn(rows, n, 2, generator=g, device="cuda"))
+    w = torch.randn(n, generator=g, device="cuda")
+    for inverse in (False, True):
+        for window in (None, w):
+            z = x.to(torch.complex128) * (1 if window is None else window.double())
+            want = torch.fft.ifft(z) if inverse else torch.fft.fft(z)
+            got = spectral.fft(x, inverse=inverse, window=window)
+            assert ((got - want).abs().pow(2).sum() / want.abs().pow(2).sum()).sqrt().item() < 4e-7
+    # two-level batch with gaps between the rows on both sides
+    b0, b1, pad = rows // 2, 2, 4
+    src = torch.view_as_complex(torch.randn(b0, b1, n + pad, 2, generator=g, device="cuda"))
+    dst = torch.zeros(b0, b1, n + 1, dtype=torch.complex64, device="cuda")
+    a = spectral._FftArgs(src.data_ptr(), dst.data_ptr(), None, 2 * b1 * (n + pad), 2 * (n + pad), 2, 2 * b1 * (n + 1), 2 * (n + 1), 2,
+                   n, b0, b1, 1, 0)
+    native.check(native.lib().st_fft_1d(ctypes.byref(a), native.stream_ptr(src.device)), "st_fft_1d")
+    want = torch.fft.fft(src[..., :n].to(torch.complex128))
+    assert ((dst[..., :n] - want).abs().pow(2).sum() / want.abs().pow(2).sum()).sqrt().item() < 4e-7
+    assert dst[..., n].abs().max().item() == 0
+    native.raise_on_device_error()
