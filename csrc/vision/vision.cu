@@ -59,11 +59,59 @@ __device__ __forceinline__ void jitter_rgb(const Jitter& j, float& r, float& g, 
   }
 }
 
+// Per-channel means of x * brightness over images and pixels, for the contrast step: partial sums per (image, channel,
+// chunk), then one warp per channel adds them in order.  The means stay on the device; read back by the host they cost a
+// conversion launch, a reduction and a synchronisation in the middle of the pipeline.
+constexpr int kMeanThreads = 256;
+__global__ void __launch_bounds__(kMeanThreads)
+channel_sums_kernel(const float* __restrict__ x, float* __restrict__ part, long long plane, int C, float brightness, int chunks) {
+  const int c = blockIdx.y, b = blockIdx.z, chunk = blockIdx.x;
+  const float* p = x + ((long long)b * C + c) * plane;
+  const long long per = (plane + chunks - 1) / chunks, lo = chunk * per, hi = lo + per < plane ? lo + per : plane;
+  float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+  long long i = lo + threadIdx.x;
+  for (; i + 3 * kMeanThreads < hi; i += 4 * kMeanThreads) {
+    s0 += p[i] * brightness; s1 += p[i + kMeanThreads] * brightness;
+    s2 += p[i + 2 * kMeanThreads] * brightness; s3 += p[i + 3 * kMeanThreads] * brightness;
+  }
+  for (; i < hi; i += kMeanThreads) s0 += p[i] * brightness;
+  __shared__ float sh[kMeanThreads / 32];
+  float s = st::warp_sum((s0 + s1) + (s2 + s3));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s = 0.0f;
+    for (int w = 0; w < kMeanThreads / 32; ++w) s += sh[w];
+    part[((long long)c * gridDim.z + b) * chunks + chunk] = s;
+  }
+}
+
+// Sum of one channel's partials, in every lane of the calling warp
+__device__ __forceinline__ float channel_mean(const float* part, int c, int parts, float inv_count) {
+  float s = 0.0f;
+  for (int i = threadIdx.x & 31; i < parts; i += 32) s += part[(long long)c * parts + i];
+  return st::warp_sum(s) * inv_count;
+}
+
 // One thread per output pixel (all channels).  The pipeline is expressed as coordinate
 // maps applied back to front: flip → crop offset → resize sample, then the colour math.
 __global__ void preprocess_kernel(const float* __restrict__ in, float* __restrict__ out, int B, int C,
                                   int sh, int sw, int rh, int rw, int oh, int ow, int crop_y, int crop_x,
-                                  int flip, Jitter jit, int do_jitter) {
+                                  int flip, Jitter jit, int do_jitter, const float* __restrict__ part, int parts,
+                                  float inv_count) {
+  __shared__ float sh_mean[4];
+  if (part) {                                       // the first warps sum the partials, a few dozen values per channel
+    const int w = threadIdx.x >> 5;
+    if (w < 4 && w < C) {
+      const float m = channel_mean(part, w, parts, inv_count);
+      if ((threadIdx.x & 31) == 0) sh_mean[w] = m;
+    } else if (w < 4 && (threadIdx.x & 31) == 0) {
+      sh_mean[w] = 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) jit.mean[c] = sh_mean[c];
+  }
   const long long total = (long long)B * oh * ow;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -231,21 +279,48 @@ struct StPreprocessArgs {
   float mean[4];
 };
 
-// out[b, c, y, x] for the pipeline resize(src → resize_h x resize_w) → crop(out_h x out_w at crop_y, crop_x)
-// → colour jitter → horizontal flip.  Single transforms are special cases of the arguments.
-ST_API int st_preprocess(const float* in, float* out, const StPreprocessArgs* a, void* stream_v) {
+namespace {
+int mean_chunks(long long plane) {
+  const long long n = (plane + 8191) / 8192;
+  return (int)(n < 1 ? 1 : (n > 32 ? 32 : n));
+}
+int preprocess_run(const float* in, float* out, const StPreprocessArgs* a, float* part, void* stream_v) {
   if (!a || a->B <= 0 || a->C <= 0 || a->C > 16) return st::fail(ST_ERR_INVALID, "preprocess: bad batch/channels");
   if (a->crop_y < 0 || a->crop_x < 0 || a->crop_y + a->out_h > a->resize_h || a->crop_x + a->out_w > a->resize_w)
     return st::fail(ST_ERR_INVALID, "preprocess: crop window outside the resized image");
   Jitter j;
   j.brightness = a->brightness; j.contrast = a->contrast; j.saturation = a->saturation; j.hue = a->hue;
   for (int i = 0; i < 4; ++i) j.mean[i] = a->mean[i];
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  const long long plane = (long long)a->src_h * a->src_w;
+  const int chunks = mean_chunks(plane);
+  if (part) {
+    if (a->B > 65535) return st::fail(ST_ERR_TOO_LARGE, "preprocess: more than 65535 images");
+    channel_sums_kernel<<<dim3(chunks, a->C < 4 ? a->C : 4, a->B), kMeanThreads, 0, s>>>(in, part, plane, a->C, a->brightness, chunks);
+    ST_CUDA_CHECK(cudaGetLastError());
+  }
   const long long total = (long long)a->B * a->out_h * a->out_w;
-  preprocess_kernel<<<grid_for(total, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  preprocess_kernel<<<grid_for(total, 256), 256, 0, s>>>(
       in, out, a->B, a->C, a->src_h, a->src_w, a->resize_h, a->resize_w, a->out_h, a->out_w, a->crop_y, a->crop_x,
-      a->flip, j, a->do_jitter);
+      a->flip, j, a->do_jitter, part, a->B * chunks, 1.0f / ((float)a->B * (float)plane));
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
+}
+}  // namespace
+
+// out[b, c, y, x] for the pipeline resize(src → resize_h x resize_w) → crop(out_h x out_w at crop_y, crop_x)
+// → colour jitter → horizontal flip.  Single transforms are special cases of the arguments.
+ST_API int st_preprocess(const float* in, float* out, const StPreprocessArgs* a, void* stream_v) {
+  return preprocess_run(in, out, a, nullptr, stream_v);
+}
+
+// The same with the contrast step's means taken from the images themselves: workspace of st_preprocess_workspace floats.
+ST_API long long st_preprocess_workspace(int B, int src_h, int src_w) {
+  return 4ll * B * mean_chunks((long long)src_h * src_w);
+}
+ST_API int st_preprocess_own_means(const float* in, float* out, const StPreprocessArgs* a, float* workspace, void* stream_v) {
+  if (!workspace) return st::fail(ST_ERR_INVALID, "preprocess: workspace missing");
+  return preprocess_run(in, out, a, workspace, stream_v);
 }
 
 ST_API int st_nerf_sample(const float* rays, float* points, float* ts, float* deltas, int R, int S,

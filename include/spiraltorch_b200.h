@@ -296,6 +296,8 @@ int st_norm_fwd(int rms, const void* x, const void* residual, const void* gamma,
 int st_norm_fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y, float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
 int st_poincare_project(const float* x, float* y, int rows, int cols, float curvature, void* stream_v);   /* csrc/optim/optim.cu */
 int st_preprocess(const float* in, float* out, const StPreprocessArgs* a, void* stream_v);   /* csrc/vision/vision.cu */
+int st_preprocess_own_means(const float* in, float* out, const StPreprocessArgs* a, float* workspace, void* stream_v);   /* csrc/vision/vision.cu */
+long long st_preprocess_workspace(int B, int src_h, int src_w);   /* csrc/vision/vision.cu */
 int st_rank_select(const float* in, float* out_v, int* out_i, int rows, int cols, int k, int mode, void* stream_v);   /* csrc/rank/rank.cu */
 int st_rank_topk(const float* in, float* out_v, int* out_i, int rows, int cols, int k, int mode, void* workspace, void* stream_v);   /* csrc/rank/rank.cu */
 long long st_rank_topk_workspace(int rows, int cols, int k);   /* csrc/rank/rank.cu */

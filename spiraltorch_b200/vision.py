@@ -105,10 +105,12 @@ def preprocess(img: torch.Tensor, *, resize: Optional[tuple[int, int]] = None, c
     if oh > rh or ow > rw:
         raise ValueError("crop size exceeds the (resized) image")
     cy, cx = (rh - oh) // 2, (rw - ow) // 2
-    means = [0.0] * 4
+    means, own_means = [0.0] * 4, False
     if jitter is not None:
         if jitter.means is not None:
             means = list(jitter.means) + [0.0] * (4 - len(jitter.means))
+        elif jitter.contrast != 1.0 and native.use_native(x) and B <= 65535:
+            own_means = True
         elif jitter.contrast != 1.0:
             mm = (x * jitter.brightness).mean(dim=(0, 2, 3)).tolist()
             means = (mm + [0.0] * 4)[:4]
@@ -130,9 +132,16 @@ def preprocess(img: torch.Tensor, *, resize: Optional[tuple[int, int]] = None, c
         for i in range(4):
             a.mean[i] = means[i]
         y = torch.empty((B, C, oh, ow), dtype=torch.float32, device=x.device)
-        st = native.lib().st_preprocess(native.ptr(x), native.ptr(y), ctypes.byref(a), native.stream_ptr(x.device))
-        native.check(st, "st_preprocess")
-        launch_count += 1
+        lib, stream = native.lib(), native.stream_ptr(x.device)
+        if own_means:
+            lib.st_preprocess_workspace.restype = ctypes.c_longlong
+            work = torch.empty(lib.st_preprocess_workspace(ctypes.c_int(B), ctypes.c_int(sh), ctypes.c_int(sw)), device=x.device)
+            native.check(lib.st_preprocess_own_means(native.ptr(x), native.ptr(y), ctypes.byref(a), native.ptr(work), stream),
+                         "st_preprocess_own_means")
+            launch_count += 2
+        else:
+            native.check(lib.st_preprocess(native.ptr(x), native.ptr(y), ctypes.byref(a), stream), "st_preprocess")
+            launch_count += 1
     return y[0] if squeeze else y
 
 

@@ -208,3 +208,13 @@ def test_fractional_gl(dev):
     ref = frac.fracdiff_gl(xr.cpu(), 0.7, h=0.5, m=64)
     assert torch.allclose(y.cpu(), ref, atol=1e-4)
     assert abs(frac.mellin_log_grid(torch.exp(-torch.exp(torch.linspace(math.log(1e-4), math.log(40), 4000))), 1e-4, 40, 2 + 0j) - 1.0) < 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,C,H,W", [(1, 3, 230, 231), (5, 3, 97, 1024), (2, 1, 8, 9), (3, 6, 300, 400)])
+def test_jitter_means_taken_on_the_device(B, C, H, W):
+    """Contrast around the images' own means: odd planes, several chunks, fewer and more than four channels."""
+    x = torch.rand(B, C, H, W)
+    kw = dict(resize=(H, W), crop=(H // 2, W // 2), jitter=vision.ColorJitter(1.1, 1.3, 1.0, 0.0), flip=True)
+    want, got = vision.preprocess(x.double().float(), **kw), vision.preprocess(x.cuda(), **kw)
+    assert torch.allclose(got.cpu(), want, rtol=1e-5, atol=2e-6)      # the means differ by the order of their sums
