@@ -51,7 +51,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 
 // RMS: y = x * rstd * gamma.   LN: y = (x - mean) * rstd * gamma + beta.
 // Optional fused residual: x := x + residual is written to `sum_out` before normalising.
-template <bool RMS, int MV>
+template <bool RMS, int MV, bool GELU = false>
 __global__ void __launch_bounds__(NT)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                 const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
@@ -124,6 +124,10 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = (v[i][j] - mean) * rstd * g[j];
+      }
+      if (GELU) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = gelu_tanh(__bfloat162float(__float2bfloat16(o[j])));
       }
       store8(y + (size_t)row * d + vi * 8, o);
     }
@@ -239,6 +243,9 @@ struct Raw8<__nv_bfloat16> {
     const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
     f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
   }
+  __device__ __forceinline__ void set(const float (&f)[8]) {
+    u = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+  }
 };
 template <>
 struct Raw8<float> {
@@ -252,7 +259,8 @@ struct Raw8<float> {
   }
 };
 
-template <typename T, bool RMS, int MV>
+// GELU: the normalised row is rounded to T and goes through the activation before it is stored.
+template <typename T, bool RMS, int MV, bool GELU = false>
 __global__ void __launch_bounds__(NT)
 norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ gamma,
                      const T* __restrict__ beta, T* __restrict__ y, T* __restrict__ sum_out, float* __restrict__ mean_out,
@@ -322,6 +330,10 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, co
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = (v[i][j] - mean) * rstd * g[j];
       }
+      if (GELU) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = gelu_tanh(as_stored(o[j], x));
+      }
       store8(y + base + vi * 8, o);
     }
   }
@@ -331,11 +343,14 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, co
 // per step.  The gradient sums of a column then need 16 registers, not 16 per vector of a whole row (a warp per row spilled
 // at 1024 features and kept 16 rows in flight per SM), all loads of a step are issued together, and its row sums cost one
 // barrier: two to four per row with a block per row.
-template <typename T, bool RMS, int ROWS>
+// GELU: dy is the gradient behind an activation of the (rounded) normalised row, which is formed again from x here; the
+// product with the activation's derivative is rounded to T as a pass of its own would store it.
+template <typename T, bool RMS, int ROWS, bool GELU = false>
 __global__ void __launch_bounds__(NT)
 norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
-                     T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta, int rows, int d) {
+                     T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta, int rows, int d,
+                     const T* __restrict__ beta = nullptr) {
   __shared__ float sh[2][NT / 32][2 * ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int c0 = threadIdx.x * 8;
@@ -344,6 +359,12 @@ norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T*
 #pragma unroll
   for (int j = 0; j < 8; ++j) g[j] = dg[j] = db[j] = 0.0f;
   if (live) load8(gamma + c0, g);
+  float shift[GELU ? 8 : 1];
+  if constexpr (GELU) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) shift[j] = 0.0f;
+    if (live) load8(beta + c0, shift);
+  }
   int buf = 0;
   for (long long row0 = (long long)blockIdx.x * ROWS; row0 < rows; row0 += (long long)gridDim.x * ROWS, buf ^= 1) {
     Raw8<T> xr[ROWS], yr[ROWS], rr[ROWS];
@@ -370,6 +391,12 @@ norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T*
         float xv[8], dv[8];
         xr[r].get(xv);
         yr[r].get(dv);
+        if constexpr (GELU) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            dv[j] = as_stored(dv[j] * gelu_tanh_grad(as_stored((xv[j] - mean[r]) * rstd[r] * g[j] + shift[j], x)), x);
+          yr[r].set(dv);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float xh = (xv[j] - mean[r]) * rstd[r], gy = dv[j] * g[j];
@@ -583,6 +610,49 @@ ST_API int st_reduce_partials(const float* partial, float* out, int parts, int n
   reduce_partials_kernel<<<(n + 31) / 32, 1024, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, nullptr, nullptr, parts, n, accumulate);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
+}
+
+// LayerNorm followed by GELU (tanh form), bf16, rows of at most 2048 features: y = gelu(round(LayerNorm(x))), and its
+// backward from x and the row statistics.  scratch: st_norm_bwd_scratch_elems floats.
+ST_API int st_norm_gelu_max_features() { return NT * 8; }
+ST_API int st_norm_gelu_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int rows, int d,
+                            float eps, void* stream_v) {
+  if (int e = check_dims(rows, d)) return e;
+  if (d > NT * 8) return st::fail(ST_ERR_TOO_LARGE, "norm_gelu: feature dimension above 2048");
+  if (!beta) return st::fail(ST_ERR_INVALID, "norm_gelu: LayerNorm with offset only");
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  auto X = static_cast<const __nv_bfloat16*>(x);
+  auto G = static_cast<const __nv_bfloat16*>(gamma);
+  auto B = static_cast<const __nv_bfloat16*>(beta);
+  auto Y = static_cast<__nv_bfloat16*>(y);
+  const __nv_bfloat16* none = nullptr;
+  __nv_bfloat16* no_sum = nullptr;
+  const int grid = (rows + WARP_ROWS - 1) / WARP_ROWS;
+#define ST_NORM_GELU(MVV) norm_fwd_warp_kernel<__nv_bfloat16, false, MVV, true><<<grid, NT, 0, s>>>(X, none, G, B, Y, no_sum, mean, rstd, rows, d, eps)
+  if (d > kWarpRowFeatures) norm_fwd_kernel<false, 1, true><<<rows, NT, 0, s>>>(X, none, G, B, Y, no_sum, mean, rstd, rows, d, eps);
+  else if (d > 768) ST_NORM_GELU(4);
+  else if (d > 512) ST_NORM_GELU(3);
+  else if (d > 256) ST_NORM_GELU(2);
+  else ST_NORM_GELU(1);
+#undef ST_NORM_GELU
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+ST_API int st_norm_gelu_bwd(const void* dy, const void* x, const void* gamma, const void* beta, const float* mean, const float* rstd,
+                            void* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v) {
+  if (int e = check_dims(rows, d)) return e;
+  if (d > NT * 8) return st::fail(ST_ERR_TOO_LARGE, "norm_gelu: feature dimension above 2048");
+  if (!beta || !dbeta || !scratch) return st::fail(ST_ERR_INVALID, "norm_gelu: offset, its gradient and scratch are required");
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  int grid = st::norm_bwd_grid_for(rows, d);
+  if (d > kWarpRowFeatures && grid > st::sm_count() * 3) grid = st::sm_count() * 3;
+  float* pb = scratch + (size_t)grid * d;
+  const __nv_bfloat16* none = nullptr;
+  norm_bwd_rows_kernel<__nv_bfloat16, false, 2, true><<<grid, bwd_threads(d), 0, s>>>(
+      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean, rstd,
+      none, static_cast<__nv_bfloat16*>(dx), scratch, pb, rows, d, static_cast<const __nv_bfloat16*>(beta));
+  ST_CUDA_CHECK(cudaGetLastError());
+  return reduce_param_grads(0, scratch, pb, dgamma, dbeta, grid, d, accumulate, s);
 }
 
 // fp32 tensors throughout, rows of at most 1024 features, 16-byte aligned: the layer protocol's LayerNorm without

@@ -249,6 +249,7 @@ int st_ce_stats(const void* logits, const long long* target, float* row_max, flo
 int st_clip_coef(const float* sumsq, float norm_scale, float max_norm, float* coef, float* norm_out, void* stream_v);   /* csrc/optim/optim.cu */
 int st_colsum(const void* x, float* out, long long rows, int cols, long long ld, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_compact_rows(const float* in, float* out_v, int* out_i, int* counts, int rows, int cols, float low, float high, void* stream_v);   /* csrc/rank/rank.cu */
+int st_contrastive_views(const float* base, const float* n1, const float* n2, float noise, void* out, long long n, void* stream_v);   /* csrc/elementwise/embed.cu */
 int st_conv3x3_dgrad_weights(const void* w, void* wt, int OC, int IC, void* stream_v);   /* csrc/conv/conv.cu */
 int st_conv3x3_fwd(const StConvArgs* a, void* stream_v);   /* csrc/conv/conv.cu */
 int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v);   /* csrc/conv/conv.cu */
@@ -283,6 +284,7 @@ int st_multi(int op, int count, const void* const* src, void* const* dst, const 
 int st_multi_blocks(long long most);   /* csrc/elementwise/multi.cu */
 int st_multi_cast_bf16(int count, const void* const* src, void* const* dst, const long long* n, void* stream_v);   /* csrc/elementwise/multi.cu */
 int st_multi_max();   /* csrc/elementwise/multi.cu */
+int st_nce_rows(float* s, float* loss, int rows, float temperature, void* stream_v);   /* csrc/elementwise/embed.cu */
 int st_nd_indexer(const unsigned* positions, unsigned* out_index, unsigned* out_segment, long long n, const unsigned* dims4, const unsigned* strides4, unsigned segments, unsigned segment_stride, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_nerf_composite_bwd(const float* sigma, const float* rad, const float* deltas, const float* accum, const float* d_accum, float* d_sigma, float* d_rad, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */
 int st_nerf_composite_fwd(const float* sigma, const float* rad, const float* deltas, float* accum, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */
@@ -294,6 +296,9 @@ long long st_norm_bwd_scratch_elems(int rows, int d);   /* csrc/norm/norm.cu */
 int st_norm_f32_max_features();   /* csrc/norm/norm.cu */
 int st_norm_fwd(int rms, const void* x, const void* residual, const void* gamma, const void* beta, void* y, void* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y, float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
+int st_norm_gelu_bwd(const void* dy, const void* x, const void* gamma, const void* beta, const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v);   /* csrc/norm/norm.cu */
+int st_norm_gelu_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
+int st_norm_gelu_max_features();   /* csrc/norm/norm.cu */
 int st_poincare_project(const float* x, float* y, int rows, int cols, float curvature, void* stream_v);   /* csrc/optim/optim.cu */
 int st_preprocess(const float* in, float* out, const StPreprocessArgs* a, void* stream_v);   /* csrc/vision/vision.cu */
 int st_preprocess_own_means(const float* in, float* out, const StPreprocessArgs* a, float* workspace, void* stream_v);   /* csrc/vision/vision.cu */
@@ -306,6 +311,8 @@ int st_reduce_partials(const float* partial, float* out, int parts, int n, int a
 int st_rnn_scan(const StRnnScanArgs* a, void* stream_v);   /* csrc/recurrent/scan.cu */
 int st_rnn_scan_supported(int H, int cell);   /* csrc/recurrent/scan.cu */
 int st_rope(void* x, const float* cos_t, const float* sin_t, long long T, int heads, int D, long long ld, int seq_len, int pos_offset, int backward, void* stream_v);   /* csrc/elementwise/elementwise.cu */
+int st_row_normalize(const void* z, float* y, float* norm, int rows, int d, void* stream_v);   /* csrc/elementwise/embed.cu */
+int st_row_normalize_bwd(const float* g, const float* y, const float* norm, void* dz, int rows, int d, void* stream_v);   /* csrc/elementwise/embed.cu */
 int st_row_softmax_f32(const float* x, float* y, float* hard, int rows, int cols, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_row_softmax_spiral_f32(const float* x, float* y, float* hard, float* spiral, float* metrics, float* zmetrics, int rows, int cols, float phi, float phi_conj, float phi_bias, float leech_scale, float ramanujan_ratio, float golden_angle, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_sequence_last_step(const float* src, float* dst, int B, int steps, int dim, int scatter, void* stream);   /* csrc/recurrent/recurrent.cu */

@@ -11,6 +11,7 @@ selfsup.rs:591-706) and docs/benchmarks/selfsup.md for the expected metric range
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Optional
 
@@ -19,6 +20,8 @@ import torch.nn as nn
 
 from ..ops import elementwise as ew
 from ..ops import gemm as gemm_ops
+from ..ops import multi
+from ..ops import native
 from ..ops import norm as norm_ops
 from ..selfsup import info_nce_torch
 
@@ -59,9 +62,99 @@ def make_views(base: torch.Tensor, noise: float = 0.1, seed: Optional[int] = Non
     return base + noise * n1, base + noise * n2
 
 
+def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
+    """Whether a step can be written out over the kernels with the same outcome as running autograd over the encoder: the
+    encoder as defined here, without hooks that would see its modules, parameters or saved tensors."""
+    if type(encoder) is not ContrastiveEncoder or not torch.is_grad_enabled() or not temperature > 0:
+        return False
+    params = list(encoder.parameters())
+    dev = base.device
+    if not (base.is_cuda and base.dtype == torch.float32 and base.dim() == 2 and base.is_contiguous() and base.data_ptr() % 16 == 0
+            and not base.requires_grad and 0 < base.shape[0] <= 12000 and len(params) == 10):
+        return False
+    for m in encoder.modules():
+        if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m.__dict__.get("forward"):
+            return False
+    module_hooks = torch.nn.modules.module
+    if module_hooks._global_forward_hooks or module_hooks._global_forward_pre_hooks or module_hooks._global_backward_hooks \
+            or module_hooks._global_backward_pre_hooks or torch.is_anomaly_enabled() \
+            or torch._C._autograd._top_saved_tensors_default_hooks(False) is not None:
+        return False
+    for p in params:
+        if not (p.device == dev and p.dtype == torch.bfloat16 and p.requires_grad and p.is_leaf and p.is_contiguous()
+                and p.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in p.shape)
+                and not p._backward_hooks and not getattr(p, "_post_accumulate_grad_hooks", None)
+                and not hasattr(p, "main_grad")):
+            return False
+    w = encoder.weights
+    return base.shape[1] == w[0].shape[1] and w[0].shape[0] <= 2048 and all(
+        a.shape[0] == b.shape[1] for a, b in zip(w[:-1], w[1:]))
+
+
+def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: float, seed: Optional[int]) -> torch.Tensor:
+    """Loss and gradients of one batch with forward and backward written out: both views go through the encoder as one
+    batch, LayerNorm and GELU are one pass in each direction, and the softmax rows of the similarities turn into their
+    gradient in place.  163 launches become about 35; the similarity products stay in fp32."""
+    lib, dev, g = native.lib(), base.device, None
+    stream = native.stream_ptr(dev)
+    B, width = base.shape
+    if seed is not None:
+        g = torch.Generator(device=dev).manual_seed(seed)
+    n1 = torch.randn(base.shape, generator=g, device=dev)
+    n2 = torch.randn(base.shape, generator=g, device=dev)
+    w, b, gamma, beta = encoder.weights, encoder.biases, encoder.gammas, encoder.betas
+    x = torch.empty((2 * B, width), dtype=torch.bfloat16, device=dev)
+    native.check(lib.st_contrastive_views(native.ptr(base), native.ptr(n1), native.ptr(n2), ctypes.c_float(noise), native.ptr(x),
+                                          ctypes.c_longlong(B * width), stream), "st_contrastive_views")
+    inputs, pre, stats = [x], [], []
+    for i in range(2):
+        h = gemm_ops.gemm(inputs[-1], w[i], bias=b[i])
+        y, mean, rstd = norm_ops.norm_gelu_forward(h, gamma[i], beta[i], 1e-5)
+        pre.append(h)
+        stats.append((mean, rstd))
+        inputs.append(y)
+    z = gemm_ops.gemm(inputs[-1], w[2], bias=b[2])
+    out = z.shape[1]
+    unit = torch.empty((2 * B, out), dtype=torch.float32, device=dev)
+    norms = torch.empty(2 * B, dtype=torch.float32, device=dev)
+    native.check(lib.st_row_normalize(native.ptr(z), native.ptr(unit), native.ptr(norms), ctypes.c_int(2 * B), ctypes.c_int(out),
+                                      stream), "st_row_normalize")
+    anchors, positives = unit[:B], unit[B:]
+    sim = anchors @ positives.t()
+    rows = torch.empty(B, dtype=torch.float32, device=dev)
+    native.check(lib.st_nce_rows(native.ptr(sim), native.ptr(rows), ctypes.c_int(B), ctypes.c_float(temperature), stream), "st_nce_rows")
+    loss = rows.mean()
+    d_unit = torch.empty_like(unit)
+    torch.mm(sim, positives, out=d_unit[:B])
+    torch.mm(sim.t(), anchors, out=d_unit[B:])
+    d = torch.empty_like(z)
+    native.check(lib.st_row_normalize_bwd(native.ptr(d_unit), native.ptr(unit), native.ptr(norms), native.ptr(d), ctypes.c_int(2 * B),
+                                          ctypes.c_int(out), stream), "st_row_normalize_bwd")
+    # vector gradients: fp32 sums side by side, rounded to bf16 in one launch
+    vectors = [*b, *gamma, *beta]
+    flat = torch.zeros(sum(v.numel() for v in vectors), dtype=torch.float32, device=dev)
+    sums = list(flat.split([v.numel() for v in vectors]))
+    d_w = [None] * 3
+    for i in (2, 1, 0):
+        ew.colsum(d, sums[i], accumulate=True)
+        d_w[i] = gemm_ops.gemm(d, inputs[i], a_mn=True, b_mn=True, out_dtype=torch.bfloat16)
+        if i:
+            da = gemm_ops.gemm(d, w[i], b_mn=True)
+            d = norm_ops.norm_gelu_backward(da, pre[i - 1], gamma[i - 1], beta[i - 1], *stats[i - 1], sums[2 + i], sums[4 + i])
+    for p, grad in zip([*w, *vectors], d_w + multi.to_bf16(sums)):
+        if p.grad is None:
+            p.grad = grad
+        else:
+            p.grad.add_(grad)
+    return loss
+
+
 def contrastive_step(encoder: ContrastiveEncoder, base: torch.Tensor, temperature: float = 0.1,
                      fused_loss=None, noise: float = 0.1, seed: Optional[int] = None) -> torch.Tensor:
     """Forward + backward of one batch; returns the loss (gradients are in ``.grad``)."""
+    if fused_loss is None and _schedulable(encoder, base, temperature):
+        with torch.no_grad():
+            return _scheduled_step(encoder, base, temperature, noise, seed)
     v1, v2 = make_views(base, noise, seed)
     za, zp = encoder(v1), encoder(v2)
     if fused_loss is not None:

@@ -118,6 +118,37 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
     return dx
 
 
+def norm_gelu_forward(x2: torch.Tensor, gamma, beta, eps: float):
+    """``gelu(layer_norm(x2))`` of contiguous bf16 rows of at most 2048 features on CUDA: ``(y, mean, rstd)``."""
+    global launch_count
+    native.require_cuda("norm_gelu_forward", x2, gamma, beta)
+    rows, d = x2.shape
+    y = torch.empty_like(x2)
+    mean, rstd = (torch.empty(rows, dtype=torch.float32, device=x2.device) for _ in range(2))
+    native.check(native.lib().st_norm_gelu_fwd(
+        native.ptr(x2), native.ptr(gamma), native.ptr(beta), native.ptr(y), native.ptr(mean), native.ptr(rstd), ctypes.c_int(rows),
+        ctypes.c_int(d), ctypes.c_float(eps), native.stream_ptr(x2.device)), "st_norm_gelu_fwd")
+    launch_count += 1
+    return y, mean, rstd
+
+
+def norm_gelu_backward(dy2, x2, gamma, beta, mean, rstd, dgamma: torch.Tensor, dbeta: torch.Tensor) -> torch.Tensor:
+    """Backward of :func:`norm_gelu_forward`: returns dx, writes the fp32 ``dgamma`` and ``dbeta``."""
+    global launch_count
+    native.require_cuda("norm_gelu_backward", dy2, x2, gamma, beta, mean, rstd, dgamma, dbeta)
+    rows, d = x2.shape
+    lib = native.lib()
+    lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
+    scratch = _get_scratch(x2.device, int(lib.st_norm_bwd_scratch_elems(ctypes.c_int(rows), ctypes.c_int(d))))
+    dx = torch.empty_like(x2)
+    native.check(lib.st_norm_gelu_bwd(
+        native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(beta), native.ptr(mean), native.ptr(rstd), native.ptr(dx),
+        native.ptr(dgamma), native.ptr(dbeta), ctypes.c_int(0), native.ptr(scratch), ctypes.c_int(rows), ctypes.c_int(d),
+        native.stream_ptr(x2.device)), "st_norm_gelu_bwd")
+    launch_count += 2
+    return dx
+
+
 class _NormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gamma, beta, eps, rms):

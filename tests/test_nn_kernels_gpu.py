@@ -431,3 +431,47 @@ def test_attention_backward_does_not_read_the_returned_output():
     with torch.no_grad():
         y.detach().zero_()
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, (q, k, v), g), want))
+
+
+@pytest.mark.parametrize("B,width,hidden,out", [(1, 8, 8, 8), (37, 72, 264, 64), (130, 128, 1032, 256), (1000, 512, 2048, 512)])
+def test_contrastive_step_written_out_over_the_kernels(B, width, hidden, out):
+    """Against the autograd form (which a hook selects), both measured from 64 bits: gradients are sums of bf16 products, so
+    neither may be further off than the rounding of its operands, and the written-out form not further than the other."""
+    from spiraltorch_b200.models import contrastive as M
+    enc = M.ContrastiveEncoder(width, hidden, out, device=DEV, seed=B)
+    for p in list(enc.gammas) + list(enc.betas) + list(enc.biases):
+        p.data.add_(0.1 * torch.randn(p.shape, device=DEV).to(p.dtype))
+    base = torch.randn(B, width, device=DEV)
+    assert M._schedulable(enc, base, 0.1) and not M._schedulable(enc, base.double(), 0.1)
+
+    def step():
+        enc.zero_grad(set_to_none=True)
+        loss = M.contrastive_step(enc, base, 0.1, seed=5)
+        assert not loss.requires_grad
+        return loss.item(), [p.grad.clone() for p in enc.parameters()]
+    loss, grads = step()
+    handle = enc.register_forward_hook(lambda *a: None)
+    assert not M._schedulable(enc, base, 0.1)
+    loss_a, grads_a = step()
+    handle.remove()
+    p64 = [p.detach().double().requires_grad_(True) for p in enc.parameters()]
+    g = torch.Generator(device=DEV).manual_seed(5)
+    z = []
+    for n in [torch.randn(base.shape, generator=g, device=DEV) for _ in range(2)]:
+        h = base.double() + 0.1 * n.double()
+        for i in range(3):
+            h = h @ p64[i].t() + p64[3 + i]
+            if i < 2:
+                h = torch.nn.functional.gelu(torch.nn.functional.layer_norm(h, h.shape[-1:], p64[6 + i], p64[8 + i], 1e-5), approximate="tanh")
+        z.append(torch.nn.functional.normalize(h, dim=-1))
+    want = torch.nn.functional.cross_entropy(z[0] @ z[1].t() / 0.1, torch.arange(B, device=DEV))
+    want.backward()
+    assert abs(loss - want.item()) <= 2e-2 * max(want.item(), 1.0)
+    for a, b, p in zip(grads, grads_a, p64):
+        scale = p.grad.norm()
+        assert a.dtype == torch.bfloat16 and a.shape == p.shape
+        if B > 1:       # one pair has no negatives: its gradients are rounding noise around zero
+            assert (a - p.grad).norm() <= max(1.3 * (b - p.grad).norm().item(), 0.01 * scale.item())
+    first = [p.grad.clone() for p in enc.parameters()]
+    M.contrastive_step(enc, base, 0.1, seed=5)                        # gradients accumulate
+    assert all((p.grad - 2 * f).norm() <= 0.02 * (2 * f).norm() + 1e-6 for p, f in zip(enc.parameters(), first)) or B == 1
