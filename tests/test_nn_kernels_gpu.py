@@ -475,3 +475,29 @@ def test_contrastive_step_written_out_over_the_kernels(B, width, hidden, out):
     first = [p.grad.clone() for p in enc.parameters()]
     M.contrastive_step(enc, base, 0.1, seed=5)                        # gradients accumulate
     assert all((p.grad - 2 * f).norm() <= 0.02 * (2 * f).norm() + 1e-6 for p, f in zip(enc.parameters(), first)) or B == 1
+
+
+@pytest.mark.parametrize("cell,B,T,H,dilation", [
+    ("tanh", 1, 1, 1, 1), ("tanh", 5, 9, 33, 1), ("tanh", 900, 3, 128, 1), ("tanh", 3, 5, 129, 1), ("wave", 7, 12, 5, 1),
+    ("wave", 6, 40, 64, 2), ("wave", 9, 11, 96, 3), ("wave", 900, 7, 72, 5), ("wave", 3, 130, 100, 60), ("wave", 2, 4, 128, 9),
+    ("lstm", 4, 7, 32, 1), ("lstm", 5, 6, 65, 1), ("lstm", 700, 4, 96, 1), ("lstm", 2, 3, 97, 1)])
+def test_recurrent_scans_with_weights_in_registers(cell, B, T, H, dilation):
+    """Sizes at and past the register forms' edges, units that do not fill a warp, one and four rows per CTA, skip histories
+    in shared and in global memory, dilations of 1 and beyond the sequence.  The scan is fp32 between bf16 projections:
+    2^-8 of the largest value, per step of error growth at most."""
+    from spiraltorch_b200.ops import recurrent as R
+    torch.manual_seed(H + B)
+    gates, width = {"tanh": 1, "wave": 2, "lstm": 4}[cell], 16
+    x = torch.randn(B, T, width, device=DEV).bfloat16().float()
+    w_ih, w_hh, b = (((torch.rand(s, device=DEV) * 2 - 1) / H ** 0.5).bfloat16().float() for s in
+                     ((width, gates * H), (H, gates * H), (1, gates * H)))
+    leaves = [t.requires_grad_(True) for t in (x, w_ih, w_hh, b)]
+    assert R.scan_supported(H, cell)
+    h = R.rnn_sequence(*leaves, cell, dilation)
+    g = torch.randn(B, H, device=DEV)
+    grads = torch.autograd.grad(h, leaves, g)
+    wide = [t.detach().double().requires_grad_(True) for t in leaves]
+    want = R.rnn_sequence_reference(*wide, cell, dilation)
+    assert (h - want).abs().max() <= 1e-4
+    for a, r in zip(grads, torch.autograd.grad(want, wide, g.double())):
+        assert (a - r).norm() <= 5e-3 * r.norm() + 1e-6
