@@ -38,6 +38,14 @@ __device__ __forceinline__ float load_grad<__nv_bfloat16>(const __nv_bfloat16* g
   return __bfloat162float(g[i]);
 }
 
+__device__ __forceinline__ void adamw_one(float g, float& w, float& m, float& v, const AdamArgs& a) {
+  m = a.beta1 * m + (1.0f - a.beta1) * g;
+  v = a.beta2 * v + (1.0f - a.beta2) * g * g;
+  const float mhat = m / a.bc1;
+  const float vhat = v / a.bc2;
+  w = w - a.lr * (mhat / (sqrtf(vhat) + a.eps) + a.weight_decay * w);
+}
+
 template <typename GradT>
 __global__ void adamw_kernel(GradT* __restrict__ grad, float* __restrict__ master,
                              float* __restrict__ m, float* __restrict__ v,
@@ -46,18 +54,44 @@ __global__ void adamw_kernel(GradT* __restrict__ grad, float* __restrict__ maste
   const float gs = a.grad_scale * (scale_ptr ? *scale_ptr : 1.0f);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const float g = load_grad<GradT>(grad, i) * gs;
-    float w = master[i];
-    float mi = a.beta1 * m[i] + (1.0f - a.beta1) * g;
-    float vi = a.beta2 * v[i] + (1.0f - a.beta2) * g * g;
+    float w = master[i], mi = m[i], vi = v[i];
+    adamw_one(load_grad<GradT>(grad, i) * gs, w, mi, vi, a);
     m[i] = mi;
     v[i] = vi;
-    const float mhat = mi / a.bc1;
-    const float vhat = vi / a.bc2;
-    w = w - a.lr * (mhat / (sqrtf(vhat) + a.eps) + a.weight_decay * w);
     master[i] = w;
     if (weight) weight[i] = __float2bfloat16(w);
     if (zero_grad) grad[i] = GradT(0.0f);
+  }
+}
+
+// Four parameters per thread and step: the step is its bytes (34 per parameter with fp32 gradients that are cleared), and
+// 4-byte accesses left it at 5.3 TB/s.  0.5 G parameters: 3.43 -> 3.00 ms, 6.1 TB/s.  n % 4 == 0, pointers aligned to a vector.
+template <typename GradT>
+__global__ void __launch_bounds__(256)
+adamw4_kernel(GradT* __restrict__ grad, float4* __restrict__ master, float4* __restrict__ m, float4* __restrict__ v,
+              uint2* __restrict__ weight, long long n4, AdamArgs a, const float* __restrict__ scale_ptr, int zero_grad) {
+  const float gs = a.grad_scale * (scale_ptr ? *scale_ptr : 1.0f);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    float4 w = master[i], mi = m[i], vi = v[i], g;
+    if constexpr (sizeof(GradT) == 4) {
+      g = reinterpret_cast<const float4*>(grad)[i];
+    } else {
+      const uint2 u = reinterpret_cast<const uint2*>(grad)[i];
+      const float2 lo = unpack_bf16x2(u.x), hi = unpack_bf16x2(u.y);
+      g = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    adamw_one(g.x * gs, w.x, mi.x, vi.x, a);
+    adamw_one(g.y * gs, w.y, mi.y, vi.y, a);
+    adamw_one(g.z * gs, w.z, mi.z, vi.z, a);
+    adamw_one(g.w * gs, w.w, mi.w, vi.w, a);
+    m[i] = mi;
+    v[i] = vi;
+    master[i] = w;
+    if (weight) weight[i] = make_uint2(pack_bf16x2(w.x, w.y), pack_bf16x2(w.z, w.w));
+    if (zero_grad) {
+      if constexpr (sizeof(GradT) == 4) reinterpret_cast<float4*>(grad)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      else reinterpret_cast<uint2*>(grad)[i] = make_uint2(0, 0);
+    }
   }
 }
 
@@ -225,6 +259,20 @@ ST_API int st_adamw(void* grad, int grad_is_bf16, float* master, float* m, float
   a.bc2 = 1.0f - powf(beta2, (float)step);
   a.grad_scale = grad_scale;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  const uintptr_t wide = reinterpret_cast<uintptr_t>(master) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v) |
+                         (grad_is_bf16 ? 0 : reinterpret_cast<uintptr_t>(grad));
+  const uintptr_t half = reinterpret_cast<uintptr_t>(weight) | (grad_is_bf16 ? reinterpret_cast<uintptr_t>(grad) : 0);
+  if ((n & 3) == 0 && (wide & 15) == 0 && (half & 7) == 0) {
+    auto run = [&](auto* g) {
+      adamw4_kernel<<<grid_for(n / 4, 256), 256, 0, s>>>(g, reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m),
+                                                         reinterpret_cast<float4*>(v), static_cast<uint2*>(weight), n / 4, a,
+                                                         scale_ptr, zero_grad);
+    };
+    if (grad_is_bf16) run(static_cast<__nv_bfloat16*>(grad));
+    else run(static_cast<float*>(grad));
+    ST_CUDA_CHECK(cudaGetLastError());
+    return ST_OK;
+  }
   if (grad_is_bf16)
     adamw_kernel<__nv_bfloat16><<<grid_for(n, 256), 256, 0, s>>>(
         static_cast<__nv_bfloat16*>(grad), master, m, v, static_cast<__nv_bfloat16*>(weight), n, a,
