@@ -248,19 +248,24 @@ __device__ __forceinline__ void epilogue_bar() {
   asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM>
+// CG = 2 (COMM_NONE only): a cluster of two CTAs works on one tile of 256 x BN.  Each CTA brings its 128 rows of A and its half
+// of B into its own shared memory, the even CTA's MMA warp issues for both, and each CTA's epilogue stores its own 128 rows.
+// A K block then costs an SM 32 KB of loads instead of 48 (BN = 256), and the ring holds six stages instead of four.
+template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM, int CG = 1>
 __global__ void __launch_bounds__(COMM == COMM_AG ? NUM_THREADS_AG : NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ OutMaps tmC, const __grid_constant__ CUtensorMap tmA_local,
                  const GemmParams p, const GemmComm cm) {
-  using L = SmemLayout<BN, STAGES>;
+  static_assert(CG == 1 || COMM == COMM_NONE, "CTA pairs run the plain product only");
+  using L = SmemLayout<BN / CG, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  const int gemm_bid = blockIdx.x;
+  const int cta = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int gemm_bid = CG == 2 ? blockIdx.x >> 1 : blockIdx.x;
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
   uint64_t* full_bar = bars;
@@ -270,12 +275,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tiles_m = (p.M + BM - 1) / BM;
+  const int tiles_m = (p.M + BM * CG - 1) / (BM * CG);
   const int tiles_n = (p.N + BN - 1) / BN;
   const int tiles_per_batch = tiles_m * tiles_n;
   const int total_tiles = tiles_per_batch * p.batch;
   const int k_blocks = (p.K + BK - 1) / BK;
-  const int grid_stride = gridDim.x;
+  const int grid_stride = gridDim.x / CG;
   constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32 : (2 * BN <= 64) ? 64 : (2 * BN <= 128) ? 128
                                  : (2 * BN <= 256) ? 256 : 512;
 
@@ -286,7 +291,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tfull_bar[a]), 1);
-      mbar_init(smem_u32(&tempty_bar[a]), 4);
+      mbar_init(smem_u32(&tempty_bar[a]), 4 * CG);
     }
     *abort_flag = 0;
     if constexpr (COMM == COMM_AG) {
@@ -306,11 +311,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (CG == 2) {
+      tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS);
+    } else {
+      tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  if constexpr (CG == 2) cluster_sync(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -331,7 +341,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     for (int t = gemm_bid; t < total_tiles && ok; t += grid_stride) {
       int b, tm, tn;
       map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
-      const int m0 = tm * BM, n0 = tn * BN;
+      const int m0 = tm * BM * CG + cta * BM, n0 = tn * BN + cta * (BN / CG);      // this CTA's rows of A and of B
       const CUtensorMap* mapA = &tmA;
       int m_coord = m0;
       if constexpr (COMM == COMM_AG) {
@@ -358,9 +368,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       auto k_loop = [&](uint32_t bytes, auto&& copies) {
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u, abort_flag)) return false;
-          const uint32_t fb = full0 + stage * 8;
+          const uint32_t fb = CG == 2 ? (full0 + stage * 8) & kPairLeaderMask : full0 + stage * 8;
           const uint32_t sa = smem0 + stage * L::STAGE_BYTES;
-          if (leader) mbar_arrive_expect_tx(fb, bytes);
+          if (leader && cta == 0) mbar_arrive_expect_tx(fb, bytes * CG);       // the even CTA's barrier counts both CTAs' bytes
           copies(kb, fb, sa, sa + L::A_BYTES);
           if (++stage == STAGES) {
             stage = 0;
@@ -371,21 +381,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       };
       // MN-major operands arrive as 64-wide boxes: a box wholly outside the matrix is not fetched (what the shared
       // memory holds in its place only reaches rows or columns of the accumulator that are never stored)
-      const int boxes_a = (A_MN && COMM == COMM_NONE) ? min(BM / 64, (p.M - m0 + 63) / 64) : BM / 64;
-      const int boxes_b = (B_MN && COMM == COMM_NONE) ? min(BN / 64, (p.N - n0 + 63) / 64) : BN / 64;
-      const bool whole = boxes_a == BM / 64 && boxes_b == BN / 64;
+      constexpr int BNC = BN / CG;         // rows of B per CTA
+      const int boxes_a = (A_MN && COMM == COMM_NONE && CG == 1) ? min(BM / 64, (p.M - m0 + 63) / 64) : BM / 64;
+      const int boxes_b = (B_MN && COMM == COMM_NONE && CG == 1) ? min(BN / 64, (p.N - n0 + 63) / 64) : BNC / 64;
+      const bool whole = boxes_a == BM / 64 && boxes_b == BNC / 64;
       const uint32_t stage_bytes = (boxes_a + boxes_b) * (64 * BK * 2);
+      auto load3 = [](uint32_t dst, const CUtensorMap* map, uint32_t fb, int c0, int c1, int c2) {
+        if constexpr (CG == 2) tma_load_3d_pair(dst, map, fb, c0, c1, c2); else tma_load_3d(dst, map, fb, c0, c1, c2);
+      };
+      auto load4 = [](uint32_t dst, const CUtensorMap* map, uint32_t fb, int c0, int c1, int c2, int c3) {
+        if constexpr (CG == 2) tma_load_4d_pair(dst, map, fb, c0, c1, c2, c3); else tma_load_4d(dst, map, fb, c0, c1, c2, c3);
+      };
       // Convolution coordinates advance by additions: six divisions per K block took about 950 SM cycles, twice the
       // tensor work of the largest tile.
       if (!A_MN && !B_MN && p.conv.mode == 1) {
         // A: 128 output pixels (Nb images x Hb rows x W) shifted by the tap, 64 channels
         const int hblocks = p.conv.H / p.conv.Hb;
-        const int img = (tm / hblocks) * p.conv.Nb, h0 = (tm % hblocks) * p.conv.Hb;
+        const int block = tm * CG + cta;
+        const int img = (block / hblocks) * p.conv.Nb, h0 = (block % hblocks) * p.conv.Hb;
         int tap_w = -1, tap_h = -1, chunk = 0;
         ok = k_loop(stage_bytes, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (leader) {
-            tma_load_4d(sa, mapA, fb, chunk * 64, tap_w, h0 + tap_h, img);
-            tma_load_3d(sb, &tmB, fb, kb * BK, n0, 0);
+            load4(sa, mapA, fb, chunk * 64, tap_w, h0 + tap_h, img);
+            load3(sb, &tmB, fb, kb * BK, n0, 0);
           }
           if (++chunk == p.conv.c_chunks) {
             chunk = 0;
@@ -402,10 +420,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (leader) {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              if (j < boxes_a) tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, pix_block * BK, 0);
+              if (j < boxes_a) load3(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, pix_block * BK, 0);
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              if (j < boxes_b) tma_load_4d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, tap_w, h0 + tap_h, img);
+            for (int j = 0; j < BNC / 64; ++j)
+              if (j < boxes_b) load4(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, tap_w, h0 + tap_h, img);
           }
           ++pix_block;
           h0 += p.conv.Hb;
@@ -415,36 +433,36 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         ok = k_loop(L::STAGE_BYTES, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (!leader) return;
           if constexpr (!A_MN) {
-            tma_load_3d(sa, mapA, fb, kb * BK, m_coord, b);
+            load3(sa, mapA, fb, kb * BK, m_coord, b);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kb * BK, b);
+              load3(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kb * BK, b);
           }
           if constexpr (!B_MN) {
-            tma_load_3d(sb, &tmB, fb, kb * BK, n0, b);
+            load3(sb, &tmB, fb, kb * BK, n0, b);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_3d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, kb * BK, b);
+            for (int j = 0; j < BNC / 64; ++j)
+              load3(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, kb * BK, b);
           }
         });
       } else {
         ok = k_loop(stage_bytes, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (!leader) return;
           if constexpr (!A_MN) {
-            tma_load_3d(sa, mapA, fb, kb * BK, m_coord, b);
+            load3(sa, mapA, fb, kb * BK, m_coord, b);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              if (j < boxes_a) tma_load_3d(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kb * BK, b);
+              if (j < boxes_a) load3(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, kb * BK, b);
           }
           if constexpr (!B_MN) {
-            tma_load_3d(sb, &tmB, fb, kb * BK, n0, b);
+            load3(sb, &tmB, fb, kb * BK, n0, b);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              if (j < boxes_b) tma_load_3d(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, kb * BK, b);
+            for (int j = 0; j < BNC / 64; ++j)
+              if (j < boxes_b) load3(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, kb * BK, b);
           }
         });
       }
@@ -452,7 +470,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == 1) {
     // ------------------------------- MMA issuer ---------------------------------------
     const bool leader = elect_one();
-    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+    constexpr uint32_t idesc = make_idesc_bf16(BM * CG, BN, A_MN, B_MN);
     // descriptor words are formed once: the high word is common, the low word advances by constants
     constexpr uint32_t desc_hi = smem_desc_hi(1024);
     constexpr uint32_t a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4, b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
@@ -466,7 +484,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t phase = 0;
     int iter = 0;
     bool ok = true;
-    for (int t = gemm_bid; t < total_tiles && ok; t += grid_stride, ++iter) {
+    for (int t = cta == 0 ? gemm_bid : total_tiles; t < total_tiles && ok; t += grid_stride, ++iter) {      // the even CTA issues
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1;
       if (!mbar_wait_warp(tempty0 + acc * 8, acc_phase ^ 1u, abort_flag)) break;
@@ -482,9 +500,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (leader) {
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16_ss_split(tmem_d, a_lo + k * a_step, desc_hi, b_lo + k * b_step, desc_hi, idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit(empty0 + stage * 8);  // frees the smem stage when MMAs finish
-          if (kb + 1 == k_blocks) umma_commit(tfull0 + acc * 8);
+            if constexpr (CG == 2)
+              umma_bf16_ss_split_pair(tmem_d, a_lo + k * a_step, desc_hi, b_lo + k * b_step, desc_hi, idesc, (kb | k) != 0 ? 1u : 0u);
+            else
+              umma_bf16_ss_split(tmem_d, a_lo + k * a_step, desc_hi, b_lo + k * b_step, desc_hi, idesc, (kb | k) != 0 ? 1u : 0u);
+          // frees the smem stage (of both CTAs) when the MMAs finish
+          if constexpr (CG == 2) umma_commit_pair(empty0 + stage * 8); else umma_commit(empty0 + stage * 8);
+          if (kb + 1 == k_blocks) {
+            if constexpr (CG == 2) umma_commit_pair(tfull0 + acc * 8); else umma_commit(tfull0 + acc * 8);
+          }
         }
         __syncwarp();
         if (++stage == STAGES) {
@@ -524,7 +548,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     for (int t = gemm_bid; t < total_tiles && alive; t += grid_stride, ++iter) {
       int b, tm, tn;
       map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
-      const int m0 = tm * BM, n0 = tn * BN;
+      const int m0 = tm * BM * CG + cta * BM, n0 = tn * BN;
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1;
       if (!mbar_wait_warp(smem_u32(&tfull_bar[acc]), acc_phase, abort_flag)) break;
@@ -796,7 +820,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // hand the accumulator back to the MMA warp
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
+      if (lane == 0) {
+        if constexpr (CG == 2) mbar_arrive_cluster(smem_u32(&tempty_bar[acc]) & kPairLeaderMask);
+        else mbar_arrive(smem_u32(&tempty_bar[acc]));
+      }
       if constexpr (COMM == COMM_RS) {
         // Publish this warp's 32 rows to the owner (the counter counts warp arrivals, so no
         // CTA-wide barrier is needed).  Waiting for the stores of the tile just issued would put
@@ -978,7 +1005,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (cm.trace && threadIdx.x == 64) cm.trace[blockIdx.x * 4 + 3] = globaltimer_ns();
   }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  if constexpr (CG == 2) cluster_sync(); else __syncthreads();      // the pair's barriers and tensor memory outlive both CTAs' use
   if (*abort_flag) {
     if (threadIdx.x == 0) report_error(p.err, ERR_MBAR_TIMEOUT, 0x6E00u);
     // give copies that are still in flight a bounded time to land before smem is released
@@ -986,8 +1014,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, TMEM_COLS); else tmem_dealloc(tmem_base, TMEM_COLS);
   }
+}
+
+// Launch of the CTA-pair form: an even grid of at most one CTA per SM, in clusters of two.
+template <bool A_MN, bool B_MN>
+int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
+  constexpr int BN = 256, STAGES = 6;
+  using L = SmemLayout<BN / 2, STAGES>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, COMM_NONE, 2>;
+  static bool configured[st::kMaxDevices] = {false};   // the attribute is per device
+  const int dev = st::current_device();
+  if (!configured[dev]) {
+    ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+    configured[dev] = true;
+  }
+  const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch;
+  const int pairs = st::sm_count() / 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * (tiles < pairs ? tiles : pairs));
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = L::TOTAL;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  GemmComm none{};
+  ST_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, tmA, p, none));
+  return ST_OK;
 }
 
 }  // namespace gemm

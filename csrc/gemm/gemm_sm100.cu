@@ -91,6 +91,14 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
   // the narrowest tile that covers N: a wider one multiplies and fetches columns that are not there
   const int BN = a->N <= 64 ? 64 : (a->N <= 128 ? 128 : 256);
 
+  // CTA pairs where they need no more rounds of tiles than single CTAs do
+  auto rounds = [](long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
+  const long long tn = (a->N + 255) / 256;
+  const bool pair = BN == 256 && a->M > BM && a->max_ctas <= 0 && st::sm_count() >= 2 &&
+                    rounds((long long)((a->M + 2 * BM - 1) / (2 * BM)) * tn * a->batch, st::sm_count() / 2) <=
+                        rounds((long long)((a->M + BM - 1) / BM) * tn * a->batch, st::sm_count());
+  const int b_rows = pair ? BN / 2 : BN;      // rows of B that one CTA loads
+
   CUtensorMap tmA, tmB;
   {
     const uint64_t bsa = a->batch > 1 ? (uint64_t)a->batch_stride_a * 2 : (uint64_t)a->lda * 2 * (a->a_mn_major ? a->K : a->M);
@@ -108,7 +116,7 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
                          CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
     if (!a->b_mn_major) {
-      dims[0] = a->K; dims[1] = a->N; box[0] = BK; box[1] = BN;
+      dims[0] = a->K; dims[1] = a->N; box[0] = BK; box[1] = b_rows;
     } else {
       dims[0] = a->N; dims[1] = a->K; box[0] = 64; box[1] = BK;
     }
@@ -151,6 +159,12 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
       return ST_ERR_CUDA;
   }
 
+  if (pair) {
+    if (!a->a_mn_major && !a->b_mn_major) return launch_pair<false, false>(tmA, tmB, tmC, p, stream);
+    if (!a->a_mn_major) return launch_pair<false, true>(tmA, tmB, tmC, p, stream);
+    if (!a->b_mn_major) return launch_pair<true, false>(tmA, tmB, tmC, p, stream);
+    return launch_pair<true, true>(tmA, tmB, tmC, p, stream);
+  }
   if (BN == 64)
     return dispatch_major<64, 8>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
   if (BN == 128)
