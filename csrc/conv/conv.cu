@@ -336,11 +336,12 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   const int P = a->N * a->H * a->W;
   CUtensorMap tmA, tmB;
   if (!nhwc_map(&tmA, a->x, a->N, a->H, a->W, a->C, a->W, Hb, Nb)) return ST_ERR_CUDA;
-  const int BN = a->OC <= 64 ? 64 : (a->OC <= 128 ? 128 : 256);
+  const TileChoice tile = choose_tile(P, a->OC, 9ll * a->C, 1, st::sm_count());
+  const int BN = tile.bn;
   {
     uint64_t dims[3] = {(uint64_t)9 * a->C, (uint64_t)a->OC, 1};
     uint64_t strides[2] = {(uint64_t)9 * a->C * 2, (uint64_t)9 * a->C * 2 * a->OC};
-    uint32_t box[3] = {BK, (uint32_t)BN, 1};
+    uint32_t box[3] = {BK, (uint32_t)(tile.pair ? BN / 2 : BN), 1};
     if (!encode_tmap(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
   }
@@ -366,6 +367,7 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   p.use_tma_store = 1;
   p.err = st::error_word();
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  if (tile.pair) return launch_pair<false, false>(tmA, tmB, tmC, p, s);
   if (BN == 64) return launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s);
   if (BN == 128) return launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, false, false>(tmA, tmB, tmC, p, s);

@@ -1018,6 +1018,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// Tile width of a product.  Time is about a + rounds * K blocks * c: a covers launch, fill and the last epilogue, c a K block
+// of one tile on one SM (the pair's on two), both measured in microseconds with bf16 outputs:
+//   tile          128 x 64   128 x 128   128 x 256   256 x 256 on a pair
+//   a, c          5.0, 0.228   5.6, 0.262   4.1, 0.40    7.6, 0.33
+// Narrow tiles lose throughput (their K block costs more than its share) but fill the chip where wide ones leave SMs without
+// a tile: 777 x 2048 x 8192 takes 39 us with 112 tiles of 128 x 128 and 53 with 56 of 128 x 256, 1536 x 512 x 4608 22 against
+// 30, while 16384 x 6144 x 2048 takes 659 / 378 / 291 / 269 us in the order of the table.  Against 24 shapes the rule is off
+// by one choice with 3 % between the two.
+struct TileChoice {
+  int bn;
+  bool pair;
+};
+inline TileChoice choose_tile(long long M, long long N, long long K, long long batch, int ctas) {
+  const long long kb = (K + BK - 1) / BK;
+  auto rounds = [](long long tiles, long long at_once) { return (tiles + at_once - 1) / at_once; };
+  auto cost = [&](int bm, int bn, long long at_once, double a, double c) {
+    return a + c * (double)(rounds(((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch, at_once) * kb);
+  };
+  TileChoice best{64, false};
+  double t = cost(BM, 64, ctas, 5.0, 0.228);
+  if (N > 64) {
+    const double u = cost(BM, 128, ctas, 5.6, 0.262);
+    if (u <= t) { t = u; best = {128, false}; }
+  }
+  if (N > 128) {
+    const double u = cost(BM, 256, ctas, 4.1, 0.40);
+    if (u <= t) { t = u; best = {256, false}; }
+    const double w = M > BM && ctas >= 2 ? cost(2 * BM, 256, ctas / 2, 7.6, 0.33) : 1e30;
+    if (w < t) best = {256, true};
+  }
+  return best;
+}
+
 // Launch of the CTA-pair form: an even grid of at most one CTA per SM, in clusters of two.
 template <bool A_MN, bool B_MN>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {

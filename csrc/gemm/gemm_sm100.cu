@@ -88,15 +88,11 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "gemm: backward activation needs aux_in");
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
 
-  // the narrowest tile that covers N: a wider one multiplies and fetches columns that are not there
-  const int BN = a->N <= 64 ? 64 : (a->N <= 128 ? 128 : 256);
-
-  // CTA pairs where they need no more rounds of tiles than single CTAs do
-  auto rounds = [](long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
-  const long long tn = (a->N + 255) / 256;
-  const bool pair = BN == 256 && a->M > BM && a->max_ctas <= 0 && st::sm_count() >= 2 &&
-                    rounds((long long)((a->M + 2 * BM - 1) / (2 * BM)) * tn * a->batch, st::sm_count() / 2) <=
-                        rounds((long long)((a->M + BM - 1) / BM) * tn * a->batch, st::sm_count());
+  const bool limited = a->max_ctas > 0 && a->max_ctas < st::sm_count();
+  TileChoice tile = choose_tile(a->M, a->N, a->K, a->batch, limited ? a->max_ctas : st::sm_count());
+  if (a->max_ctas > 0) tile.pair = false;      // a limited grid runs beside another kernel: single CTAs find room anywhere
+  const int BN = tile.bn;
+  const bool pair = tile.pair;
   const int b_rows = pair ? BN / 2 : BN;      // rows of B that one CTA loads
 
   CUtensorMap tmA, tmB;

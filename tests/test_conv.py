@@ -99,7 +99,7 @@ def test_classifier_cuda_tracks_cpu():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N,H,W,Cin,OC", [(2, 6, 10, 3, 64), (1, 4, 4, 5, 72), (3, 12, 6, 8, 40), (2, 24, 24, 64, 64), (2, 64, 64, 64, 8)])
+@pytest.mark.parametrize("N,H,W,Cin,OC", [(2, 6, 10, 3, 64), (1, 4, 4, 5, 72), (3, 12, 6, 8, 40), (2, 24, 24, 64, 64), (2, 64, 64, 64, 8), (64, 16, 16, 64, 256), (130, 32, 32, 64, 264)])
 def test_conv_steps_off_the_main_sizes(N, H, W, Cin, OC):
     """Column matrices with odd and vectorised channel counts, output tiles 64 columns wide, the data gradient's weights,
     and the fused pool / ReLU / bias backward."""

@@ -384,3 +384,31 @@ def test_cuda_graph_replay_matches_eager_forward_backward():
     torch.cuda.synchronize()
     assert g.replays == 3
     assert ((a.flat_grad - b.flat_grad).norm() / a.flat_grad.norm()).item() < 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(257, 264, 64), (300, 520, 1000), (129, 2048, 4096), (777, 6144, 2048), (2048, 256, 2304), (1, 8, 8),
+                                   (1536, 512, 192), (640, 1024, 8192)])
+@pytest.mark.parametrize("major", [(False, False), (False, True), (True, False), (True, True)])
+def test_gemm_tile_forms(M, N, K, major):
+    """Every tile width and the CTA pairs, with rows, columns and K blocks that do not fill them, epilogues included: bf16
+    output is one rounding (2^-9) of the fp32 result, gradient accumulation is fp32."""
+    from spiraltorch_b200.ops import gemm as G
+    from spiraltorch_b200.ops import native
+    a_mn, b_mn = major
+    torch.manual_seed(M + N)
+    a = torch.randn(*((K, M) if a_mn else (M, K)), device="cuda").bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device="cuda").bfloat16()
+    bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    y = G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, act="relu", residual=res)
+    want = torch.relu(ref + bias.double()) + res.double()
+    assert ((y - want).norm() / want.norm()).item() < 2.5e-3
+    out = torch.full((M, N), 0.5, device="cuda")
+    G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=True)
+    assert ((out - ref - 0.5).norm() / ref.norm()).item() < 1e-5
+    aux = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    z = G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, aux_out=aux, act="gelu", max_ctas=7 if M < 700 else 0)
+    assert ((aux - ref).norm() / ref.norm()).item() < 2.5e-3
+    assert ((z - torch.nn.functional.gelu(ref, approximate="tanh")).norm() / ref.norm()).item() < 4e-3
+    native.raise_on_device_error()
