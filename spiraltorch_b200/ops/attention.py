@@ -112,9 +112,9 @@ def _bias_args(a, q, k, key_bias, attn_bias, lengths, keep: list) -> None:
 
 
 def set_pair_kernel(on: bool) -> None:
-    """Plain (no bias, no lengths) forward attention runs the pair kernel by default: two 128-row query tiles per
-    CTA share every K / V tile, with the probabilities and the output accumulator in tensor memory.  ``False``
-    selects the single-tile kernel, which the biased / variable-length cases always use."""
+    """Forward attention without a bias per (query, key) runs the pair kernel by default, where its pairs fill the chip:
+    two 128-row query tiles per CTA share every K / V tile, with the probabilities and the output accumulator in tensor
+    memory.  ``False`` selects the single-tile kernel for every case."""
     native.lib().st_attn_fwd_set_pair_kernel(1 if on else 0)
 
 
