@@ -111,6 +111,8 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __rest
 // columns of the block and the rest of the 256 are row lanes, so narrow matrices (64 channels: 8 of 32 threads had
 // columns, 47 us for 134 MB) keep every thread loading.  Four rows are in flight per thread.  Needs cols % 8 == 0 and
 // 16-byte aligned rows.
+// STORE (one chunk of rows only): the sums replace what is there, so the caller needs no cleared output.
+template <bool STORE>
 __global__ void __launch_bounds__(256)
 colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long rows, int cols, long long ld) {
   __shared__ float sh[256 * 8 + 32];
@@ -158,7 +160,9 @@ colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, lon
   float s = 0.0f;
   for (int y = 0; y < lanes; ++y) s += sh[y * (width + 1) + t];
   const int c = blockIdx.x * width + t;
-  if (c < cols) atomicAdd(out + c, s);
+  if (c >= cols) return;
+  if (STORE) out[c] = s;
+  else atomicAdd(out + c, s);
 }
 
 // ------------------------------------------------------------------------------------
@@ -560,7 +564,7 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
     if (chunks > 512) chunks = 512;
     int bx = 8;
     while (bx < 32 && bx * 8 < cols) bx <<= 1;
-    colsum8_kernel<<<dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+    colsum8_kernel<false><<<dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
         static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
@@ -571,6 +575,18 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
   if (chunks > 256) chunks = 256;
   dim3 grid((cols + 31) / 32, chunks);
   colsum_kernel<<<grid, block, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+      static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
+  ST_CUDA_CHECK(cudaGetLastError());
+  return ST_OK;
+}
+
+// out (fp32 [cols]) = column sums of a short matrix: at most 1024 rows, cols and ld multiples of 8, x 16-byte aligned.  One
+// launch and a fixed order of summation, where st_colsum wants a cleared output and joins row chunks with atomics.
+ST_API int st_colsum_short(const void* x, float* out, long long rows, int cols, long long ld, void* stream_v) {
+  if (!x || !out || rows <= 0 || rows > 1024 || cols <= 0 || (cols & 7) || (ld & 7) || (reinterpret_cast<uintptr_t>(x) & 15))
+    return st::fail(ST_ERR_INVALID, "colsum_short: bad arguments");
+  const int bx = 8;       // 32 row lanes per column group, and as many CTAs as the columns give
+  colsum8_kernel<true><<<dim3((cols + bx * 8 - 1) / (bx * 8), 1), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
       static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;

@@ -18,6 +18,7 @@ constexpr int kMultiBlocks = 32;     // blocks per tensor at most; 32 x 256 thre
 struct MultiTable {
   const float* src[kMultiMax];
   float* dst[kMultiMax];
+  __nv_bfloat16* half[kMultiMax];      // STEP: receives the updated values rounded to bf16, or null
   long long n[kMultiMax];
 };
 
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(kMultiThreads)
 multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict__ bad) {
   const float* __restrict__ src = t.src[blockIdx.y];
   float* dst = t.dst[blockIdx.y];
+  __nv_bfloat16* half = OP == MULTI_STEP ? t.half[blockIdx.y] : nullptr;
   const long long n = t.n[blockIdx.y], stride = (long long)gridDim.x * kMultiThreads;
   bool odd = false;
   for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n; i += 4 * stride) {
@@ -42,7 +44,11 @@ multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict_
       if (OP != MULTI_STEP) odd |= !isfinite(v[u]);
       if (at < n) {
         if (OP == MULTI_DIV) dst[at] = __fdiv_rn(v[u], value);
-        if (OP == MULTI_STEP) dst[at] = __fsub_rn(dst[at], __fmul_rn(value, v[u]));
+        if (OP == MULTI_STEP) {
+          const float w = __fsub_rn(dst[at], __fmul_rn(value, v[u]));
+          dst[at] = w;
+          if (half) half[at] = __float2bfloat16(w);
+        }
       }
     }
   }
@@ -137,10 +143,26 @@ int blocks_for(long long n, int most) {
 ST_API int st_multi_max() { return kMultiMax; }
 ST_API int st_multi_blocks(long long most) { return blocks_for(most, kMultiBlocks); }
 
+namespace {
+int run_multi(int op, int count, const void* const* src, void* const* dst, void* const* half, const long long* n, float value,
+              int* bad, void* stream_v);
+}
+
 // op 0: finite check of src; 1: dst = src / value and finite check of src; 2: dst -= value * src.  `bad` (op 0 and 1):
 // count * st_multi_blocks(largest n) ints, tensor by tensor, in memory that the device can write (pinned host memory).
 ST_API int st_multi(int op, int count, const void* const* src, void* const* dst, const long long* n, float value, int* bad,
                     void* stream_v) {
+  return run_multi(op, count, src, dst, nullptr, n, value, bad, stream_v);
+}
+// dst -= value * src, and where half[i] is not null the updated values as bf16 there.
+ST_API int st_multi_step_bf16(int count, const void* const* src, void* const* dst, void* const* half, const long long* n, float value,
+                              void* stream_v) {
+  return run_multi(MULTI_STEP, count, src, dst, half, n, value, nullptr, stream_v);
+}
+
+namespace {
+int run_multi(int op, int count, const void* const* src, void* const* dst, void* const* half, const long long* n, float value,
+              int* bad, void* stream_v) {
   if (count <= 0) return ST_OK;
   if (count > kMultiMax) return st::fail(ST_ERR_TOO_LARGE, "multi: too many tensors for one launch");
   if (op < MULTI_CHECK || op > MULTI_STEP || !src || !n || (op != MULTI_CHECK && !dst) || (op != MULTI_STEP && !bad))
@@ -150,6 +172,7 @@ ST_API int st_multi(int op, int count, const void* const* src, void* const* dst,
   for (int i = 0; i < count; ++i) {
     t.src[i] = static_cast<const float*>(src[i]);
     t.dst[i] = dst ? static_cast<float*>(dst[i]) : nullptr;
+    t.half[i] = half ? static_cast<__nv_bfloat16*>(half[i]) : nullptr;
     t.n[i] = n[i];
     most = n[i] > most ? n[i] : most;
   }
@@ -161,6 +184,8 @@ ST_API int st_multi(int op, int count, const void* const* src, void* const* dst,
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
+
+}  // namespace
 
 // bf16 copies of fp32 tensors; every pointer 16-byte aligned.
 ST_API int st_multi_cast_bf16(int count, const void* const* src, void* const* dst, const long long* n, void* stream_v) {

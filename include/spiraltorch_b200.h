@@ -248,6 +248,7 @@ int st_ce_grad(const void* logits, const long long* target, const float* lse, co
 int st_ce_stats(const void* logits, const long long* target, float* row_max, float* row_sum, float* tgt_logit, long long rows, long long ld, int V, int vocab_start, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_clip_coef(const float* sumsq, float norm_scale, float max_norm, float* coef, float* norm_out, void* stream_v);   /* csrc/optim/optim.cu */
 int st_colsum(const void* x, float* out, long long rows, int cols, long long ld, void* stream_v);   /* csrc/elementwise/elementwise.cu */
+int st_colsum_short(const void* x, float* out, long long rows, int cols, long long ld, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_compact_rows(const float* in, float* out_v, int* out_i, int* counts, int rows, int cols, float low, float high, void* stream_v);   /* csrc/rank/rank.cu */
 int st_contrastive_views(const float* base, const float* n1, const float* n2, float noise, void* out, long long n, void* stream_v);   /* csrc/elementwise/embed.cu */
 int st_conv3x3_dgrad_weights(const void* w, void* wt, int OC, int IC, void* stream_v);   /* csrc/conv/conv.cu */
@@ -284,6 +285,7 @@ int st_multi(int op, int count, const void* const* src, void* const* dst, const 
 int st_multi_blocks(long long most);   /* csrc/elementwise/multi.cu */
 int st_multi_cast_bf16(int count, const void* const* src, void* const* dst, const long long* n, void* stream_v);   /* csrc/elementwise/multi.cu */
 int st_multi_max();   /* csrc/elementwise/multi.cu */
+int st_multi_step_bf16(int count, const void* const* src, void* const* dst, void* const* half, const long long* n, float value, void* stream_v);   /* csrc/elementwise/multi.cu */
 int st_nce_rows(float* s, float* loss, int rows, float temperature, void* stream_v);   /* csrc/elementwise/embed.cu */
 int st_nd_indexer(const unsigned* positions, unsigned* out_index, unsigned* out_segment, long long n, const unsigned* dims4, const unsigned* strides4, unsigned segments, unsigned segment_stride, void* stream_v);   /* csrc/elementwise/elementwise.cu */
 int st_nerf_composite_bwd(const float* sigma, const float* rad, const float* deltas, const float* accum, const float* d_accum, float* d_sigma, float* d_rad, int R, int S, float delta_scale, void* stream_v);   /* csrc/vision/vision.cu */

@@ -130,6 +130,8 @@ class _MovedModule:
 
 
 class Module:
+    _grads_finite = False      # set by backward: every accumulator holds what that call has just checked
+
     def __init__(self):
         self._params: list[Parameter] = []
         self.training = True
@@ -190,6 +192,9 @@ class Module:
         else:
             assert_finite(found, lambda i: f"non-finite gradient for parameter {live[i][0].name}")
             means = [gp / batch for gp in found]
+        # nothing was accumulated before: what follows holds exactly these checked means
+        self._grads_finite = all(type(p) is Parameter and p.gradient is None and p.hypergrad is None and p.realgrad is None
+                                 for p in self.parameters())
         for (p, _), mean in zip(live, means):
             if p.gradient is None and p.hypergrad is None and p.realgrad is None and type(p) is Parameter:
                 p.gradient = mean.reshape(p.value.shape)            # a fresh tensor: nothing to clone

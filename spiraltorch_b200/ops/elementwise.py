@@ -116,6 +116,13 @@ def colsum(x2: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: boo
     """fp32 column sums of a bf16 ``[rows, cols]`` matrix (bias gradients)."""
     global launch_count
     rows, cols = x2.shape
+    if out is None and 0 < rows <= 1024 and cols % 8 == 0 and cols > 0 and native.use_native(x2) and x2.dtype == torch.bfloat16 \
+            and x2.stride(-1) == 1 and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0:
+        out = torch.empty(cols, dtype=torch.float32, device=x2.device)
+        native.check(native.lib().st_colsum_short(native.ptr(x2), native.ptr(out), ctypes.c_longlong(rows), ctypes.c_int(cols),
+                                                  ctypes.c_longlong(x2.stride(0)), native.stream_ptr(x2.device)), "st_colsum_short")
+        launch_count += 1
+        return out
     if out is None:
         out = torch.zeros(cols, dtype=torch.float32, device=x2.device)
     elif not accumulate:

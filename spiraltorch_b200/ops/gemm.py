@@ -140,6 +140,20 @@ def cached_bf16(t: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def has_cached_bf16(t: torch.Tensor) -> bool:
+    """Whether ``t``'s current values have a cached copy."""
+    hit = _bf16_cache.get((t.data_ptr(), tuple(t.shape), tuple(t.stride()), t.dtype, t.device))
+    return hit is not None and hit[0] == t._version
+
+
+def renew_cached_bf16(t: torch.Tensor, copy: torch.Tensor) -> None:
+    """``copy`` holds the bf16 form of ``t``'s values as they are now: it takes the place of the cached one."""
+    key = (t.data_ptr(), tuple(t.shape), tuple(t.stride()), t.dtype, t.device)
+    hit = _bf16_cache.get(key)
+    if hit is not None:
+        _bf16_cache[key] = (t._version, copy, hit[2], hit[3])
+
+
 def clear_bf16_cache() -> None:
     """Drops every cached bf16 copy (CUDA-graph capture calls this so that the casts it needs are captured too)."""
     global _bf16_cache_bytes

@@ -67,9 +67,24 @@ def divided(tensors: Sequence[torch.Tensor], value: float):
 
 def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: float) -> None:
     """``v -= lr * g`` for every pair, in place."""
-    _run(_STEP, grads, values, lr)
-    for v in values:
+    global launch_count
+    from . import gemm
+    lib, stream = native.lib(), native.stream_ptr(values[0].device)
+    # values whose bf16 copy is in use get the next one in the same launch (a new tensor: a graph may still hold the old one)
+    halves = [torch.empty(v.shape, dtype=torch.bfloat16, device=v.device) if gemm.has_cached_bf16(v) else None for v in values]
+    for at in range(0, len(values), _MAX):
+        v, g, h = values[at:at + _MAX], grads[at:at + _MAX], halves[at:at + _MAX]
+        n = len(v)
+        array = ctypes.c_void_p * n
+        native.check(lib.st_multi_step_bf16(
+            ctypes.c_int(n), array(*[t.data_ptr() for t in g]), array(*[t.data_ptr() for t in v]),
+            array(*[None if t is None else t.data_ptr() for t in h]), (ctypes.c_longlong * n)(*[t.numel() for t in v]),
+            ctypes.c_float(lr), stream), "st_multi_step_bf16")
+        launch_count += 1
+    for v, h in zip(values, halves):
         torch.autograd.graph.increment_version(v)      # copies of the values are cached by version
+        if h is not None:
+            gemm.renew_cached_bf16(v, h)
 
 
 def to_bf16(tensors: Sequence[torch.Tensor]):

@@ -501,3 +501,41 @@ def test_recurrent_scans_with_weights_in_registers(cell, B, T, H, dilation):
     assert (h - want).abs().max() <= 1e-4
     for a, r in zip(grads, torch.autograd.grad(want, wide, g.double())):
         assert (a - r).norm() <= 5e-3 * r.norm() + 1e-6
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (33, 72), (1000, 264), (1024, 64)])
+def test_column_sums_of_short_matrices(rows, cols):
+    from spiraltorch_b200.ops import elementwise as E
+    x = torch.randn(rows, cols, device=DEV).bfloat16()
+    s = E.colsum(x)
+    assert torch.allclose(s.double(), x.double().sum(0), rtol=1e-5, atol=1e-4) and torch.equal(s, E.colsum(x))
+
+
+def test_updates_renew_the_cached_bf16_values():
+    """The copy that the next forward reads is that of the updated values, and a graph built before keeps the old one."""
+    from spiraltorch_b200.ops import multi
+    w, other, g = (torch.randn(40, 24, device=DEV) for _ in range(3))
+    old = G.cached_bf16(w)
+    kept = old.clone()
+    multi.descend_([w, other], [g, g], 0.5)
+    new = G.cached_bf16(w)
+    assert torch.equal(old, kept) and new.data_ptr() != old.data_ptr() and torch.equal(new, w.bfloat16())
+    assert not G.has_cached_bf16(other)
+    w.mul_(2.0)                                      # a change the cache has not seen
+    assert not G.has_cached_bf16(w) and torch.equal(G.cached_bf16(w), w.bfloat16())
+
+
+def test_trainer_still_refuses_gradients_that_overflow_in_accumulation():
+    class Doubled(st.nn.Linear):
+        def backward(self, x, grad):
+            out = super().backward(x, grad)
+            self.weight.gradient.mul_(float("inf"))
+            return out
+    lin = Doubled("fc", 8, 8)
+    lin.init_normal(0.1, seed=1)
+    trainer = st.SpiralSession("cuda", seed=1).trainer(fallback_learning_rate=0.1)
+    trainer.prepare(lin)
+    batch = (st.Tensor(torch.randn(16, 8, device=DEV)), st.Tensor(torch.randn(16, 8, device=DEV)))
+    with pytest.raises(Exception, match="non-finite gradient"):
+        trainer.train_epoch(lin, st.nn.MeanSquaredError(), [batch])
+    assert all(p.gradient is None for p in lin.parameters())
