@@ -9,7 +9,7 @@
 //                  — the same kernel on dY with the flipped/transposed weights Wt and the ReLU mask of
 //                  the layer input fused in the epilogue
 //   weight gradient dW[oc, tap, ic] += Σ_p dY[p, oc] · X[p + tap, ic]
-//                  — K runs over pixels, one (tap, K-split) per batch index, fp32 atomics into dW
+//                  — K runs over pixels and N over (tap, ic), one K split per batch index, fp32 atomics into dW
 // The first layer (3 input channels) uses a small explicit im2col (K padded to 32).
 //
 // Pooling: 2x2 max pool forward/backward and global average pool forward/backward on NHWC bf16.
@@ -389,14 +389,35 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "conv3x3_wgrad: image width must divide 64 and the batch must fill whole pixel blocks");
   const int P = a->N * a->H * a->W;
   const int kblocks_total = P / BK;
-  const int BNv = a->C <= 64 ? 64 : (a->C <= 128 ? 128 : 256);
-  const int tiles = ((a->OC + BM - 1) / BM) * ((a->C + BNv - 1) / BNv) * 9;
-  int splits = a->splits;
-  if (splits <= 0) {
-    splits = (2 * st::sm_count() + tiles - 1) / tiles;
-    while (splits > 1 && (kblocks_total % splits != 0 || kblocks_total / splits < 8)) --splits;
+  // One product over N = 9 C columns: a wide tile of them reads dY once where a tile per tap read it nine times (C = 64 in
+  // tiles of 192: 96 KB of loads per 64 pixels instead of 144).  The form (tile width, or pairs over 256 output channels) and
+  // the splits by the cost of a K block as in choose_tile, plus about 6 us of atomics for each tile of an SM.  A caller's own
+  // split count fixes the summation order with one CTA per tile and split; narrow tiles then keep more SMs at work.
+  // Measured, with a tile per tap and now: 256 x 64 x 64 pixels, C = OC = 64: 240 -> 115 us (672 TFLOP/s; half of the 128
+  // rows of a tile are padding); 256 x 32 x 32, 128 to 128: 134 -> 66; 256 x 16 x 16, 256 to 256: 86 -> 55 (1399 TFLOP/s).
+  struct Form { int bn, rows, sms; double c; };
+  static const Form forms[4] = {{192, BM, 1, 0.33}, {256, BM, 1, 0.40}, {256, 2 * BM, 2, 0.33}, {64, BM, 1, 0.228}};
+  const long long N9 = 9ll * a->C;
+  int splits = a->splits, form = 0;
+  if (splits > 0) {
+    if (kblocks_total % splits != 0) return st::fail(ST_ERR_INVALID, "conv3x3_wgrad: splits must divide the pixel blocks");
+    form = a->C <= 192 ? 3 : 1;
+  } else {
+    double best = 1e30;
+    const long long most = kblocks_total / 8 > 0 ? kblocks_total / 8 : 1;      // at least eight K blocks per split
+    for (int f = 0; f < 4; ++f) {
+      if (forms[f].rows > BM && a->OC <= BM) continue;
+      const long long tiles = (a->OC + forms[f].rows - 1) / forms[f].rows * ((N9 + forms[f].bn - 1) / forms[f].bn);
+      const int at_once = st::sm_count() / forms[f].sms;
+      for (int r = 1; r <= 3; ++r) {
+        long long n = (long long)r * at_once / tiles;
+        n = n < 1 ? 1 : (n > most ? most : n);
+        const double rounds = (double)((tiles * n + at_once - 1) / at_once);
+        const double t = rounds * ((double)((kblocks_total + n - 1) / n) * forms[f].c + 6.0);
+        if (t < best) { best = t; splits = (int)n; form = f; }
+      }
+    }
   }
-  if (kblocks_total % splits != 0) return st::fail(ST_ERR_INVALID, "conv3x3_wgrad: splits must divide the pixel blocks");
   CUtensorMap tmA, tmB;
   {
     uint64_t dims[3] = {(uint64_t)a->OC, (uint64_t)P, 1};
@@ -411,15 +432,16 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
   GemmParams p{};
   p.conv.mode = 2;
   p.conv.H = a->H; p.conv.W = a->W; p.conv.Hb = Hb; p.conv.Nb = Nb;
-  p.conv.c_chunks = a->C / 64; p.conv.taps = 9;
-  p.C = a->dw; p.ldc = 9ll * a->C;
-  p.M = a->OC; p.N = a->C; p.K = (kblocks_total / splits) * BK;
-  p.alpha = 1.0f; p.batch = 9 * splits; p.batch_stride_c = a->C;
+  p.conv.c_chunks = a->C / 64; p.conv.taps = 9; p.conv.blocks = kblocks_total;
+  p.C = a->dw; p.ldc = N9;
+  p.M = a->OC; p.N = (int)N9; p.K = P;
+  p.alpha = 1.0f; p.batch = splits; p.batch_stride_c = 0;
   p.out_fp32 = 1; p.accumulate = 2;
   p.err = st::error_word();
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (BNv == 64) return launch_gemm<64, 8, true, true>(tmA, tmB, tmC, p, s);
-  if (BNv == 128) return launch_gemm<128, 6, true, true>(tmA, tmB, tmC, p, s);
+  if (form == 0) return launch_gemm<192, 4, true, true>(tmA, tmB, tmC, p, s);
+  if (form == 2) return launch_pair<true, true>(tmA, tmB, tmC, p, s);
+  if (form == 3) return launch_gemm<64, 8, true, true>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, true, true>(tmA, tmB, tmC, p, s);
 }
 

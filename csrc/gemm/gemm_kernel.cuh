@@ -69,14 +69,16 @@ struct GemmComm {
 //   mode 1 (forward / data gradient): the A tile of 128 output pixels is a 4-D TMA box
 //          {64 channels, W, Hb, Nb} taken at the tap's (kh-1, kw-1) offset; pixels outside the image
 //          are zero-filled by TMA.  K = 9 * C runs tap-major, matching weights stored [OC][tap][C].
-//   mode 2 (weight gradient): K runs over pixels; the B tile (64 pixels x 64-channel blocks of the
-//          shifted input) is the 4-D box, A is dYᵀ; the batch index enumerates (tap, K split).
+//   mode 2 (weight gradient): K runs over pixels, N over (tap, channel); the B tile is a row of 4-D boxes, one per
+//          64 columns (64 pixels x 64 channels of the input shifted by the column's tap), A is dYᵀ; the batch index
+//          is the K split, whose share of the pixel blocks need not be the same for all.
 struct ConvGeom {
   int mode;
   int H, W;          // image size
   int Hb, Nb;        // rows / images per pixel block (mode 1: 128 pixels, mode 2: 64 pixels)
-  int c_chunks;      // input channels / 64 (mode 1)
+  int c_chunks;      // input channels / 64
   int taps;          // 9
+  int blocks;        // pixel blocks over all splits (mode 2)
 };
 
 struct GemmParams {
@@ -248,6 +250,12 @@ __device__ __forceinline__ void epilogue_bar() {
   asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
+// Pixel blocks of split b of a convolution's weight gradient
+__device__ __forceinline__ int split_begin(const GemmParams& p, int b) {
+  return static_cast<int>((long long)p.conv.blocks * b / p.batch);
+}
+__device__ __forceinline__ int split_blocks(const GemmParams& p, int b) { return split_begin(p, b + 1) - split_begin(p, b); }
+
 // CG = 2 (COMM_NONE only): a cluster of two CTAs works on one tile of 256 x BN.  Each CTA brings its 128 rows of A and its half
 // of B into its own shared memory, the even CTA's MMA warp issues for both, and each CTA's epilogue stores its own 128 rows.
 // A K block then costs an SM 32 KB of loads instead of 48 (BN = 256), and the ring holds six stages instead of four.
@@ -329,8 +337,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // The whole warp walks the schedule and one lane issues.  With warp-uniform control flow the loop's addresses and
     // coordinates sit in uniform registers, which TMA and tcgen05 instructions read; issued from inside a one-lane
     // branch, with descriptors rebuilt per instruction, these two loops set the pace of short or narrow K blocks: the weight
-    // gradient of a 64-channel 3x3 convolution over a million pixels took 315 us and takes 240, a training step of the
-    // conv classifier (256 x 64 x 64) 2.55 ms and takes 2.27.  Wide products of the language models did not change.
+    // gradient of a 64-channel 3x3 convolution over a million pixels, in tiles of 64 columns, went from 315 to 240 us (its
+    // wider tiles of today take 115), a training step of the conv classifier (256 x 64 x 64) from 2.55 to 2.27 ms.  Wide products of the language models did not change.
     const bool leader = COMM == COMM_AG ? lane == 0 : elect_one();
     const uint32_t smem0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const uint32_t full0 = __shfl_sync(0xffffffffu, smem_u32(full_bar), 0);
@@ -364,9 +372,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         if (leader) fence_proxy_async_global();
       }
+      const int k_count = A_MN && B_MN && p.conv.mode == 2 ? split_blocks(p, b) : k_blocks;
       // one K block per ring stage: wait until its MMAs have read it, then hand the copies to the TMA unit
       auto k_loop = [&](uint32_t bytes, auto&& copies) {
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        for (int kb = 0; kb < k_count; ++kb) {
           if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u, abort_flag)) return false;
           const uint32_t fb = CG == 2 ? (full0 + stage * 8) & kPairLeaderMask : full0 + stage * 8;
           const uint32_t sa = smem0 + stage * L::STAGE_BYTES;
@@ -411,11 +420,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         });
       } else if (A_MN && B_MN && p.conv.mode == 2) {
-        // batch index = tap + taps * split; K block = 64 consecutive pixels
-        const int tap = b % p.conv.taps, hblocks = p.conv.H / p.conv.Hb;
-        int pix_block = (b / p.conv.taps) * k_blocks;
+        // K block = 64 consecutive pixels; each 64 columns of B are one tap and channel block
+        const int hblocks = p.conv.H / p.conv.Hb;
+        int tap_w[BNC / 64], tap_h[BNC / 64], chan[BNC / 64];
+#pragma unroll
+        for (int j = 0; j < BNC / 64; ++j) {
+          const int col = n0 / 64 + j, tap = col / p.conv.c_chunks;
+          chan[j] = (col - tap * p.conv.c_chunks) * 64;
+          tap_w[j] = tap % 3 - 1;
+          tap_h[j] = tap / 3 - 1;
+        }
+        int pix_block = split_begin(p, b);
         int img = (pix_block / hblocks) * p.conv.Nb, h0 = (pix_block % hblocks) * p.conv.Hb;
-        const int tap_w = tap % 3 - 1, tap_h = tap / 3 - 1;
         ok = k_loop(stage_bytes, [&](int, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (leader) {
 #pragma unroll
@@ -423,7 +439,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               if (j < boxes_a) load3(sa + j * (64 * BK * 2), mapA, fb, m_coord + 64 * j, pix_block * BK, 0);
 #pragma unroll
             for (int j = 0; j < BNC / 64; ++j)
-              if (j < boxes_b) load4(sb + j * (64 * BK * 2), &tmB, fb, n0 + 64 * j, tap_w, h0 + tap_h, img);
+              if (j < boxes_b) load4(sb + j * (64 * BK * 2), &tmB, fb, chan[j], tap_w[j], h0 + tap_h[j], img);
           }
           ++pix_block;
           h0 += p.conv.Hb;
@@ -490,7 +506,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait_warp(tempty0 + acc * 8, acc_phase ^ 1u, abort_flag)) break;
       tc_fence_after();
       const uint32_t tmem_d = tmem0 + acc * BN;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      const int k_count = A_MN && B_MN && p.conv.mode == 2 ? split_blocks(p, t / tiles_per_batch) : k_blocks;
+      for (int kb = 0; kb < k_count; ++kb) {
         if (!mbar_wait_warp(full0 + stage * 8, phase, abort_flag)) {
           ok = false;
           break;
@@ -506,7 +523,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               umma_bf16_ss_split(tmem_d, a_lo + k * a_step, desc_hi, b_lo + k * b_step, desc_hi, idesc, (kb | k) != 0 ? 1u : 0u);
           // frees the smem stage (of both CTAs) when the MMAs finish
           if constexpr (CG == 2) umma_commit_pair(empty0 + stage * 8); else umma_commit(empty0 + stage * 8);
-          if (kb + 1 == k_blocks) {
+          if (kb + 1 == k_count) {
             if constexpr (CG == 2) umma_commit_pair(tfull0 + acc * 8); else umma_commit(tfull0 + acc * 8);
           }
         }
@@ -557,8 +574,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int row = m0 + quad * 32 + lane;
       const bool row_ok = row < p.M;
       void* c_ptr = p.C;
-      const int cbatch = (p.conv.mode == 2) ? (b % p.conv.taps) : b;
-      long long c_base = (long long)cbatch * p.batch_stride_c + (long long)row * p.ldc;
+      long long c_base = (long long)b * p.batch_stride_c + (long long)row * p.ldc;
       int owner = 0;
       bool local_tile = false;
       int n_srcs = 0;             // RS local tile: staged partials + residual to add

@@ -148,3 +148,23 @@ def test_column_sums_of_narrow_matrices(rows, cols):
     from spiraltorch_b200.ops import elementwise as E
     x = torch.randn(rows, cols, device="cuda").bfloat16()
     assert torch.allclose(E.colsum(x).double(), x.double().sum(0), rtol=1e-5, atol=1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,H,W,Cin,OC", [(1, 8, 8, 64, 64), (3, 16, 16, 64, 72), (5, 32, 32, 128, 200), (7, 16, 16, 128, 320), (2, 8, 64, 320, 136)])
+def test_weight_gradient_over_taps_and_channels(monkeypatch, N, H, W, Cin, OC):
+    """Columns run over (tap, channel), so tiles of 192 and 256 cross taps and end past the last one, and the pixel splits
+    need not be equal; the caller's fixed order takes the narrow tiles."""
+    torch.manual_seed(OC + N)
+    x, dy = torch.randn(N, H, W, Cin).bfloat16(), torch.randn(N, H, W, OC).bfloat16()
+    want = torch.zeros(OC, 9 * Cin, dtype=torch.float64)
+    xp = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1))
+    for tap in range(9):
+        shifted = xp[:, tap // 3:tap // 3 + H, tap % 3:tap % 3 + W]
+        want[:, tap * Cin:(tap + 1) * Cin] = dy.double().reshape(-1, OC).t() @ shifted.reshape(-1, Cin)
+    bound = N * H * W * 2.0 ** -24 * 4 * (N * H * W) ** 0.5          # fp32 sums of about sqrt(pixels), one rounding per term
+    for fixed in ("0", "1"):
+        monkeypatch.setenv("SPIRAL_DETERMINISTIC_REDUCTION", fixed)
+        got = torch.zeros(OC, 9 * Cin, device="cuda")
+        C.conv3x3_wgrad(dy.cuda(), x.cuda(), got)
+        assert (got.cpu().double() - want).abs().max().item() <= bound
