@@ -81,9 +81,10 @@ class ConvClassifier(nn.Module):
         P = self.p
         x = images.to(self.flat_w.device, self.dtype).permute(0, 2, 3, 1).contiguous()
         acts, pools = [x], []
+        col = C.im2col(x, STAGES[0])                # the stem's column matrix, kept for its weight gradient
         for s in range(4):
             for i in range(2):
-                x = C.conv3x3(x, P[f"conv{s}_{i}.weight"], P[f"conv{s}_{i}.bias"], relu=True)
+                x = C.conv3x3(x, P[f"conv{s}_{i}.weight"], P[f"conv{s}_{i}.bias"], relu=True, col=col if s + i == 0 else None)
                 acts.append(x)
             x, idx = C.maxpool2(x)
             pools.append((idx, acts[-1].shape[1], acts[-1].shape[2]))
@@ -119,7 +120,7 @@ class ConvClassifier(nn.Module):
                 xin = acts[k - 1]
                 w = P[f"conv{s}_{i}.weight"]
                 ic = xin.shape[-1]
-                C.conv3x3_wgrad(d, xin, w.main_grad)
+                C.conv3x3_wgrad(d, xin, w.main_grad, col if s + i == 0 else None)
                 if i == 0:
                     ew.colsum(d.reshape(-1, d.shape[-1]), P[f"conv{s}_0.bias"].main_grad, accumulate=True)
                 if k - 1 > 0:

@@ -69,6 +69,22 @@ def implicit_ok(N: int, H: int, W: int, C: int, OC: int, pixels: int = 128) -> b
     return H % hb == 0 and N % nb == 0
 
 
+def im2col(x: torch.Tensor, OC: int) -> Optional[torch.Tensor]:
+    """The column matrix that :func:`conv3x3` and :func:`conv3x3_wgrad` both build where the implicit kernels do not take the
+    geometry, for a caller that runs both on the same input; None where neither needs it."""
+    global launch_count
+    N, H, W, C = x.shape
+    if not native.use_native(x) or (implicit_ok(N, H, W, C, OC, 128) and implicit_ok(N, H, W, C, OC, 64)):
+        return None
+    kpad = (9 * C + 31) // 32 * 32
+    col = torch.empty((N * H * W, kpad), dtype=torch.bfloat16, device=x.device)
+    native.check(native.lib().st_im2col3x3_small(native.ptr(x), native.ptr(col), ctypes.c_int(N), ctypes.c_int(H), ctypes.c_int(W),
+                                                 ctypes.c_int(C), ctypes.c_int(kpad), native.stream_ptr(x.device)),
+                 "st_im2col3x3_small")
+    launch_count += 1
+    return col
+
+
 def _conv_ref(x, w_tap, bias, act, aux_in):
     N, H, W, C = x.shape
     oc = w_tap.shape[0]
@@ -83,10 +99,10 @@ def _conv_ref(x, w_tap, bias, act, aux_in):
 
 
 def conv3x3(x: torch.Tensor, w_tap: torch.Tensor, bias: Optional[torch.Tensor] = None, *, relu: bool = False,
-            relu_mask_of: Optional[torch.Tensor] = None) -> torch.Tensor:
+            relu_mask_of: Optional[torch.Tensor] = None, col: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x`` NHWC ``[N,H,W,C]``, ``w_tap`` ``[OC, 9*C]`` → NHWC ``[N,H,W,OC]``.
     ``relu_mask_of`` (same shape as the output) zeroes the output where that tensor is <= 0
-    (used by the data gradient)."""
+    (used by the data gradient).  ``col``: :func:`im2col` of ``x``, if the caller has it."""
     global launch_count
     N, H, W, C = x.shape
     OC = w_tap.shape[0]
@@ -101,12 +117,8 @@ def conv3x3(x: torch.Tensor, w_tap: torch.Tensor, bias: Optional[torch.Tensor] =
         # few input channels (the RGB stem) or a geometry the 4-D TMA boxes cannot tile: explicit im2col
         # with K padded to a multiple of 32, then the plain GEMM
         kpad = (9 * C + 31) // 32 * 32
-        col = torch.empty((N * H * W, kpad), dtype=torch.bfloat16, device=x.device)
-        st = native.lib().st_im2col3x3_small(native.ptr(x), native.ptr(col), ctypes.c_int(N), ctypes.c_int(H),
-                                             ctypes.c_int(W), ctypes.c_int(C), ctypes.c_int(kpad),
-                                             native.stream_ptr(x.device))
-        native.check(st, "st_im2col3x3_small")
-        launch_count += 1
+        if col is None:
+            col = im2col(x, OC)
         wp = torch.zeros((OC, kpad), dtype=torch.bfloat16, device=x.device)
         wp[:, : 9 * C] = w_tap
         if relu_mask_of is not None:
@@ -125,8 +137,9 @@ def conv3x3(x: torch.Tensor, w_tap: torch.Tensor, bias: Optional[torch.Tensor] =
     return y
 
 
-def conv3x3_wgrad(dy: torch.Tensor, x: torch.Tensor, dw_tap: torch.Tensor) -> None:
-    """``dw_tap[oc, tap, ic] += sum_p dy[p, oc] * x[p + tap, ic]`` (fp32 accumulation)."""
+def conv3x3_wgrad(dy: torch.Tensor, x: torch.Tensor, dw_tap: torch.Tensor, col: Optional[torch.Tensor] = None) -> None:
+    """``dw_tap[oc, tap, ic] += sum_p dy[p, oc] * x[p + tap, ic]`` (fp32 accumulation).
+    ``col``: :func:`im2col` of ``x``, if the caller has it."""
     global launch_count
     N, H, W, C = x.shape
     OC = dy.shape[-1]
@@ -139,13 +152,8 @@ def conv3x3_wgrad(dy: torch.Tensor, x: torch.Tensor, dw_tap: torch.Tensor) -> No
     assert dw_tap.dtype == torch.float32 and dw_tap.is_contiguous() and dw_tap.numel() == OC * 9 * C
     assert dy.shape[:3] == x.shape[:3] and dy.is_contiguous() and x.is_contiguous()
     if not implicit_ok(N, H, W, C, OC, 64):
-        kpad = (9 * C + 31) // 32 * 32
-        col = torch.empty((N * H * W, kpad), dtype=torch.bfloat16, device=x.device)
-        st = native.lib().st_im2col3x3_small(native.ptr(x), native.ptr(col), ctypes.c_int(N), ctypes.c_int(H),
-                                             ctypes.c_int(W), ctypes.c_int(C), ctypes.c_int(kpad),
-                                             native.stream_ptr(x.device))
-        native.check(st, "st_im2col3x3_small")
-        launch_count += 1
+        if col is None:
+            col = im2col(x, OC)
         tmp = gemm(dy.reshape(-1, OC), col, a_mn=True, b_mn=True, out_dtype=torch.float32)
         dw_tap += tmp[:, : 9 * C]
         return

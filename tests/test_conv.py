@@ -168,3 +168,14 @@ def test_weight_gradient_over_taps_and_channels(monkeypatch, N, H, W, Cin, OC):
         got = torch.zeros(OC, 9 * Cin, device="cuda")
         C.conv3x3_wgrad(dy.cuda(), x.cuda(), got)
         assert (got.cpu().double() - want).abs().max().item() <= bound
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,H,W,Cin", [(1, 1, 1, 3), (2, 5, 51, 1), (3, 7, 13, 2), (1, 16, 16, 3), (2, 9, 29, 3), (3, 10, 9, 4)])
+def test_column_matrix_of_images(N, H, W, Cin):
+    """Pixels that do not fill the last block, borders on every side, channel counts with and without padding: exact copies."""
+    x = torch.randn(N, H, W, Cin, device="cuda").bfloat16()
+    col = C.im2col(x, 64).float().cpu()
+    want = torch.nn.functional.unfold(x.float().cpu().permute(0, 3, 1, 2), 3, padding=1)
+    want = want.reshape(N, Cin, 9, H * W).permute(0, 3, 2, 1).reshape(N * H * W, 9 * Cin)
+    assert torch.equal(col[:, :9 * Cin], want) and not col[:, 9 * Cin:].any()
