@@ -17,7 +17,7 @@
 // Reference parity: fused_im2col_matmul.wgsl, fused_grad_input_col2im.wgsl (crates/st-tensor/src/
 // wgpu_shaders), CPU im2col path of crates/st-nn/src/layers/conv.rs:607-1017, pooling entry points
 // of tensor_utils.wgsl.
-#include "../gemm/gemm_kernel.cuh"
+#include "conv_halo.cuh"
 #include <cstring>
 
 namespace {
@@ -370,6 +370,43 @@ struct StConvArgs {
   int act;             // 0 none, 1 relu, 4 relu_bwd(aux_in)
 };
 
+// Plan of the shared-row form (conv_halo.cuh): false where the geometry or the shared memory does not allow it.  `us` is its
+// modelled time, about 4.2 (64 channels) or 5.5 us plus 1.0 us for every box of rows that an SM walks.  It loses where tiles
+// of 256 pixels leave most SMs without one: 1 x 32 x 32, 64 to 128 channels, takes 8.7 us and 7.0 in 16 tiles of 128 x 64;
+// 24 x 32 x 32, 128 to 128: 12.2 and 16.6; 256 x 32 x 32: 57 and 87; 256 x 64 x 64, 64 to 64: 88 and 149 (data gradient 93
+// and 161).
+struct HaloPlan {
+  int bn, resident, smem;
+  double us;
+  st::conv::HaloParams p;
+};
+static bool halo_plan(const StConvArgs* a, HaloPlan* out) {
+  using namespace st::conv;
+  if (a->OC > 128 || (reinterpret_cast<uintptr_t>(a->aux_in) & 15) != 0 || a->W < 8 || kHaloPixels % a->W != 0) return false;
+  const int rows = kHaloPixels / a->W;
+  if (a->H % rows != 0) return false;
+  HaloPlan& h = *out;
+  h.bn = a->OC <= 64 ? 64 : 128;
+  const int b_tile = h.bn * BK * 2, a_bytes = (rows + 2) * a->W * BK * 2, fixed = kHaloCStage + kHaloTail;
+  h.resident = a->C == 64 && h.bn == 64 && 9 * b_tile + 2 * a_bytes + fixed <= kSmemLimit;
+  const int base = fixed + (h.resident ? 9 * b_tile : 0), stage = a_bytes + (h.resident ? 0 : 3 * b_tile);
+  int stages = (kSmemLimit - base) / stage;
+  if (stages < 2) return false;
+  if (stages > kHaloMaxStages) stages = kHaloMaxStages;
+  h.smem = base + stages * stage;
+  h.p = HaloParams{};
+  h.p.hblocks = a->H / rows;
+  h.p.tiles = a->N * h.p.hblocks;
+  h.p.rows = rows; h.p.W = a->W;
+  h.p.chunks = a->C / 64; h.p.C = a->C; h.p.OC = a->OC;
+  h.p.act = a->act; h.p.stages = stages;
+  h.p.bias = static_cast<const __nv_bfloat16*>(a->bias);
+  h.p.aux_in = static_cast<const __nv_bfloat16*>(a->aux_in);
+  h.p.err = st::error_word();
+  h.us = (h.bn == 64 ? 4.2 : 5.5) + 3.0 * h.p.chunks * ((h.p.tiles + st::sm_count() - 1) / st::sm_count());
+  return true;
+}
+
 ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   if (!a || !a->x || !a->w || !a->y) return st::fail(ST_ERR_INVALID, "conv3x3: null pointer");
   if (a->C % 64 != 0) return st::fail(ST_ERR_INVALID, "conv3x3: input channels must be a multiple of 64");
@@ -379,13 +416,16 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "conv3x3: image width must divide 128 and the batch must fill whole pixel blocks");
   const int P = a->N * a->H * a->W;
   CUtensorMap tmA, tmB;
-  if (!nhwc_map(&tmA, a->x, a->N, a->H, a->W, a->C, a->W, Hb, Nb)) return ST_ERR_CUDA;
   const TileChoice tile = choose_tile(P, a->OC, 9ll * a->C, 1, st::sm_count());
-  const int BN = tile.bn;
+  HaloPlan halo;
+  const bool use_halo = halo_plan(a, &halo) && halo.us <= tile.us;
+  const int BN = use_halo ? halo.bn : tile.bn;
+  const bool pair = tile.pair && !use_halo;
+  if (!nhwc_map(&tmA, a->x, a->N, a->H, a->W, a->C, a->W, use_halo ? halo.p.rows + 2 : Hb, use_halo ? 1 : Nb)) return ST_ERR_CUDA;
   {
     uint64_t dims[3] = {(uint64_t)9 * a->C, (uint64_t)a->OC, 1};
     uint64_t strides[2] = {(uint64_t)9 * a->C * 2, (uint64_t)9 * a->C * 2 * a->OC};
-    uint32_t box[3] = {BK, (uint32_t)(tile.pair ? BN / 2 : BN), 1};
+    uint32_t box[3] = {BK, (uint32_t)(pair ? BN / 2 : BN), 1};
     if (!encode_tmap(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
   }
@@ -397,6 +437,12 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
     uint32_t box[3] = {64, 32, 1};
     if (!encode_tmap(&tmC.m[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->y, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
+  }
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  if (use_halo) {
+    if (halo.resident) return st::conv::launch_halo<64, true>(tmA, tmB, tmC.m[0], halo.p, halo.smem, s);
+    if (BN == 64) return st::conv::launch_halo<64, false>(tmA, tmB, tmC.m[0], halo.p, halo.smem, s);
+    return st::conv::launch_halo<128, false>(tmA, tmB, tmC.m[0], halo.p, halo.smem, s);
   }
   GemmParams p{};
   p.conv.mode = 1;
@@ -410,8 +456,7 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   p.alpha = 1.0f; p.act = a->act; p.batch = 1;
   p.use_tma_store = 1;
   p.err = st::error_word();
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (tile.pair) return launch_pair<false, false>(tmA, tmB, tmC, p, s);
+  if (pair) return launch_pair<false, false>(tmA, tmB, tmC, p, s);
   if (BN == 64) return launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s);
   if (BN == 128) return launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, false, false>(tmA, tmB, tmC, p, s);

@@ -1045,6 +1045,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 struct TileChoice {
   int bn;
   bool pair;
+  double us;      // modelled time
 };
 inline TileChoice choose_tile(long long M, long long N, long long K, long long batch, int ctas) {
   const long long kb = (K + BK - 1) / BK;
@@ -1052,17 +1053,17 @@ inline TileChoice choose_tile(long long M, long long N, long long K, long long b
   auto cost = [&](int bm, int bn, long long at_once, double a, double c) {
     return a + c * (double)(rounds(((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch, at_once) * kb);
   };
-  TileChoice best{64, false};
   double t = cost(BM, 64, ctas, 5.0, 0.228);
+  TileChoice best{64, false, t};
   if (N > 64) {
     const double u = cost(BM, 128, ctas, 5.6, 0.262);
-    if (u <= t) { t = u; best = {128, false}; }
+    if (u <= t) { t = u; best = {128, false, u}; }
   }
   if (N > 128) {
     const double u = cost(BM, 256, ctas, 4.1, 0.40);
-    if (u <= t) { t = u; best = {256, false}; }
+    if (u <= t) { t = u; best = {256, false, u}; }
     const double w = M > BM && ctas >= 2 ? cost(2 * BM, 256, ctas / 2, 7.6, 0.33) : 1e30;
-    if (w < t) best = {256, true};
+    if (w < t) best = {256, true, w};
   }
   return best;
 }

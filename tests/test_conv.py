@@ -179,3 +179,20 @@ def test_column_matrix_of_images(N, H, W, Cin):
     want = torch.nn.functional.unfold(x.float().cpu().permute(0, 3, 1, 2), 3, padding=1)
     want = want.reshape(N, Cin, 9, H * W).permute(0, 3, 2, 1).reshape(N * H * W, 9 * Cin)
     assert torch.equal(col[:, :9 * Cin], want) and not col[:, 9 * Cin:].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,H,W,Cin,OC", [(80, 4, 64, 64, 64), (5, 64, 64, 64, 8), (80, 8, 32, 128, 64), (80, 16, 16, 192, 72),
+                                          (80, 32, 8, 64, 128), (30, 6, 128, 64, 64), (40, 4, 128, 64, 128), (40, 32, 32, 64, 128)])
+def test_conv_with_shared_row_blocks(N, H, W, Cin, OC):
+    """Up to 128 output channels over whole tiles of 256 pixels: resident and streamed weights, every width, channels that do
+    not fill the tile, one and several tiles per SM, and both epilogues; the seventh does not fit in shared memory."""
+    torch.manual_seed(H * W + OC)
+    x = torch.randn(N, H, W, Cin).bfloat16()
+    w = (torch.randn(OC, 9 * Cin) * (9 * Cin) ** -0.5).bfloat16()
+    bias, mask = torch.randn(OC).bfloat16(), torch.randn(N, H, W, OC).bfloat16()
+    want = C._conv_ref(x.float(), w.float(), None, 0, None)
+    for act, got in (("relu", C.conv3x3(x.cuda(), w.cuda(), bias.cuda(), relu=True)), ("mask", C.conv3x3(x.cuda(), w.cuda(), relu_mask_of=mask.cuda()))):
+        ref = torch.relu(want + bias.float()) if act == "relu" else torch.where(mask.float() > 0, want, torch.zeros(()))
+        err = (got.float().cpu() - ref).abs()
+        assert (err <= 2.0 ** -8 * ref.abs() + 1e-4).all()            # one bf16 rounding, fp32 sums of terms of order one
