@@ -611,16 +611,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // loads left this bandwidth-bound pass at a quarter of the copy rate.
 // With F32 the gradient arrives in fp32: this pass also writes the bf16 form that the tensor cores read (strides do_*) and
 // takes the products with it.
-template <int D, bool F32>
+// Index is 32-bit wherever the row count allows it: with 64-bit divisions 8 x 2048 x 16 rows of 128 took 38.5 us,
+// with 32-bit ones 35.1 (20.5 of bytes).
+template <int D, bool F32, typename Index>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ O, __nv_bfloat16* __restrict__ dO, const float* __restrict__ dO32,
                   float* __restrict__ delta, int B, int S, int H, long long o_sb, long long o_ss, long long o_sh,
                   long long do_sb, long long do_ss, long long do_sh) {
   constexpr int LPR = D / 8;                       // lanes per row
-  const long long total = (long long)B * S * H;
+  const Index total = (Index)B * S * H;
   const int sub = threadIdx.x % LPR;
-  const long long stride = (long long)gridDim.x * (blockDim.x / LPR);
-  for (long long w = blockIdx.x * (long long)(blockDim.x / LPR) + threadIdx.x / LPR; ; w += stride) {
+  const Index stride = (Index)gridDim.x * (blockDim.x / LPR);
+  for (Index w = blockIdx.x * (Index)(blockDim.x / LPR) + threadIdx.x / LPR; ; w += stride) {
     // every lane of a warp takes the same number of trips: the shuffles below need the full warp
     const bool live = w < total;
     if (!__any_sync(0xffffffffu, live)) break;
@@ -628,14 +630,14 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ O, __nv_bfloat16* __restrict
     int hh = 0, s = 0, bb = 0;
     if (live) {
       hh = (int)(w % H);
-      const long long bs = w / H;
+      const Index bs = w / H;
       s = (int)(bs % S);
       bb = (int)(bs / S);
       const uint4 a = *reinterpret_cast<const uint4*>(O + bb * o_sb + s * o_ss + hh * o_sh + sub * 8);
       __nv_bfloat16* gp = dO + bb * do_sb + s * do_ss + hh * do_sh + sub * 8;
       uint4 g;
       if constexpr (F32) {
-        const float4* src = reinterpret_cast<const float4*>(dO32 + w * D + sub * 8);
+        const float4* src = reinterpret_cast<const float4*>(dO32 + (long long)w * D + sub * 8);
         const float4 u = src[0], v = src[1];
         g = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
         *reinterpret_cast<uint4*>(gp) = g;
@@ -701,8 +703,13 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
       kernel<<<(unsigned)blocks, 256, 0, s>>>(Op, dOp, dO32, a->delta, a->B, a->Sq, a->H, a->o_sb, a->o_ss, a->o_sh, a->do_sb,
                                               a->do_ss, a->do_sh);
     };
-    if (a->D == 128) { if (dO32) delta(attn_delta_kernel<128, true>); else delta(attn_delta_kernel<128, false>); }
-    else { if (dO32) delta(attn_delta_kernel<64, true>); else delta(attn_delta_kernel<64, false>); }
+    const bool narrow = rows + blocks * rows_per_block < (1ll << 31);      // the last step's index must not wrap either
+    auto pick = [&](auto d) {
+      constexpr int D = decltype(d)::value;
+      if (narrow) { if (dO32) delta(attn_delta_kernel<D, true, unsigned>); else delta(attn_delta_kernel<D, false, unsigned>); }
+      else { if (dO32) delta(attn_delta_kernel<D, true, long long>); else delta(attn_delta_kernel<D, false, long long>); }
+    };
+    if (a->D == 128) pick(std::integral_constant<int, 128>{}); else pick(std::integral_constant<int, 64>{});
     ST_CUDA_CHECK(cudaGetLastError());
   }
 
