@@ -48,7 +48,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, c
     ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     configured[dev] = true;
   }
-  kern<<<grid, COMM == COMM_AG ? NUM_THREADS_AG : NUM_THREADS, SMEM, stream>>>(tmA, tmB, tmC, tmA_local, p, cm);
+  kern<<<grid, COMM == COMM_AG ? NUM_THREADS_AG : COMM == COMM_RS ? NUM_THREADS_RS : NUM_THREADS, SMEM, stream>>>(tmA, tmB, tmC, tmA_local, p, cm);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }

@@ -30,7 +30,8 @@ namespace gemm {
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int NUM_THREADS = 192;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: epilogue
+constexpr int NUM_THREADS = 320;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-9: epilogue, two per 32 lanes
+constexpr int NUM_THREADS_RS = 192;  // reduce-scatter variant: one epilogue warp per 32 lanes
 constexpr int NUM_THREADS_AG = 256;  // all-gather variant: + warp 6 (shard push) and warp 7 (arrival publisher)
 constexpr int AG_RING_CHUNK = 16384;  // bytes per bulk copy of the push ring
 constexpr int AG_RING_SLOTS = 3;      // the ring sits behind the barriers of the 3-stage GEMM layout
@@ -113,7 +114,7 @@ struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int CSTAGE_OFFSET = STAGES * STAGE_BYTES;       // 4 warps x 2 buffers x 4 KiB
+  static constexpr int CSTAGE_OFFSET = STAGES * STAGE_BYTES;       // one 4 KiB block per epilogue warp (two of four warps)
   static constexpr int CSTAGE_BYTES = 4 * 2 * 4096;
   static constexpr int BAR_OFFSET = CSTAGE_OFFSET + CSTAGE_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;  // barriers + alignment slack
@@ -260,12 +261,19 @@ __device__ __forceinline__ int split_blocks(const GemmParams& p, int b) { return
 // of B into its own shared memory, the even CTA's MMA warp issues for both, and each CTA's epilogue stores its own 128 rows.
 // A K block then costs an SM 32 KB of loads instead of 48 (BN = 256), and the ring holds six stages instead of four.
 template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM, int CG = 1>
-__global__ void __launch_bounds__(COMM == COMM_AG ? NUM_THREADS_AG : NUM_THREADS, 1)
+__global__ void __launch_bounds__(COMM == COMM_AG ? NUM_THREADS_AG : COMM == COMM_RS ? NUM_THREADS_RS : NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ OutMaps tmC, const __grid_constant__ CUtensorMap tmA_local,
                  const GemmParams p, const GemmComm cm) {
   static_assert(CG == 1 || COMM == COMM_NONE, "CTA pairs run the plain product only");
   using L = SmemLayout<BN / CG, STAGES>;
+  // Epilogue warps per 32 lanes of the accumulator.  Two of them take 64-column groups in turn, or, where a tile has only one
+  // group, whole tiles in turn.  One warp took about 0.6 us for 32 columns, 1 us and more with a fused activation, which a
+  // short K does not cover: 16384 x 3072 x 768 takes 65 us and took 69, with GELU and its saved input 114 (141), with GELU'
+  // 140 (193); 16384 x 768 x 768 plus residual 32 (41); 16384 x 8192 x 2048 with GELU' 438 (525); 2^20 x 64 x 32 with bias and
+  // ReLU 78 (92).  Fetching the epilogue's operand a column group ahead did not help on top (144 and 126 us with GELU' and GELU).
+  constexpr int SETS = COMM == COMM_NONE ? 2 : 1;
+  constexpr bool SPLIT = SETS == 2 && BN > 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -299,7 +307,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tfull_bar[a]), 1);
-      mbar_init(smem_u32(&tempty_bar[a]), 4 * CG);
+      mbar_init(smem_u32(&tempty_bar[a]), (SPLIT ? 8 : 4) * CG);
     }
     *abort_flag = 0;
     if constexpr (COMM == COMM_AG) {
@@ -534,13 +542,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
     }
-  } else if (warp < 6) {
+  } else if (warp < 2 + 4 * SETS) {
     // ------------------------------- epilogue warps -----------------------------------
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
+    const int set = (warp - 2) >> 2;
     int iter = 0;
-    // staging buffers per warp: two, except in the 4-stage all-gather variant, whose push ring takes
-    // the upper half of the staging area
-    constexpr int CSB = (COMM == COMM_AG && STAGES == 4) ? 1 : 2;
+    // staging buffers per warp: two of four warps, one of eight, and one in the 4-stage all-gather variant, whose push ring
+    // takes the upper half of the staging area
+    constexpr int CSB = (SETS == 2 || (COMM == COMM_AG && STAGES == 4)) ? 1 : 2;
+    uint8_t* const cs_warp = smem + L::CSTAGE_OFFSET + (set * 4 + quad) * CSB * 4096;
     int store_seq = 0;          // TMA stores issued by this warp (selects the staging buffer)
     int tile_seq0 = 0;          // value of store_seq when the current tile started
     constexpr int kPubBatch = 3;
@@ -563,6 +573,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     if (tracer) cm.trace[blockIdx.x * 4 + 1] = globaltimer_ns();
     for (int t = gemm_bid; t < total_tiles && alive; t += grid_stride, ++iter) {
+      if (SETS == 2 && !SPLIT && (iter & 1) != set) continue;
       int b, tm, tn;
       map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
       const int m0 = tm * BM * CG + cta * BM, n0 = tn * BN;
@@ -642,7 +653,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) {
           const CUtensorMap* om = &tmC.m[COMM == COMM_RS ? owner : 0];
           const int r0 = (COMM == COMM_RS ? m0 - owner * cm.rows_per_chunk : m0) + quad * 32;
-          tma_store_3d(om, smem_u32(smem + L::CSTAGE_OFFSET + (quad * CSB + (store_seq % CSB)) * 4096),
+          tma_store_3d(om, smem_u32(cs_warp + (store_seq % CSB) * 4096),
                        n0 + (c >> 1) * 64, r0, b);
           tma_store_commit();
         }
@@ -652,6 +663,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int c = 0; c < BN / 32; ++c) {
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) break;  // uniform across the warp
+        if (SPLIT && ((c >> 1) & 1) != set) continue;
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + c * 32, r);
         tmem_ld_wait();
@@ -773,7 +785,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (p.use_tma_store) {
           // stage this warp's 32 rows x 64 columns (128-byte swizzle) and store them by TMA
           const int half = c & 1;
-          uint8_t* cs = smem + L::CSTAGE_OFFSET + (quad * CSB + (store_seq % CSB)) * 4096;
+          uint8_t* cs = cs_warp + (store_seq % CSB) * 4096;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint4 o;

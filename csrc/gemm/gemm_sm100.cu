@@ -1,10 +1,10 @@
 // Persistent bf16 GEMM for sm_100a: C[M,N] = epilogue(alpha * A·Bᵀ).
 //
-//   * operands arrive by TMA (128-byte swizzle) into a 4-stage shared-memory ring;
-//   * one elected thread issues tcgen05.mma (128 x BN x 16, cta_group::1) with fp32
+//   * operands arrive by TMA (128-byte swizzle) into a shared-memory ring of 4 to 8 stages;
+//   * one elected thread issues tcgen05.mma (128 x BN x 16, or 256 x 256 x 16 over a CTA pair) with fp32
 //     accumulators in TMEM; two accumulator buffers let the epilogue of tile i overlap the
 //     main loop of tile i+1;
-//   * four epilogue warps read TMEM with tcgen05.ld and apply the fused epilogue:
+//   * eight epilogue warps read TMEM with tcgen05.ld and apply the fused epilogue:
 //     +bias, ReLU / GELU(tanh), store of the pre-activation, multiply by GELU'/ReLU' of a
 //     saved pre-activation (backward), +residual, C += (gradient accumulation), bf16 or
 //     fp32 output.

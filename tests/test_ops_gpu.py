@@ -393,8 +393,6 @@ def test_cuda_graph_replay_matches_eager_forward_backward():
 def test_gemm_tile_forms(M, N, K, major):
     """Every tile width and the CTA pairs, with rows, columns and K blocks that do not fill them, epilogues included: bf16
     output is one rounding (2^-9) of the fp32 result, gradient accumulation is fp32."""
-    from spiraltorch_b200.ops import gemm as G
-    from spiraltorch_b200.ops import native
     a_mn, b_mn = major
     torch.manual_seed(M + N)
     a = torch.randn(*((K, M) if a_mn else (M, K)), device="cuda").bfloat16()
@@ -412,3 +410,22 @@ def test_gemm_tile_forms(M, N, K, major):
     assert ((aux - ref).norm() / ref.norm()).item() < 2.5e-3
     assert ((z - torch.nn.functional.gelu(ref, approximate="tanh")).norm() / ref.norm()).item() < 4e-3
     native.raise_on_device_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(40000, 64, 32), (20100, 40, 72), (20000, 136, 64), (19000, 200, 136), (5000, 712, 40), (130, 264, 64)])
+def test_gemm_epilogue_warps_share_columns_and_tiles(M, N, K):
+    """Two epilogue warps per 32 rows: whole tiles in turn at 64 columns, 64-column groups in turn above, with a ragged last
+    group; several tiles per CTA, single tiles, every bf16 epilogue operand and the fp32 accumulation."""
+    torch.manual_seed(M + N)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    pre = a.double() @ b.double().t() + bias.double()
+    aux = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    got = G.gemm(a, b, bias=bias, act="gelu", aux_out=aux, residual=res)
+    want = torch.nn.functional.gelu(pre, approximate="tanh") + res.double()
+    for x, y in ((aux, pre), (got, want)):
+        assert ((x.double() - y).abs() <= 2.0 ** -8 * y.abs() + 1e-5).all()        # one bf16 rounding of an fp32 value
+    acc = torch.ones(M, N, device="cuda")
+    G.gemm(a, b, out=acc, accumulate=True)
+    assert ((acc.double() - 1 - (pre - bias.double())).abs() <= 1e-5 * K ** 0.5).all()      # fp32 sums of terms of order one
