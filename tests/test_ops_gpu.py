@@ -429,3 +429,21 @@ def test_gemm_epilogue_warps_share_columns_and_tiles(M, N, K):
     acc = torch.ones(M, N, device="cuda")
     G.gemm(a, b, out=acc, accumulate=True)
     assert ((acc.double() - 1 - (pre - bias.double())).abs() <= 1e-5 * K ** 0.5).all()      # fp32 sums of terms of order one
+
+
+@pytest.mark.gpu
+def test_gelu_and_its_derivative_in_fp32():
+    """Through the GEMM's epilogue with an identity product: both signs, tiny and large arguments, infinity and NaN."""
+    x = torch.cat([torch.linspace(-9, 9, 8192), torch.tensor([0.0, -0.0, 1e-20, -1e-20, 30.0, -30.0, 1e30, -1e30])])
+    x = x.cuda().bfloat16().view(-1, 8)
+    one = torch.eye(8, device="cuda").bfloat16()
+    xd = x.double().requires_grad_()
+    want = torch.nn.functional.gelu(xd, approximate="tanh")
+    want.sum().backward()
+    got = G.gemm(x, one, act="gelu", out_dtype=torch.float32)
+    grad = G.gemm(torch.ones_like(x), one, act="gelu_bwd", aux_in=x, out_dtype=torch.float32)
+    assert ((got.double() - want).abs() <= 3e-7 * (1 + want.abs())).all()                      # a few roundings of fp32
+    assert ((grad.double() - xd.grad).abs() <= 6e-7)[x.abs() < 1e4].all()                      # x^2 overflows beyond
+    special = torch.tensor([float("inf"), float("-inf"), float("nan"), 1.0] * 8, device="cuda").bfloat16()
+    y, ref = E.gelu(special).float(), torch.nn.functional.gelu(special.float(), approximate="tanh")
+    assert torch.equal(y.isnan(), ref.isnan()) and (y[special == float("inf")] == float("inf")).all()
