@@ -291,6 +291,25 @@ __device__ __forceinline__ void store8(float* p, const float (&f)[8]) {
 __device__ __forceinline__ float as_stored(float v, const __nv_bfloat16*) { return __bfloat162float(__float2bfloat16(v)); }
 __device__ __forceinline__ float as_stored(float v, const float*) { return v; }
 
+// fp32 tensors whose values count as bf16: rounded when read and when written, so that the results are those of the bf16 form
+// between two conversion passes.  The layer protocol takes this form: a pre-activation that keeps more bits may fall on the
+// other side of the ReLU behind it, which a gradient summed over a few rows shows.
+struct F32AsBf16 {
+  float v;
+};
+__device__ __forceinline__ float as_stored(float v, const F32AsBf16*) { return __bfloat162float(__float2bfloat16(v)); }
+__device__ __forceinline__ void load8(const F32AsBf16* p, float (&f)[8]) {
+  load8(reinterpret_cast<const float*>(p), f);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = as_stored(f[j], p);
+}
+__device__ __forceinline__ void store8(F32AsBf16* p, const float (&f)[8]) {
+  float r[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] = as_stored(f[j], p);
+  store8(reinterpret_cast<float*>(p), r);
+}
+
 // Eight elements as they lie in memory
 template <typename T>
 struct Raw8;
@@ -315,6 +334,16 @@ struct Raw8<float> {
   }
   __device__ __forceinline__ void get(float (&f)[8]) const {
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+  }
+};
+template <>
+struct Raw8<F32AsBf16> {
+  Raw8<float> raw;
+  __device__ __forceinline__ void load(const F32AsBf16* p) { raw.load(reinterpret_cast<const float*>(p)); }
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    raw.get(f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = as_stored(f[j], static_cast<const F32AsBf16*>(nullptr));
   }
 };
 
@@ -715,26 +744,54 @@ ST_API int st_norm_gelu_bwd(const void* dy, const void* x, const void* gamma, co
   return reduce_param_grads(0, scratch, pb, dgamma, dbeta, grid, d, accumulate, s);
 }
 
-// fp32 tensors throughout, rows of at most 1024 features, 16-byte aligned: the layer protocol's LayerNorm without
-// conversion passes.  scratch: st_norm_bwd_scratch_elems floats.
-ST_API int st_norm_f32_max_features() { return kWarpRowFeatures; }
-ST_API int st_norm_fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y,
-                           float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v) {
+// fp32 tensors, rows of at most 1024 features, 16-byte aligned: the layer protocol's LayerNorm without conversion passes.
+// scratch: st_norm_bwd_scratch_elems floats.
+namespace {
+template <typename T>
+int fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y, float* sum_out,
+            float* mean, float* rstd, int rows, int d, float eps, void* stream_v) {
   if (int e = check_dims(rows, d)) return e;
   if (d > kWarpRowFeatures) return st::fail(ST_ERR_TOO_LARGE, "norm_f32: feature dimension above 1024");
-  return fwd_warp<float>(rms, x, residual, gamma, beta, y, sum_out, mean, rstd, rows, d, eps, reinterpret_cast<cudaStream_t>(stream_v));
+  auto in = [](const float* p) { return reinterpret_cast<const T*>(p); };
+  return fwd_warp<T>(rms, in(x), in(residual), in(gamma), in(beta), reinterpret_cast<T*>(y), reinterpret_cast<T*>(sum_out), mean, rstd,
+                     rows, d, eps, reinterpret_cast<cudaStream_t>(stream_v));
 }
-ST_API int st_norm_bwd_f32(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd,
-                           const float* dres, float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows,
-                           int d, void* stream_v) {
+template <typename T>
+int bwd_f32(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd, const float* dres,
+            float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v) {
   if (int e = check_dims(rows, d)) return e;
   if (d > kWarpRowFeatures) return st::fail(ST_ERR_TOO_LARGE, "norm_f32: feature dimension above 1024");
   if (!scratch) return st::fail(ST_ERR_INVALID, "norm_f32: scratch buffer is required");
   const int grid = st::norm_bwd_grid_for(rows, d);
   float* pb = scratch + (size_t)grid * d;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (int e = bwd_rows<float>(rms, dy, x, gamma, mean, rstd, dres, dx, scratch, rms ? nullptr : pb, rows, d, grid, s)) return e;
+  auto in = [](const float* p) { return reinterpret_cast<const T*>(p); };
+  if (int e = bwd_rows<T>(rms, in(dy), in(x), in(gamma), mean, rstd, in(dres), reinterpret_cast<T*>(dx), scratch, rms ? nullptr : pb,
+                          rows, d, grid, s))
+    return e;
   return reduce_param_grads(rms, scratch, pb, dgamma, dbeta, grid, d, accumulate, s);
+}
+}  // namespace
+
+ST_API int st_norm_f32_max_features() { return kWarpRowFeatures; }
+ST_API int st_norm_fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y,
+                           float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v) {
+  return fwd_f32<float>(rms, x, residual, gamma, beta, y, sum_out, mean, rstd, rows, d, eps, stream_v);
+}
+ST_API int st_norm_bwd_f32(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd,
+                           const float* dres, float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows,
+                           int d, void* stream_v) {
+  return bwd_f32<float>(rms, dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate, scratch, rows, d, stream_v);
+}
+// The same with every operand and result rounded to bf16 (F32AsBf16).
+ST_API int st_norm_fwd_f32_rounded(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y,
+                                   float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v) {
+  return fwd_f32<F32AsBf16>(rms, x, residual, gamma, beta, y, sum_out, mean, rstd, rows, d, eps, stream_v);
+}
+ST_API int st_norm_bwd_f32_rounded(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd,
+                                   const float* dres, float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch,
+                                   int rows, int d, void* stream_v) {
+  return bwd_f32<F32AsBf16>(rms, dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate, scratch, rows, d, stream_v);
 }
 
 // dgamma / dbeta are fp32 [d]; with accumulate != 0 the kernel adds to them.

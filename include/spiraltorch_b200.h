@@ -293,11 +293,13 @@ int st_nerf_composite_fwd(const float* sigma, const float* rad, const float* del
 int st_nerf_sample(const float* rays, float* points, float* ts, float* deltas, int R, int S, int stratified, unsigned seed, void* stream_v);   /* csrc/vision/vision.cu */
 int st_norm_bwd(int rms, const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* dres, void* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_bwd_f32(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd, const float* dres, float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v);   /* csrc/norm/norm.cu */
+int st_norm_bwd_f32_rounded(int rms, const float* dy, const float* x, const float* gamma, const float* mean, const float* rstd, const float* dres, float* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_bwd_noalloc(int rms, const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* dres, void* dx, float* dgamma, float* dbeta, int accumulate, int rows, int d, void* stream_v);   /* csrc/norm/norm.cu */
 long long st_norm_bwd_scratch_elems(int rows, int d);   /* csrc/norm/norm.cu */
 int st_norm_f32_max_features();   /* csrc/norm/norm.cu */
 int st_norm_fwd(int rms, const void* x, const void* residual, const void* gamma, const void* beta, void* y, void* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_fwd_f32(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y, float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
+int st_norm_fwd_f32_rounded(int rms, const float* x, const float* residual, const float* gamma, const float* beta, float* y, float* sum_out, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_gelu_bwd(const void* dy, const void* x, const void* gamma, const void* beta, const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int rows, int d, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_gelu_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int rows, int d, float eps, void* stream_v);   /* csrc/norm/norm.cu */
 int st_norm_gelu_max_features();   /* csrc/norm/norm.cu */

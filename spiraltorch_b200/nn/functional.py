@@ -104,7 +104,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 # layer norm (optionally with a residual added first)
 # ------------------------------------------------------------------------------------------------------
 class _LayerNormFn(torch.autograd.Function):
-    """The tensors stay fp32 where the kernels take them so (rows of up to 1024 features); wider rows pass through bf16."""
+    """Operands and results are bf16 values, like those of the layers around it.  Where the kernels take fp32 tensors (rows of up
+    to 1024 features) they round inside; wider rows pass through bf16 tensors."""
 
     @staticmethod
     def forward(ctx, x, gamma, beta, eps, residual):
@@ -120,7 +121,7 @@ class _LayerNormFn(torch.autograd.Function):
             g, b = bf16_of(gamma).reshape(-1), bf16_of(beta).reshape(-1)
         # the backward reads copies, as with the bf16 operands: the caller may go on to change x or the gain in place
         keep = ctx.fp32 and any(ctx.needs_input_grad)
-        y, summed, mean, rstd = _norm.norm_forward(xd, g, b, float(eps), False, rd, copy_input=keep)
+        y, summed, mean, rstd = _norm.norm_forward(xd, g, b, float(eps), False, rd, copy_input=keep, rounded=ctx.fp32)
         ctx.save_for_backward(xd if summed is None else summed, g.clone() if keep else g, mean, rstd)
         return y if ctx.fp32 else y.float()
 
@@ -135,7 +136,7 @@ class _LayerNormFn(torch.autograd.Function):
             d = dy.to(torch.bfloat16).contiguous()
         dg = torch.empty(xin.shape[1], dtype=torch.float32, device=xin.device)
         db = torch.empty_like(dg)
-        dx = _norm.norm_backward(d, xin, g, mean, rstd, False, dg, db, False).float()
+        dx = _norm.norm_backward(d, xin, g, mean, rstd, False, dg, db, False, rounded=ctx.fp32).float()
         return dx, dg.reshape(ctx.pshape), db.reshape(ctx.pshape), None, (dx if ctx.has_residual else None)
 
 

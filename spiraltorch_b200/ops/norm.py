@@ -35,6 +35,10 @@ def takes_f32(d: int, *tensors: Optional[torch.Tensor]) -> bool:
         t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in tensors)
 
 
+def _form(lib, entry: str, x2: torch.Tensor, rounded: bool):
+    return getattr(lib, entry if x2.dtype != torch.float32 else entry + ("_f32_rounded" if rounded else "_f32"))
+
+
 def norm_reference(x, gamma, beta, eps, rms, residual=None):
     xf = x.float()
     if residual is not None:
@@ -53,9 +57,11 @@ def norm_reference(x, gamma, beta, eps, rms, residual=None):
     return y, xf, mean.squeeze(-1), rstd.squeeze(-1)
 
 
-def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=None, out=None, copy_input: bool = False):
-    """x2: [rows, d] bf16, or fp32 throughout where :func:`takes_f32`.  Returns (y, summed_input_or_None, mean, rstd); ``out`` (contiguous, same shape and
-    dtype) receives y when given.  ``copy_input`` (fp32 form): without a residual the second result is a copy of x2."""
+def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=None, out=None, copy_input: bool = False,
+                 rounded: bool = False):
+    """x2: [rows, d] bf16, or fp32 throughout where :func:`takes_f32`.  Returns (y, summed_input_or_None, mean, rstd); ``out``
+    (contiguous, same shape and dtype) receives y when given.  fp32 form on CUDA: with ``copy_input`` and no residual the second
+    result is a copy of x2; with ``rounded`` operands and results are rounded to bf16, as the bf16 form has them."""
     global launch_count
     rows, d = x2.shape
     if out is not None:
@@ -70,8 +76,7 @@ def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=
     s = torch.empty_like(x2) if residual is not None or (copy_input and x2.dtype == torch.float32) else None
     mean = torch.empty(rows, dtype=torch.float32, device=x2.device)
     rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
-    entry = native.lib().st_norm_fwd_f32 if x2.dtype == torch.float32 else native.lib().st_norm_fwd
-    st = entry(
+    st = _form(native.lib(), "st_norm_fwd", x2, rounded)(
         ctypes.c_int(int(rms)), native.ptr(x2), native.ptr(residual), native.ptr(gamma), native.ptr(beta),
         native.ptr(y), native.ptr(s), native.ptr(mean), native.ptr(rstd), ctypes.c_int(rows),
         ctypes.c_int(d), ctypes.c_float(eps), native.stream_ptr(x2.device))
@@ -81,8 +86,9 @@ def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=
 
 
 def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
-                  dbeta: Optional[torch.Tensor], accumulate: bool, dres=None, out=None):
-    """Writes dx (returned; into ``out`` when given) and fp32 dgamma/dbeta (in place, ``+=`` when ``accumulate``)."""
+                  dbeta: Optional[torch.Tensor], accumulate: bool, dres=None, out=None, rounded: bool = False):
+    """Writes dx (returned; into ``out`` when given) and fp32 dgamma/dbeta (in place, ``+=`` when ``accumulate``).
+    ``rounded`` as in :func:`norm_forward`."""
     global launch_count
     rows, d = x2.shape
     if out is not None:
@@ -108,7 +114,7 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
     lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
     need = lib.st_norm_bwd_scratch_elems(ctypes.c_int(rows), ctypes.c_int(d))
     scratch = _get_scratch(x2.device, int(need))
-    st = (lib.st_norm_bwd_f32 if x2.dtype == torch.float32 else lib.st_norm_bwd)(
+    st = _form(lib, "st_norm_bwd", x2, rounded)(
         ctypes.c_int(int(rms)), native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(mean),
         native.ptr(rstd), native.ptr(dres), native.ptr(dx), native.ptr(dgamma), native.ptr(dbeta),
         ctypes.c_int(int(accumulate)), native.ptr(scratch), ctypes.c_int(rows), ctypes.c_int(d),

@@ -539,3 +539,22 @@ def test_trainer_still_refuses_gradients_that_overflow_in_accumulation():
     with pytest.raises(Exception, match="non-finite gradient"):
         trainer.train_epoch(lin, st.nn.MeanSquaredError(), [batch])
     assert all(p.gradient is None for p in lin.parameters())
+
+
+@pytest.mark.parametrize("rows,d,residual", [(1, 8, False), (33, 128, True), (2500, 264, False), (640, 1024, True)])
+def test_layer_norm_of_fp32_tensors_has_the_values_of_the_bf16_form(rows, d, residual):
+    """Bit for bit: operands, output and input gradient are bf16 values wherever the tensors are fp32.  A wider result moved
+    elements across the ReLU behind it, and with them whole gradients of small batches."""
+    torch.manual_seed(rows + d)
+    x, dy = torch.randn(rows, d, device=DEV), torch.randn(rows, d, device=DEV)
+    g, b, r = (torch.randn(s, device=DEV) for s in ((1, d), (1, d), (rows, d)))
+    r = r if residual else None
+    leaves = [t.requires_grad_(True) for t in (x, g, b)]
+    y = Fn.layer_norm(*leaves, residual=r)
+    got = torch.autograd.grad(y, leaves, dy)
+    xb, gb, bb, rb = (None if t is None else t.detach().bfloat16() for t in (x, g.reshape(-1), b.reshape(-1), r))
+    want, summed, mean, rstd = N.norm_forward(xb, gb, bb, 1e-5, False, rb)
+    dg, db = torch.empty(d, device=DEV), torch.empty(d, device=DEV)
+    dx = N.norm_backward(dy.bfloat16(), xb if summed is None else summed, gb, mean, rstd, False, dg, db, False)
+    assert torch.equal(y, want.float()) and torch.equal(got[0], dx.float())
+    assert torch.equal(got[1].reshape(-1), dg) and torch.equal(got[2].reshape(-1), db)
