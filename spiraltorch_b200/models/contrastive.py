@@ -67,6 +67,8 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
     encoder as defined here, without hooks that would see its modules, parameters or saved tensors."""
     if type(encoder) is not ContrastiveEncoder or not torch.is_grad_enabled() or not temperature > 0:
         return False
+    if torch.is_autocast_enabled(base.device.type):      # the similarity products would change their type under the fp32 kernels
+        return False
     params = list(encoder.parameters())
     dev = base.device
     if not (base.is_cuda and base.dtype == torch.float32 and base.dim() == 2 and base.is_contiguous() and base.data_ptr() % 16 == 0

@@ -558,3 +558,23 @@ def test_layer_norm_of_fp32_tensors_has_the_values_of_the_bf16_form(rows, d, res
     dx = N.norm_backward(dy.bfloat16(), xb if summed is None else summed, gb, mean, rstd, False, dg, db, False)
     assert torch.equal(y, want.float()) and torch.equal(got[0], dx.float())
     assert torch.equal(got[1].reshape(-1), dg) and torch.equal(got[2].reshape(-1), db)
+
+
+def test_contrastive_step_under_autocast_takes_the_autograd_form():
+    """Its similarity products come out in 16 bits there, which the kernels of the written-out form must never see."""
+    from spiraltorch_b200.models import contrastive as M
+    enc = M.ContrastiveEncoder(64, 128, 64, device=DEV, seed=1)
+    base = torch.randn(48, 64, device=DEV)
+
+    def step(hooked):
+        enc.zero_grad(set_to_none=True)
+        handle = enc.register_forward_hook(lambda *a: None) if hooked else None
+        loss = M.contrastive_step(enc, base, 0.1, seed=5)
+        if handle is not None:
+            handle.remove()
+        return [loss] + [p.grad.clone() for p in enc.parameters()]
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert not M._schedulable(enc, base, 0.1)
+        got, want = step(False), step(True)
+    assert M._schedulable(enc, base, 0.1)
+    assert all(torch.isfinite(a).all() and (a.float() - b.float()).norm() <= 1e-2 * b.float().norm() for a, b in zip(got, want))
