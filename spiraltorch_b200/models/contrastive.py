@@ -102,8 +102,8 @@ def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: floa
     B, width = base.shape
     if seed is not None:
         g = torch.Generator(device=dev).manual_seed(seed)
-    n1 = torch.randn(base.shape, generator=g, device=dev)
-    n2 = torch.randn(base.shape, generator=g, device=dev)
+    n1 = torch.randn(base.shape, generator=g, device=dev, dtype=base.dtype)
+    n2 = torch.randn(base.shape, generator=g, device=dev, dtype=base.dtype)
     w, b, gamma, beta = encoder.weights, encoder.biases, encoder.gammas, encoder.betas
     x = torch.empty((2 * B, width), dtype=torch.bfloat16, device=dev)
     native.check(lib.st_contrastive_views(native.ptr(base), native.ptr(n1), native.ptr(n2), ctypes.c_float(noise), native.ptr(x),

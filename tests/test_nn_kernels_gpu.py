@@ -578,3 +578,22 @@ def test_contrastive_step_under_autocast_takes_the_autograd_form():
         got, want = step(False), step(True)
     assert M._schedulable(enc, base, 0.1)
     assert all(torch.isfinite(a).all() and (a.float() - b.float()).norm() <= 1e-2 * b.float().norm() for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float64])
+def test_contrastive_step_does_not_depend_on_the_default_dtype(dtype):
+    from spiraltorch_b200.models import contrastive as M
+    enc = M.ContrastiveEncoder(64, 128, 64, device=DEV, seed=1)
+    base = torch.randn(48, 64, device=DEV)
+
+    def step():
+        enc.zero_grad(set_to_none=True)
+        assert M._schedulable(enc, base, 0.1)
+        return [M.contrastive_step(enc, base, 0.1, seed=5)] + [p.grad.clone() for p in enc.parameters()]
+    want = step()
+    torch.set_default_dtype(dtype)
+    try:
+        got = step()
+    finally:
+        torch.set_default_dtype(torch.float32)
+    assert all(a.dtype == b.dtype and torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-5) for a, b in zip(got, want))
