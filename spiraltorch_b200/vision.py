@@ -135,7 +135,8 @@ def preprocess(img: torch.Tensor, *, resize: Optional[tuple[int, int]] = None, c
         lib, stream = native.lib(), native.stream_ptr(x.device)
         if own_means:
             lib.st_preprocess_workspace.restype = ctypes.c_longlong
-            work = torch.empty(lib.st_preprocess_workspace(ctypes.c_int(B), ctypes.c_int(sh), ctypes.c_int(sw)), device=x.device)
+            work = torch.empty(lib.st_preprocess_workspace(ctypes.c_int(B), ctypes.c_int(sh), ctypes.c_int(sw)), dtype=torch.float32,
+                               device=x.device)
             native.check(lib.st_preprocess_own_means(native.ptr(x), native.ptr(y), ctypes.byref(a), native.ptr(work), stream),
                          "st_preprocess_own_means")
             launch_count += 2

@@ -218,3 +218,16 @@ def test_jitter_means_taken_on_the_device(B, C, H, W):
     kw = dict(resize=(H, W), crop=(H // 2, W // 2), jitter=vision.ColorJitter(1.1, 1.3, 1.0, 0.0), flip=True)
     want, got = vision.preprocess(x.double().float(), **kw), vision.preprocess(x.cuda(), **kw)
     assert torch.allclose(got.cpu(), want, rtol=1e-5, atol=2e-6)      # the means differ by the order of their sums
+
+
+@pytest.mark.gpu
+def test_preprocessing_does_not_depend_on_the_default_dtype():
+    x = torch.rand(2, 3, 300, 400, device="cuda")
+    kw = dict(resize=(256, 256), crop=(224, 224), jitter=vision.ColorJitter(1.1, 1.3, 1.0, 0.0))
+    want = vision.preprocess(x, **kw)
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        got = vision.preprocess(x, **kw)
+    finally:
+        torch.set_default_dtype(torch.float32)
+    assert got.dtype == torch.float32 and torch.equal(got, want)
