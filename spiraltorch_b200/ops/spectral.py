@@ -41,7 +41,7 @@ def window_coefficients(kind: str, n: int, device=None) -> torch.Tensor:
     if kind not in WINDOWS:
         raise ValueError(f"unknown window '{kind}', expected one of {WINDOWS}")
     if n <= 1 or kind == "rectangular":
-        return torch.ones(max(n, 0), device=device)
+        return torch.ones(max(n, 0), dtype=torch.float32, device=device)
     r = torch.arange(n, dtype=torch.float32, device=device) / (n - 1)
     c = torch.cos(2 * math.pi * r)
     if kind == "hann":
@@ -113,7 +113,7 @@ def fft_field_interleaved(field: torch.Tensor, axis: str, inverse: bool = False,
             z = z * (win.reshape(1, W, 1) if axis == "row" else win.reshape(H, 1, 1))
         z = torch.fft.ifft(z, dim=d) if inverse else torch.fft.fft(z, dim=d)
         return torch.view_as_real(z).reshape(H, W, 2 * C)
-    out = torch.empty(H, W, 2 * C, device=f.device)
+    out = torch.empty(H, W, 2 * C, dtype=torch.float32, device=f.device)
     if axis == "row":       # batch0 = row, batch1 = channel, element = column
         _launch(f, out, win, W, H, C, (W * C, 1, C), (W * 2 * C, 2, 2 * C), False, inverse)
     else:                   # batch0 = column, batch1 = channel, element = row
@@ -194,7 +194,7 @@ def temporal_render(voxels: torch.Tensor, harmonics: Optional[torch.Tensor], dec
         dd = torch.where(torch.isfinite(d), d.clamp(min=0.0), torch.ones_like(d)).reshape(1, -1)
         out = torch.where(dd <= 1.1920929e-07, torch.zeros_like(base), base * torch.exp(-dd * t[:, None]))
         return out.reshape(frames, *voxels.shape)
-    out = torch.empty(frames, v.numel(), device=v.device)
+    out = torch.empty(frames, v.numel(), dtype=torch.float32, device=v.device)
     hp = harmonics.float().contiguous() if channels else None
     st = native.lib().st_temporal_render(native.ptr(v), native.ptr(hp), native.ptr(d), native.ptr(out),
                                          ctypes.c_longlong(v.numel()), ctypes.c_int(channels), ctypes.c_int(frames),

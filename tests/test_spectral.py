@@ -196,3 +196,20 @@ def test_fft_of_long_batches(n):
     assert ((dst[..., :n] - want).abs().pow(2).sum() / want.abs().pow(2).sum()).sqrt().item() < 4e-7
     assert dst[..., n].abs().max().item() == 0
     native.raise_on_device_error()
+
+
+@pytest.mark.gpu
+def test_spectral_outputs_do_not_depend_on_the_default_dtype():
+    field = torch.randn(16, 32, 3, device="cuda")
+    vox, harm, decay = _temporal_case("cuda")
+
+    def run():
+        return (spectral.fft_field_interleaved(field, "row", window="rectangular"), spectral.fft_field_interleaved(field, "col"),
+                spectral.temporal_render(vox, harm, decay, 7, 12.0))
+    want = run()
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        got = run()
+    finally:
+        torch.set_default_dtype(torch.float32)
+    assert all(a.dtype == torch.float32 and torch.equal(a, b) for a, b in zip(got, want))
