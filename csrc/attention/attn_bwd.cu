@@ -407,8 +407,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float lse2 = 0.0f, dlt = 0.0f;
     int row_g = own * BLK + r;
     bool row_ok = row_g < p.Sq;
-    int q_live = p.Sq;                          // queries from here on are masked
-    if (BIAS == BIAS_KEYS && p.lengths) q_live = min(p.Sq, max(0, min(p.Sk, p.lengths[b])));
+    int q_live = p.Sq, kv_live = p.Sk;          // queries and keys from here on are masked
+    if (BIAS == BIAS_KEYS && p.lengths) {
+      kv_live = max(0, min(p.Sk, p.lengths[b]));
+      q_live = min(p.Sq, kv_live);
+    }
     if (MODE == MODE_Q && row_ok) {
       const long long stat_idx = ((long long)b * p.H + h) * p.Sq + row_g;
       lse2 = p.lse[stat_idx] * LOG2E;
@@ -459,10 +462,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld_32x32(tmem_base + lane_off + S_COL + part * 32, s_r);
         tmem_ld_wait();
         if constexpr (BIAS == BIAS_KEYS) {
-          // exp2(S c + bias - lse): masked keys carry -inf in the bias, masked rows +inf in the subtrahend (a fully masked
-          // row has lse = -inf and contributes nothing)
-          const float sub = row_g < q_live && lse2 > -INFINITY ? lse2 : INFINITY;
-          const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), ns2 = make_float2(-sub, -sub);
+          // exp2(S c + bias - lse): masked keys carry -inf in the bias; a fully masked row has lse = -inf and contributes
+          // nothing.  Padded queries and keys may hold values that are not finite: their rows, and their columns in the
+          // tile that holds the length, are set to zero by comparison.
+          const bool row_live = row_g < q_live && lse2 > -INFINITY;
+          const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), ns2 = make_float2(-lse2, -lse2);
           const float4* bias = reinterpret_cast<const float4*>(p.kb_pad + b * p.kp_sb + h * p.kp_sh + kv0 + part * 32);
 #pragma unroll
           for (int q = 0; q < 32; q += 4) {
@@ -472,10 +476,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             pv[q] = fast_exp2(x.x); pv[q + 1] = fast_exp2(x.y);
             pv[q + 2] = fast_exp2(y.x); pv[q + 3] = fast_exp2(y.y);
           }
-          if (p.causal && kv_tile >= q_tile) {
+          if ((p.causal && kv_tile >= q_tile) || kv0 + BLK > kv_live) {
 #pragma unroll
-            for (int q = 0; q < 32; ++q)
-              if (kv0 + part * 32 + q > row_g) pv[q] = 0.0f;
+            for (int q = 0; q < 32; ++q) {
+              const int colg = kv0 + part * 32 + q;
+              if (colg >= kv_live || (p.causal && colg > row_g)) pv[q] = 0.0f;
+            }
+          }
+          if (!row_live) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) pv[q] = 0.0f;
           }
         } else if (plain) {
 #pragma unroll

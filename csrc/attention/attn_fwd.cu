@@ -441,7 +441,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // operand reads per product, K and V written per tile, P written and read) to 128 KB.
 // With a key bias or valid lengths (KEYB) the logits take them from a padded fp32 row per batch entry (and head), already
 // in the log2 domain and minus infinity wherever a key is masked: 16-byte loads that all lanes share, one packed multiply-
-// add per two logits and no comparisons.  The single-tile kernel loaded and compared per element: 244 us for 96 contexts of
+// add per two logits and no comparisons, except in the tile that holds the length, where a padded key may have given a logit
+// that is not finite and is replaced by comparison.  The single-tile kernel loaded and compared per element: 244 us for 96 contexts of
 // up to 1000 keys, D = 64, where this form takes 99.  A bias per (query, key) stays with the single-tile kernel.
 // ------------------------------------------------------------------------------------------------------------------
 // Phase clocks of CTA 0 (SM cycles summed over the launch), written when tracing is switched on:
@@ -759,7 +760,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         continue;
       }
-      const bool row_live = !KEYB || !p.lengths || row_g < min(p.Sk, p.lengths[b]);
+      int kv_len = p.Sk;
+      if (KEYB && p.lengths) kv_len = max(0, min(p.Sk, p.lengths[b]));
+      const bool row_live = !KEYB || !p.lengths || row_g < kv_len;
       const float4* bias_row = KEYB ? reinterpret_cast<const float4*>(p.kb_pad + b * p.kp_sb + h * p.kp_sh) : nullptr;
       float m = -INFINITY, l = 0.0f;
       for (int j = 0; j < n_kv; ++j) {
@@ -781,7 +784,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         if (tr) { c1 = static_cast<uint32_t>(clock()); tacc[2] += c1 - c0; c0 = c1; }
         const int col0 = j * BLK;
-        float mx = -INFINITY;
         if constexpr (KEYB) {      // to the log2 domain, bias added; keys that are masked or past the end become -inf
           const float2 sc2 = make_float2(sc, sc);
 #pragma unroll
@@ -793,27 +795,22 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             sr[c + 2] = __float_as_uint(y.x); sr[c + 3] = __float_as_uint(y.y);
           }
         }
-        if ((p.causal && j == q_tile) || (!KEYB && col0 + BLK > p.Sk)) {
+        if ((p.causal && j == q_tile) || col0 + BLK > kv_len) {
+          const int live = p.causal && j == q_tile ? min(kv_len - col0, r + 1) : kv_len - col0;      // columns this row sees
 #pragma unroll
-          for (int c = 0; c < BLK; ++c) {
-            const int col = col0 + c;
-            const bool dead = (col >= p.Sk) || (p.causal && col > row_g);
-            const float s = dead ? -INFINITY : __uint_as_float(sr[c]);
-            sr[c] = __float_as_uint(s);
-            mx = fmaxf(mx, s);
-          }
-        } else {
-          float mc[8];                                 // eight independent chains
-#pragma unroll
-          for (int q = 0; q < 8; ++q) mc[q] = fmaxf(__uint_as_float(sr[2 * q]), __uint_as_float(sr[2 * q + 1]));
-#pragma unroll
-          for (int c = 16; c < BLK; c += 16) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              mc[q] = max3(mc[q], __uint_as_float(sr[c + 2 * q]), __uint_as_float(sr[c + 2 * q + 1]));
-          }
-          mx = fmaxf(fmaxf(max3(mc[0], mc[1], mc[2]), max3(mc[3], mc[4], mc[5])), fmaxf(mc[6], mc[7]));
+          for (int c = 0; c < BLK; ++c)
+            if (c >= live) sr[c] = __float_as_uint(-INFINITY);
         }
+        float mc[8];                                   // eight independent chains
+#pragma unroll
+        for (int q = 0; q < 8; ++q) mc[q] = fmaxf(__uint_as_float(sr[2 * q]), __uint_as_float(sr[2 * q + 1]));
+#pragma unroll
+        for (int c = 16; c < BLK; c += 16) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            mc[q] = max3(mc[q], __uint_as_float(sr[c + 2 * q]), __uint_as_float(sr[c + 2 * q + 1]));
+        }
+        const float mx = fmaxf(fmaxf(max3(mc[0], mc[1], mc[2]), max3(mc[3], mc[4], mc[5])), fmaxf(mc[6], mc[7]));
         const float m_new = fmaxf(m, KEYB ? mx : mx * sc);
         bool raise = false;
         float alpha = 1.0f;
@@ -889,6 +886,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         uint32_t v[32];
         tmem_ld_32x32(o_addr + ch * 32, v);
         tmem_ld_wait();
+        if (KEYB && !row_live) {      // zeros by value: what a padded query summed up need not be finite
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] = 0;
+        }
         if (row_g < p.Sq) {
           if (o32) {
 #pragma unroll

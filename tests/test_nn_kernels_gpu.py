@@ -597,3 +597,31 @@ def test_contrastive_step_does_not_depend_on_the_default_dtype(dtype):
     finally:
         torch.set_default_dtype(torch.float32)
     assert all(a.dtype == b.dtype and torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-5) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("Sq,Sk,D,causal,lengths", [(200, 200, 64, False, [130, 64, 1, 200]), (300, 300, 128, True, [129, 256, 127, 0]),
+                                                    (100, 385, 64, False, [90, 385, 260, 5])])
+def test_padding_that_is_not_finite_stays_out_of_attention_with_lengths(Sq, Sk, D, causal, lengths, bad):
+    """Queries at and beyond the length give zeros and queries below it do not see the keys beyond it, whatever stands there;
+    the padded queries leave nothing in dV and in the live rows of dQ."""
+    torch.manual_seed(Sq + D)
+    B, ln = len(lengths), torch.tensor(lengths, device=DEV, dtype=torch.int32)
+    q, do = torch.randn(B, Sq, D, device=DEV), torch.randn(B, Sq, D, device=DEV)
+    k, v = torch.randn(B, Sk, D, device=DEV), torch.randn(B, Sk, D, device=DEV)
+    zb = torch.randn(B, Sk, device=DEV)
+    dead_q = torch.arange(Sq, device=DEV) >= ln[:, None]
+    dead_k = torch.arange(Sk, device=DEV) >= ln[:, None]
+
+    def run(q, k):
+        leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        o = Fn.scaled_dot_attention(*leaves, z_bias=zb, causal=causal, lengths=ln)
+        return [o.detach()] + list(torch.autograd.grad(o, leaves, do))
+    fill = lambda t, dead: torch.where(dead[..., None], torch.full_like(t, bad), t)  # noqa: E731
+    clean, spoilt_q, spoilt = run(q, k), run(fill(q, dead_q), k), run(fill(q, dead_q), fill(k, dead_k))
+    assert not clean[0][dead_q].any()
+    for got in (spoilt_q, spoilt):
+        assert torch.equal(got[0], clean[0])
+    assert torch.equal(spoilt_q[1][~dead_q], clean[1][~dead_q]) and torch.equal(spoilt_q[3], clean[3])
+    ref = Fn.scaled_dot_attention(fill(q, dead_q).cpu(), fill(k, dead_k).cpu(), v.cpu(), z_bias=zb.cpu(), causal=causal, lengths=ln.cpu())
+    assert torch.isfinite(ref).all() and (clean[0].cpu() - ref).abs().max() <= 2e-2 * ref.abs().max()
