@@ -69,6 +69,8 @@ def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: 
     """``v -= lr * g`` for every pair, in place."""
     global launch_count
     from . import gemm
+    if len(values) != len(grads) or any(v.numel() != g.numel() for v, g in zip(values, grads)):
+        raise ValueError("descend_: every value needs a gradient of its own size")
     lib, stream = native.lib(), native.stream_ptr(values[0].device)
     # values whose bf16 copy is in use get the next one in the same launch (a new tensor: a graph may still hold the old one)
     halves = [torch.empty(v.shape, dtype=torch.bfloat16, device=v.device) if gemm.has_cached_bf16(v) else None for v in values]

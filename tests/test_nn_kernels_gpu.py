@@ -625,3 +625,22 @@ def test_padding_that_is_not_finite_stays_out_of_attention_with_lengths(Sq, Sk, 
     assert torch.equal(spoilt_q[1][~dead_q], clean[1][~dead_q]) and torch.equal(spoilt_q[3], clean[3])
     ref = Fn.scaled_dot_attention(fill(q, dead_q).cpu(), fill(k, dead_k).cpu(), v.cpu(), z_bias=zb.cpu(), causal=causal, lengths=ln.cpu())
     assert torch.isfinite(ref).all() and (clean[0].cpu() - ref).abs().max() <= 2e-2 * ref.abs().max()
+
+
+def test_updates_refuse_or_broadcast_gradients_of_another_shape():
+    """As ``value.sub_(lr * gradient)`` does; the launch over all parameters reads as many elements as the value has."""
+    from spiraltorch_b200.ops import multi
+    lin = st.nn.Linear("fc", 8, 16)
+    lin.init_normal(0.1, seed=1)
+    lin.to(DEV)
+    before = [p.value.clone() for p in lin.parameters()]
+    for p in lin.parameters():
+        p.gradient = torch.ones_like(p.value)
+    lin.weight.gradient = torch.arange(16.0, device=DEV).reshape(1, 16)
+    lin.apply_step(0.5)
+    assert torch.equal(lin.weight.value, before[0] - 0.5 * torch.arange(16.0, device=DEV)) and torch.equal(lin.bias.value, before[1] - 0.5)
+    lin.weight.gradient = torch.ones(3, 5, device=DEV)
+    with pytest.raises(RuntimeError):
+        lin.apply_step(0.5)
+    with pytest.raises(ValueError):
+        multi.descend_([lin.weight.value], [torch.ones(16, device=DEV)], 0.5)
