@@ -222,9 +222,11 @@ class Module:
     def apply_step(self, fallback_lr: float = 1e-2) -> None:
         plain = [p for p in self.parameters() if type(p) is Parameter and p.trainable and p.hypergrad is None
                  and p.realgrad is None and p.gradient is not None]
-        # a gradient of another shape broadcasts, or is refused, in the parameter's own step
-        if plain and len({id(p) for p in plain}) == len(plain) and _multi.takes([t for p in plain for t in (p.value, p.gradient)]) \
-                and not any(p.value.requires_grad or p.gradient.shape != p.value.shape for p in plain):
+        # a gradient of another shape broadcasts, or is refused, in the parameter's own step, and updates that share memory
+        # follow one another there
+        if plain and _multi.takes([t for p in plain for t in (p.value, p.gradient)]) \
+                and not any(p.value.requires_grad or p.gradient.shape != p.value.shape for p in plain) \
+                and _multi.disjoint([p.value for p in plain], [p.gradient for p in plain]):
             _multi.descend_([p.value for p in plain], [p.gradient for p in plain], fallback_lr)
             for p in plain:
                 p.gradient = None

@@ -65,8 +65,22 @@ def divided(tensors: Sequence[torch.Tensor], value: float):
     return out, _run(_DIV, tensors, out, value)
 
 
+def disjoint(written: Sequence[torch.Tensor], read: Sequence[torch.Tensor]) -> bool:
+    """Whether no memory of the dense tensors ``written`` belongs to another of them or to one of ``read``: the blocks of one
+    launch run in any order."""
+    spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size(), own) for ts, own in ((written, True), (read, False)) for t in ts)
+    end = end_written = 0
+    for begin, stop, own in spans:
+        if begin < (end if own else end_written):
+            return False
+        end = max(end, stop)
+        if own:
+            end_written = max(end_written, stop)
+    return True
+
+
 def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: float) -> None:
-    """``v -= lr * g`` for every pair, in place."""
+    """``v -= lr * g`` for every pair, in place; values and gradients :func:`disjoint`."""
     global launch_count
     from . import gemm
     if len(values) != len(grads) or any(v.numel() != g.numel() for v, g in zip(values, grads)):

@@ -644,3 +644,31 @@ def test_updates_refuse_or_broadcast_gradients_of_another_shape():
         lin.apply_step(0.5)
     with pytest.raises(ValueError):
         multi.descend_([lin.weight.value], [torch.ones(16, device=DEV)], 0.5)
+
+
+def test_parameters_over_one_storage_get_both_updates():
+    from spiraltorch_b200.nn.modules import Parameter
+
+    class Tied(st.nn.Linear):
+        twin = None
+
+        def parameters(self):
+            return super().parameters() + ([self.twin] if self.twin else [])
+    lin = Tied("fc", 300, 400)
+    lin.init_normal(0.1, seed=1)
+    lin.to(DEV)
+    for twin in (lin.weight.value, lin.weight.value.view(-1)[1000:].view(-1, 1)):      # the whole storage, and a part of it
+        lin.twin = Parameter("twin", twin)
+        assert lin.twin.value.data_ptr() == twin.data_ptr()
+        want = lin.weight.value.clone()
+        for p in lin.parameters():
+            p.gradient = torch.randn_like(p.value)
+        want -= 0.5 * lin.weight.gradient
+        want.view(-1)[want.numel() - twin.numel():] -= 0.5 * lin.twin.gradient.reshape(-1)
+        lin.apply_step(0.5)
+        assert torch.equal(lin.weight.value, want)
+    lin.twin = Parameter("twin", torch.zeros(300, 400, device=DEV))
+    lin.twin.gradient, lin.weight.gradient = lin.weight.value, torch.ones(300, 400, device=DEV)      # read as another step writes it
+    want = lin.weight.value - 0.5
+    lin.apply_step(0.5)
+    assert torch.equal(lin.weight.value, want) and torch.equal(lin.twin.value, -0.5 * want)
