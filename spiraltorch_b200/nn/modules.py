@@ -122,6 +122,12 @@ class Parameter:
             self.gradient = None
 
 
+def _plain(p) -> bool:
+    """Whether a parameter accumulates and steps as :class:`Parameter` does: nothing of it overridden or replaced, no tape."""
+    return type(p) is Parameter and p.hypergrad is None and p.realgrad is None and "accumulate" not in p.__dict__ \
+        and "apply_step" not in p.__dict__
+
+
 class _MovedModule:
     """What a Python handle turns into after ``Sequential.add`` took the layer."""
 
@@ -193,10 +199,9 @@ class Module:
             assert_finite(found, lambda i: f"non-finite gradient for parameter {live[i][0].name}")
             means = [gp / batch for gp in found]
         # nothing was accumulated before: what follows holds exactly these checked means
-        self._grads_finite = all(type(p) is Parameter and p.gradient is None and p.hypergrad is None and p.realgrad is None
-                                 for p in self.parameters())
+        self._grads_finite = all(_plain(p) and p.gradient is None for p in self.parameters())
         for (p, _), mean in zip(live, means):
-            if p.gradient is None and p.hypergrad is None and p.realgrad is None and type(p) is Parameter:
+            if _plain(p) and p.gradient is None:
                 p.gradient = mean.reshape(p.value.shape)            # a fresh tensor: nothing to clone
             else:
                 p.accumulate(mean)
@@ -220,8 +225,7 @@ class Module:
             p.zero()
 
     def apply_step(self, fallback_lr: float = 1e-2) -> None:
-        plain = [p for p in self.parameters() if type(p) is Parameter and p.trainable and p.hypergrad is None
-                 and p.realgrad is None and p.gradient is not None]
+        plain = [p for p in self.parameters() if _plain(p) and p.trainable and p.gradient is not None]
         # a gradient of another shape broadcasts, or is refused, in the parameter's own step, and updates that share memory
         # follow one another there
         if plain and _multi.takes([t for p in plain for t in (p.value, p.gradient)]) \

@@ -429,7 +429,9 @@ class ModuleTrainer:
             if schedule is not None:
                 self.last_band_energy = schedule.band_energy(grad)
             weights = self._spectral_band_weights(module) if schedule is not None else None
-            module._grads_finite = False
+            own_backward = getattr(type(module), "backward", None) is Module.backward and "backward" not in vars(module)
+            if own_backward:
+                module._grads_finite = False
             if schedule is not None and (self.band_backward or weights is not None):
                 bands = schedule.split(grad)
                 if weights is not None:
@@ -443,7 +445,7 @@ class ModuleTrainer:
             else:
                 module.backward(x, grad)
             # a backward into empty accumulators has just checked what they hold; anything else is checked here
-            finite = getattr(type(module), "backward", None) is Module.backward and module._grads_finite
+            finite = own_backward and module._grads_finite
             held = [] if finite else [(p, a) for p in module.parameters() for a in p.accumulators()]
             try:
                 assert_finite([a for _, a in held],

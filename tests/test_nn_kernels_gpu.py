@@ -672,3 +672,29 @@ def test_parameters_over_one_storage_get_both_updates():
     want = lin.weight.value - 0.5
     lin.apply_step(0.5)
     assert torch.equal(lin.weight.value, want) and torch.equal(lin.twin.value, -0.5 * want)
+
+
+def test_replaced_methods_of_one_module_or_parameter_are_still_heard():
+    def trained(lin):
+        trainer = st.SpiralSession("cuda", seed=1).trainer(fallback_learning_rate=0.1)
+        trainer.prepare(lin)
+        trainer.train_epoch(lin, st.nn.MeanSquaredError(), [(st.Tensor(torch.randn(16, 8, device=DEV)), st.Tensor(torch.randn(16, 8, device=DEV)))])
+
+    lin = st.nn.Linear("fc", 8, 8)
+    lin.init_normal(0.1, seed=1)
+    plain_backward = lin.backward
+
+    def backward(x, grad):
+        out = plain_backward(x, grad)
+        lin.weight.gradient.mul_(float("inf"))
+        return out
+    lin.backward = backward
+    with pytest.raises(Exception, match="non-finite gradient"):
+        trained(lin)
+    assert all(p.gradient is None for p in lin.parameters())
+    del lin.backward
+    before, calls = [p.value.clone() for p in lin.parameters()], []
+    lin.weight.apply_step = lambda lr: calls.append(lr)                       # a parameter that its owner froze
+    lin.bias.accumulate = lambda grad: calls.append(grad)
+    trained(lin)
+    assert len(calls) == 2 and all(torch.equal(p.value, b) for p, b in zip(lin.parameters(), before))
