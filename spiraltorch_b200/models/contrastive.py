@@ -62,9 +62,35 @@ def make_views(base: torch.Tensor, noise: float = 0.1, seed: Optional[int] = Non
     return base + noise * n1, base + noise * n2
 
 
+class _Graph(torch.autograd.Function):
+    """A graph over leaves that computes nothing."""
+
+    @staticmethod
+    def forward(ctx, *leaves):
+        return torch.empty(0, dtype=torch.float32, device="cpu")
+
+    @staticmethod
+    def backward(ctx, grad):
+        return (None,) * len(ctx.needs_input_grad)
+
+
+def _accumulation_held(leaves) -> bool:
+    """Whether anything outside holds an accumulation node of these leaves, and may have hooks on it that only a backward pass
+    runs.  A node that nobody holds ends with its graph, so a mark on it is gone in the next one."""
+    mark = object()
+
+    def nodes():
+        out = _Graph.apply(*leaves)
+        return [edge[0] for edge in out.grad_fn.next_functions]
+    for node in nodes():
+        node.metadata["contrastive_step"] = mark
+    del node
+    return any(node.metadata.get("contrastive_step") is mark for node in nodes())
+
+
 def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
     """Whether a step can be written out over the kernels with the same outcome as running autograd over the encoder: the
-    encoder as defined here, without hooks that would see its modules, parameters or saved tensors."""
+    encoder as defined here, without hooks that would see its modules, parameters, accumulation nodes or saved tensors."""
     if type(encoder) is not ContrastiveEncoder or not torch.is_grad_enabled() or not temperature > 0:
         return False
     if torch.is_autocast_enabled(base.device.type):      # the similarity products would change their type under the fp32 kernels
@@ -90,7 +116,7 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
             return False
     w = encoder.weights
     return base.shape[1] == w[0].shape[1] and w[0].shape[0] <= 2048 and all(
-        a.shape[0] == b.shape[1] for a, b in zip(w[:-1], w[1:]))
+        a.shape[0] == b.shape[1] for a, b in zip(w[:-1], w[1:])) and not _accumulation_held(params)
 
 
 def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: float, seed: Optional[int]) -> torch.Tensor:

@@ -698,3 +698,25 @@ def test_replaced_methods_of_one_module_or_parameter_are_still_heard():
     lin.bias.accumulate = lambda grad: calls.append(grad)
     trained(lin)
     assert len(calls) == 2 and all(torch.equal(p.value, b) for p, b in zip(lin.parameters(), before))
+
+
+def test_contrastive_step_runs_the_hooks_of_accumulation_nodes():
+    from spiraltorch_b200.models import contrastive as M
+    enc = M.ContrastiveEncoder(64, 128, 64, device=DEV, seed=1)
+    base = torch.randn(48, 64, device=DEV)
+    params = list(enc.parameters())
+    M.contrastive_step(enc, base, 0.1, seed=5)
+    want = [p.grad.clone() for p in params]
+    views = [p.expand_as(p) for p in params]                  # graphs that keep the nodes, and with them their hooks, alive
+    seen = []
+    for v in views:
+        v.grad_fn.next_functions[0][0].register_hook(lambda *a: seen.append(1))
+    assert not M._schedulable(enc, base, 0.1)
+    enc.zero_grad(set_to_none=True)
+    M.contrastive_step(enc, base, 0.1, seed=5)
+    assert len(seen) == len(params) == 10
+    assert all((p.grad.float() - w.float()).norm() <= 2e-2 * w.float().norm() for p, w in zip(params, want))
+    views.pop(0)
+    assert not M._schedulable(enc, base, 0.1)
+    del v, views
+    assert M._schedulable(enc, base, 0.1)
