@@ -114,7 +114,7 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
                 and not p._backward_hooks and not getattr(p, "_post_accumulate_grad_hooks", None)
                 and not hasattr(p, "main_grad")):
             return False
-    w = encoder.weights
+    w = list(encoder.weights)      # a slice of a ParameterList builds another one, 20 us each
     return base.shape[1] == w[0].shape[1] and w[0].shape[0] <= 2048 and all(
         a.shape[0] == b.shape[1] for a, b in zip(w[:-1], w[1:])) and not _accumulation_held(params)
 
@@ -130,7 +130,7 @@ def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: floa
         g = torch.Generator(device=dev).manual_seed(seed)
     n1 = torch.randn(base.shape, generator=g, device=dev, dtype=base.dtype)
     n2 = torch.randn(base.shape, generator=g, device=dev, dtype=base.dtype)
-    w, b, gamma, beta = encoder.weights, encoder.biases, encoder.gammas, encoder.betas
+    w, b, gamma, beta = (list(part) for part in (encoder.weights, encoder.biases, encoder.gammas, encoder.betas))
     x = torch.empty((2 * B, width), dtype=torch.bfloat16, device=dev)
     native.check(lib.st_contrastive_views(native.ptr(base), native.ptr(n1), native.ptr(n2), ctypes.c_float(noise), native.ptr(x),
                                           ctypes.c_longlong(B * width), stream), "st_contrastive_views")
