@@ -226,14 +226,13 @@ class Module:
 
     def apply_step(self, fallback_lr: float = 1e-2) -> None:
         plain = [p for p in self.parameters() if _plain(p) and p.trainable and p.gradient is not None]
-        # a gradient of another shape broadcasts, or is refused, in the parameter's own step, and updates that share memory
-        # follow one another there
-        if plain and _multi.takes([t for p in plain for t in (p.value, p.gradient)]) \
-                and not any(p.value.requires_grad or p.gradient.shape != p.value.shape for p in plain) \
-                and _multi.disjoint([p.value for p in plain], [p.gradient for p in plain]):
-            _multi.descend_([p.value for p in plain], [p.gradient for p in plain], fallback_lr)
-            for p in plain:
-                p.gradient = None
+        if plain:
+            values, grads = [p.value for p in plain], [p.gradient for p in plain]
+            # a gradient of another shape broadcasts, or is refused, in the parameter's own step, and updates that share memory
+            # follow one another there
+            if _multi.takes(values + grads) and not any(v.requires_grad for v in values) and _multi.descend_(values, grads, fallback_lr):
+                for p in plain:
+                    p.gradient = None
         for p in self.parameters():
             p.apply_step(fallback_lr)
 

@@ -6,6 +6,7 @@ The callers (:mod:`spiraltorch_b200.nn`) keep their PyTorch statement for tensor
 """
 from __future__ import annotations
 
+import bisect
 import ctypes
 from typing import Optional, Sequence
 
@@ -65,42 +66,38 @@ def divided(tensors: Sequence[torch.Tensor], value: float):
     return out, _run(_DIV, tensors, out, value)
 
 
-def disjoint(written: Sequence[torch.Tensor], read: Sequence[torch.Tensor]) -> bool:
-    """Whether no memory of the dense tensors ``written`` belongs to another of them or to one of ``read``: the blocks of one
-    launch run in any order."""
-    spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size(), own) for ts, own in ((written, True), (read, False)) for t in ts)
-    end = end_written = 0
-    for begin, stop, own in spans:
-        if begin < (end if own else end_written):
-            return False
-        end = max(end, stop)
-        if own:
-            end_written = max(end_written, stop)
-    return True
-
-
-def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: float) -> None:
-    """``v -= lr * g`` for every pair, in place; values and gradients :func:`disjoint`."""
+def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: float) -> bool:
+    """``v -= lr * g`` for every pair, in place.  The blocks of a launch run in any order: False, with nothing done, where memory
+    of a value also belongs to another of the tensors, or where a gradient has not its value's shape."""
     global launch_count
     from . import gemm
-    if len(values) != len(grads) or any(v.numel() != g.numel() for v, g in zip(values, grads)):
-        raise ValueError("descend_: every value needs a gradient of its own size")
+    if any(v.shape != g.shape for v, g in zip(values, grads)):
+        return False
+    at_v, at_g, sizes = [t.data_ptr() for t in values], [t.data_ptr() for t in grads], [t.numel() for t in values]
+    spans = sorted(zip(at_v, sizes))
+    begins = [begin for begin, _ in spans]
+    if any(begin + 4 * n > after for (begin, n), after in zip(spans, begins[1:])):
+        return False
+    for g, n in zip(at_g, sizes):
+        below = bisect.bisect_left(begins, g + 4 * n) - 1        # the last value that begins before the gradient ends
+        if below >= 0 and spans[below][0] + 4 * spans[below][1] > g:
+            return False
     lib, stream = native.lib(), native.stream_ptr(values[0].device)
     # values whose bf16 copy is in use get the next one in the same launch (a new tensor: a graph may still hold the old one)
     halves = [torch.empty(v.shape, dtype=torch.bfloat16, device=v.device) if gemm.has_cached_bf16(v) else None for v in values]
     for at in range(0, len(values), _MAX):
-        v, g, h = values[at:at + _MAX], grads[at:at + _MAX], halves[at:at + _MAX]
-        n = len(v)
+        part = slice(at, at + _MAX)
+        n = len(values[part])
         array = ctypes.c_void_p * n
         native.check(lib.st_multi_step_bf16(
-            ctypes.c_int(n), array(*[t.data_ptr() for t in g]), array(*[t.data_ptr() for t in v]),
-            array(*[None if t is None else t.data_ptr() for t in h]), (ctypes.c_longlong * n)(*[t.numel() for t in v]),
-            ctypes.c_float(lr), stream), "st_multi_step_bf16")
+            ctypes.c_int(n), array(*at_g[part]), array(*at_v[part]), array(*[None if t is None else t.data_ptr() for t in halves[part]]),
+            (ctypes.c_longlong * n)(*sizes[part]), ctypes.c_float(lr), stream), "st_multi_step_bf16")
         launch_count += 1
     for v, h in zip(values, halves):
         torch.autograd.graph.increment_version(v)      # copies of the values are cached by version
         if h is not None:
             gemm.renew_cached_bf16(v, h)
+    return True
 
 
 def to_bf16(tensors: Sequence[torch.Tensor]):
