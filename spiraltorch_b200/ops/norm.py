@@ -18,15 +18,14 @@ import torch
 from . import native
 
 launch_count = 0
-_scratch: dict = {}
 
 
-def _get_scratch(device, elems: int) -> torch.Tensor:
-    buf = _scratch.get(device)
-    if buf is None or buf.numel() < elems:
-        buf = torch.empty(max(elems, 1 << 20), dtype=torch.float32, device=device)
-        _scratch[device] = buf
-    return buf
+def _scratch(lib, x2: torch.Tensor) -> torch.Tensor:
+    """Partial parameter gradients of one backward call.  A tensor per call: a buffer kept for a device would be shared by its
+    streams and threads, and a captured step would go on writing to it after a larger call had replaced it."""
+    lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
+    elems = lib.st_norm_bwd_scratch_elems(ctypes.c_int(x2.shape[0]), ctypes.c_int(x2.shape[1]))
+    return torch.empty(elems, dtype=torch.float32, device=x2.device)
 
 
 def takes_f32(d: int, *tensors: Optional[torch.Tensor]) -> bool:
@@ -111,9 +110,7 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
         return dx if out is None else out.copy_(dx)
     dx = torch.empty_like(x2) if out is None else out
     lib = native.lib()
-    lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
-    need = lib.st_norm_bwd_scratch_elems(ctypes.c_int(rows), ctypes.c_int(d))
-    scratch = _get_scratch(x2.device, int(need))
+    scratch = _scratch(lib, x2)
     st = _form(lib, "st_norm_bwd", x2, rounded)(
         ctypes.c_int(int(rms)), native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(mean),
         native.ptr(rstd), native.ptr(dres), native.ptr(dx), native.ptr(dgamma), native.ptr(dbeta),
@@ -144,8 +141,7 @@ def norm_gelu_backward(dy2, x2, gamma, beta, mean, rstd, dgamma: torch.Tensor, d
     native.require_cuda("norm_gelu_backward", dy2, x2, gamma, beta, mean, rstd, dgamma, dbeta)
     rows, d = x2.shape
     lib = native.lib()
-    lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
-    scratch = _get_scratch(x2.device, int(lib.st_norm_bwd_scratch_elems(ctypes.c_int(rows), ctypes.c_int(d))))
+    scratch = _scratch(lib, x2)
     dx = torch.empty_like(x2)
     native.check(lib.st_norm_gelu_bwd(
         native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(beta), native.ptr(mean), native.ptr(rstd), native.ptr(dx),

@@ -725,3 +725,33 @@ def test_contrastive_step_runs_the_hooks_of_accumulation_nodes():
     assert not M._schedulable(enc, base, 0.1)
     del v, views
     assert M._schedulable(enc, base, 0.1)
+
+
+@pytest.mark.parametrize("form", ["bf16", "fp32", "gelu"])
+def test_captured_norm_backward_keeps_its_own_scratch(form):
+    """A larger eager backward between capture and replay, with its memory handed on to other tensors."""
+    dtype = torch.float32 if form == "fp32" else torch.bfloat16
+    g, b = torch.randn(768, device=DEV).to(dtype), torch.randn(768, device=DEV).to(dtype)
+
+    def inputs(rows):
+        return torch.randn(rows, 768, device=DEV).to(dtype), torch.randn(rows, 768, device=DEV).to(dtype)
+
+    def backward(x, dy, dg, db):
+        if form == "gelu":
+            _, mean, rstd = N.norm_gelu_forward(x, g, b, 1e-5)
+            return N.norm_gelu_backward(dy, x, g, b, mean, rstd, dg, db)
+        _, _, mean, rstd = N.norm_forward(x, g, b, 1e-5, False)
+        return N.norm_backward(dy, x, g, mean, rstd, False, dg, db, False)
+    x, dy = inputs(64)
+    dg, db, want_g, want_b = (torch.zeros(768, device=DEV) for _ in range(4))
+    want = backward(x, dy, want_g, want_b).clone()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        dx = backward(x, dy, dg, db)
+    backward(*inputs(20000), torch.zeros_like(dg), torch.zeros_like(db))
+    other = [torch.full((1 << 18,), 3.0, device=DEV) for _ in range(16)]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(dx, want) and torch.equal(dg, want_g) and torch.equal(db, want_b)
+    assert all(bool((t == 3.0).all()) for t in other)
