@@ -755,3 +755,18 @@ def test_captured_norm_backward_keeps_its_own_scratch(form):
     torch.cuda.synchronize()
     assert torch.equal(dx, want) and torch.equal(dg, want_g) and torch.equal(db, want_b)
     assert all(bool((t == 3.0).all()) for t in other)
+
+
+def test_tensor_lists_of_very_different_sizes():
+    """Blocks by size: one tensor that fills the chip between small ones, and the last element of each found."""
+    from spiraltorch_b200.ops import multi
+    sizes = [3, 40_000_003, 1, 1025, 1_300_000]
+    ts = [torch.randn(n, device=DEV) for n in sizes]
+    out, bad = multi.divided(ts, 3.0)
+    assert bad is None and all(torch.equal(o[-2000:].cpu(), t[-2000:].cpu() / 3.0) for o, t in zip(out, ts))
+    values = [torch.randn(n, device=DEV) for n in sizes]
+    want = [v - 0.25 * t for v, t in zip(values, ts)]
+    assert multi.descend_(values, ts, 0.25) and all(torch.equal(v, w) for v, w in zip(values, want))
+    for k in (4, 3, 2, 1, 0):
+        ts[k][-1] = float("nan")
+        assert multi.first_nonfinite(ts) == k and multi.divided(ts, 2.0)[1] == k
