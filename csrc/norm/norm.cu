@@ -843,6 +843,14 @@ ST_API int st_norm_bwd_noalloc(int rms, const void* dy, const void* x, const voi
     if (p == nullptr) return st::fail(ST_ERR_CUDA, "norm_bwd_noalloc: cudaGetSymbolAddress returned null");
     g_noalloc_ptr[dev] = p;
   }
-  return st::norm_bwd_launch(rms, dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate,
-                             g_noalloc_ptr[dev], rows, d, st::norm_bwd_grid(rows), reinterpret_cast<cudaStream_t>(stream_v));
+  // Up to 1024 features a CTA has 32 to 128 threads, and two of them leave an SM idle: as many as the regular entry takes, if the
+  // array holds their partials and each has 16 rows (below that the sum over the partials grows faster than the rows shrink:
+  // 1024 rows of 768 take 10.5 us with two per SM and 12.5 with 512).  16384 rows, RMSNorm, with two per SM and now: 256 features
+  // 41 and 21 us, 768 features 50 and 31, 1024 features 62 and 42.
+  const int least = st::norm_bwd_grid(rows), room = ST_NORM_BWD_NOALLOC_MAX_ELEMS / (2 * d);
+  int grid = st::norm_bwd_grid_for(rows, d);
+  grid = grid < room ? grid : room;
+  grid = grid < rows / 16 ? grid : rows / 16;
+  return st::norm_bwd_launch(rms, dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate, g_noalloc_ptr[dev], rows, d,
+                             grid > least ? grid : least, reinterpret_cast<cudaStream_t>(stream_v));
 }

@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 
 namespace st {
-// CTAs (= number of partials) used by the entry point that owns its scratch (2 per SM) and by the
+// CTAs (= number of partials) that the entry point with its own scratch takes at least (2 per SM), and those of the
 // regular entry point (as many as stay resident for this feature dimension).
 int norm_bwd_grid(int rows);
 int norm_bwd_grid_for(int rows, int d);

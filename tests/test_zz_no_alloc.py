@@ -86,6 +86,13 @@ def test_noalloc_matches_scratch_entry_point_twice_in_a_row():
     _run_pair(lib, True, 64, 8192, seed=3)
 
 
+def test_noalloc_with_as_many_partials_as_its_array_holds():
+    lib = native.lib()
+    for rms in (True, False):
+        for rows, d in ((3, 64), (5001, 64), (6000, 768), (6000, 1024), (2000, 1032)):
+            _run_pair(lib, rms, rows, d, seed=rows + d)
+
+
 def test_noalloc_rejects_oversized_problem():
     lib = native.lib()
     d, rows = 8192, 4096
