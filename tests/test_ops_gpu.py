@@ -447,3 +447,20 @@ def test_gelu_and_its_derivative_in_fp32():
     special = torch.tensor([float("inf"), float("-inf"), float("nan"), 1.0] * 8, device="cuda").bfloat16()
     y, ref = E.gelu(special).float(), torch.nn.functional.gelu(special.float(), approximate="tanh")
     assert torch.equal(y.isnan(), ref.isnan()) and (y[special == float("inf")] == float("inf")).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("std,value,slope", [(0.3, 7.3e-9, 2.18e-8), (0.5, 1.27e-8, 2.38e-8), (1.0, 2.5e-8, 3.0e-8)])
+def test_gelu_is_no_further_from_64_bits_than_with_tanhf(std, value, slope):
+    """Root mean square errors over pre-activations of the language models' spread; the bounds are those of the same expressions
+    over tanhf."""
+    torch.manual_seed(5)
+    x = (torch.randn(1 << 16, 8, device="cuda") * std).bfloat16()
+    one = torch.eye(8, device="cuda").bfloat16()
+    xd = x.double().requires_grad_()
+    want = torch.nn.functional.gelu(xd, approximate="tanh")
+    want.sum().backward()
+    got = G.gemm(x, one, act="gelu", out_dtype=torch.float32)
+    grad = G.gemm(torch.ones_like(x), one, act="gelu_bwd", aux_in=x, out_dtype=torch.float32)
+    assert (got - want).pow(2).mean().sqrt().item() <= value
+    assert (grad - xd.grad).pow(2).mean().sqrt().item() <= slope
