@@ -231,3 +231,18 @@ def test_preprocessing_does_not_depend_on_the_default_dtype():
     finally:
         torch.set_default_dtype(torch.float32)
     assert got.dtype == torch.float32 and torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 1), (7, 31), (5, 1023), (1184, 1024), (1184, 1025), (1185, 1025), (3, 4096), (3, 4097), (1300, 65)])
+def test_rank_of_one_value(rows, cols):
+    """The arg-max form and the lists on both sides of the rule between them; ties go to the lower column."""
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, cols) * 3).round() + 0.0
+    x[torch.rand(rows, cols) < 0.05] = float("inf")
+    x[torch.rand(rows, cols) < 0.05] = float("nan")
+    x[-1] = float("-inf")
+    for kind in ("topk", "bottomk"):
+        cv, ci = R.rank_select(x, 1, kind)
+        gv, gi = R.rank_select(x.cuda(), 1, kind)
+        assert torch.equal(ci, gi.cpu()) and torch.equal(torch.nan_to_num(cv, nan=-7.0), torch.nan_to_num(gv.cpu(), nan=-7.0))
