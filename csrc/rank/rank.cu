@@ -651,6 +651,21 @@ __global__ void gather_candidates_kernel(const float* const* __restrict__ vals, 
 
 }  // namespace
 
+// Whether the radix select and the sort of its range (key_slots) beat the sort of the whole row (padded columns).  The select is
+// a chain of histograms, about 17 us for one row and 150 to 200 for 4096, whatever the row's length; the sort grows with it.
+// Sort against select, in us: 4096 rows of 64: 9.6 and 160, of 256: 39 and 178, of 512: 90 and 182 (k = 32 and less), of 606:
+// 217 and 189; k = 128 217 and 214; k = 250 218 and 235.  600 rows of 1000: k = 32 45 and 41, k = 250 45 and 49; one row 16 and
+// 18.  Top and bottom have one boundary to find: 1000 rows of 606, k = 200 59 and 47, k = 500 59 and 63.  From 2048 columns on the
+// sort loses (1 x 1500 30 and 15, 4096 x 4096 1108 and 215), except for a few rows with a range of half the row (1 x 2000,
+// k = 1000: 30 and 34).
+static bool range_pays(int rows, int padded, int key_slots, int mode) {
+  const int sms = st::sm_count();
+  if (2 * key_slots > padded || padded <= 512) return false;
+  if (padded > 1024) return padded > 2048 || mode != MID || 2 * key_slots < padded || rows >= sms / 2;
+  if (mode != MID) return rows >= 4 * sms && (key_slots <= 256 || rows >= 16 * sms);
+  return rows >= (key_slots <= 32 ? 2 : 16) * sms && key_slots <= 128;
+}
+
 // mode: 0 top, 1 bottom, 2 mid.  in: fp32 [rows, cols]; out_v fp32 [rows, k]; out_i int32 [rows, k].
 ST_API int st_rank_select(const float* in, float* out_v, int* out_i, int rows, int cols, int k, int mode,
                           void* stream_v) {
@@ -679,10 +694,7 @@ ST_API int st_rank_select(const float* in, float* out_v, int* out_i, int rows, i
     ST_CUDA_CHECK(cudaFuncSetAttribute(rank_range_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4096 * 8 + 8192 * 4));
     cfg[dev] = true;
   }
-  // The select pays where the range's sort is narrower than the row's, but for a few short rows its chain of histograms is
-  // longer than the whole sort: 5 rows of 606 take 18 us against 16, 5 of 2000 23 against 30, 2000 of 606 93 against 111.
-  const bool few_short = padded <= 1024 && rows < 4 * st::sm_count();
-  if (2 * key_slots <= padded && !few_short) {
+  if (range_pays(rows, padded, key_slots, mode)) {
     const size_t range_smem = (size_t)key_slots * sizeof(unsigned long long) + (size_t)cols * sizeof(unsigned);
     rank_range_kernel<<<rows, RANGE_THREADS, range_smem, s>>>(in, out_v, out_i, cols, k, mode, key_slots);
     ST_CUDA_CHECK(cudaGetLastError());

@@ -246,3 +246,17 @@ def test_rank_of_one_value(rows, cols):
         cv, ci = R.rank_select(x, 1, kind)
         gv, gi = R.rank_select(x.cuda(), 1, kind)
         assert torch.equal(ci, gi.cpu()) and torch.equal(torch.nan_to_num(cv, nan=-7.0), torch.nan_to_num(gv.cpu(), nan=-7.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,k,kind", [(2500, 64, 8, "midk"), (700, 512, 200, "topk"), (295, 1024, 32, "midk"), (296, 513, 32, "midk"), (296, 600, 33, "midk"),
+                                              (2368, 601, 128, "midk"), (592, 700, 256, "bottomk"), (592, 1000, 500, "topk"), (2368, 1000, 500, "bottomk"),
+                                              (1, 2000, 1000, "midk"), (74, 1025, 1000, "midk"), (3, 2048, 512, "midk"), (1, 4100, 4000, "topk")])
+def test_rank_sort_and_select_on_both_sides_of_their_rule(rows, cols, k, kind):
+    """Values of few kinds, so that both boundary values of a range have ties inside and outside it."""
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, cols) * 4).round() / 2 + 0.0
+    x[0, ::3] = float("nan")
+    cv, ci = R.rank_select(x, k, kind)
+    gv, gi = R.rank_select(x.cuda(), k, kind)
+    assert torch.equal(ci, gi.cpu()) and torch.equal(torch.nan_to_num(cv, nan=-7.0), torch.nan_to_num(gv.cpu(), nan=-7.0))
