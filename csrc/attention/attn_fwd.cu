@@ -1041,9 +1041,14 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
     if (int e = st::attn_key_bias(a->key_bias, a->kb_sb, a->kb_sh, a->lengths, bias_ws, a->B, a->H, a->Sk, &p.kp_sb, &p.kp_sh, s)) return e;
     p.kb_pad = bias_ws;
   }
-  // Two query tiles per CTA halve the CTAs: while pairs do not fill the chip twice, single tiles finish earlier (16 heads of
-  // 777, D = 128: 14.6 us against 21.2; four such batches 36.3 against 37.5; 12 heads of 512, D = 64, batch 8: 20.4 against 21.2)
-  const bool few_pairs = !keyb && !out32 && (long long)((p.n_q + 1) / 2) * a->H * a->B < 2ll * st::sm_count();
+  // Two query tiles per CTA halve the CTAs.  Where single tiles need no more rounds over the chip than pairs do, they finish
+  // earlier, because each is shorter: 16 heads of 777, D = 128, 64 pairs or 112 tiles, causal: 18.8 us in pairs, 15.0 in tiles.
+  // One round more and they lose: two such batches (128 pairs, 224 tiles) 19.8 and 21.8, 2 x 2048 x 16 heads (256, 512) 42.3 and
+  // 65.5.  A single tile per head gains nothing (16 heads of 128: 7.5 and 8.5).  With two rounds of causal items the short pairs
+  // fill the second one: 40 heads of 896 (160, 280) 22.9 and 25.9 against 40.6 and 29.4 without the mask.
+  const long long pairs = (long long)((p.n_q + 1) / 2) * a->H * a->B, tiles = (long long)p.n_q * a->H * a->B, sms = st::sm_count();
+  const bool few_pairs = !keyb && !out32 && p.n_q > 1 && (tiles + sms - 1) / sms == (pairs + sms - 1) / sms &&
+                         (tiles <= sms || !a->causal || p.n_q <= 3);
   if ((!biased || keyb) && g_pair_kernel && !few_pairs) {
     // two query tiles per CTA: the items are (query pair, head, batch)
     if (g_pair_trace_on) ST_CUDA_CHECK(cudaGetSymbolAddress(reinterpret_cast<void**>(&p.trace), g_pair_trace));

@@ -770,3 +770,15 @@ def test_tensor_lists_of_very_different_sizes():
     for k in (4, 3, 2, 1, 0):
         ts[k][-1] = float("nan")
         assert multi.first_nonfinite(ts) == k and multi.divided(ts, 2.0)[1] == k
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B,S,H,D", [(1, 128, 16, 128), (1, 777, 16, 64), (2, 777, 16, 64), (1, 300, 98, 64), (1, 896, 40, 64), (1, 129, 74, 128), (1, 129, 75, 128)])
+def test_attention_in_pairs_and_single_tiles(B, S, H, D, causal):
+    """On both sides of the rule between the two kernels: one tile per head, one round of either, two rounds, one round more in
+    single tiles.  P is bf16: 2^-8 of the largest value."""
+    torch.manual_seed(S + H)
+    q, k, v = (torch.randn(B, S, H, D, device=DEV).bfloat16() for _ in range(3))
+    o, lse = A.attention_forward(q, k, v, causal)
+    ro, rlse = A.attention_reference(q, k, v, causal, 1 / math.sqrt(D))
+    assert (o.float() - ro).abs().max() <= 2e-2 * ro.abs().max() and (lse - rlse).abs().max() < 1e-2
