@@ -107,17 +107,18 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __rest
   if (threadIdx.x == 0 && cc < cols) atomicAdd(out + cc, t);
 }
 
-// Vectorised variant: each thread owns 8 adjacent columns (one 16-byte load per row); blockDim.x threads cover the
-// columns of the block and the rest of the 256 are row lanes, so narrow matrices (64 channels: 8 of 32 threads had
-// columns, 47 us for 134 MB) keep every thread loading.  Four rows are in flight per thread.  Needs cols % 8 == 0 and
-// 16-byte aligned rows.
+// Vectorised variant: each thread owns 8 adjacent columns (one 16-byte load per row); BX threads cover the columns of the
+// block and LANES row lanes share its rows, so narrow matrices (64 channels: 8 of 32 threads had columns, 47 us for 134 MB)
+// keep every thread loading.  Four rows are in flight per thread.  Needs cols % 8 == 0 and 16-byte aligned rows.  Both are
+// compile-time: with strides and the sum over the lanes left to run time, 2048 x 2048 took 6.5 us and takes 4.2.
 // STORE (one chunk of rows only): the sums replace what is there, so the caller needs no cleared output.
-template <bool STORE>
-__global__ void __launch_bounds__(256)
+template <int BX, int LANES, bool STORE>
+__global__ void __launch_bounds__(BX * LANES)
 colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long rows, int cols, long long ld) {
-  __shared__ float sh[256 * 8 + 32];
-  const int lanes = blockDim.y, width = blockDim.x * 8;
-  const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  constexpr int WIDTH = BX * 8, PARTS = BX * LANES / WIDTH, lanes = LANES;      // PARTS threads add a column's lanes
+  __shared__ float sh[LANES * (WIDTH + 1)];
+  __shared__ float part[PARTS > 1 ? PARTS * WIDTH : 1];
+  const int c0 = (blockIdx.x * BX + threadIdx.x) * 8;
   const long long rows_per = (rows + gridDim.y - 1) / gridDim.y;
   const long long r0 = blockIdx.y * rows_per;
   const long long r1 = min(rows, r0 + rows_per);
@@ -153,13 +154,21 @@ colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, lon
     }
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) sh[threadIdx.y * (width + 1) + threadIdx.x * 8 + j] = acc[j];
+  for (int j = 0; j < 8; ++j) sh[threadIdx.y * (WIDTH + 1) + threadIdx.x * 8 + j] = acc[j];
   __syncthreads();
-  const int t = threadIdx.y * blockDim.x + threadIdx.x;
-  if (t >= width) return;
+  const int t = threadIdx.y * BX + threadIdx.x, col = t % WIDTH;
   float s = 0.0f;
-  for (int y = 0; y < lanes; ++y) s += sh[y * (width + 1) + t];
-  const int c = blockIdx.x * width + t;
+#pragma unroll
+  for (int y = 0; y < LANES / PARTS; ++y) s += sh[(t / WIDTH + y * PARTS) * (WIDTH + 1) + col];
+  if constexpr (PARTS > 1) {
+    part[t] = s;
+    __syncthreads();
+    if (t >= WIDTH) return;
+    s = 0.0f;
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p) s += part[p * WIDTH + col];
+  }
+  const int c = blockIdx.x * WIDTH + col;
   if (c >= cols) return;
   if (STORE) out[c] = s;
   else atomicAdd(out + c, s);
@@ -562,9 +571,9 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
     int chunks = (int)((rows + 255) / 256);
     if (chunks < 1) chunks = 1;
     if (chunks > 512) chunks = 512;
-    int bx = 8;
-    while (bx < 32 && bx * 8 < cols) bx <<= 1;
-    colsum8_kernel<false><<<dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+    const int bx = cols <= 64 ? 8 : (cols <= 128 ? 16 : 32);
+    auto kern = bx == 8 ? colsum8_kernel<8, 32, false> : (bx == 16 ? colsum8_kernel<16, 16, false> : colsum8_kernel<32, 8, false>);
+    kern<<<dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
         static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
@@ -585,9 +594,13 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
 ST_API int st_colsum_short(const void* x, float* out, long long rows, int cols, long long ld, void* stream_v) {
   if (!x || !out || rows <= 0 || rows > 1024 || cols <= 0 || (cols & 7) || (ld & 7) || (reinterpret_cast<uintptr_t>(x) & 15))
     return st::fail(ST_ERR_INVALID, "colsum_short: bad arguments");
-  const int bx = 8;       // 32 row lanes per column group, and as many CTAs as the columns give
-  colsum8_kernel<true><<<dim3((cols + bx * 8 - 1) / (bx * 8), 1), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
-      static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
+  // As many CTAs as the columns give.  Up to one per SM, enough row lanes that each has its rows in flight at once (1024 x 264
+  // 3.5 us, with 32 lanes 6.4); above, CTAs of 1024 threads crowd one another out (256 x 32768 8.0 us, with 32 lanes 3.9).
+  auto X = static_cast<const __nv_bfloat16*>(x);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  const unsigned narrow = (cols + 63) / 64;
+  if (rows <= 128 || narrow > (unsigned)st::sm_count()) colsum8_kernel<8, 32, true><<<narrow, dim3(8, 32), 0, s>>>(X, out, rows, cols, ld);
+  else colsum8_kernel<8, 128, true><<<narrow, dim3(8, 128), 0, s>>>(X, out, rows, cols, ld);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }

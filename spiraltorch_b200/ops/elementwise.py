@@ -116,7 +116,8 @@ def colsum(x2: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: boo
     """fp32 column sums of a bf16 ``[rows, cols]`` matrix (bias gradients)."""
     global launch_count
     rows, cols = x2.shape
-    if out is None and 0 < rows <= 1024 and cols % 8 == 0 and cols > 0 and native.use_native(x2) and x2.dtype == torch.bfloat16 \
+    # one launch for a matrix that stays in L2; larger ones are read in more pieces than the columns give
+    if out is None and 0 < rows <= 1024 and rows * cols <= 1 << 25 and cols % 8 == 0 and cols > 0 and native.use_native(x2) and x2.dtype == torch.bfloat16 \
             and x2.stride(-1) == 1 and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0:
         out = torch.empty(cols, dtype=torch.float32, device=x2.device)
         native.check(native.lib().st_colsum_short(native.ptr(x2), native.ptr(out), ctypes.c_longlong(rows), ctypes.c_int(cols),

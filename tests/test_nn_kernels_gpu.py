@@ -782,3 +782,14 @@ def test_attention_in_pairs_and_single_tiles(B, S, H, D, causal):
     o, lse = A.attention_forward(q, k, v, causal)
     ro, rlse = A.attention_reference(q, k, v, causal, 1 / math.sqrt(D))
     assert (o.float() - ro).abs().max() <= 2e-2 * ro.abs().max() and (lse - rlse).abs().max() < 1e-2
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 64), (128, 72), (129, 8), (129, 9472), (513, 9480), (700, 136), (1030, 64), (1030, 72), (2000, 128), (300, 136), (1000, 37888)])
+def test_column_sums_on_both_sides_of_their_rules(rows, cols):
+    """Lanes and widths of both forms, columns and rows that fill none of them; fp32 sums of terms of order one."""
+    from spiraltorch_b200.ops import elementwise as E
+    x = torch.randn(rows, cols, device=DEV).bfloat16()
+    want = x.double().sum(0)
+    acc = torch.full((cols,), 2.0, device=DEV)
+    assert torch.allclose(E.colsum(x).double(), want, rtol=1e-5, atol=1e-4)
+    assert torch.allclose(E.colsum(x, acc, accumulate=True).double(), want + 2.0, rtol=1e-5, atol=1e-4)
