@@ -644,7 +644,11 @@ ST_API int st_norm_fwd(int rms, const void* x, const void* residual, const void*
   auto B = static_cast<const __nv_bfloat16*>(beta);
   auto Y = static_cast<__nv_bfloat16*>(y);
   auto S = static_cast<__nv_bfloat16*>(sum_out);
-  if (d <= kWarpRowFeatures) return fwd_warp<__nv_bfloat16>(rms, X, R, G, B, Y, S, mean, rstd, rows, d, eps, s);
+  // A warp per row, or a block while that leaves SMs without enough warps: 600 rows of 1024, LayerNorm 4.2 us in warps and 3.0 in
+  // blocks (RMSNorm 3.2, 2.4), of 512 both 2.9; 1500 rows 4.7 and 4.5, 3000 4.8 and 6.2.  Up to 256 features the warp has one
+  // vector per lane and never loses.
+  const bool few = rows <= (d > 512 ? 8 : 4) * st::sm_count() && d > 256;
+  if (d <= kWarpRowFeatures && !few) return fwd_warp<__nv_bfloat16>(rms, X, R, G, B, Y, S, mean, rstd, rows, d, eps, s);
 #define ST_NORM_FWD(RMSV, MVV) norm_fwd_kernel<RMSV, MVV><<<rows, NT, 0, s>>>(X, R, G, B, Y, S, mean, rstd, rows, d, eps)
   const int mv = d <= NT * 8 ? 1 : (d <= NT * 16 ? 2 : 4);
   if (rms) {

@@ -541,9 +541,9 @@ def test_trainer_still_refuses_gradients_that_overflow_in_accumulation():
     assert all(p.gradient is None for p in lin.parameters())
 
 
-@pytest.mark.parametrize("rows,d,residual", [(1, 8, False), (33, 128, True), (2500, 264, False), (640, 1024, True)])
+@pytest.mark.parametrize("rows,d,residual", [(1, 8, False), (33, 128, True), (2500, 264, False), (1300, 1024, True)])
 def test_layer_norm_of_fp32_tensors_has_the_values_of_the_bf16_form(rows, d, residual):
-    """Bit for bit: operands, output and input gradient are bf16 values wherever the tensors are fp32.  A wider result moved
+    """Bit for bit, where both take the same kernel: operands, output and input gradient are bf16 values wherever the tensors are fp32.  A wider result moved
     elements across the ReLU behind it, and with them whole gradients of small batches."""
     torch.manual_seed(rows + d)
     x, dy = torch.randn(rows, d, device=DEV), torch.randn(rows, d, device=DEV)
@@ -793,3 +793,26 @@ def test_column_sums_on_both_sides_of_their_rules(rows, cols):
     acc = torch.full((cols,), 2.0, device=DEV)
     assert torch.allclose(E.colsum(x).double(), want, rtol=1e-5, atol=1e-4)
     assert torch.allclose(E.colsum(x, acc, accumulate=True).double(), want + 2.0, rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,d", [(592, 264), (593, 512), (1184, 520), (1185, 1024), (1, 1024), (296, 64), (297, 768), (1184, 72), (1185, 72), (1, 8)])
+def test_norm_on_both_sides_of_its_rules(rows, d, rms):
+    """Forward by a block or a warp per row, backward by a block per row, in steps of two rows, and with two steps per CTA."""
+    torch.manual_seed(rows + d)
+    x, dy = (torch.randn(rows, d, device=DEV).bfloat16() for _ in range(2))
+    g, b = torch.randn(d, device=DEV).bfloat16(), (None if rms else torch.randn(d, device=DEV).bfloat16())
+    y, _, mean, rstd = N.norm_forward(x, g, b, 1e-5, rms)
+    xd = x.double()
+    mu = 0 if rms else xd.mean(-1, keepdim=True)
+    rs = torch.rsqrt((xd - mu).pow(2).mean(-1, keepdim=True) + 1e-5)
+    xh = (xd - mu) * rs
+    want = xh * g.double() + (0 if rms else b.double())
+    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all()
+    dg, db = torch.full((d,), 0.5, device=DEV), (None if rms else torch.full((d,), 0.25, device=DEV))
+    dx = N.norm_backward(dy, x, g, mean, rstd, rms, dg, db, True)
+    gy = dy.double() * g.double()
+    want = rs * (gy - (0 if rms else gy.mean(-1, keepdim=True)) - xh * (gy * xh).mean(-1, keepdim=True))
+    assert ((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2e-5).all()
+    assert torch.allclose(dg.double(), 0.5 + (dy.double() * xh).sum(0), rtol=1e-5, atol=1e-3)
+    assert rms or torch.allclose(db.double(), 0.25 + dy.double().sum(0), rtol=1e-5, atol=1e-3)
