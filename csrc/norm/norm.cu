@@ -568,6 +568,7 @@ constexpr int kWarpRowFeatures = 1024;   // forward, fp32 form
 constexpr int kRowsThreads = 768;
 inline bool rows_kernel(int rms, int d) { return d <= kWarpRowFeatures || (!rms && d <= NT * 8); }
 inline int bwd_threads(int d) { return (d + 255) / 256 * 32; }
+inline int step_grid(int grid, int rows) { return grid < (rows + 1) / 2 ? grid : (rows + 1) / 2; }      // at most a CTA per step of two rows
 
 template <typename T>
 int fwd_warp(int rms, const T* x, const T* r, const T* g, const T* b, T* y, T* s, float* mean, float* rstd, int rows, int d,
@@ -616,8 +617,11 @@ int norm_bwd_grid(int rows) {
 // CTAs for the regular entry: as many as stay resident (register footprint grows with d)
 int norm_bwd_grid_for(int rows, int d) {
   if (d <= kWarpRowFeatures) {
+    // Two rows per CTA are one step; four as soon as the chip is full, because the sum over the partials grows with the CTAs:
+    // 4000 rows of 264, RMSNorm, 12.9 us with two, 10.3 with four, 11.4 with eight; 600 rows 5.5, 6.9, 9.1.
+    if (rows <= 2 * sm_count()) return rows;
     const int resident = kRowsThreads / bwd_threads(d);
-    const int need = (rows + 1) / 2, most = sm_count() * (resident < 16 ? resident : 16);
+    const int need = rows <= 6 * sm_count() ? (rows + 1) / 2 : (rows + 3) / 4, most = sm_count() * (resident < 16 ? resident : 16);
     return need < most ? need : most;
   }
   const int per_sm = d <= 2048 ? 4 : 2;
@@ -679,7 +683,15 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   auto G = static_cast<const __nv_bfloat16*>(gamma);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
+  // few rows: a block per row is one step without a second row's share (64 x 264 4.0 us, in pairs 4.9; 600 x 264 7.4 and 5.5)
+  if (rms && rows <= 2 * st::sm_count() && d <= NT * 8) {
+    grid = grid < rows ? grid : rows;
+    rms_bwd_ahead_kernel<<<grid, NT, 0, s>>>(DY, X, G, rstd, DR, DX, pg, rows, d);
+    ST_CUDA_CHECK(cudaGetLastError());
+    return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
+  }
   if (rows_kernel(rms, d)) {
+    grid = step_grid(grid, rows);
     if (d > kWarpRowFeatures && grid > st::sm_count() * 3) grid = st::sm_count() * 3;      // 768 of 256 threads
     if (int e = bwd_rows<__nv_bfloat16>(rms, DY, X, G, mean, rstd, DR, DX, pg, rms ? nullptr : pb, rows, d, grid, s)) return e;
     return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
@@ -737,7 +749,7 @@ ST_API int st_norm_gelu_bwd(const void* dy, const void* x, const void* gamma, co
   if (d > NT * 8) return st::fail(ST_ERR_TOO_LARGE, "norm_gelu: feature dimension above 2048");
   if (!beta || !dbeta || !scratch) return st::fail(ST_ERR_INVALID, "norm_gelu: offset, its gradient and scratch are required");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  int grid = st::norm_bwd_grid_for(rows, d);
+  int grid = step_grid(st::norm_bwd_grid_for(rows, d), rows);
   if (d > kWarpRowFeatures && grid > st::sm_count() * 3) grid = st::sm_count() * 3;
   float* pb = scratch + (size_t)grid * d;
   const __nv_bfloat16* none = nullptr;
@@ -766,7 +778,7 @@ int bwd_f32(int rms, const float* dy, const float* x, const float* gamma, const 
   if (int e = check_dims(rows, d)) return e;
   if (d > kWarpRowFeatures) return st::fail(ST_ERR_TOO_LARGE, "norm_f32: feature dimension above 1024");
   if (!scratch) return st::fail(ST_ERR_INVALID, "norm_f32: scratch buffer is required");
-  const int grid = st::norm_bwd_grid_for(rows, d);
+  const int grid = step_grid(st::norm_bwd_grid_for(rows, d), rows);
   float* pb = scratch + (size_t)grid * d;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   auto in = [](const float* p) { return reinterpret_cast<const T*>(p); };
@@ -848,13 +860,11 @@ ST_API int st_norm_bwd_noalloc(int rms, const void* dy, const void* x, const voi
     g_noalloc_ptr[dev] = p;
   }
   // Up to 1024 features a CTA has 32 to 128 threads, and two of them leave an SM idle: as many as the regular entry takes, if the
-  // array holds their partials and each has 16 rows (below that the sum over the partials grows faster than the rows shrink:
-  // 1024 rows of 768 take 10.5 us with two per SM and 12.5 with 512).  16384 rows, RMSNorm, with two per SM and now: 256 features
-  // 41 and 21 us, 768 features 50 and 31, 1024 features 62 and 42.
+  // array holds their partials.  RMSNorm over 16384 rows of 256 / 768 / 1024 features, with two per SM and now: 38 / 47 / 61 and
+  // 18 / 28 / 40 us (a block per row 39 / 45 / 66).
   const int least = st::norm_bwd_grid(rows), room = ST_NORM_BWD_NOALLOC_MAX_ELEMS / (2 * d);
   int grid = st::norm_bwd_grid_for(rows, d);
   grid = grid < room ? grid : room;
-  grid = grid < rows / 16 ? grid : rows / 16;
   return st::norm_bwd_launch(rms, dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate, g_noalloc_ptr[dev], rows, d,
                              grid > least ? grid : least, reinterpret_cast<cudaStream_t>(stream_v));
 }

@@ -796,7 +796,7 @@ def test_column_sums_on_both_sides_of_their_rules(rows, cols):
 
 
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("rows,d", [(592, 264), (593, 512), (1184, 520), (1185, 1024), (1, 1024), (296, 64), (297, 768), (1184, 72), (1185, 72), (1, 8)])
+@pytest.mark.parametrize("rows,d", [(592, 264), (593, 512), (1184, 520), (1185, 1024), (1, 1024), (296, 64), (297, 768), (888, 72), (889, 72), (1, 8)])
 def test_norm_on_both_sides_of_its_rules(rows, d, rms):
     """Forward by a block or a warp per row, backward by a block per row, in steps of two rows, and with two steps per CTA."""
     torch.manual_seed(rows + d)
