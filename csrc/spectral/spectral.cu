@@ -576,8 +576,11 @@ ST_API int st_fft_1d(const StFftArgs* a, void* stream_v) {
     const bool vec = a->complex_in && a->in_i == 2 && a->out_i == 2 && a->n > 1 &&
                      ((a->in_b0 | a->in_b1 | a->out_b0 | a->out_b1) & 1) == 0 &&
                      ((reinterpret_cast<uintptr_t>(a->in) | reinterpret_cast<uintptr_t>(a->out)) & 7) == 0;
-    // 16-byte aligned rows, and at least one group of 4096 points per SM (below that, a CTA per row spreads the work wider)
-    if (vec && log2n >= 6 && log2n <= 12 && (long long)grid * a->n >= (long long)F16_POINTS * st::sm_count() &&
+    // 16-byte aligned rows, and at least one group of 4096 points per SM (below that, a CTA per row spreads the work wider).  Long
+    // rows fill the chip as well in CTAs of their own, two at once per SM: 296 of 4096 6.6 us and 6.9 streamed, 303 9.1 and 8.3;
+    // 385 of 2048 5.1 and 5.6, 473 6.1 and 5.6.
+    const long long least = a->n == 4096 ? 2ll * st::sm_count() + 1 : (a->n == 2048 ? 3ll * st::sm_count() : (long long)F16_POINTS * st::sm_count() / a->n);
+    if (vec && log2n >= 6 && log2n <= 12 && grid >= least &&
         ((a->in_b0 | a->in_b1) & 3) == 0 && (reinterpret_cast<uintptr_t>(a->in) & 15) == 0) {
       switch (log2n) {
         case 6: return launch_fft16<6>(a->in, a->out, a->window, L, a->inverse, grid, stream);

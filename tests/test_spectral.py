@@ -213,3 +213,13 @@ def test_spectral_outputs_do_not_depend_on_the_default_dtype():
     finally:
         torch.set_default_dtype(torch.float32)
     assert all(a.dtype == torch.float32 and torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,n", [(296, 4096), (297, 4096), (443, 2048), (444, 2048), (592, 1024), (591, 1024)])
+def test_fft_on_both_sides_of_the_streaming_rule(rows, n):
+    x = torch.view_as_complex(torch.randn(rows, n, 2, device="cuda"))
+    want = torch.fft.fft(x.to(torch.complex128))
+    got = spectral.fft(x)
+    assert ((got - want).abs().norm() / want.abs().norm()).item() < 1e-6
+    assert ((spectral.fft(got, inverse=True) - x).abs().norm() / x.abs().norm()).item() < 1e-6
