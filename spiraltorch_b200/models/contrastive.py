@@ -95,9 +95,13 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
         return False
     if torch.is_autocast_enabled(base.device.type):      # the similarity products would change their type under the fp32 kernels
         return False
+    # tangents, transforms, traces and modes see the operators of the autograd form
+    if torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None \
+            or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack():
+        return False
     params = list(encoder.parameters())
     dev = base.device
-    if not (base.is_cuda and base.dtype == torch.float32 and base.dim() == 2 and base.is_contiguous() and base.data_ptr() % 16 == 0
+    if not (type(base) in (torch.Tensor, nn.Parameter) and base.is_cuda and base.dtype == torch.float32 and base.dim() == 2 and base.is_contiguous() and base.data_ptr() % 16 == 0
             and not base.requires_grad and 0 < base.shape[0] <= 12000 and len(params) == 10):
         return False
     for m in encoder.modules():
@@ -109,7 +113,7 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
             or torch._C._autograd._top_saved_tensors_default_hooks(False) is not None:
         return False
     for p in params:
-        if not (p.device == dev and p.dtype == torch.bfloat16 and p.requires_grad and p.is_leaf and p.is_contiguous()
+        if not (type(p) is nn.Parameter and p.device == dev and p.dtype == torch.bfloat16 and p.requires_grad and p.is_leaf and p.is_contiguous()
                 and p.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in p.shape)
                 and not p._backward_hooks and not getattr(p, "_post_accumulate_grad_hooks", None)
                 and not hasattr(p, "main_grad")):

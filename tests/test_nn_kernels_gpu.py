@@ -816,3 +816,25 @@ def test_norm_on_both_sides_of_its_rules(rows, d, rms):
     assert ((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2e-5).all()
     assert torch.allclose(dg.double(), 0.5 + (dy.double() * xh).sum(0), rtol=1e-5, atol=1e-3)
     assert rms or torch.allclose(db.double(), 0.25 + dy.double().sum(0), rtol=1e-5, atol=1e-3)
+
+
+def test_contrastive_step_leaves_tangents_transforms_and_modes_to_the_autograd_form():
+    import torch.autograd.forward_ad as fwAD
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from spiraltorch_b200.models import contrastive as M
+    enc = M.ContrastiveEncoder(64, 128, 64, device=DEV, seed=1)
+    base = torch.randn(48, 64, device=DEV)
+
+    class Count(TorchDispatchMode):
+        ops = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            Count.ops += 1
+            return func(*args, **(kwargs or {}))
+    with Count():
+        assert not M._schedulable(enc, base, 0.1)
+    with fwAD.dual_level():
+        assert not M._schedulable(enc, base, 0.1)
+        with pytest.raises(RuntimeError):
+            M.contrastive_step(enc, fwAD.make_dual(base, torch.ones_like(base)), 0.1, seed=5)
+    assert M._schedulable(enc, base, 0.1)
