@@ -230,7 +230,7 @@ class Module:
             values, grads = [p.value for p in plain], [p.gradient for p in plain]
             # a gradient of another shape broadcasts, or is refused, in the parameter's own step, and updates that share memory
             # follow one another there
-            if _multi.takes(values + grads) and not any(v.requires_grad for v in values) and _multi.descend_(values, grads, fallback_lr):
+            if _multi.takes(values + grads) and not any(t.requires_grad for t in values + grads) and _multi.descend_(values, grads, fallback_lr):
                 for p in plain:
                     p.gradient = None
         for p in self.parameters():

@@ -21,8 +21,10 @@ _CHECK, _DIV, _STEP = 0, 1, 2
 
 def takes(tensors: Sequence[torch.Tensor]) -> bool:
     """Whether the kernels take these tensors: dense non-empty fp32 on the current CUDA device, outside a graph capture
-    (a captured stream cannot be waited for)."""
-    if not tensors or not tensors[0].is_cuda or torch.cuda.is_current_stream_capturing():
+    (a captured stream cannot be waited for) and outside function transforms and forward-mode differentiation (whose
+    tensors are more than their memory)."""
+    if not tensors or not tensors[0].is_cuda or torch.cuda.is_current_stream_capturing() \
+            or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
         return False
     dev = tensors[0].device
     return dev.index == torch.cuda.current_device() and all(

@@ -838,3 +838,21 @@ def test_contrastive_step_leaves_tangents_transforms_and_modes_to_the_autograd_f
         with pytest.raises(RuntimeError):
             M.contrastive_step(enc, fwAD.make_dual(base, torch.ones_like(base)), 0.1, seed=5)
     assert M._schedulable(enc, base, 0.1)
+
+
+def test_losses_and_updates_keep_what_belongs_to_their_tensors():
+    """Forward-mode tangents and gradients with a graph go through PyTorch's operators."""
+    import torch.autograd.forward_ad as fwAD
+    p, t = torch.randn(16, 8, device=DEV), torch.randn(16, 8, device=DEV)
+    loss, target = st.nn.MeanSquaredError(), st.Tensor._wrap(t)
+    with fwAD.dual_level():
+        value = loss.forward(st.Tensor._wrap(fwAD.make_dual(p, torch.ones_like(p))), target).torch()
+        tangent = fwAD.unpack_dual(value).tangent
+        assert torch.allclose(tangent, (2 * (p - t)).mean())
+    lin = st.nn.Linear("fc", 8, 8)
+    lin.init_normal(0.1, seed=1)
+    lin.to(DEV)
+    rate = torch.ones((), device=DEV, requires_grad=True)
+    lin.weight.gradient = rate * torch.ones_like(lin.weight.value)
+    lin.apply_step(0.5)
+    assert torch.autograd.grad(lin.weight.value.sum(), rate)[0].item() == -32.0
