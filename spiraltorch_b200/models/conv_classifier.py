@@ -124,7 +124,7 @@ class ConvClassifier(nn.Module):
                 if i == 0:
                     ew.colsum(d.reshape(-1, d.shape[-1]), P[f"conv{s}_0.bias"].main_grad, accumulate=True)
                 if k - 1 > 0:
-                    d = C.conv3x3(d, C.dgrad_weights(w, ic), relu_mask_of=xin)
+                    d = C.conv3x3(d, C.dgrad_weights(w.detach(), ic), relu_mask_of=xin)
                 if layer_done:
                     layer_done(f"conv{s}_{i}")   # after the data gradient has read the weights
                 k -= 1

@@ -46,7 +46,8 @@ def dgrad_weights(w_tap: torch.Tensor, ic: int) -> torch.Tensor:
     """Weights of the data-gradient convolution: ``Wt[ic][kh'][kw'][oc] = W[oc][2-kh'][2-kw'][ic]``."""
     global launch_count
     oc = w_tap.shape[0]
-    if native.use_native(w_tap) and w_tap.dtype == torch.bfloat16 and w_tap.is_contiguous() and w_tap.shape[1] == 9 * ic:
+    if native.use_native(w_tap) and w_tap.dtype == torch.bfloat16 and w_tap.is_contiguous() and w_tap.shape[1] == 9 * ic \
+            and not (w_tap.requires_grad and torch.is_grad_enabled()):
         out = torch.empty((ic, 9 * oc), dtype=torch.bfloat16, device=w_tap.device)
         native.check(native.lib().st_conv3x3_dgrad_weights(native.ptr(w_tap), native.ptr(out), ctypes.c_int(oc), ctypes.c_int(ic),
                                                            native.stream_ptr(w_tap.device)), "st_conv3x3_dgrad_weights")

@@ -196,3 +196,13 @@ def test_conv_with_shared_row_blocks(N, H, W, Cin, OC):
         ref = torch.relu(want + bias.float()) if act == "relu" else torch.where(mask.float() > 0, want, torch.zeros(()))
         err = (got.float().cpu() - ref).abs()
         assert (err <= 2.0 ** -8 * ref.abs() + 1e-4).all()            # one bf16 rounding, fp32 sums of terms of order one
+
+
+@pytest.mark.gpu
+def test_data_gradient_weights_stay_differentiable():
+    w = torch.randn(8, 9 * 16, device="cuda").bfloat16().requires_grad_()
+    out = C.dgrad_weights(w, 16)
+    g = torch.randn_like(out)
+    out.backward(g)
+    with torch.no_grad():
+        assert torch.equal(C.dgrad_weights(w, 16), out) and torch.equal(C.dgrad_weights(w.grad, 16), g)
