@@ -447,7 +447,7 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   GemmParams p{};
   p.conv.mode = 1;
   p.conv.H = a->H; p.conv.W = a->W; p.conv.Hb = Hb; p.conv.Nb = Nb;
-  p.conv.c_chunks = a->C / 64; p.conv.taps = 9;
+  p.conv.c_chunks = a->C / 64;
   p.C = a->y; p.ldc = a->OC;
   p.bias = static_cast<const __nv_bfloat16*>(a->bias);
   p.aux_in = static_cast<const __nv_bfloat16*>(a->aux_in);
@@ -521,7 +521,7 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
   GemmParams p{};
   p.conv.mode = 2;
   p.conv.H = a->H; p.conv.W = a->W; p.conv.Hb = Hb; p.conv.Nb = Nb;
-  p.conv.c_chunks = a->C / 64; p.conv.taps = 9; p.conv.blocks = kblocks_total;
+  p.conv.c_chunks = a->C / 64; p.conv.blocks = kblocks_total;
   p.C = a->dw; p.ldc = N9;
   p.M = a->OC; p.N = (int)N9; p.K = P;
   p.alpha = 1.0f; p.batch = splits; p.batch_stride_c = 0;

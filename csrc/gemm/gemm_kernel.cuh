@@ -78,7 +78,6 @@ struct ConvGeom {
   int H, W;          // image size
   int Hb, Nb;        // rows / images per pixel block (mode 1: 128 pixels, mode 2: 64 pixels)
   int c_chunks;      // input channels / 64
-  int taps;          // 9
   int blocks;        // pixel blocks over all splits (mode 2)
 };
 
@@ -245,10 +244,6 @@ __device__ __forceinline__ void rs_add_batch(int s0, int n_srcs, const uint4 (&b
       }
     }
   }
-}
-
-__device__ __forceinline__ void epilogue_bar() {
-  asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
 // Pixel blocks of split b of a convolution's weight gradient

@@ -119,7 +119,7 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
                 and not hasattr(p, "main_grad")):
             return False
     w = list(encoder.weights)      # a slice of a ParameterList builds another one, 20 us each
-    return base.shape[1] == w[0].shape[1] and w[0].shape[0] <= 2048 and all(
+    return base.shape[1] == w[0].shape[1] and w[0].shape[0] <= norm_ops.gelu_max_features() and all(
         a.shape[0] == b.shape[1] for a, b in zip(w[:-1], w[1:])) and not _accumulation_held(params)
 
 

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import bisect
 import ctypes
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -15,8 +16,7 @@ import torch
 from . import native
 
 launch_count = 0
-_MAX = 48
-_CHECK, _DIV, _STEP = 0, 1, 2
+_CHECK, _DIV = 0, 1
 
 
 def takes(tensors: Sequence[torch.Tensor]) -> bool:
@@ -32,28 +32,33 @@ def takes(tensors: Sequence[torch.Tensor]) -> bool:
         and t.numel() > 0 for t in tensors)
 
 
+@functools.cache
+def _most() -> int:
+    """Tensors that one launch takes."""
+    return native.lib().st_multi_max()
+
+
 def _run(op: int, src, dst, value: float) -> Optional[int]:
-    """Index of the first tensor of ``src`` with a value that is not finite, or None (always None for an update)."""
+    """Index of the first tensor of ``src`` with a value that is not finite, or None."""
     global launch_count
     lib, stream = native.lib(), torch.cuda.current_stream()
     first = None
-    for at in range(0, len(src), _MAX):
-        s = src[at:at + _MAX]
+    for at in range(0, len(src), _most()):
+        s = src[at:at + _most()]
         n = len(s)
         counts = [t.numel() for t in s]
         blocks = lib.st_multi_blocks(ctypes.c_longlong(max(counts)))
-        bad = None if op == _STEP else torch.empty(n * blocks, dtype=torch.int32, pin_memory=True)
+        bad = torch.empty(n * blocks, dtype=torch.int32, pin_memory=True)
         ptrs = (ctypes.c_void_p * n)(*[t.data_ptr() for t in s])
-        outs = None if dst is None else (ctypes.c_void_p * n)(*[t.data_ptr() for t in dst[at:at + _MAX]])
+        outs = None if dst is None else (ctypes.c_void_p * n)(*[t.data_ptr() for t in dst[at:at + _most()]])
         native.check(lib.st_multi(ctypes.c_int(op), ctypes.c_int(n), ptrs, outs, (ctypes.c_longlong * n)(*counts),
-                                  ctypes.c_float(value), None if bad is None else ctypes.c_void_p(bad.data_ptr()),
+                                  ctypes.c_float(value), ctypes.c_void_p(bad.data_ptr()),
                                   ctypes.c_void_p(stream.cuda_stream)), "st_multi")
         launch_count += 1
-        if bad is not None:
-            stream.synchronize()
-            hits = bad.nonzero()
-            if first is None and hits.numel():
-                first = at + int(hits[0]) // blocks
+        stream.synchronize()
+        hits = bad.nonzero()
+        if first is None and hits.numel():
+            first = at + int(hits[0]) // blocks
     return first
 
 
@@ -87,8 +92,8 @@ def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: 
     lib, stream = native.lib(), native.stream_ptr(values[0].device)
     # values whose bf16 copy is in use get the next one in the same launch (a new tensor: a graph may still hold the old one)
     halves = [torch.empty(v.shape, dtype=torch.bfloat16, device=v.device) if gemm.has_cached_bf16(v) else None for v in values]
-    for at in range(0, len(values), _MAX):
-        part = slice(at, at + _MAX)
+    for at in range(0, len(values), _most()):
+        part = slice(at, at + _most())
         n = len(values[part])
         array = ctypes.c_void_p * n
         native.check(lib.st_multi_step_bf16(

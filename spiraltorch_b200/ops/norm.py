@@ -11,6 +11,7 @@ RMSNorm has no counterpart in the reference.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -28,10 +29,21 @@ def _scratch(lib, x2: torch.Tensor) -> torch.Tensor:
     return torch.empty(elems, dtype=torch.float32, device=x2.device)
 
 
+@functools.cache
+def _limit(entry: str) -> int:
+    return getattr(native.lib(), entry)()
+
+
+def gelu_max_features() -> int:
+    """Widest rows of :func:`norm_gelu_forward` and its backward."""
+    return _limit("st_norm_gelu_max_features")
+
+
 def takes_f32(d: int, *tensors: Optional[torch.Tensor]) -> bool:
     """Whether the fp32 form of the kernels takes these tensors (``None`` entries are skipped)."""
-    return d % 8 == 0 and 0 < d <= 1024 and all(
-        t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in tensors)
+    return d % 8 == 0 and d > 0 and all(
+        t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in tensors) \
+        and d <= _limit("st_norm_f32_max_features")
 
 
 def _form(lib, entry: str, x2: torch.Tensor, rounded: bool):
@@ -122,7 +134,7 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
 
 
 def norm_gelu_forward(x2: torch.Tensor, gamma, beta, eps: float):
-    """``gelu(layer_norm(x2))`` of contiguous bf16 rows of at most 2048 features on CUDA: ``(y, mean, rstd)``."""
+    """``gelu(layer_norm(x2))`` of contiguous bf16 rows of at most :func:`gelu_max_features` on CUDA: ``(y, mean, rstd)``."""
     global launch_count
     native.require_cuda("norm_gelu_forward", x2, gamma, beta)
     rows, d = x2.shape
