@@ -416,7 +416,7 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "conv3x3: image width must divide 128 and the batch must fill whole pixel blocks");
   const int P = a->N * a->H * a->W;
   CUtensorMap tmA, tmB;
-  const TileChoice tile = choose_tile(P, a->OC, 9ll * a->C, 1, st::sm_count());
+  const TileChoice tile = choose_tile(P, a->OC, 9ll * a->C, 1, st::sm_count(), a->act == ACT_RELU_BWD ? EPI_OPERAND : EPI_PLAIN);
   HaloPlan halo;
   const bool use_halo = halo_plan(a, &halo) && halo.us <= tile.us;
   const int BN = use_halo ? halo.bn : tile.bn;

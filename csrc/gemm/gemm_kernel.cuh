@@ -1041,37 +1041,47 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
-// Tile width of a product.  Time is about a + rounds * K blocks * c: a covers launch, fill and the last epilogue, c a K block
-// of one tile on one SM (the pair's on two), both measured in microseconds with bf16 outputs:
-//   tile          128 x 64   128 x 128   128 x 256   256 x 256 on a pair
-//   a, c          5.0, 0.228   5.6, 0.262   4.1, 0.40    7.6, 0.33
-// Narrow tiles lose throughput (their K block costs more than its share) but fill the chip where wide ones leave SMs without
-// a tile: 777 x 2048 x 8192 takes 39 us with 112 tiles of 128 x 128 and 53 with 56 of 128 x 256, 1536 x 512 x 4608 22 against
-// 30, while 16384 x 6144 x 2048 takes 659 / 378 / 291 / 269 us in the order of the table.  Against 24 shapes the rule is off
-// by one choice with 3 % between the two.
+// Tile width of a product.  A tile's main loop takes about c per K block (c2 from the 33rd on, where the start-up of the ring no
+// longer counts) and its epilogue e, which runs beside the next tile's main loop; what does not overlap is the first main loop and
+// the last epilogue:
+//   time = a + (rounds - 1) max(main, e) + main + e
+// in microseconds, fitted to 1314 products of 64 to 32768 rows, 64 to 50304 columns and K of 128 to 16384 with every epilogue.
+// Narrow tiles lose throughput but fill the chip where wide ones leave SMs without a tile: 777 x 2048 x 8192 takes 39 us with 112
+// tiles of 128 x 128 and 53 with 56 of 128 x 256; their short epilogues matter where K is short: 777 x 256 x 256 5.3 us in tiles of
+// 64 columns, 7.4 of 256, with GELU' 8.2 and 13.5.  128 x 256 and the pair come out within a few percent of one another over much
+// of the range, timed alone; inside a training step, under the power limit, the pair is the faster one (the products of the 85 M
+// byte model's step, K = 768 and 3072: 7.87 ms against 8.10), so it is taken up to 7 % above.
+// Against the fastest form of each, timed alone, the rule takes 0.3 to 0.7 % longer on average with bf16 outputs (1.0 with GELU')
+// and 1.0 to 1.4 % with fp32 ones, at most 16 %.
+enum TileEpilogue : int { EPI_PLAIN, EPI_OPERAND, EPI_GELU, EPI_GELU_BWD, EPI_FP32, EPI_FP32_ADD, EPI_FP32_ATOMIC };
+struct TileCost {
+  double a, c, c2, e[7];
+};
+constexpr TileCost kTileCost[4] = {
+    //  a    c      c2     plain operand gelu gelu'  fp32  add   atomics
+    {3.37, 0.253, 0.224, {1.04, 1.85, 2.15, 3.75, 2.00, 6.27, 1.26}},       // 128 x 64
+    {2.43, 0.290, 0.248, {2.25, 3.25, 3.75, 5.86, 4.55, 11.56, 3.23}},      // 128 x 128
+    {1.49, 0.376, 0.302, {3.98, 5.77, 6.87, 10.39, 8.14, 20.0, 5.42}},      // 128 x 256
+    {2.18, 0.366, 0.301, {4.30, 6.27, 7.21, 11.06, 8.54, 20.0, 6.45}}};     // 256 x 256 on a pair
 struct TileChoice {
   int bn;
   bool pair;
   double us;      // modelled time
 };
-inline TileChoice choose_tile(long long M, long long N, long long K, long long batch, int ctas) {
-  const long long kb = (K + BK - 1) / BK;
-  auto rounds = [](long long tiles, long long at_once) { return (tiles + at_once - 1) / at_once; };
-  auto cost = [&](int bm, int bn, long long at_once, double a, double c) {
-    return a + c * (double)(rounds(((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch, at_once) * kb);
+inline TileChoice choose_tile(long long M, long long N, long long K, long long batch, int ctas, TileEpilogue epi) {
+  const double kb = (double)((K + BK - 1) / BK);
+  auto cost = [&](const TileCost& t, int bm, int bn, long long at_once) {
+    const long long tiles = ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch;
+    const double main = t.c * (kb < 32 ? kb : 32) + t.c2 * (kb > 32 ? kb - 32 : 0), e = t.e[epi];
+    return t.a + (double)((tiles + at_once - 1) / at_once - 1) * (main > e ? main : e) + main + e;
   };
-  double t = cost(BM, 64, ctas, 5.0, 0.228);
-  TileChoice best{64, false, t};
-  if (N > 64) {
-    const double u = cost(BM, 128, ctas, 5.6, 0.262);
-    if (u <= t) { t = u; best = {128, false, u}; }
-  }
-  if (N > 128) {
-    const double u = cost(BM, 256, ctas, 4.1, 0.40);
-    if (u <= t) { t = u; best = {256, false, u}; }
-    const double w = M > BM && ctas >= 2 ? cost(2 * BM, 256, ctas / 2, 7.6, 0.33) : 1e30;
-    if (w < t) best = {256, true, w};
-  }
+  TileChoice best{64, false, cost(kTileCost[0], BM, 64, ctas)};
+  auto take = [&](int bn, bool pair, double us) {
+    if (us <= best.us) best = {bn, pair, us};
+  };
+  if (N > 64) take(128, false, cost(kTileCost[1], BM, 128, ctas));
+  if (N > 128) take(256, false, cost(kTileCost[2], BM, 256, ctas));
+  if (N > 128 && M > BM && ctas >= 2) take(256, true, 0.93 * cost(kTileCost[3], 2 * BM, 256, ctas / 2));
   return best;
 }
 

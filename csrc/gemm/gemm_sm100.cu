@@ -89,7 +89,13 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
 
   const bool limited = a->max_ctas > 0 && a->max_ctas < st::sm_count();
-  TileChoice tile = choose_tile(a->M, a->N, a->K, a->batch, limited ? a->max_ctas : st::sm_count());
+  const TileEpilogue epi = a->accumulate == 2 ? EPI_FP32_ATOMIC
+                           : a->out_fp32      ? (a->accumulate ? EPI_FP32_ADD : EPI_FP32)
+                           : a->act == ACT_GELU_BWD ? EPI_GELU_BWD
+                           : a->act == ACT_GELU     ? EPI_GELU
+                           : a->residual || a->aux_out || a->aux_in || a->accumulate ? EPI_OPERAND
+                                                                                     : EPI_PLAIN;
+  TileChoice tile = choose_tile(a->M, a->N, a->K, a->batch, limited ? a->max_ctas : st::sm_count(), epi);
   if (a->max_ctas > 0) tile.pair = false;      // a limited grid runs beside another kernel: single CTAs find room anywhere
   const int BN = tile.bn;
   const bool pair = tile.pair;
