@@ -428,7 +428,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Pair kernel (no bias / lengths): one CTA owns TWO adjacent 128-row query tiles of one (batch, head), so every K and
+// Pair kernel (no bias per query and key): one CTA owns TWO adjacent 128-row query tiles of one (batch, head), so every K and
 // V tile that TMA brings in feeds two products, and the probabilities never touch shared memory:
 //   S_t = Q_t·Kᵀ          tcgen05.mma (both operands from shared memory), fp32 in TMEM, one S buffer per query tile
 //   P_t = exp2(S_t·c − m)  one softmax warpgroup per query tile, one thread per row; P is written back as bf16 over
@@ -443,7 +443,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // in the log2 domain and minus infinity wherever a key is masked: 16-byte loads that all lanes share, one packed multiply-
 // add per two logits and no comparisons, except in the tile that holds the length, where a padded key may have given a logit
 // that is not finite and is replaced by comparison.  The single-tile kernel loaded and compared per element: 244 us for 96 contexts of
-// up to 1000 keys, D = 64, where this form takes 99.  A bias per (query, key) stays with the single-tile kernel.
+// up to 1000 keys, D = 64, where this form takes 95.  A bias per (query, key) stays with the single-tile kernel.
 // ------------------------------------------------------------------------------------------------------------------
 // Phase clocks of CTA 0 (SM cycles summed over the launch), written when tracing is switched on:
 //   softmax warp 0:  0 steps, 1 wait for S, 2 S load, 3 maximum / rescale, 4 first half of P, 5 second half of P,
@@ -482,8 +482,7 @@ __global__ void attn_key_bias_kernel(const float* __restrict__ kb, long long kb_
   }
 }
 
-// FP32: the launch may ask for an fp32 copy of the output; its stores cost the plain form 2 % (192 against 188 us, 8 x 2048 x
-// 16 heads, D = 128, causal).
+// FP32: the launch may ask for an fp32 copy of the output; its stores cost the plain form 2 %.
 template <int D, bool KEYB, bool FP32>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,

@@ -372,9 +372,9 @@ struct StConvArgs {
 
 // Plan of the shared-row form (conv_halo.cuh): false where the geometry or the shared memory does not allow it.  `us` is its
 // modelled time, about 4.2 (64 channels) or 5.5 us plus 1.0 us for every box of rows that an SM walks.  It loses where tiles
-// of 256 pixels leave most SMs without one: 1 x 32 x 32, 64 to 128 channels, takes 8.7 us and 7.0 in 16 tiles of 128 x 64;
-// 24 x 32 x 32, 128 to 128: 12.2 and 16.6; 256 x 32 x 32: 57 and 87; 256 x 64 x 64, 64 to 64: 88 and 149 (data gradient 93
-// and 161).
+// of 256 pixels leave most SMs without one: 1 x 32 x 32, 64 to 128 channels, takes 8.6 us and 7.2 in 16 tiles of 128 x 64;
+// 24 x 32 x 32, 128 to 128: 12.2 and 15.8; 256 x 32 x 32: 58 and 80; 256 x 64 x 64, 64 to 64: 88 and 141 (data gradient 95
+// and 153).
 struct HaloPlan {
   int bn, resident, smem;
   double us;
@@ -482,8 +482,8 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
   // tiles of 192: 96 KB of loads per 64 pixels instead of 144).  The form (tile width, or pairs over 256 output channels) and
   // the splits by the cost of a K block as in choose_tile, plus about 6 us of atomics for each tile of an SM.  A caller's own
   // split count fixes the summation order with one CTA per tile and split; narrow tiles then keep more SMs at work.
-  // Measured, with a tile per tap and now: 256 x 64 x 64 pixels, C = OC = 64: 240 -> 115 us (672 TFLOP/s; half of the 128
-  // rows of a tile are padding); 256 x 32 x 32, 128 to 128: 134 -> 66; 256 x 16 x 16, 256 to 256: 86 -> 55 (1399 TFLOP/s).
+  // Measured, with a tile per tap and in this form: 256 x 64 x 64 pixels, C = OC = 64: 240 and 118 us (655 TFLOP/s; half of the
+  // 128 rows of a tile are padding); 256 x 32 x 32, 128 to 128: 134 and 66; 256 x 16 x 16, 256 to 256: 86 and 55 (1399 TFLOP/s).
   struct Form { int bn, rows, sms; double c; };
   static const Form forms[4] = {{192, BM, 1, 0.33}, {256, BM, 1, 0.40}, {256, 2 * BM, 2, 0.33}, {64, BM, 1, 0.228}};
   const long long N9 = 9ll * a->C;

@@ -263,10 +263,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   static_assert(CG == 1 || COMM == COMM_NONE, "CTA pairs run the plain product only");
   using L = SmemLayout<BN / CG, STAGES>;
   // Epilogue warps per 32 lanes of the accumulator.  Two of them take 64-column groups in turn, or, where a tile has only one
-  // group, whole tiles in turn.  One warp took about 0.6 us for 32 columns, 1 us and more with a fused activation, which a
-  // short K does not cover: 16384 x 3072 x 768 takes 65 us and took 69, with GELU and its saved input 114 (141), with GELU'
-  // 140 (193); 16384 x 768 x 768 plus residual 32 (41); 16384 x 8192 x 2048 with GELU' 438 (525); 2^20 x 64 x 32 with bias and
-  // ReLU 78 (92).  Fetching the epilogue's operand a column group ahead did not help on top (144 and 126 us with GELU' and GELU).
+  // group, whole tiles in turn.  One warp needs about 0.6 us for 32 columns, 1 us and more with a fused activation, which a
+  // short K does not cover.  With two warps and with one: 16384 x 3072 x 768 65 and 69 us, with GELU and its saved input 105 and
+  // 141, with GELU' 135 and 193; 16384 x 768 x 768 plus residual 30 and 41; 16384 x 8192 x 2048 with GELU' 446 and 525; 2^20 x
+  // 64 x 32 with bias and ReLU 78 and 92.  Fetching the epilogue's operand a column group ahead makes it slower (144 and 126 us
+  // with GELU' and GELU).
   constexpr int SETS = COMM == COMM_NONE ? 2 : 1;
   constexpr bool SPLIT = SETS == 2 && BN > 64;
   extern __shared__ uint8_t smem_raw[];
@@ -339,9 +340,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------- TMA producer -------------------------------------
     // The whole warp walks the schedule and one lane issues.  With warp-uniform control flow the loop's addresses and
     // coordinates sit in uniform registers, which TMA and tcgen05 instructions read; issued from inside a one-lane
-    // branch, with descriptors rebuilt per instruction, these two loops set the pace of short or narrow K blocks: the weight
-    // gradient of a 64-channel 3x3 convolution over a million pixels, in tiles of 64 columns, went from 315 to 240 us (its
-    // wider tiles of today take 115), a training step of the conv classifier (256 x 64 x 64) from 2.55 to 2.27 ms.  Wide products of the language models did not change.
+    // branch, with descriptors rebuilt per instruction, the producer's and the issuer's loops set the pace of short or narrow
+    // K blocks: the weight gradient of a 64-channel 3x3 convolution over a million pixels, in tiles of 64 columns, takes 240 us
+    // this way and 315 in the other.  Wide products do not change.
     const bool leader = COMM == COMM_AG ? lane == 0 : elect_one();
     const uint32_t smem0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const uint32_t full0 = __shfl_sync(0xffffffffu, smem_u32(full_bar), 0);

@@ -10,7 +10,8 @@
 // the smallest key is the best and the order is total and deterministic.  Four forms:
 //   * top / bottom, k = 1: block arg-max over a row of up to 4096 columns (rank_k1_kernel);
 //   * top / bottom, k <= 128: a sorted list of the best 32, 64 or 128 keys per warp, kept in registers while the warp
-//     streams its share of the row; one to 32 warps share a row (rank_topk_kernel);
+//     streams its share of the row; up to 16 warps of a CTA share a row, and eight in each of up to 64 CTAs a wide one
+//     (rank_topk_kernel);
 //   * mid, and larger k: a radix select over the row in shared memory finds the two boundary values of the wanted
 //     range of ranks, and only the keys inside it are sorted (rank_range_kernel);
 //   * k so large that the range's sort would be as wide as the row's: one bitonic sort (rank_select_kernel).
@@ -388,7 +389,7 @@ rank_merge_kernel(const u64* __restrict__ lists, float* __restrict__ out_v, int*
 }
 
 // CTAs that share a row: fewer than 16 warps per SM over all rows leaves loads unissued, so a wide row (above the
-// 8192 columns one CTA of 32 warps reads in a microsecond) is split until there are enough, but not below 256 columns
+// 8192 columns that one CTA of 16 warps reads in a few microseconds) is split until there are enough, but not below 256 columns
 // per warp of an 8-warp CTA.
 int topk_parts(int rows, int cols) {
   if (cols <= 8192 || (long long)rows * 32 >= 16ll * st::sm_count()) return 1;

@@ -160,7 +160,8 @@ def conv3x3_wgrad(dy: torch.Tensor, x: torch.Tensor, dw_tap: torch.Tensor, col: 
         return
     a = _WgradArgs()
     a.dy, a.x, a.dw = dy.data_ptr(), x.data_ptr(), dw_tap.data_ptr()
-    # one CTA per (tap, tile) when the summation order must be fixed; 0 lets the launcher split the pixel loop
+    # one CTA per tile of output channels x (tap, channel) columns when the summation order must be fixed; 0 lets the
+    # launcher split the pixel loop
     a.N, a.H, a.W, a.C, a.OC, a.splits = N, H, W, C, OC, (1 if native.deterministic_reduction() else 0)
     native.check(native.lib().st_conv3x3_wgrad(ctypes.byref(a), native.stream_ptr(x.device)), "st_conv3x3_wgrad")
     launch_count += 1

@@ -72,7 +72,7 @@ def test_rank_two_stage_for_wide_rows_matches_cpu(rows, cols, k):
 @pytest.mark.parametrize("rows,cols,k", [(1, 33, 1), (3, 64, 31), (9, 127, 32), (2600, 130, 33), (5, 511, 64), (5, 513, 65), (2, 2048, 128),
                                          (70, 8192, 128), (6, 8190, 129), (2, 8193, 32), (80, 8196, 7), (1, 50001, 128), (3, 30000, 2)])
 def test_rank_forms_at_their_edges(rows, cols, k):
-    """List lengths 32 / 64 / 128 and the step past them, odd and unaligned rows, one to 32 warps per row and rows split
+    """List lengths 32 / 64 / 128 and the step past them, odd and unaligned rows, one to 16 warps per row and rows split
     over CTAs; ties, infinities and NaN included.  Selections are exact."""
     torch.manual_seed(rows + cols)
     x = torch.randn(rows * cols + 1)
