@@ -145,13 +145,13 @@ int blocks_for(long long n, int most) {
   const long long b = (n + 4 * kMultiThreads - 1) / (4 * kMultiThreads);
   return (int)(b < 1 ? 1 : (b > most ? most : b));
 }
-int multi_blocks(long long n) { return blocks_for(n, 8 * st::sm_count()); }
+int multi_cap() { return 8 * st::sm_count(); }      // blocks of one tensor at most
 
 }  // namespace
 
 // Tensors per st_multi call, and ints of result a call over tensors of at most `most` elements writes per tensor.
 ST_API int st_multi_max() { return kMultiMax; }
-ST_API int st_multi_blocks(long long most) { return multi_blocks(most); }
+ST_API int st_multi_blocks(long long most) { return blocks_for(most, multi_cap()); }
 
 namespace {
 int run_multi(int op, int count, const void* const* src, void* const* dst, void* const* half, const long long* n, float value,
@@ -179,6 +179,7 @@ int run_multi(int op, int count, const void* const* src, void* const* dst, void*
     return st::fail(ST_ERR_INVALID, "multi: bad arguments");
   MultiTable t;
   long long most = 0;
+  const int cap = multi_cap();
   int grid = 0;
   for (int i = 0; i < count; ++i) {
     t.src[i] = static_cast<const float*>(src[i]);
@@ -186,11 +187,11 @@ int run_multi(int op, int count, const void* const* src, void* const* dst, void*
     t.half[i] = half ? static_cast<__nv_bfloat16*>(half[i]) : nullptr;
     t.n[i] = n[i];
     t.first[i] = grid;
-    grid += multi_blocks(n[i]);
+    grid += blocks_for(n[i], cap);
     most = n[i] > most ? n[i] : most;
   }
   for (int i = count; i <= kMultiMax; ++i) t.first[i] = i == count ? grid : 0x7FFFFFFF;
-  const int slots = multi_blocks(most);
+  const int slots = blocks_for(most, cap);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   if (op == MULTI_CHECK) multi_kernel<MULTI_CHECK><<<grid, kMultiThreads, 0, s>>>(t, value, bad, slots);
   else if (op == MULTI_DIV) multi_kernel<MULTI_DIV><<<grid, kMultiThreads, 0, s>>>(t, value, bad, slots);

@@ -143,7 +143,8 @@ __global__ void rank_k1_kernel(const float* __restrict__ in, float* __restrict__
 // A row is read once, so the bound is its bytes.  What made the full sort slow was shared memory: 78 exchange stages
 // over 4096 keys per row.  Here an element costs one comparison with a bound on the k-th best value; the few that pass
 // go to a small queue, and a full queue is sorted in registers and merged into the list.  4096 x 4096, k = 32: 22 us
-// (the bytes take 10), two sorts of row halves and the merge of their lists took 669; issue slots bound it now.
+// (the bytes take 10) with half of the issue slots busy and the rest waiting for loads; two sorts of row halves and the merge of
+// their lists took 669.
 using u64 = unsigned long long;
 constexpr int TOPK_MAX_K = 128;
 constexpr int TOPK_GROUP = 128;             // columns of a warp-wide load: four per lane
