@@ -38,7 +38,7 @@ constexpr int AG_EXTRA_SMEM = AG_RING_SLOTS * AG_RING_CHUNK + 64;
 template <bool B_MN, int COMM, int ST = STAGES>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const CUtensorMap& tmA_local,
            const GemmParams& p, const GemmComm& cm, int grid, cudaStream_t stream) {
-  using L = SmemLayout<BN, ST>;
+  using L = SmemLayout<BN, ST, 1>;
   constexpr int SMEM = L::TOTAL + ((COMM == COMM_AG && ST == AG_STAGES) ? AG_EXTRA_SMEM : 0);
   static_assert(SMEM <= 232448, "dynamic shared memory above the 227 KB limit");
   auto kern = gemm_bf16_kernel<BN, ST, false, B_MN, COMM>;

@@ -193,6 +193,12 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sr
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+// TMA tiled addition shared -> global (the element type is the map's).
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
 // Untiled bulk copies (both addresses 16-byte aligned, size a multiple of 16 bytes).
 __device__ __forceinline__ void bulk_load_g2s(uint32_t dst_smem, const void* src_gmem, uint32_t bytes,
                                               uint32_t bar) {
@@ -530,6 +536,43 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
+}
+
+// gelu_tanh and gelu_tanh_grad of two values with packed arithmetic: the same operations in the same order, so the same bits.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float2 splat2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ void gelu_parts_pair(float2 x, float2 z, float2& q, float2& p) {
+  constexpr double c = 2.0 * 0.7978845608028654 * 1.4426950408889634;
+  constexpr float c0 = static_cast<float>(c), c1 = static_cast<float>(c * 0.044715);
+  const float2 a = mul2(make_float2(-fabsf(x.x), -fabsf(x.y)), fma2(splat2(c1), z, splat2(c0)));
+  const float2 e = make_float2(exp2_ftz(a.x), exp2_ftz(a.y));
+  const float2 d = add2(splat2(1.0f), e);
+  p = make_float2(rcp_approx(d.x), rcp_approx(d.y));
+  q = mul2(e, p);
+}
+__device__ __forceinline__ void gelu_tanh_pair(float& x0, float& x1) {
+  const float2 x = make_float2(x0, x1), z = mul2(x, x);
+  float2 q, p;
+  gelu_parts_pair(x, z, q, p);
+  x0 = x.x > 0.0f ? x.x - fminf(x.x, 3.402823466e38f) * q.x : x.x * q.x;
+  x1 = x.y > 0.0f ? x.y - fminf(x.y, 3.402823466e38f) * q.y : x.y * q.y;
+}
+__device__ __forceinline__ float2 gelu_tanh_grad_pair(float2 x) {
+  constexpr float d0 = static_cast<float>(2.0 * 0.7978845608028654), d1 = static_cast<float>(6.0 * 0.7978845608028654 * 0.044715);
+  const float2 z = mul2(x, x);
+  float2 q, p;
+  gelu_parts_pair(x, z, q, p);
+  const float2 t = fma2(fma2(fma2(fma2(splat2(-7.50559184e-06f), z, splat2(1.18915079e-04f)), z, splat2(-1.24431029e-03f)), z,
+                             splat2(1.02022300e-02f)), z, splat2(-6.68196306e-02f));
+  const float2 h = fma2(splat2(3.98942292e-01f), x, mul2(mul2(x, z), t));
+  const float2 w = fma2(make_float2(-h.x, -h.y), h, splat2(0.25f)), qp = mul2(q, p), g = mul2(x, fma2(splat2(d1), z, splat2(d0)));
+  const bool n0 = fabsf(x.x) < 1.0f, n1 = fabsf(x.y) < 1.0f;
+  const float s0 = n0 ? 0.5f + h.x : (x.x > 0.0f ? 1.0f - q.x : q.x), s1 = n1 ? 0.5f + h.y : (x.y > 0.0f ? 1.0f - q.y : q.y);
+  return fma2(g, make_float2(n0 ? w.x : qp.x, n1 ? w.y : qp.y), make_float2(s0, s1));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

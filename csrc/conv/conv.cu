@@ -429,20 +429,17 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
     if (!encode_tmap(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
   }
-  OutMaps tmC;
-  memset(&tmC, 0, sizeof(tmC));
-  {
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
+  if (use_halo) {
+    CUtensorMap tmY;
     uint64_t dims[3] = {(uint64_t)a->OC, (uint64_t)P, 1};
     uint64_t strides[2] = {(uint64_t)a->OC * 2, (uint64_t)a->OC * 2 * P};
     uint32_t box[3] = {64, 32, 1};
-    if (!encode_tmap(&tmC.m[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->y, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (!encode_tmap(&tmY, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->y, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
       return ST_ERR_CUDA;
-  }
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (use_halo) {
-    if (halo.resident) return st::conv::launch_halo<64, true>(tmA, tmB, tmC.m[0], halo.p, halo.smem, s);
-    if (BN == 64) return st::conv::launch_halo<64, false>(tmA, tmB, tmC.m[0], halo.p, halo.smem, s);
-    return st::conv::launch_halo<128, false>(tmA, tmB, tmC.m[0], halo.p, halo.smem, s);
+    if (halo.resident) return st::conv::launch_halo<64, true>(tmA, tmB, tmY, halo.p, halo.smem, s);
+    if (BN == 64) return st::conv::launch_halo<64, false>(tmA, tmB, tmY, halo.p, halo.smem, s);
+    return st::conv::launch_halo<128, false>(tmA, tmB, tmY, halo.p, halo.smem, s);
   }
   GemmParams p{};
   p.conv.mode = 1;
@@ -454,11 +451,13 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   p.ld_aux_in = a->OC;
   p.M = P; p.N = a->OC; p.K = 9 * a->C;
   p.alpha = 1.0f; p.act = a->act; p.batch = 1;
-  p.use_tma_store = 1;
   p.err = st::error_word();
+  OutMaps tmC;
+  if (!plan_epilogue(p, tmC)) return ST_ERR_CUDA;
   if (pair) return launch_pair<false, false>(tmA, tmB, tmC, p, s);
-  if (BN == 64) return launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s);
-  if (BN == 128) return launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s);
+  const bool plain = plain_epilogue(p);
+  if (BN == 64) return plain ? launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s) : launch_gemm<64, 6, false, false>(tmA, tmB, tmC, p, s);
+  if (BN == 128) return plain ? launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s) : launch_gemm<128, 5, false, false>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, false, false>(tmA, tmB, tmC, p, s);
 }
 
@@ -516,8 +515,6 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
       return ST_ERR_CUDA;
   }
   if (!nhwc_map(&tmB, a->x, a->N, a->H, a->W, a->C, a->W, Hb, Nb)) return ST_ERR_CUDA;
-  OutMaps tmC;
-  memset(&tmC, 0, sizeof(tmC));
   GemmParams p{};
   p.conv.mode = 2;
   p.conv.H = a->H; p.conv.W = a->W; p.conv.Hb = Hb; p.conv.Nb = Nb;
@@ -527,10 +524,12 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
   p.alpha = 1.0f; p.batch = splits; p.batch_stride_c = 0;
   p.out_fp32 = 1; p.accumulate = 2;
   p.err = st::error_word();
+  OutMaps tmC;
+  if (!plan_epilogue(p, tmC)) return ST_ERR_CUDA;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   if (form == 0) return launch_gemm<192, 4, true, true>(tmA, tmB, tmC, p, s);
   if (form == 2) return launch_pair<true, true>(tmA, tmB, tmC, p, s);
-  if (form == 3) return launch_gemm<64, 8, true, true>(tmA, tmB, tmC, p, s);
+  if (form == 3) return launch_gemm<64, 6, true, true>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, true, true>(tmA, tmB, tmC, p, s);
 }
 

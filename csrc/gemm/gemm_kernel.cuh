@@ -23,6 +23,7 @@
 #include "../common/host.h"
 #include "../common/ptx.cuh"
 #include "../comm/comm.cuh"
+#include <cstring>
 
 namespace st {
 namespace gemm {
@@ -99,24 +100,37 @@ struct GemmParams {
   int accumulate;
   int batch;
   long long batch_stride_c;
-  int use_tma_store;   // bf16 output without accumulation: stage through smem, store by TMA
+  int use_tma_store;   // StoreMode: the output goes through shared memory and the copy engine
+  int operand_tma;     // the epilogue's operand (aux_in of a derivative, else the residual) arrives by TMA, OutMaps.m[1]
+  int aux_tma;         // aux_out leaves by TMA, OutMaps.m[2]
   unsigned* err;
 };
+enum StoreMode : int { STORE_DIRECT = 0, STORE_BF16 = 1, STORE_FP32 = 2, STORE_FP32_ADD = 3 };
 
-// Tensor maps of the output: [0] for a plain GEMM, one per owner rank for GEMM → reduce-scatter.
+// Tensor maps of the output, one per owner rank for GEMM → reduce-scatter.  Plain product: [0] the output, [1] the epilogue's
+// operand, [2] the saved pre-activation.
 struct OutMaps {
   CUtensorMap m[kMaxRanks];
 };
 
-template <int BN, int STAGES>
+// CBUF: 4 KiB staging blocks per epilogue warp of the plain product (eight warps), as many as fit beside the operand ring; the
+// tensor-parallel variants have four warps with two blocks each, which is the room of CBUF = 1.
+constexpr int kSmemMax = 232448;      // 227 KiB
+template <int BN, int STAGES, int CB = 0>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int CSTAGE_OFFSET = STAGES * STAGE_BYTES;       // one 4 KiB block per epilogue warp (two of four warps)
-  static constexpr int CSTAGE_BYTES = 4 * 2 * 4096;
+  static constexpr int BAR_BYTES = 512;                            // barriers
+  static constexpr int SLACK = BAR_BYTES + 1024;                   // and alignment
+  static constexpr int ROOM = (kSmemMax - SLACK - STAGES * STAGE_BYTES) / (8 * 4096);
+  static constexpr int CBUF = CB ? CB : ROOM < 4 ? ROOM : 4;
+  static_assert(CBUF >= 1, "no room for the staged output");
+  static constexpr int CSTAGE_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int CSTAGE_BYTES = 8 * CBUF * 4096;
   static constexpr int BAR_OFFSET = CSTAGE_OFFSET + CSTAGE_BYTES;
-  static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;  // barriers + alignment slack
+  static constexpr int OPBAR_OFFSET = BAR_OFFSET + 256;            // one barrier per epilogue warp and staging block (at most 32)
+  static constexpr int TOTAL = BAR_OFFSET + SLACK;
 };
 
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
@@ -252,6 +266,39 @@ __device__ __forceinline__ int split_begin(const GemmParams& p, int b) {
 }
 __device__ __forceinline__ int split_blocks(const GemmParams& p, int b) { return split_begin(p, b + 1) - split_begin(p, b); }
 
+// ---- epilogue of the plain product -----------------------------------------------------------
+__device__ __forceinline__ uint4 pack8_bf16(const float* v) {
+  return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+__device__ __forceinline__ void add8_bf16(float* v, const uint4& u) {
+  const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
+  v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
+  v[4] += f2.x; v[5] += f2.y; v[6] += f3.x; v[7] += f3.y;
+}
+// Whether a row segment starting at `p`, on a 32-column boundary of its matrix, may be accessed 16 bytes at a time
+__device__ __forceinline__ bool vec8(const __nv_bfloat16* p, long long ld) {
+  return (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+}
+// 32 values of a row, of which `n` exist (the rest is zero)
+__device__ __forceinline__ void load32_bf16(uint4 (&x)[4], const __nv_bfloat16* a, long long ld, bool full, int n) {
+  if (full && n > 0 && vec8(a, ld)) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = reinterpret_cast<const uint4*>(a)[q];
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int j = q * 8 + i * 2;
+      const uint32_t lo = j < n ? __bfloat16_as_ushort(a[j]) : 0u, hi = j + 1 < n ? __bfloat16_as_ushort(a[j + 1]) : 0u;
+      w[i] = lo | (hi << 16);
+    }
+    x[q] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 // CG = 2 (COMM_NONE only): a cluster of two CTAs works on one tile of 256 x BN.  Each CTA brings its 128 rows of A and its half
 // of B into its own shared memory, the even CTA's MMA warp issues for both, and each CTA's epilogue stores its own 128 rows.
 // A K block then costs an SM 32 KB of loads instead of 48 (BN = 256), and the ring holds six stages instead of four.
@@ -261,13 +308,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const __grid_constant__ OutMaps tmC, const __grid_constant__ CUtensorMap tmA_local,
                  const GemmParams p, const GemmComm cm) {
   static_assert(CG == 1 || COMM == COMM_NONE, "CTA pairs run the plain product only");
-  using L = SmemLayout<BN / CG, STAGES>;
+  using L = SmemLayout<BN / CG, STAGES, COMM == COMM_NONE ? 0 : 1>;
   // Epilogue warps per 32 lanes of the accumulator.  Two of them take 64-column groups in turn, or, where a tile has only one
-  // group, whole tiles in turn.  One warp needs about 0.6 us for 32 columns, 1 us and more with a fused activation, which a
-  // short K does not cover.  With two warps and with one: 16384 x 3072 x 768 65 and 69 us, with GELU and its saved input 105 and
-  // 141, with GELU' 135 and 193; 16384 x 768 x 768 plus residual 30 and 41; 16384 x 8192 x 2048 with GELU' 446 and 525; 2^20 x
-  // 64 x 32 with bias and ReLU 78 and 92.  Fetching the epilogue's operand a column group ahead makes it slower (144 and 126 us
-  // with GELU' and GELU).
+  // group, whole tiles in turn: one warp's loads, arithmetic and stores for a tile are longer than the main loop of a short K.
   constexpr int SETS = COMM == COMM_NONE ? 2 : 1;
   constexpr bool SPLIT = SETS == 2 && BN > 64;
   extern __shared__ uint8_t smem_raw[];
@@ -305,6 +348,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(smem_u32(&tfull_bar[a]), 1);
       mbar_init(smem_u32(&tempty_bar[a]), (SPLIT ? 8 : 4) * CG);
     }
+    if constexpr (COMM == COMM_NONE)
+      for (int i = 0; i < 8 * L::CBUF; ++i) mbar_init(smem_u32(smem + L::OPBAR_OFFSET) + i * 8, 1);
     *abort_flag = 0;
     if constexpr (COMM == COMM_AG) {
       tmem_slot[2] = 0;   // items whose stores are complete (push warp → publisher warp)
@@ -538,15 +583,262 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
     }
-  } else if (warp < 2 + 4 * SETS) {
-    // ------------------------------- epilogue warps -----------------------------------
+  } else if (COMM == COMM_NONE) {
+    // ------------------------------- epilogue warps, plain product ----------------------------------------
+    // A warp takes 32 rows and 64 columns at a time.  Everything that is wide leaves and arrives through the copy engine and
+    // this warp's staging blocks: a lane that reads or writes its own row of global memory touches a 16-byte piece of 32
+    // lines per instruction.
+    //   operand (saved pre-activation or residual): the warp's blocks land in its staging blocks in turn, asked for ahead of the
+    //     arithmetic, and are replaced there by the result, which is stored from the same place;
+    //   saved pre-activation out: a staging block beside the result's;
+    //   fp32: 32 x 32 blocks, stored, or added by the copy engine (one adder per element unless K is split).
+    // Outputs, operands and leading dimensions that TMA cannot take keep the element-wise accesses.
+    constexpr int CBUF = L::CBUF;
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
     const int set = (warp - 2) >> 2;
+    uint8_t* const bufs = smem + L::CSTAGE_OFFSET + (set * 4 + quad) * (CBUF * 4096);
+    const uint32_t op_bar = smem_u32(smem + L::OPBAR_OFFSET) + (set * 4 + quad) * (CBUF * 8);
+    const bool tma_op = CBUF >= 2 && p.operand_tma, tma_aux = CBUF >= 2 && p.aux_tma;
+    const bool bwd = p.act == ACT_GELU_BWD || p.act == ACT_RELU_BWD;
+    int iter = 0, blocks = 0;       // blocks staged by this warp
+    // the warp's 64-column groups of tile t: set, set + 2, ... (SPLIT), or the only one of every second tile
+    auto groups_of = [&](int t, int& m0, int& n0, int& b) {
+      int tm, tn;
+      map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
+      m0 = tm * BM * CG + cta * BM + quad * 32;
+      n0 = tn * BN;
+      return m0 < p.M ? min(BN / 64, (p.N - n0 + 63) >> 6) : 0;
+    };
+    // operand requests run up to CBUF - 1 blocks ahead of the arithmetic
+    int req_t = SPLIT ? gemm_bid : gemm_bid + set * grid_stride, req_g = SPLIT ? set : 0, requested = 0;
+    auto request = [&]() {
+      int m0, n0, b;
+      while (req_t < total_tiles && req_g >= groups_of(req_t, m0, n0, b)) {
+        req_t += SPLIT ? grid_stride : 2 * grid_stride;
+        req_g = SPLIT ? set : 0;
+      }
+      if (req_t >= total_tiles) return;
+      if (lane == 0) {
+        const uint32_t bar = op_bar + (requested % CBUF) * 8;
+        mbar_arrive_expect_tx(bar, 4096);
+        tma_load_3d(smem_u32(bufs + (requested % CBUF) * 4096), &tmC.m[1], bar, n0 + req_g * 64, m0, 0);
+      }
+      ++requested;
+      req_g += SPLIT ? 2 : BN / 64;
+    };
+    if (tma_op)
+      for (int i = 1; i < CBUF; ++i) request();
+    for (int t = gemm_bid; t < total_tiles; t += grid_stride, ++iter) {
+      if (!SPLIT && (iter & 1) != set) continue;
+      int m0, n0, b;
+      const int groups = groups_of(t, m0, n0, b);
+      const int acc = iter & 1;
+      if (!mbar_wait_warp(smem_u32(&tfull_bar[acc]), (iter >> 1) & 1, abort_flag)) break;
+      tc_fence_after();
+      const int row = m0 + lane;
+      const bool row_ok = row < p.M;
+      bool held = true, alive = true;
+      auto release = [&]() {       // hands the accumulator back to the MMA warp
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (CG == 2) mbar_arrive_cluster(smem_u32(&tempty_bar[acc]) & kPairLeaderMask);
+          else mbar_arrive(smem_u32(&tempty_bar[acc]));
+        }
+        held = false;
+      };
+#pragma unroll 1
+      for (int g = SPLIT ? set : 0; g < groups; g += SPLIT ? 2 : 1) {
+        // saved pre-activation and result take turns
+        const int at = tma_aux ? (2 * blocks) % (CBUF & ~1) : blocks % CBUF;
+        uint8_t* const cs = bufs + (tma_aux ? at + 1 : at) * 4096;
+        uint8_t* const aux_block = bufs + at * 4096;
+        if (tma_op && !mbar_wait_warp(op_bar + (blocks % CBUF) * 8, (blocks / CBUF) & 1, abort_flag)) {
+          alive = false;
+          break;
+        }
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          const int col0 = n0 + g * 64 + half * 32;
+          if (col0 >= p.N) {
+            if (held && g + (SPLIT ? 2 : 1) >= groups) release();
+            break;  // uniform across the warp
+          }
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + g * 64 + half * 32, r);
+          tmem_ld_wait();
+          if (half == 1 && g + (SPLIT ? 2 : 1) >= groups) release();
+          const bool full = col0 + 32 <= p.N;
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+          if (p.bias) {
+            if (full && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) add8_bf16(v + q * 8, __ldg(reinterpret_cast<const uint4*>(p.bias + col0) + q));
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (full || col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+            }
+          }
+          // the staging blocks written below were handed to the copy engine a block or more ago
+          if (half == 0 && p.use_tma_store == STORE_BF16 && !tma_op) {
+            if (lane == 0) {
+              if (tma_aux) tma_store_wait_read<(CBUF >= 4 ? 1 : 0)>(); else tma_store_wait_read<CBUF - 1>();
+            }
+            __syncwarp();
+          }
+          if (p.aux_out) {
+            if (tma_aux) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(aux_block + sw128_offset(lane, half * 4 + q)) = pack8_bf16(v + q * 8);
+            } else if (row_ok) {
+              __nv_bfloat16* a = p.aux_out + (long long)row * p.ld_aux_out + col0;
+              if (full && vec8(a, p.ld_aux_out)) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(a)[q] = pack8_bf16(v + q * 8);
+              } else {
+                for (int j = 0; j < 32; ++j)
+                  if (col0 + j < p.N) a[j] = __float2bfloat16(v[j]);
+              }
+            }
+          }
+          if (p.act == ACT_RELU) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+          } else if (p.act == ACT_GELU) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) gelu_tanh_pair(v[j], v[j + 1]);
+          } else if (bwd) {
+            uint4 x[4];
+            if (tma_op) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) x[q] = *reinterpret_cast<const uint4*>(cs + sw128_offset(lane, half * 4 + q));
+            } else {
+              load32_bf16(x, p.aux_in + (long long)row * p.ld_aux_in + col0, p.ld_aux_in, full, row_ok ? p.N - col0 : 0);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t w[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 f = unpack_bf16x2(w[i]);
+                float* const d = v + q * 8 + i * 2;
+                if (p.act == ACT_GELU_BWD) {
+                  const float2 s = gelu_tanh_grad_pair(f);
+                  d[0] *= s.x;
+                  d[1] *= s.y;
+                } else {
+                  d[0] = f.x > 0.0f ? d[0] : 0.0f;
+                  d[1] = f.y > 0.0f ? d[1] : 0.0f;
+                }
+              }
+            }
+          }
+          if (p.residual) {
+            if (tma_op && !bwd) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) add8_bf16(v + q * 8, *reinterpret_cast<const uint4*>(cs + sw128_offset(lane, half * 4 + q)));
+            } else {
+              uint4 x[4];
+              load32_bf16(x, p.residual + (long long)row * p.ldr + col0, p.ldr, full, row_ok ? p.N - col0 : 0);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) add8_bf16(v + q * 8, x[q]);
+            }
+          }
+          if (p.use_tma_store == STORE_BF16) {
+            // 32 rows x 64 columns (128-byte swizzle)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(cs + sw128_offset(lane, half * 4 + q)) = pack8_bf16(v + q * 8);
+          } else if (p.use_tma_store) {
+            uint8_t* const fs = bufs + (blocks % CBUF) * 4096;
+            if (lane == 0) tma_store_wait_read<CBUF - 1>();
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              *reinterpret_cast<float4*>(fs + sw128_offset(lane, q)) = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              const int bc = p.batch_stride_c ? b : 0;       // the parts of a split sum meet in the same place
+              if (p.use_tma_store == STORE_FP32_ADD) tma_reduce_add_3d(&tmC.m[0], smem_u32(fs), col0, m0, bc);
+              else tma_store_3d(&tmC.m[0], smem_u32(fs), col0, m0, bc);
+              tma_store_commit();
+            }
+            ++blocks;
+          } else if (row_ok) {
+            const long long at0 = (long long)b * p.batch_stride_c + (long long)row * p.ldc + col0;
+            if (p.out_fp32) {
+              float* cp = reinterpret_cast<float*>(p.C) + at0;
+              if (full && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                  float4 o = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                  if (p.accumulate == 2) {  // split-K: several CTAs add into the same tile
+                    atomicAdd(reinterpret_cast<float4*>(cp) + q, o);
+                    continue;
+                  }
+                  if (p.accumulate) {
+                    float4 old = reinterpret_cast<float4*>(cp)[q];
+                    o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+                  }
+                  reinterpret_cast<float4*>(cp)[q] = o;
+                }
+              } else {
+                for (int j = 0; j < 32; ++j)
+                  if (col0 + j < p.N) {
+                    if (p.accumulate == 2) atomicAdd(cp + j, v[j]); else cp[j] = p.accumulate ? cp[j] + v[j] : v[j];
+                  }
+              }
+            } else {
+              __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + at0;
+              if (full && vec8(cp, p.ldc)) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  if (p.accumulate) add8_bf16(v + q * 8, reinterpret_cast<const uint4*>(cp)[q]);
+                  reinterpret_cast<uint4*>(cp)[q] = pack8_bf16(v + q * 8);
+                }
+              } else {
+                for (int j = 0; j < 32; ++j)
+                  if (col0 + j < p.N) {
+                    float o = v[j];
+                    if (p.accumulate) o += __bfloat162float(cp[j]);
+                    cp[j] = __float2bfloat16(o);
+                  }
+              }
+            }
+          }
+          if (half == 0 && tma_op) {
+            // the block before this one has been handed over half a block's time ago: its place takes another operand
+            if (lane == 0) tma_store_wait_read<0>();
+            request();
+          }
+        }
+        if (p.use_tma_store == STORE_BF16) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (tma_aux) tma_store_3d(&tmC.m[2], smem_u32(aux_block), n0 + g * 64, m0, 0);
+            tma_store_3d(&tmC.m[0], smem_u32(cs), n0 + g * 64, m0, b);
+            tma_store_commit();
+          }
+          ++blocks;
+        }
+      }
+      if (!alive) break;
+      if (held) release();
+    }
+    if (p.use_tma_store && lane == 0) tma_store_wait<0>();
+  } else if (warp < 6) {
+    // ------------------------------- epilogue warps, tensor-parallel variants ------------------------------
+    const int quad = warp & 3;  // TMEM lane quadrant this warp may read
     int iter = 0;
-    // staging buffers per warp: two of four warps, one of eight, and one in the 4-stage all-gather variant, whose push ring
-    // takes the upper half of the staging area
-    constexpr int CSB = (SETS == 2 || (COMM == COMM_AG && STAGES == 4)) ? 1 : 2;
-    uint8_t* const cs_warp = smem + L::CSTAGE_OFFSET + (set * 4 + quad) * CSB * 4096;
+    // staging buffers per warp: two, and one in the 4-stage all-gather variant, whose push ring takes the upper half of the
+    // staging area
+    constexpr int CSB = (COMM == COMM_AG && STAGES == 4) ? 1 : 2;
+    uint8_t* const cs_warp = smem + L::CSTAGE_OFFSET + quad * CSB * 4096;
     int store_seq = 0;          // TMA stores issued by this warp (selects the staging buffer)
     int tile_seq0 = 0;          // value of store_seq when the current tile started
     constexpr int kPubBatch = 3;
@@ -569,10 +861,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     if (tracer) cm.trace[blockIdx.x * 4 + 1] = globaltimer_ns();
     for (int t = gemm_bid; t < total_tiles && alive; t += grid_stride, ++iter) {
-      if (SETS == 2 && !SPLIT && (iter & 1) != set) continue;
       int b, tm, tn;
       map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
-      const int m0 = tm * BM * CG + cta * BM, n0 = tn * BN;
+      const int m0 = tm * BM, n0 = tn * BN;
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1;
       if (!mbar_wait_warp(smem_u32(&tfull_bar[acc]), acc_phase, abort_flag)) break;
@@ -659,7 +950,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int c = 0; c < BN / 32; ++c) {
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) break;  // uniform across the warp
-        if (SPLIT && ((c >> 1) & 1) != set) continue;
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + c * 32, r);
         tmem_ld_wait();
@@ -844,10 +1134,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // hand the accumulator back to the MMA warp
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        if constexpr (CG == 2) mbar_arrive_cluster(smem_u32(&tempty_bar[acc]) & kPairLeaderMask);
-        else mbar_arrive(smem_u32(&tempty_bar[acc]));
-      }
+      if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
       if constexpr (COMM == COMM_RS) {
         // Publish this warp's 32 rows to the owner (the counter counts warp arrivals, so no
         // CTA-wide barrier is needed).  Waiting for the stores of the tile just issued would put
@@ -1042,6 +1329,51 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// How the output leaves and the epilogue's operands arrive: tensor maps where leading dimensions and addresses allow them.
+// Returns false after recording an error.
+inline bool plan_epilogue(GemmParams& p, OutMaps& maps) {
+  memset(&maps, 0, sizeof(maps));
+  p.use_tma_store = STORE_DIRECT;
+  p.operand_tma = p.aux_tma = 0;
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  auto bf16_map = [&](CUtensorMap* m, const void* base, long long ld, long long batch, long long stride) {
+    const uint64_t dims[3] = {(uint64_t)p.N, (uint64_t)p.M, (uint64_t)batch};
+    const uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)(batch > 1 ? stride : ld * p.M) * 2};
+    const uint32_t box[3] = {64, 32, 1};
+    return st::encode_tmap(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  const int per16 = p.out_fp32 ? 4 : 8;
+  const long long batch = p.batch_stride_c ? p.batch : 1;      // without a stride every part of the batch has the same output
+  if (p.ldc % per16 != 0 || !aligned(p.C) || p.batch_stride_c % per16 != 0 || p.batch_stride_c < 0) return true;
+  if (p.out_fp32) {
+    if (p.batch > 1 && batch == 1 && p.accumulate != 2) return true;
+    const uint64_t dims[3] = {(uint64_t)p.N, (uint64_t)p.M, (uint64_t)batch};
+    const uint64_t strides[2] = {(uint64_t)p.ldc * 4, (uint64_t)(batch > 1 ? p.batch_stride_c : p.ldc * p.M) * 4};
+    const uint32_t box[3] = {32, 32, 1};
+    p.use_tma_store = p.accumulate ? STORE_FP32_ADD : STORE_FP32;
+    return st::encode_tmap(&maps.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, p.C, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+  }
+  if (p.accumulate || (p.batch > 1 && batch == 1)) return true;
+  p.use_tma_store = STORE_BF16;
+  if (!bf16_map(&maps.m[0], p.C, p.ldc, batch, p.batch_stride_c)) return false;
+  const bool bwd = p.act == ACT_GELU_BWD || p.act == ACT_RELU_BWD;
+  const __nv_bfloat16* operand = bwd ? p.aux_in : p.residual;
+  const long long ld = bwd ? p.ld_aux_in : p.ldr;
+  if (operand && (ld & 7) == 0 && ld >= p.N && aligned(operand)) {
+    p.operand_tma = 1;
+    if (!bf16_map(&maps.m[1], operand, ld, 1, 0)) return false;
+  } else if (p.aux_out && (p.ld_aux_out & 7) == 0 && p.ld_aux_out >= p.N && aligned(p.aux_out)) {
+    p.aux_tma = 1;
+    if (!bf16_map(&maps.m[2], p.aux_out, p.ld_aux_out, 1, 0)) return false;
+  }
+  return true;
+}
+// Whether the epilogue only writes the bf16 output.  One staging block per warp is enough then, and the operand ring gets the
+// room: its depth covers the latency of weights that come from HBM.
+inline bool plain_epilogue(const GemmParams& p) {
+  return !p.out_fp32 && !p.accumulate && !p.residual && !p.aux_out && p.act != ACT_GELU_BWD && p.act != ACT_RELU_BWD;
+}
+
 // Tile width of a product.  A tile's main loop takes about c per K block (c2 from the 33rd on, where the start-up of the ring no
 // longer counts) and its epilogue e, which runs beside the next tile's main loop; what does not overlap is the first main loop and
 // the last epilogue:
@@ -1087,9 +1419,9 @@ inline TileChoice choose_tile(long long M, long long N, long long K, long long b
 }
 
 // Launch of the CTA-pair form: an even grid of at most one CTA per SM, in clusters of two.
-template <bool A_MN, bool B_MN>
-int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
-  constexpr int BN = 256, STAGES = 6;
+template <bool A_MN, bool B_MN, int STAGES>
+int launch_pair_ring(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
+  constexpr int BN = 256;
   using L = SmemLayout<BN / 2, STAGES>;
   auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, COMM_NONE, 2>;
   static bool configured[st::kMaxDevices] = {false};   // the attribute is per device
@@ -1115,6 +1447,12 @@ int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& t
   GemmComm none{};
   ST_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, tmA, p, none));
   return ST_OK;
+}
+
+template <bool A_MN, bool B_MN>
+int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
+  if (plain_epilogue(p)) return launch_pair_ring<A_MN, B_MN, 6>(tmA, tmB, tmC, p, stream);
+  return launch_pair_ring<A_MN, B_MN, 5>(tmA, tmB, tmC, p, stream);
 }
 
 }  // namespace gemm

@@ -18,7 +18,6 @@
 // (crates/st-tensor/src/wgpu_shaders) and rocBLAS sgemm + hip_gemm_epilogue.cu
 // (crates/st-backend-hip/src/real.rs:759-960).
 #include "gemm_kernel.cuh"
-#include <cstring>
 
 namespace {
 
@@ -144,22 +143,10 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
   p.out_fp32 = a->out_fp32;
   p.accumulate = a->accumulate;
   p.batch = a->batch;
-  p.batch_stride_c = a->batch_stride_c;
+  p.batch_stride_c = a->batch > 1 ? a->batch_stride_c : 0;
   p.err = st::error_word();
-  p.use_tma_store = (!a->out_fp32 && !a->accumulate && (a->ldc & 7) == 0 &&
-                     (reinterpret_cast<uintptr_t>(a->C) & 15) == 0 &&
-                     (a->batch == 1 || (a->batch_stride_c & 7) == 0)) ? 1 : 0;
   OutMaps tmC;
-  memset(&tmC, 0, sizeof(tmC));
-  if (p.use_tma_store) {
-    uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)a->M, (uint64_t)a->batch};
-    uint64_t strides[2] = {(uint64_t)a->ldc * 2,
-                           a->batch > 1 ? (uint64_t)a->batch_stride_c * 2 : (uint64_t)a->ldc * 2 * a->M};
-    uint32_t box[3] = {64, 32, 1};
-    if (!st::encode_tmap(&tmC.m[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->C, dims, strides, box,
-                         CU_TENSOR_MAP_SWIZZLE_128B))
-      return ST_ERR_CUDA;
-  }
+  if (!plan_epilogue(p, tmC)) return ST_ERR_CUDA;
 
   if (pair) {
     if (!a->a_mn_major && !a->b_mn_major) return launch_pair<false, false>(tmA, tmB, tmC, p, stream);
@@ -167,9 +154,12 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
     if (!a->b_mn_major) return launch_pair<true, false>(tmA, tmB, tmC, p, stream);
     return launch_pair<true, true>(tmA, tmB, tmC, p, stream);
   }
+  const bool plain = plain_epilogue(p), a_mn = a->a_mn_major != 0, b_mn = a->b_mn_major != 0;
   if (BN == 64)
-    return dispatch_major<64, 8>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
+    return plain ? dispatch_major<64, 8>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas)
+                 : dispatch_major<64, 6>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
   if (BN == 128)
-    return dispatch_major<128, 6>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
-  return dispatch_major<256, 4>(a->a_mn_major != 0, a->b_mn_major != 0, tmA, tmB, tmC, p, stream, a->max_ctas);
+    return plain ? dispatch_major<128, 6>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas)
+                 : dispatch_major<128, 5>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
+  return dispatch_major<256, 4>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
 }
