@@ -226,6 +226,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();      // set up beside the previous kernel's end; global memory is touched from here on
 
   if (warp == EW_WARPS) {
     // ---------------------------- TMA producer -----------------------------------------
@@ -628,6 +629,7 @@ __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ O, __nv_bfloat16* __restrict__ dO, const float* __restrict__ dO32,
                   float* __restrict__ delta, int B, int S, int H, long long o_sb, long long o_ss, long long o_sh,
                   long long do_sb, long long do_ss, long long do_sh) {
+  chain_begin(O, dO32);
   constexpr int LPR = D / 8;                       // lanes per row
   const Index total = (Index)B * S * H;
   const int sub = threadIdx.x % LPR;
@@ -710,7 +712,7 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
     auto Op = static_cast<const __nv_bfloat16*>(a->O);
     auto dOp = static_cast<__nv_bfloat16*>(const_cast<void*>(a->dO));        // written only from dO32
     auto delta = [&](auto kernel) {
-      kernel<<<(unsigned)blocks, 256, 0, s>>>(Op, dOp, dO32, a->delta, a->B, a->Sq, a->H, a->o_sb, a->o_ss, a->o_sh, a->do_sb,
+      st::chained(kernel, (unsigned)blocks, 256, 0, s)(Op, dOp, dO32, a->delta, a->B, a->Sq, a->H, a->o_sb, a->o_ss, a->o_sh, a->do_sb,
                                               a->do_ss, a->do_sh);
     };
     const bool narrow = rows + blocks * rows_per_block < (1ll << 31);      // the last step's index must not wrap either
@@ -765,7 +767,7 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
   const dim3 grid_q(items_q < num_sms ? items_q : num_sms);
   auto launch = [&](auto kernel, int smem_bytes, dim3 grid) -> int {
     ST_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    kernel<<<grid, NUM_THREADS, smem_bytes, s>>>(tq, tk, tv, tdo, p);
+    st::chained(kernel, grid, NUM_THREADS, smem_bytes, s)(tq, tk, tv, tdo, p);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
   };

@@ -148,6 +148,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();      // set up beside the previous kernel's end; global memory is touched from here on
 
   if (warp == 8) {
     // ---------------------------- TMA producer -----------------------------------------
@@ -470,6 +471,7 @@ struct PairSmem {
 // out[b, (h,) key] = key_bias * log2(e) for the keys below the valid length, minus infinity from there to the padded end
 __global__ void attn_key_bias_kernel(const float* __restrict__ kb, long long kb_sb, long long kb_sh, const int* __restrict__ lengths,
                                      float* __restrict__ out, int heads, int Sk, int padded, long long total) {
+  chain_begin(kb, lengths);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int key = (int)(i % padded);
     const long long row = i / padded;
@@ -564,6 +566,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();      // set up beside the previous kernel's end; global memory is touched from here on
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PAIR_REGS_AUX));
@@ -958,7 +961,7 @@ int attn_key_bias(const float* kb, long long kb_sb, long long kb_sh, const int* 
   *out_sh = heads > 1 ? padded : 0;
   long long blocks = (total + 255) / 256;
   if (blocks > 16ll * sm_count()) blocks = 16ll * sm_count();
-  attn_key_bias_kernel<<<(unsigned)blocks, 256, 0, stream>>>(kb, kb_sb, kb_sh, lengths, ws, heads, Sk, padded, total);
+  st::chained(attn_key_bias_kernel, (unsigned)blocks, 256, 0, stream)(kb, kb_sb, kb_sh, lengths, ws, heads, Sk, padded, total);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -1061,7 +1064,7 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
         ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         cfg[dev] = true;
       }
-      kern<<<pgrid, PAIR_THREADS, smem_bytes, s>>>(tq, tk, tv, p);
+      st::chained(kern, pgrid, PAIR_THREADS, smem_bytes, s)(tq, tk, tv, p);
       return ST_OK;
     };
     static bool pcfg[6][st::kMaxDevices] = {{false}};
@@ -1087,7 +1090,7 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
       ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
       cfg[st::current_device()] = true;
     }
-    kern<<<grid, NUM_THREADS, smem_bytes, s>>>(tq, tk, tv, p);
+    st::chained(kern, grid, NUM_THREADS, smem_bytes, s)(tq, tk, tv, p);
     return ST_OK;
   };
   static bool cfg[4][st::kMaxDevices] = {{false}};

@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 #include <cuda.h>
 #include <stdint.h>
+#include "chain.cuh"
 
 #ifndef ST_WAIT_TIMEOUT_NS
 #define ST_WAIT_TIMEOUT_NS 2000000000ull  // 2 s

@@ -38,7 +38,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& t
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
   const int grid = tiles < st::sm_count() ? tiles : st::sm_count();
   GemmComm none{};
-  kern<<<grid, NUM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmC, tmA, p, none);
+  st::chained(kern, grid, NUM_THREADS, L::TOTAL, stream)(tmA, tmB, tmC, tmA, p, none);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -73,6 +73,7 @@ template <typename Index>
 __global__ void __launch_bounds__(256)
 im2col3x3_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col,
                        int N, int H, int W, int C, int Kpad, int aligned) {
+  chain_begin(x);
   const int K8 = Kpad / 8;
   const Index total = (Index)N * H * W * K8;
   for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (Index)gridDim.x * blockDim.x) {
@@ -109,6 +110,7 @@ im2col3x3_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __res
 template <int C>
 __global__ void __launch_bounds__(256)
 im2col3x3_image_kernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ col, long long pixels, int H, int W) {
+  chain_begin(x);
   constexpr int K8 = (9 * C + 31) / 32 * 4;
   __shared__ uint4 rows[256 * K8];
   const __nv_bfloat16 zero = __float2bfloat16(0.0f);
@@ -150,6 +152,7 @@ im2col3x3_image_kernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ 
 template <typename Index>
 __global__ void __launch_bounds__(256)
 im2col3x3_c8_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, int N, int H, int W, int C8, int K8) {
+  chain_begin(x);
   const Index total = (Index)N * H * W * K8;
   for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (Index)gridDim.x * blockDim.x) {
     const int k = (int)(i % K8);
@@ -167,6 +170,7 @@ im2col3x3_c8_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, int N,
 // Weights of the data-gradient convolution: out[ic][8 - tap][oc] = in[oc][tap][ic], 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256)
 dgrad_weights_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int OC, int IC) {
+  chain_begin(in);
   __shared__ __nv_bfloat16 tile[32][33];
   const int tap = blockIdx.z, ic0 = blockIdx.x * 32, oc0 = blockIdx.y * 32;
   for (int r = threadIdx.y; r < 32; r += 8)
@@ -180,6 +184,7 @@ dgrad_weights_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __rest
 __global__ void __launch_bounds__(256)
 maxpool2_fwd8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                      unsigned char* __restrict__ idx, int N, int H, int W, int C) {
+  chain_begin(x);
   const int OH = H / 2, OW = W / 2, C8 = C / 8;
   const long long total = (long long)N * OH * OW * C8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -222,6 +227,7 @@ maxpool2_fwd8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
 // y[n, h/2, w/2, c] = max over the 2x2 window; idx (uint8) records the arg-max for the backward pass
 __global__ void maxpool2_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                     unsigned char* __restrict__ idx, int N, int H, int W, int C) {
+  chain_begin(x);
   const int OH = H / 2, OW = W / 2;
   const long long total = (long long)N * OH * OW * (C / 2);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -256,6 +262,7 @@ __global__ void maxpool2_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bf
 __global__ void __launch_bounds__(256)
 maxpool2_bwd8_kernel(const uint4* __restrict__ dy, const uint2* __restrict__ idx, const uint4* __restrict__ pooled,
                      uint4* __restrict__ dx, float* __restrict__ dbias, int N, int H, int W, int C8) {
+  chain_begin(dy, idx, pooled);
   const int OH = H / 2, OW = W / 2;
   const long long total = (long long)N * OH * OW * C8;
   float sum[8];
@@ -312,6 +319,7 @@ maxpool2_bwd8_kernel(const uint4* __restrict__ dy, const uint2* __restrict__ idx
 
 __global__ void maxpool2_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const unsigned char* __restrict__ idx,
                                     __nv_bfloat16* __restrict__ dx, int N, int H, int W, int C) {
+  chain_begin(dy, idx);
   const int OH = H / 2, OW = W / 2;
   const long long total = (long long)N * OH * OW * C;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -333,6 +341,7 @@ __global__ void maxpool2_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const 
 // y[n, c] = mean over H*W
 __global__ void avgpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int N,
                                    int HW, int C) {
+  chain_begin(x);
   const int n = blockIdx.x;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     float s = 0.0f;
@@ -342,6 +351,7 @@ __global__ void avgpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfl
 }
 __global__ void avgpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, int N,
                                    int HW, int C) {
+  chain_begin(dy);
   const long long total = (long long)N * HW * C;
   const float inv = 1.0f / HW;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -543,13 +553,13 @@ ST_API int st_im2col3x3_small(const void* x, void* col, int N, int H, int W, int
   if (aligned && C >= 1 && C <= 4 && Kpad == (9 * C + 31) / 32 * 32) {
     const long long pixels = (long long)N * H * W;
     auto kern = C == 1 ? im2col3x3_image_kernel<1> : C == 2 ? im2col3x3_image_kernel<2> : C == 3 ? im2col3x3_image_kernel<3> : im2col3x3_image_kernel<4>;
-    kern<<<grid_for(pixels, 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<uint4*>(col), pixels, H, W);
+    st::chained(kern, grid_for(pixels, 256), 256, 0, s)(static_cast<const __nv_bfloat16*>(x), static_cast<uint4*>(col), pixels, H, W);
   } else if (aligned && (C & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     auto kern = narrow ? im2col3x3_c8_kernel<unsigned> : im2col3x3_c8_kernel<long long>;
-    kern<<<grid, 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<uint4*>(col), N, H, W, C / 8, Kpad / 8);
+    st::chained(kern, grid, 256, 0, s)(static_cast<const uint4*>(x), static_cast<uint4*>(col), N, H, W, C / 8, Kpad / 8);
   } else {
     auto kern = narrow ? im2col3x3_small_kernel<unsigned> : im2col3x3_small_kernel<long long>;
-    kern<<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), N, H, W, C, Kpad, aligned);
+    st::chained(kern, grid, 256, 0, s)(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), N, H, W, C, Kpad, aligned);
   }
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -559,14 +569,14 @@ ST_API int st_maxpool2_fwd(const void* x, void* y, void* idx, int N, int H, int 
   if ((H & 1) || (W & 1) || (C & 1)) return st::fail(ST_ERR_INVALID, "maxpool2: H, W and C must be even");
   if ((C & 7) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(idx) & 7) == 0) {
-    maxpool2_fwd8_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0,
-                           reinterpret_cast<cudaStream_t>(stream_v)>>>(
+    st::chained(maxpool2_fwd8_kernel, grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0,
+                           reinterpret_cast<cudaStream_t>(stream_v))(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), static_cast<unsigned char*>(idx), N, H, W, C);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
   }
-  maxpool2_fwd_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * (C / 2), 256), 256, 0,
-                        reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(maxpool2_fwd_kernel, grid_for((long long)N * (H / 2) * (W / 2) * (C / 2), 256), 256, 0,
+                        reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), static_cast<unsigned char*>(idx), N, H, W, C);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -574,7 +584,7 @@ ST_API int st_maxpool2_fwd(const void* x, void* y, void* idx, int N, int H, int 
 // Weights [OC][9][IC] (tap-major) to those of the data gradient, [IC][9][OC] with the taps reversed.
 ST_API int st_conv3x3_dgrad_weights(const void* w, void* wt, int OC, int IC, void* stream_v) {
   if (!w || !wt || OC <= 0 || IC <= 0) return st::fail(ST_ERR_INVALID, "conv3x3_dgrad_weights: bad arguments");
-  dgrad_weights_kernel<<<dim3((IC + 31) / 32, (OC + 31) / 32, 9), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(dgrad_weights_kernel, dim3((IC + 31) / 32, (OC + 31) / 32, 9), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(wt), OC, IC);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -590,7 +600,7 @@ ST_API int st_maxpool2_relu_bwd(const void* dy, const void* idx, const void* poo
   if (((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(pooled) | reinterpret_cast<uintptr_t>(dx)) & 15) ||
       (reinterpret_cast<uintptr_t>(idx) & 7))
     return st::fail(ST_ERR_INVALID, "maxpool2_relu_bwd: tensors must be 16-byte aligned");
-  maxpool2_bwd8_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(maxpool2_bwd8_kernel, grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const uint4*>(dy), static_cast<const uint2*>(idx), static_cast<const uint4*>(pooled),
       static_cast<uint4*>(dx), dbias, N, H, W, C / 8);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -600,26 +610,26 @@ ST_API int st_maxpool2_relu_bwd(const void* dy, const void* idx, const void* poo
 ST_API int st_maxpool2_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, void* stream_v) {
   if ((H & 1) == 0 && (W & 1) == 0 && (C & 7) == 0 &&
       ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0 && (reinterpret_cast<uintptr_t>(idx) & 7) == 0) {
-    maxpool2_bwd8_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+    st::chained(maxpool2_bwd8_kernel, grid_for((long long)N * (H / 2) * (W / 2) * (C / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
         static_cast<const uint4*>(dy), static_cast<const uint2*>(idx), nullptr, static_cast<uint4*>(dx), nullptr, N, H, W, C / 8);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
   }
-  maxpool2_bwd_kernel<<<grid_for((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0,
-                        reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(maxpool2_bwd_kernel, grid_for((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0,
+                        reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const unsigned char*>(idx), static_cast<__nv_bfloat16*>(dx),
       N, H, W, C);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
 ST_API int st_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream_v) {
-  avgpool_fwd_kernel<<<N, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(avgpool_fwd_kernel, N, 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), N, HW, C);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
 ST_API int st_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, void* stream_v) {
-  avgpool_bwd_kernel<<<grid_for((long long)N * HW * C, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(avgpool_bwd_kernel, grid_for((long long)N * HW * C, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), N, HW, C);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;

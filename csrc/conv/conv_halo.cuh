@@ -76,6 +76,7 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();      // set up beside the previous kernel's end; global memory is touched from here on
 
   if (warp == 0) {
     // ------------------------------- TMA producer (converged warp, one lane issues) -------------------------------
@@ -237,7 +238,7 @@ int launch_halo(const CUtensorMap& tmX, const CUtensorMap& tmW, const CUtensorMa
     ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     configured[dev] = true;
   }
-  kern<<<p.tiles < st::sm_count() ? p.tiles : st::sm_count(), kHaloThreads, smem, stream>>>(tmX, tmW, tmY, p);
+  st::chained(kern, p.tiles < st::sm_count() ? p.tiles : st::sm_count(), kHaloThreads, smem, stream)(tmX, tmW, tmY, p);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }

@@ -30,6 +30,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cs,
                             const float* __restrict__ sn, long long T, int heads, int D,
                             long long ld, int seq_len, int pos_offset, float sign) {
+  chain_begin(cs, sn);
   const int half = D >> 1;
   const int vec_per_head = half >> 3;
   const long long total = T * heads * vec_per_head;
@@ -66,6 +67,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // ------------------------------------------------------------------------------------
 __global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                 long long n8, int relu) {
+  chain_begin(x);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
     float v[8];
@@ -77,6 +79,7 @@ __global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat
 }
 __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                                 __nv_bfloat16* __restrict__ dx, long long n8, int relu) {
+  chain_begin(x, dy);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
     float v[8], g[8];
@@ -91,6 +94,7 @@ __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 // out[c] (+)= sum_r x[r, c]; grid (ceil(cols/32), row_chunks); fp32 atomics across chunks.
 __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out,
                               long long rows, int cols, long long ld) {
+  chain_begin(x);
   __shared__ float sh[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   const long long rows_per = (rows + gridDim.y - 1) / gridDim.y;
@@ -115,6 +119,7 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __rest
 template <int BX, int LANES, bool STORE>
 __global__ void __launch_bounds__(BX * LANES)
 colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long rows, int cols, long long ld) {
+  chain_begin(x);
   constexpr int WIDTH = BX * 8, PARTS = BX * LANES / WIDTH, lanes = LANES;      // PARTS threads add a column's lanes
   __shared__ float sh[LANES * (WIDTH + 1)];
   __shared__ float part[PARTS > 1 ? PARTS * WIDTH : 1];
@@ -181,6 +186,7 @@ colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, lon
 __global__ void embedding_fwd_kernel(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ W,
                                      const __nv_bfloat16* __restrict__ pos, __nv_bfloat16* __restrict__ out,
                                      long long T, int d, int vocab_start, int vocab_local, int seq_len) {
+  chain_begin(idx, W, pos);
   const int vec = d >> 3;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < T * vec;
        i += (long long)gridDim.x * blockDim.x) {
@@ -207,6 +213,7 @@ __device__ __forceinline__ void red_add4(float* addr, float a, float b, float c,
 __global__ void embedding_bwd_kernel(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ dy,
                                      float* __restrict__ dW, float* __restrict__ dpos, long long T, int d,
                                      int vocab_start, int vocab_local, int seq_len, int vec4) {
+  chain_begin(idx, dy);
   // vec4: both tables start on a 16-byte boundary, so the additions can go out four at a time
   const int vec = d >> 3;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < T * vec;
@@ -246,6 +253,7 @@ __global__ void embedding_bwd_sorted_kernel(const long long* __restrict__ uniq_i
                                             const long long* __restrict__ seg_count, const long long* __restrict__ perm,
                                             const __nv_bfloat16* __restrict__ dy, float* __restrict__ dW, int d,
                                             int vocab_start, int vocab_local) {
+  chain_begin(uniq_ids, seg_start, seg_count, perm, dy);
   const long long id = uniq_ids[blockIdx.x] - vocab_start;
   if (id < 0 || id >= vocab_local) return;
   const long long start = seg_start[blockIdx.x], count = seg_count[blockIdx.x];
@@ -268,6 +276,7 @@ __global__ void embedding_bwd_sorted_kernel(const long long* __restrict__ uniq_i
 // ------------------------------------------------------------------------------------
 __global__ void row_softmax_kernel(const float* __restrict__ x, float* __restrict__ y,
                                    float* __restrict__ hard, int rows, int cols) {
+  chain_begin(x);
   __shared__ float sh[32];
   __shared__ int shi[32];
   const int row = blockIdx.x;
@@ -332,6 +341,7 @@ struct SpiralConsts {
 __global__ void row_softmax_spiral_kernel(const float* __restrict__ x, float* __restrict__ y, float* __restrict__ hard,
                                           float* __restrict__ spiral, float* __restrict__ metrics,
                                           float* __restrict__ zmetrics, int rows, int cols, SpiralConsts k) {
+  chain_begin(x);
   __shared__ float sh[32];
   __shared__ int shi[32];
   __shared__ float red[5][32];
@@ -443,6 +453,7 @@ __global__ void __launch_bounds__(512)
 ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
                 float* __restrict__ row_max, float* __restrict__ row_sum, float* __restrict__ tgt_logit,
                 long long ld, int V, int vocab_start) {
+  chain_begin(logits, target);
   __shared__ float shm[16], shs[16];
   const long long row = blockIdx.x;
   const __nv_bfloat16* lr = logits + row * ld;
@@ -504,6 +515,7 @@ ce_grad_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __rest
                const float* __restrict__ lse, const float* __restrict__ coef_ptr, float coef,
                __nv_bfloat16* __restrict__ dlogits, long long ld, int V, int vocab_start,
                long long ignore_index) {
+  chain_begin(logits, target, lse, coef_ptr);
   const long long row = blockIdx.x;
   const __nv_bfloat16* lr = logits + row * ld;
   __nv_bfloat16* dr = dlogits + row * ld;
@@ -541,7 +553,7 @@ ST_API int st_rope(void* x, const float* cos_t, const float* sin_t, long long T,
   if (D % 16 != 0 || (ld & 7) || (reinterpret_cast<uintptr_t>(x) & 15))
     return st::fail(ST_ERR_INVALID, "rope: head_dim must be a multiple of 16 and rows 16-byte aligned");
   const long long total = T * heads * (D / 16);
-  rope_kernel<<<grid_for(total, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(rope_kernel, grid_for(total, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<__nv_bfloat16*>(x), cos_t, sin_t, T, heads, D, ld, seq_len, pos_offset,
       backward ? -1.0f : 1.0f);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -550,14 +562,14 @@ ST_API int st_rope(void* x, const float* cos_t, const float* sin_t, long long T,
 
 ST_API int st_act_fwd(const void* x, void* y, long long n, int relu, void* stream_v) {
   if (n & 7) return st::fail(ST_ERR_INVALID, "act: element count must be a multiple of 8");
-  gelu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(gelu_fwd_kernel, grid_for(n / 8, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), n / 8, relu);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
 ST_API int st_act_bwd(const void* x, const void* dy, void* dx, long long n, int relu, void* stream_v) {
   if (n & 7) return st::fail(ST_ERR_INVALID, "act: element count must be a multiple of 8");
-  gelu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(gelu_bwd_kernel, grid_for(n / 8, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy),
       static_cast<__nv_bfloat16*>(dx), n / 8, relu);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -573,7 +585,7 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
     if (chunks > 512) chunks = 512;
     const int bx = cols <= 64 ? 8 : (cols <= 128 ? 16 : 32);
     auto kern = bx == 8 ? colsum8_kernel<8, 32, false> : (bx == 16 ? colsum8_kernel<16, 16, false> : colsum8_kernel<32, 8, false>);
-    kern<<<dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+    st::chained(kern, dim3((cols + bx * 8 - 1) / (bx * 8), chunks), dim3(bx, 256 / bx), 0, reinterpret_cast<cudaStream_t>(stream_v))(
         static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
@@ -583,7 +595,7 @@ ST_API int st_colsum(const void* x, float* out, long long rows, int cols, long l
   if (chunks < 1) chunks = 1;
   if (chunks > 256) chunks = 256;
   dim3 grid((cols + 31) / 32, chunks);
-  colsum_kernel<<<grid, block, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(colsum_kernel, grid, block, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(x), out, rows, cols, ld);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -599,8 +611,8 @@ ST_API int st_colsum_short(const void* x, float* out, long long rows, int cols, 
   auto X = static_cast<const __nv_bfloat16*>(x);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   const unsigned narrow = (cols + 63) / 64;
-  if (rows <= 128 || narrow > (unsigned)st::sm_count()) colsum8_kernel<8, 32, true><<<narrow, dim3(8, 32), 0, s>>>(X, out, rows, cols, ld);
-  else colsum8_kernel<8, 128, true><<<narrow, dim3(8, 128), 0, s>>>(X, out, rows, cols, ld);
+  if (rows <= 128 || narrow > (unsigned)st::sm_count()) st::chained(colsum8_kernel<8, 32, true>, narrow, dim3(8, 32), 0, s)(X, out, rows, cols, ld);
+  else st::chained(colsum8_kernel<8, 128, true>, narrow, dim3(8, 128), 0, s)(X, out, rows, cols, ld);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -609,7 +621,7 @@ ST_API int st_embedding_fwd(const long long* idx, const void* W, const void* pos
                             long long T, int d, int vocab_start, int vocab_local, int seq_len,
                             void* stream_v) {
   if (d & 7) return st::fail(ST_ERR_INVALID, "embedding: dim must be a multiple of 8");
-  embedding_fwd_kernel<<<grid_for(T * (d / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(embedding_fwd_kernel, grid_for(T * (d / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       idx, static_cast<const __nv_bfloat16*>(W), static_cast<const __nv_bfloat16*>(pos),
       static_cast<__nv_bfloat16*>(out), T, d, vocab_start, vocab_local, seq_len > 0 ? seq_len : 1);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -618,7 +630,7 @@ ST_API int st_embedding_fwd(const long long* idx, const void* W, const void* pos
 ST_API int st_embedding_bwd(const long long* idx, const void* dy, float* dW, float* dpos, long long T,
                             int d, int vocab_start, int vocab_local, int seq_len, void* stream_v) {
   if (d & 7) return st::fail(ST_ERR_INVALID, "embedding: dim must be a multiple of 8");
-  embedding_bwd_kernel<<<grid_for(T * (d / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(embedding_bwd_kernel, grid_for(T * (d / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       idx, static_cast<const __nv_bfloat16*>(dy), dW, dpos, T, d, vocab_start, vocab_local,
       seq_len > 0 ? seq_len : 1,
       ((reinterpret_cast<uintptr_t>(dW) | reinterpret_cast<uintptr_t>(dpos)) & 15) == 0 ? 1 : 0);
@@ -634,7 +646,7 @@ ST_API int st_embedding_bwd_sorted(const long long* uniq_ids, const long long* s
   if (d & 7) return st::fail(ST_ERR_INVALID, "embedding: dim must be a multiple of 8");
   if (n_unique <= 0) return ST_OK;
   const int threads = d >= 2048 ? 256 : (d >= 512 ? 64 : 32);
-  embedding_bwd_sorted_kernel<<<(unsigned)n_unique, threads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(embedding_bwd_sorted_kernel, (unsigned)n_unique, threads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       uniq_ids, seg_start, seg_count, perm, static_cast<const __nv_bfloat16*>(dy), dW, d, vocab_start, vocab_local);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -643,7 +655,7 @@ ST_API int st_embedding_bwd_sorted(const long long* uniq_ids, const long long* s
 ST_API int st_row_softmax_f32(const float* x, float* y, float* hard, int rows, int cols, void* stream_v) {
   if (rows <= 0 || cols <= 0) return st::fail(ST_ERR_INVALID, "softmax: empty input");
   int threads = cols >= 1024 ? 256 : (cols >= 128 ? 128 : 32);
-  row_softmax_kernel<<<rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(x, y, hard, rows, cols);
+  st::chained(row_softmax_kernel, rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v))(x, y, hard, rows, cols);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -655,7 +667,7 @@ ST_API int st_row_softmax_spiral_f32(const float* x, float* y, float* hard, floa
   if (!x || !y) return st::fail(ST_ERR_INVALID, "softmax: null pointer");
   int threads = cols >= 1024 ? 256 : (cols >= 128 ? 128 : 32);
   SpiralConsts k{phi, phi_conj, phi_bias, leech_scale, ramanujan_ratio, golden_angle};
-  row_softmax_spiral_kernel<<<rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(x, y, hard, spiral, metrics,
+  st::chained(row_softmax_spiral_kernel, rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v))(x, y, hard, spiral, metrics,
                                                                                            zmetrics, rows, cols, k);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -667,7 +679,7 @@ ST_API int st_ce_stats(const void* logits, const long long* target, float* row_m
   if ((ld & 7) || (reinterpret_cast<uintptr_t>(logits) & 15))
     return st::fail(ST_ERR_INVALID, "ce: logits rows must be 16-byte aligned");
   const int threads = V >= 8192 ? 512 : 128;
-  ce_stats_kernel<<<(unsigned)rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(ce_stats_kernel, (unsigned)rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(logits), target, row_max, row_sum, tgt_logit, ld, V, vocab_start);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -678,7 +690,7 @@ ST_API int st_ce_grad(const void* logits, const long long* target, const float* 
   if ((ld & 7) || (reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(dlogits) & 15))
     return st::fail(ST_ERR_INVALID, "ce: logits rows must be 16-byte aligned");
   const int threads = V >= 8192 ? 512 : 128;
-  ce_grad_kernel<<<(unsigned)rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(ce_grad_kernel, (unsigned)rows, threads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(logits), target, lse, coef_ptr, coef,
       static_cast<__nv_bfloat16*>(dlogits), ld, V, vocab_start, ignore_index);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -697,6 +709,7 @@ struct NdIndexerParams {
 
 __global__ void nd_indexer_kernel(const unsigned* __restrict__ positions, unsigned* __restrict__ out_index,
                                   unsigned* __restrict__ out_segment, long long n, NdIndexerParams p) {
+  chain_begin(positions);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     unsigned remaining = positions[i], flat = 0;
 #pragma unroll
@@ -723,7 +736,7 @@ ST_API int st_nd_indexer(const unsigned* positions, unsigned* out_index, unsigne
   p.segments = segments; p.segment_stride = segment_stride;
   long long blocks = (n + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  nd_indexer_kernel<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(positions, out_index, out_segment, n, p);
+  st::chained(nd_indexer_kernel, (unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(positions, out_index, out_segment, n, p);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }

@@ -14,6 +14,7 @@ constexpr int kThreads = 256;
 __global__ void __launch_bounds__(kThreads)
 views_kernel(const float4* __restrict__ base, const float4* __restrict__ n1, const float4* __restrict__ n2, float noise,
              uint2* __restrict__ out, long long n4) {
+  st::chain_begin(base, n1, n2);
   for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < n4; i += (long long)gridDim.x * kThreads) {
     const float4 b = base[i], u = n1[i], v = n2[i];
     auto at = [noise](float x, float z) { return __fadd_rn(x, __fmul_rn(noise, z)); };
@@ -27,6 +28,7 @@ constexpr float kTiny = 1e-12f;
 // y = z / max(|z|, 1e-12) per row in fp32, and |z|; one warp per row
 __global__ void __launch_bounds__(kThreads)
 row_normalize_kernel(const __nv_bfloat16* __restrict__ z, float* __restrict__ y, float* __restrict__ norm, int rows, int d) {
+  st::chain_begin(z);
   const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const __nv_bfloat16* zr = z + (size_t)row * d;
@@ -44,6 +46,7 @@ row_normalize_kernel(const __nv_bfloat16* __restrict__ z, float* __restrict__ y,
 __global__ void __launch_bounds__(kThreads)
 row_normalize_bwd_kernel(const float* __restrict__ g, const float* __restrict__ y, const float* __restrict__ norm,
                          __nv_bfloat16* __restrict__ dz, int rows, int d) {
+  st::chain_begin(g, y, norm);
   const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const size_t base = (size_t)row * d;
@@ -61,6 +64,7 @@ row_normalize_bwd_kernel(const float* __restrict__ g, const float* __restrict__ 
 // temperature), the gradient of the mean loss.  The row waits in shared memory between the passes.
 __global__ void __launch_bounds__(kThreads)
 nce_rows_kernel(float* __restrict__ s, float* __restrict__ loss, int rows, int cols, float temperature) {
+  st::chain_begin();
   extern __shared__ float x[];
   __shared__ float sh[kThreads / 32];
   float* row = s + (size_t)blockIdx.x * cols;
@@ -99,7 +103,7 @@ ST_API int st_contrastive_views(const float* base, const float* n1, const float*
     return st::fail(ST_ERR_INVALID, "contrastive_views: tensors must be 16-byte aligned");
   long long blocks = (n / 4 + kThreads - 1) / kThreads;
   if (blocks > 8ll * st::sm_count()) blocks = 8ll * st::sm_count();
-  views_kernel<<<(unsigned)blocks, kThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(views_kernel, (unsigned)blocks, kThreads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       reinterpret_cast<const float4*>(base), reinterpret_cast<const float4*>(n1), reinterpret_cast<const float4*>(n2), noise,
       static_cast<uint2*>(out), n / 4);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -108,7 +112,7 @@ ST_API int st_contrastive_views(const float* base, const float* n1, const float*
 
 ST_API int st_row_normalize(const void* z, float* y, float* norm, int rows, int d, void* stream_v) {
   if (!z || !y || !norm || rows <= 0 || d <= 0) return st::fail(ST_ERR_INVALID, "row_normalize: bad arguments");
-  row_normalize_kernel<<<(rows + 7) / 8, kThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(row_normalize_kernel, (rows + 7) / 8, kThreads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       static_cast<const __nv_bfloat16*>(z), y, norm, rows, d);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -116,7 +120,7 @@ ST_API int st_row_normalize(const void* z, float* y, float* norm, int rows, int 
 
 ST_API int st_row_normalize_bwd(const float* g, const float* y, const float* norm, void* dz, int rows, int d, void* stream_v) {
   if (!g || !y || !norm || !dz || rows <= 0 || d <= 0) return st::fail(ST_ERR_INVALID, "row_normalize_bwd: bad arguments");
-  row_normalize_bwd_kernel<<<(rows + 7) / 8, kThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(row_normalize_bwd_kernel, (rows + 7) / 8, kThreads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       g, y, norm, static_cast<__nv_bfloat16*>(dz), rows, d);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -126,7 +130,7 @@ ST_API int st_row_normalize_bwd(const float* g, const float* y, const float* nor
 ST_API int st_nce_rows(float* s, float* loss, int rows, float temperature, void* stream_v) {
   if (!s || !loss || rows <= 0 || !(temperature > 0.0f)) return st::fail(ST_ERR_INVALID, "nce_rows: bad arguments");
   if (rows > 12000) return st::fail(ST_ERR_TOO_LARGE, "nce_rows: the row does not fit in shared memory");
-  nce_rows_kernel<<<rows, kThreads, rows * sizeof(float), reinterpret_cast<cudaStream_t>(stream_v)>>>(s, loss, rows, rows, temperature);
+  st::chained(nce_rows_kernel, rows, kThreads, rows * sizeof(float), reinterpret_cast<cudaStream_t>(stream_v))(s, loss, rows, rows, temperature);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }

@@ -31,6 +31,7 @@ enum MultiOp : int { MULTI_CHECK = 0, MULTI_DIV = 1, MULTI_STEP = 2 };
 template <int OP>
 __global__ void __launch_bounds__(kMultiThreads)
 multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict__ bad, int slots) {
+  st::chain_begin();
   int which = 0;
 #pragma unroll
   for (int step = 32; step > 0; step >>= 1)
@@ -70,6 +71,7 @@ multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict_
 // dst (bf16) = src (fp32) for a list of tensors, eight elements per thread and step; the tail element by element
 __global__ void __launch_bounds__(kMultiThreads)
 multi_cast_kernel(const __grid_constant__ MultiTable t) {
+  st::chain_begin();
   const float* __restrict__ src = t.src[blockIdx.y];
   __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(t.dst[blockIdx.y]);
   const long long n = t.n[blockIdx.y], n8 = n / 8;
@@ -96,6 +98,7 @@ __device__ __forceinline__ float block_sum_256(float v, float* sh) {
 __global__ void __launch_bounds__(kMultiThreads)
 mse_forward_kernel(const float* __restrict__ p, const float* __restrict__ t, long long n, float* __restrict__ value,
                    float* __restrict__ part, unsigned* __restrict__ arrived, int* __restrict__ bad) {
+  st::chain_begin(p, t);
   __shared__ float sh[kMultiThreads / 32];
   __shared__ bool last;
   float s = 0.0f;
@@ -131,6 +134,7 @@ mse_forward_kernel(const float* __restrict__ p, const float* __restrict__ t, lon
 __global__ void __launch_bounds__(kMultiThreads)
 mse_backward_kernel(const float* __restrict__ p, const float* __restrict__ t, long long n, float inv_n, float* __restrict__ g,
                     int* __restrict__ bad) {
+  st::chain_begin(p, t);
   bool odd = false;
   for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kMultiThreads) {
     const float a = p[i], b = t[i];
@@ -193,9 +197,9 @@ int run_multi(int op, int count, const void* const* src, void* const* dst, void*
   for (int i = count; i <= kMultiMax; ++i) t.first[i] = i == count ? grid : 0x7FFFFFFF;
   const int slots = blocks_for(most, cap);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
-  if (op == MULTI_CHECK) multi_kernel<MULTI_CHECK><<<grid, kMultiThreads, 0, s>>>(t, value, bad, slots);
-  else if (op == MULTI_DIV) multi_kernel<MULTI_DIV><<<grid, kMultiThreads, 0, s>>>(t, value, bad, slots);
-  else multi_kernel<MULTI_STEP><<<grid, kMultiThreads, 0, s>>>(t, value, bad, slots);
+  if (op == MULTI_CHECK) st::chained(multi_kernel<MULTI_CHECK>, grid, kMultiThreads, 0, s)(t, value, bad, slots);
+  else if (op == MULTI_DIV) st::chained(multi_kernel<MULTI_DIV>, grid, kMultiThreads, 0, s)(t, value, bad, slots);
+  else st::chained(multi_kernel<MULTI_STEP>, grid, kMultiThreads, 0, s)(t, value, bad, slots);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -218,7 +222,7 @@ ST_API int st_multi_cast_bf16(int count, const void* const* src, void* const* ds
     most = n[i] > most ? n[i] : most;
   }
   const dim3 grid(blocks_for(most / 2, 8 * st::sm_count()), count);
-  multi_cast_kernel<<<grid, kMultiThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(t);
+  st::chained(multi_cast_kernel, grid, kMultiThreads, 0, reinterpret_cast<cudaStream_t>(stream_v))(t);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -234,14 +238,14 @@ ST_API int st_mse_forward(const float* p, const float* t, long long n, float* va
   unsigned* arrived = reinterpret_cast<unsigned*>(part + kMultiThreads);
   const int blocks = blocks_for(n, kMultiThreads);
   if (blocks > 1) ST_CUDA_CHECK(cudaMemsetAsync(arrived, 0, sizeof(unsigned), s));
-  mse_forward_kernel<<<blocks, kMultiThreads, 0, s>>>(p, t, n, value, part, arrived, bad);
+  st::chained(mse_forward_kernel, blocks, kMultiThreads, 0, s)(p, t, n, value, part, arrived, bad);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
 
 ST_API int st_mse_backward(const float* p, const float* t, long long n, float* g, int* bad, void* stream_v) {
   if (!p || !t || !g || !bad || n <= 0) return st::fail(ST_ERR_INVALID, "mse: bad arguments");
-  mse_backward_kernel<<<blocks_for(n, kMultiThreads), kMultiThreads, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(mse_backward_kernel, blocks_for(n, kMultiThreads), kMultiThreads, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       p, t, n, 1.0f / (float)n, g, bad);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;

@@ -380,6 +380,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if constexpr (CG == 2) cluster_sync(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // barriers, tensor memory and descriptors are set up beside the previous kernel's end; global memory is touched from here on
+  if constexpr (COMM == COMM_NONE) chain_begin();
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------------
@@ -1432,20 +1434,8 @@ int launch_pair_ring(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMa
   }
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch;
   const int pairs = st::sm_count() / 2;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(2 * (tiles < pairs ? tiles : pairs));
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = L::TOTAL;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
   GemmComm none{};
-  ST_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, tmA, p, none));
+  ST_CUDA_CHECK(st::chained(kern, 2 * (tiles < pairs ? tiles : pairs), NUM_THREADS, L::TOTAL, stream, 2)(tmA, tmB, tmC, tmA, p, none));
   return ST_OK;
 }
 

@@ -58,6 +58,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ sum_out,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int d,
                 float eps) {
+  chain_begin(x, residual, gamma, beta);
   __shared__ float sh[NT / 32];
   const int row = blockIdx.x;
   if (row >= rows) return;
@@ -142,6 +143,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ partial_dgamma,
                 float* __restrict__ partial_dbeta, int rows, int d) {
+  chain_begin(dy, x, gamma, mean_in, rstd_in, dres);
   __shared__ float sh[NT / 32];
   const int nvec = d >> 3;
   float g[MV][8], dg[MV][8], db[MV][8];
@@ -222,6 +224,7 @@ __global__ void __launch_bounds__(NT, 4)
 rms_bwd_ahead_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                      const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ partial_dgamma, int rows, int d) {
+  chain_begin(dy, x, gamma, rstd_in, dres);
   __shared__ __align__(16) float sh[2][NT / 32];
   const uint4 zero = make_uint4(0, 0, 0, 0);
   const bool live = threadIdx.x < (d >> 3);
@@ -353,6 +356,7 @@ __global__ void __launch_bounds__(NT)
 norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ gamma,
                      const T* __restrict__ beta, T* __restrict__ y, T* __restrict__ sum_out, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, int rows, int d, float eps) {
+  chain_begin(x, residual, gamma, beta);
   const int row = blockIdx.x * WARP_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const int nvec = d >> 3;
@@ -439,6 +443,7 @@ norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T*
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
                      T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta, int rows, int d,
                      const T* __restrict__ beta = nullptr) {
+  chain_begin(dy, x, gamma, mean_in, rstd_in, dres, beta);
   __shared__ float sh[2][NT / 32][2 * ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int c0 = threadIdx.x * 8;
@@ -537,6 +542,7 @@ norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T*
 __global__ void __launch_bounds__(1024)
 reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, const float* __restrict__ partial2,
                        float* __restrict__ out2, int parts, int d, int accumulate) {
+  chain_begin(partial, partial2);
   if (blockIdx.y) {
     partial = partial2;
     out = out2;
@@ -575,8 +581,8 @@ int fwd_warp(int rms, const T* x, const T* r, const T* g, const T* b, T* y, T* s
              float eps, cudaStream_t stream) {
   const int grid = (rows + WARP_ROWS - 1) / WARP_ROWS;
 #define ST_FWD_WARP(MVV) \
-  if (rms) norm_fwd_warp_kernel<T, true, MVV><<<grid, NT, 0, stream>>>(x, r, g, b, y, s, mean, rstd, rows, d, eps); \
-  else norm_fwd_warp_kernel<T, false, MVV><<<grid, NT, 0, stream>>>(x, r, g, b, y, s, mean, rstd, rows, d, eps)
+  if (rms) st::chained(norm_fwd_warp_kernel<T, true, MVV>, grid, NT, 0, stream)(x, r, g, b, y, s, mean, rstd, rows, d, eps); \
+  else st::chained(norm_fwd_warp_kernel<T, false, MVV>, grid, NT, 0, stream)(x, r, g, b, y, s, mean, rstd, rows, d, eps)
   switch ((d + 255) / 256) {
     case 1: ST_FWD_WARP(1); break;
     case 2: ST_FWD_WARP(2); break;
@@ -593,8 +599,8 @@ int bwd_rows(int rms, const T* dy, const T* x, const T* g, const float* mean, co
              float* pg, float* pb, int rows, int d, int grid, cudaStream_t stream) {
   constexpr int ROWS = 2;
   const int threads = bwd_threads(d);
-  if (rms) norm_bwd_rows_kernel<T, true, ROWS><<<grid, threads, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, nullptr, rows, d);
-  else norm_bwd_rows_kernel<T, false, ROWS><<<grid, threads, 0, stream>>>(dy, x, g, mean, rstd, dres, dx, pg, pb, rows, d);
+  if (rms) st::chained(norm_bwd_rows_kernel<T, true, ROWS>, grid, threads, 0, stream)(dy, x, g, mean, rstd, dres, dx, pg, nullptr, rows, d, nullptr);
+  else st::chained(norm_bwd_rows_kernel<T, false, ROWS>, grid, threads, 0, stream)(dy, x, g, mean, rstd, dres, dx, pg, pb, rows, d, nullptr);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -602,7 +608,7 @@ int bwd_rows(int rms, const T* dy, const T* x, const T* g, const float* mean, co
 int reduce_param_grads(int rms, const float* pg, const float* pb, float* dgamma, float* dbeta, int grid, int d, int accumulate,
                        cudaStream_t stream) {
   const bool both = !rms && dbeta;
-  reduce_partials_kernel<<<dim3((d + 31) / 32, both ? 2 : 1), 1024, 0, stream>>>(pg, dgamma, pb, dbeta, grid, d, accumulate);
+  st::chained(reduce_partials_kernel, dim3((d + 31) / 32, both ? 2 : 1), 1024, 0, stream)(pg, dgamma, pb, dbeta, grid, d, accumulate);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -653,7 +659,7 @@ ST_API int st_norm_fwd(int rms, const void* x, const void* residual, const void*
   // vector per lane and never loses.
   const bool few = rows <= (d > 512 ? 8 : 4) * st::sm_count() && d > 256;
   if (d <= kWarpRowFeatures && !few) return fwd_warp<__nv_bfloat16>(rms, X, R, G, B, Y, S, mean, rstd, rows, d, eps, s);
-#define ST_NORM_FWD(RMSV, MVV) norm_fwd_kernel<RMSV, MVV><<<rows, NT, 0, s>>>(X, R, G, B, Y, S, mean, rstd, rows, d, eps)
+#define ST_NORM_FWD(RMSV, MVV) st::chained(norm_fwd_kernel<RMSV, MVV>, rows, NT, 0, s)(X, R, G, B, Y, S, mean, rstd, rows, d, eps)
   const int mv = d <= NT * 8 ? 1 : (d <= NT * 16 ? 2 : 4);
   if (rms) {
     if (mv == 1) ST_NORM_FWD(true, 1); else if (mv == 2) ST_NORM_FWD(true, 2); else ST_NORM_FWD(true, 4);
@@ -686,7 +692,7 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
   // few rows: a block per row is one step without a second row's share (64 x 264 4.0 us, in pairs 4.9; 600 x 264 7.4 and 5.5)
   if (rms && rows <= 2 * st::sm_count() && d <= NT * 8) {
     grid = grid < rows ? grid : rows;
-    rms_bwd_ahead_kernel<<<grid, NT, 0, s>>>(DY, X, G, rstd, DR, DX, pg, rows, d);
+    st::chained(rms_bwd_ahead_kernel, grid, NT, 0, s)(DY, X, G, rstd, DR, DX, pg, rows, d);
     ST_CUDA_CHECK(cudaGetLastError());
     return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
   }
@@ -696,10 +702,10 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
     if (int e = bwd_rows<__nv_bfloat16>(rms, DY, X, G, mean, rstd, DR, DX, pg, rms ? nullptr : pb, rows, d, grid, s)) return e;
     return reduce_param_grads(rms, pg, pb, dgamma, dbeta, grid, d, accumulate, s);
   }
-#define ST_NORM_BWD(RMSV, MVV, PB) norm_bwd_kernel<RMSV, MVV><<<grid, NT, 0, s>>>(DY, X, G, mean, rstd, DR, DX, pg, PB, rows, d)
+#define ST_NORM_BWD(RMSV, MVV, PB) st::chained(norm_bwd_kernel<RMSV, MVV>, grid, NT, 0, s)(DY, X, G, mean, rstd, DR, DX, pg, PB, rows, d)
   const int mv = d <= NT * 8 ? 1 : (d <= NT * 16 ? 2 : 4);
   if (rms) {
-    if (mv == 1) rms_bwd_ahead_kernel<<<grid, NT, 0, s>>>(DY, X, G, rstd, DR, DX, pg, rows, d);
+    if (mv == 1) st::chained(rms_bwd_ahead_kernel, grid, NT, 0, s)(DY, X, G, rstd, DR, DX, pg, rows, d);
     else if (mv == 2) ST_NORM_BWD(true, 2, nullptr); else ST_NORM_BWD(true, 4, nullptr);
   } else {
     if (mv == 2) ST_NORM_BWD(false, 2, pb); else ST_NORM_BWD(false, 4, pb);
@@ -712,7 +718,7 @@ int st::norm_bwd_launch(int rms, const void* dy, const void* x, const void* gamm
 // out[i] (+)= sum over p of partial[p * n + i], in a fixed order.
 ST_API int st_reduce_partials(const float* partial, float* out, int parts, int n, int accumulate, void* stream_v) {
   if (!partial || !out || parts <= 0 || n <= 0) return st::fail(ST_ERR_INVALID, "reduce_partials: bad arguments");
-  reduce_partials_kernel<<<(n + 31) / 32, 1024, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(partial, out, nullptr, nullptr, parts, n, accumulate);
+  st::chained(reduce_partials_kernel, (n + 31) / 32, 1024, 0, reinterpret_cast<cudaStream_t>(stream_v))(partial, out, nullptr, nullptr, parts, n, accumulate);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
@@ -733,8 +739,8 @@ ST_API int st_norm_gelu_fwd(const void* x, const void* gamma, const void* beta, 
   const __nv_bfloat16* none = nullptr;
   __nv_bfloat16* no_sum = nullptr;
   const int grid = (rows + WARP_ROWS - 1) / WARP_ROWS;
-#define ST_NORM_GELU(MVV) norm_fwd_warp_kernel<__nv_bfloat16, false, MVV, true><<<grid, NT, 0, s>>>(X, none, G, B, Y, no_sum, mean, rstd, rows, d, eps)
-  if (d > kWarpRowFeatures) norm_fwd_kernel<false, 1, true><<<rows, NT, 0, s>>>(X, none, G, B, Y, no_sum, mean, rstd, rows, d, eps);
+#define ST_NORM_GELU(MVV) st::chained(norm_fwd_warp_kernel<__nv_bfloat16, false, MVV, true>, grid, NT, 0, s)(X, none, G, B, Y, no_sum, mean, rstd, rows, d, eps)
+  if (d > kWarpRowFeatures) st::chained(norm_fwd_kernel<false, 1, true>, rows, NT, 0, s)(X, none, G, B, Y, no_sum, mean, rstd, rows, d, eps);
   else if (d > 768) ST_NORM_GELU(4);
   else if (d > 512) ST_NORM_GELU(3);
   else if (d > 256) ST_NORM_GELU(2);
@@ -753,7 +759,7 @@ ST_API int st_norm_gelu_bwd(const void* dy, const void* x, const void* gamma, co
   if (d > kWarpRowFeatures && grid > st::sm_count() * 3) grid = st::sm_count() * 3;
   float* pb = scratch + (size_t)grid * d;
   const __nv_bfloat16* none = nullptr;
-  norm_bwd_rows_kernel<__nv_bfloat16, false, 2, true><<<grid, bwd_threads(d), 0, s>>>(
+  st::chained(norm_bwd_rows_kernel<__nv_bfloat16, false, 2, true>, grid, bwd_threads(d), 0, s)(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean, rstd,
       none, static_cast<__nv_bfloat16*>(dx), scratch, pb, rows, d, static_cast<const __nv_bfloat16*>(beta));
   ST_CUDA_CHECK(cudaGetLastError());

@@ -51,6 +51,7 @@ __global__ void adamw_kernel(GradT* __restrict__ grad, float* __restrict__ maste
                              float* __restrict__ m, float* __restrict__ v,
                              __nv_bfloat16* __restrict__ weight, long long n, AdamArgs a,
                              const float* __restrict__ scale_ptr, int zero_grad) {
+  chain_begin(scale_ptr);
   const float gs = a.grad_scale * (scale_ptr ? *scale_ptr : 1.0f);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -70,6 +71,7 @@ template <typename GradT>
 __global__ void __launch_bounds__(256)
 adamw4_kernel(GradT* __restrict__ grad, float4* __restrict__ master, float4* __restrict__ m, float4* __restrict__ v,
               uint2* __restrict__ weight, long long n4, AdamArgs a, const float* __restrict__ scale_ptr, int zero_grad) {
+  chain_begin(scale_ptr);
   const float gs = a.grad_scale * (scale_ptr ? *scale_ptr : 1.0f);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     float4 w = master[i], mi = m[i], vi = v[i], g;
@@ -100,6 +102,7 @@ __global__ void sgd_kernel(GradT* __restrict__ grad, float* __restrict__ master,
                            float* __restrict__ mom, __nv_bfloat16* __restrict__ weight, long long n,
                            float lr, float momentum, float weight_decay, float grad_scale,
                            const float* __restrict__ scale_ptr, int nesterov, int zero_grad) {
+  chain_begin(scale_ptr);
   const float gs = grad_scale * (scale_ptr ? *scale_ptr : 1.0f);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -119,6 +122,7 @@ __global__ void sgd_kernel(GradT* __restrict__ grad, float* __restrict__ master,
 
 template <typename T>
 __global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __restrict__ out) {
+  chain_begin(x);
   __shared__ float sh[32];
   float s = 0.0f;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -140,6 +144,7 @@ __global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __rest
 // coef = min(1, max_norm / (sqrt(sumsq * norm_scale^2) + 1e-6)); also stores the norm.
 __global__ void clip_coef_kernel(const float* sumsq, float norm_scale, float max_norm, float* coef,
                                  float* norm_out) {
+  chain_begin();
   const float nrm = sqrtf(*sumsq) * norm_scale;
   if (norm_out) *norm_out = nrm;
   *coef = (max_norm > 0.0f) ? fminf(1.0f, max_norm / (nrm + 1e-6f)) : 1.0f;
@@ -165,6 +170,7 @@ __device__ __forceinline__ float porous_mix(float value, float saturation, float
 __global__ void hyper_accumulate_kernel(float* __restrict__ g, const float* __restrict__ v,
                                         long long n, float curvature, float tol, float saturation,
                                         float porosity, int conformal, float scale) {
+  chain_begin(v);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const float x = v[i] * scale;
@@ -180,6 +186,7 @@ __global__ void __launch_bounds__(256)
 hyper_apply_kernel(float* __restrict__ w, float* __restrict__ g, float* __restrict__ g_real,
                    int rows, int cols, float curvature, float lr, float lr_real, float tol,
                    float saturation, float porosity, int use_hyper) {
+  chain_begin();
   __shared__ float sh[8];
   const int row = blockIdx.x;
   float* wr = w + (size_t)row * cols;
@@ -227,6 +234,7 @@ hyper_apply_kernel(float* __restrict__ w, float* __restrict__ g, float* __restri
 __global__ void __launch_bounds__(256)
 poincare_project_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int cols,
                         float curvature) {
+  chain_begin(x);
   __shared__ float sh[8];
   const int row = blockIdx.x;
   const float* xr = x + (size_t)row * cols;
@@ -264,7 +272,7 @@ ST_API int st_adamw(void* grad, int grad_is_bf16, float* master, float* m, float
   const uintptr_t half = reinterpret_cast<uintptr_t>(weight) | (grad_is_bf16 ? reinterpret_cast<uintptr_t>(grad) : 0);
   if ((n & 3) == 0 && (wide & 15) == 0 && (half & 7) == 0) {
     auto run = [&](auto* g) {
-      adamw4_kernel<<<grid_for(n / 4, 256), 256, 0, s>>>(g, reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m),
+      st::chained(adamw4_kernel<std::remove_pointer_t<decltype(g)>>, grid_for(n / 4, 256), 256, 0, s)(g, reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m),
                                                          reinterpret_cast<float4*>(v), static_cast<uint2*>(weight), n / 4, a,
                                                          scale_ptr, zero_grad);
     };
@@ -274,11 +282,11 @@ ST_API int st_adamw(void* grad, int grad_is_bf16, float* master, float* m, float
     return ST_OK;
   }
   if (grad_is_bf16)
-    adamw_kernel<__nv_bfloat16><<<grid_for(n, 256), 256, 0, s>>>(
+    st::chained(adamw_kernel<__nv_bfloat16>, grid_for(n, 256), 256, 0, s)(
         static_cast<__nv_bfloat16*>(grad), master, m, v, static_cast<__nv_bfloat16*>(weight), n, a,
         scale_ptr, zero_grad);
   else
-    adamw_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(
+    st::chained(adamw_kernel<float>, grid_for(n, 256), 256, 0, s)(
         static_cast<float*>(grad), master, m, v, static_cast<__nv_bfloat16*>(weight), n, a, scale_ptr,
         zero_grad);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -291,11 +299,11 @@ ST_API int st_sgd(void* grad, int grad_is_bf16, float* master, float* mom, void*
   if (n <= 0) return ST_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   if (grad_is_bf16)
-    sgd_kernel<__nv_bfloat16><<<grid_for(n, 256), 256, 0, s>>>(
+    st::chained(sgd_kernel<__nv_bfloat16>, grid_for(n, 256), 256, 0, s)(
         static_cast<__nv_bfloat16*>(grad), master, mom, static_cast<__nv_bfloat16*>(weight), n, lr,
         momentum, weight_decay, grad_scale, scale_ptr, nesterov, zero_grad);
   else
-    sgd_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(
+    st::chained(sgd_kernel<float>, grid_for(n, 256), 256, 0, s)(
         static_cast<float*>(grad), master, mom, static_cast<__nv_bfloat16*>(weight), n, lr, momentum,
         weight_decay, grad_scale, scale_ptr, nesterov, zero_grad);
   ST_CUDA_CHECK(cudaGetLastError());
@@ -307,16 +315,16 @@ ST_API int st_sumsq(const void* x, int is_bf16, long long n, float* out, void* s
   if (n <= 0) return ST_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   if (is_bf16)
-    sumsq_kernel<__nv_bfloat16><<<grid_for(n, 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), n, out);
+    st::chained(sumsq_kernel<__nv_bfloat16>, grid_for(n, 256), 256, 0, s)(static_cast<const __nv_bfloat16*>(x), n, out);
   else
-    sumsq_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(static_cast<const float*>(x), n, out);
+    st::chained(sumsq_kernel<float>, grid_for(n, 256), 256, 0, s)(static_cast<const float*>(x), n, out);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
 
 ST_API int st_clip_coef(const float* sumsq, float norm_scale, float max_norm, float* coef,
                         float* norm_out, void* stream_v) {
-  clip_coef_kernel<<<1, 1, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(sumsq, norm_scale, max_norm,
+  st::chained(clip_coef_kernel, 1, 1, 0, reinterpret_cast<cudaStream_t>(stream_v))(sumsq, norm_scale, max_norm,
                                                                           coef, norm_out);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -326,7 +334,7 @@ ST_API int st_hyper_accumulate(float* g, const float* v, long long n, float curv
                                float saturation, float porosity, int conformal, float scale,
                                void* stream_v) {
   if (n <= 0) return ST_OK;
-  hyper_accumulate_kernel<<<grid_for(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(hyper_accumulate_kernel, grid_for(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       g, v, n, curvature, tol, saturation, porosity, conformal, scale);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -337,7 +345,7 @@ ST_API int st_hyper_apply(float* w, float* g, float* g_real, int rows, int cols,
                           void* stream_v) {
   if (rows <= 0 || cols <= 0) return ST_OK;
   if (g && !(curvature < 0.0f)) return st::fail(ST_ERR_INVALID, "hypergrad: curvature must be negative");
-  hyper_apply_kernel<<<rows, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  st::chained(hyper_apply_kernel, rows, 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
       w, g, g_real, rows, cols, curvature, lr, lr_real, tol, saturation, porosity, g != nullptr);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
@@ -346,7 +354,7 @@ ST_API int st_hyper_apply(float* w, float* g, float* g_real, int rows, int cols,
 ST_API int st_poincare_project(const float* x, float* y, int rows, int cols, float curvature,
                                void* stream_v) {
   if (!(curvature < 0.0f)) return st::fail(ST_ERR_INVALID, "project_to_poincare: curvature must be negative");
-  poincare_project_kernel<<<rows, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(x, y, rows, cols, curvature);
+  st::chained(poincare_project_kernel, rows, 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(x, y, rows, cols, curvature);
   ST_CUDA_CHECK(cudaGetLastError());
   return ST_OK;
 }
