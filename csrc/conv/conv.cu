@@ -426,7 +426,7 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
     return st::fail(ST_ERR_INVALID, "conv3x3: image width must divide 128 and the batch must fill whole pixel blocks");
   const int P = a->N * a->H * a->W;
   CUtensorMap tmA, tmB;
-  const TileChoice tile = choose_tile(P, a->OC, 9ll * a->C, 1, st::sm_count(), a->act == ACT_RELU_BWD ? EPI_OPERAND : EPI_PLAIN);
+  const TileChoice tile = choose_tile(P, a->OC, 9ll * a->C, 1, st::sm_count(), a->act == ACT_RELU_BWD ? EPI_OPERAND : EPI_PLAIN, true);
   HaloPlan halo;
   const bool use_halo = halo_plan(a, &halo) && halo.us <= tile.us;
   const int BN = use_halo ? halo.bn : tile.bn;
@@ -465,9 +465,10 @@ ST_API int st_conv3x3_fwd(const StConvArgs* a, void* stream_v) {
   OutMaps tmC;
   if (!plan_epilogue(p, tmC)) return ST_ERR_CUDA;
   if (pair) return launch_pair<false, false>(tmA, tmB, tmC, p, s);
-  const bool plain = plain_epilogue(p);
-  if (BN == 64) return plain ? launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s) : launch_gemm<64, 6, false, false>(tmA, tmB, tmC, p, s);
-  if (BN == 128) return plain ? launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s) : launch_gemm<128, 5, false, false>(tmA, tmB, tmC, p, s);
+  if (tile.parts > 1) return launch_parts<false, false>(BN, tile.parts, tmA, tmB, tmC, p, s);
+  if (BN == 64) return launch_gemm<64, 8, false, false>(tmA, tmB, tmC, p, s);
+  if (BN == 128)
+    return staged_epilogue(p) ? launch_gemm<128, 5, false, false>(tmA, tmB, tmC, p, s) : launch_gemm<128, 6, false, false>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, false, false>(tmA, tmB, tmC, p, s);
 }
 
@@ -539,7 +540,7 @@ ST_API int st_conv3x3_wgrad(const StConvWgradArgs* a, void* stream_v) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   if (form == 0) return launch_gemm<192, 4, true, true>(tmA, tmB, tmC, p, s);
   if (form == 2) return launch_pair<true, true>(tmA, tmB, tmC, p, s);
-  if (form == 3) return launch_gemm<64, 6, true, true>(tmA, tmB, tmC, p, s);
+  if (form == 3) return launch_gemm<64, 8, true, true>(tmA, tmB, tmC, p, s);
   return launch_gemm<256, 4, true, true>(tmA, tmB, tmC, p, s);
 }
 

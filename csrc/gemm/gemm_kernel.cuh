@@ -299,15 +299,17 @@ __device__ __forceinline__ void load32_bf16(uint4 (&x)[4], const __nv_bfloat16* 
   }
 }
 
+// KS > 1 (COMM_NONE only): a cluster of KS CTAs shares one tile, each with a KS-th of its K blocks; they add their fp32 sums through
+// shared memory in a fixed order, and each finishes a KS-th of the rows.  One tile per cluster.
 // CG = 2 (COMM_NONE only): a cluster of two CTAs works on one tile of 256 x BN.  Each CTA brings its 128 rows of A and its half
 // of B into its own shared memory, the even CTA's MMA warp issues for both, and each CTA's epilogue stores its own 128 rows.
 // A K block then costs an SM 32 KB of loads instead of 48 (BN = 256), and the ring holds six stages instead of four.
-template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM, int CG = 1>
+template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM, int CG = 1, int KS = 1>
 __global__ void __launch_bounds__(COMM == COMM_AG ? NUM_THREADS_AG : COMM == COMM_RS ? NUM_THREADS_RS : NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ OutMaps tmC, const __grid_constant__ CUtensorMap tmA_local,
                  const GemmParams p, const GemmComm cm) {
-  static_assert(CG == 1 || COMM == COMM_NONE, "CTA pairs run the plain product only");
+  static_assert((CG == 1 && KS == 1) || (COMM == COMM_NONE && (CG == 1 || KS == 1)), "CTA pairs and K parts run the plain product only");
   using L = SmemLayout<BN / CG, STAGES, COMM == COMM_NONE ? 0 : 1>;
   // Epilogue warps per 32 lanes of the accumulator.  Two of them take 64-column groups in turn, or, where a tile has only one
   // group, whole tiles in turn: one warp's loads, arithmetic and stores for a tile are longer than the main loop of a short K.
@@ -320,7 +322,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int lane = threadIdx.x & 31;
 
   const int cta = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
-  const int gemm_bid = CG == 2 ? blockIdx.x >> 1 : blockIdx.x;
+  const int kpart = KS > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int gemm_bid = blockIdx.x / (CG * KS);
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
   uint64_t* full_bar = bars;
@@ -335,7 +338,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int tiles_per_batch = tiles_m * tiles_n;
   const int total_tiles = tiles_per_batch * p.batch;
   const int k_blocks = (p.K + BK - 1) / BK;
-  const int grid_stride = gridDim.x / CG;
+  const int grid_stride = gridDim.x / (CG * KS);
+  const int k_first = KS > 1 ? k_blocks * kpart / KS : 0;
+  const int k_own = KS > 1 ? k_blocks * (kpart + 1) / KS - k_first : k_blocks;       // K blocks of this CTA
   constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32 : (2 * BN <= 64) ? 64 : (2 * BN <= 128) ? 128
                                  : (2 * BN <= 256) ? 256 : 512;
 
@@ -423,7 +428,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         if (leader) fence_proxy_async_global();
       }
-      const int k_count = A_MN && B_MN && p.conv.mode == 2 ? split_blocks(p, b) : k_blocks;
+      const int k_count = A_MN && B_MN && p.conv.mode == 2 ? split_blocks(p, b) : k_own;
       // one K block per ring stage: wait until its MMAs have read it, then hand the copies to the TMA unit
       auto k_loop = [&](uint32_t bytes, auto&& copies) {
         for (int kb = 0; kb < k_count; ++kb) {
@@ -460,10 +465,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int block = tm * CG + cta;
         const int img = (block / hblocks) * p.conv.Nb, h0 = (block % hblocks) * p.conv.Hb;
         int tap_w = -1, tap_h = -1, chunk = 0;
+        if constexpr (KS > 1) {
+          const int tap = k_first / p.conv.c_chunks;
+          chunk = k_first - tap * p.conv.c_chunks;
+          tap_w = tap % 3 - 1;
+          tap_h = tap / 3 - 1;
+        }
         ok = k_loop(stage_bytes, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (leader) {
             load4(sa, mapA, fb, chunk * 64, tap_w, h0 + tap_h, img);
-            load3(sb, &tmB, fb, kb * BK, n0, 0);
+            load3(sb, &tmB, fb, (k_first + kb) * BK, n0, 0);
           }
           if (++chunk == p.conv.c_chunks) {
             chunk = 0;
@@ -499,6 +510,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else if (whole) {
         ok = k_loop(L::STAGE_BYTES, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (!leader) return;
+          kb += k_first;
           if constexpr (!A_MN) {
             load3(sa, mapA, fb, kb * BK, m_coord, b);
           } else {
@@ -517,6 +529,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else {
         ok = k_loop(stage_bytes, [&](int kb, uint32_t fb, uint32_t sa, uint32_t sb) {
           if (!leader) return;
+          kb += k_first;
           if constexpr (!A_MN) {
             load3(sa, mapA, fb, kb * BK, m_coord, b);
           } else {
@@ -533,6 +546,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         });
       }
+    }
+    if constexpr (KS > 1) {       // the epilogue warps' two meetings
+      __syncwarp();
+      cluster_sync();
+      cluster_sync();
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer ---------------------------------------
@@ -557,7 +575,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait_warp(tempty0 + acc * 8, acc_phase ^ 1u, abort_flag)) break;
       tc_fence_after();
       const uint32_t tmem_d = tmem0 + acc * BN;
-      const int k_count = A_MN && B_MN && p.conv.mode == 2 ? split_blocks(p, t / tiles_per_batch) : k_blocks;
+      const int k_count = A_MN && B_MN && p.conv.mode == 2 ? split_blocks(p, t / tiles_per_batch) : k_own;
       for (int kb = 0; kb < k_count; ++kb) {
         if (!mbar_wait_warp(full0 + stage * 8, phase, abort_flag)) {
           ok = false;
@@ -585,6 +603,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
     }
+    if constexpr (KS > 1) {
+      __syncwarp();
+      cluster_sync();
+      cluster_sync();
+    }
   } else if (COMM == COMM_NONE) {
     // ------------------------------- epilogue warps, plain product ----------------------------------------
     // A warp takes 32 rows and 64 columns at a time.  Everything that is wide leaves and arrives through the copy engine and
@@ -609,8 +632,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
       m0 = tm * BM * CG + cta * BM + quad * 32;
       n0 = tn * BN;
+      if (KS > 1 && quad / (4 / KS) != kpart) return 0;
       return m0 < p.M ? min(BN / 64, (p.N - n0 + 63) >> 6) : 0;
     };
+    // K parts: CTA i of the cluster finishes rows [i, i + 1) * 128 / KS of the tile.  Once every CTA's products are complete the
+    // operand ring is idle and takes the others' partial sums of those rows, [source][column / 4][row] in 16-byte pieces.
+    constexpr int OWN_ROWS = BM / KS, PART_ELEMS = OWN_ROWS * BN;
+    static_assert(KS == 1 || (KS - 1) * PART_ELEMS * 4 <= STAGES * L::STAGE_BYTES, "the ring is too small for the partial sums");
+    if constexpr (KS > 1) {
+      const bool done = mbar_wait_warp(smem_u32(&tfull_bar[0]), 0, abort_flag);
+      tc_fence_after();
+      cluster_sync();
+      const int owner = quad / (4 / KS);
+      if (done && owner != kpart) {
+        int b, tm, tn;
+        map_tile<COMM>(gemm_bid, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
+        const int slot = kpart < owner ? kpart : kpart - 1;
+        const uint32_t dst = cluster_map(smem_u32(smem), owner) + (slot * PART_ELEMS + ((quad % (4 / KS)) * 32 + lane) * 4) * 4;
+        for (int c = set; c < BN / 32 && tn * BN + c * 32 < p.N; c += 2) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) cluster_store_16(dst + (c * 8 + q) * (OWN_ROWS * 16), r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
+        }
+      }
+      cluster_sync();
+    }
     // operand requests run up to CBUF - 1 blocks ahead of the arithmetic
     int req_t = SPLIT ? gemm_bid : gemm_bid + set * grid_stride, req_g = SPLIT ? set : 0, requested = 0;
     auto request = [&]() {
@@ -670,6 +718,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + g * 64 + half * 32, r);
           tmem_ld_wait();
           if (half == 1 && g + (SPLIT ? 2 : 1) >= groups) release();
+          if constexpr (KS > 1) {
+            const float4* part = reinterpret_cast<const float4*>(smem) + (g * 64 + half * 32) / 4 * OWN_ROWS + (quad % (4 / KS)) * 32 + lane;
+#pragma unroll
+            for (int i = 0; i < KS - 1; ++i)
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float4 u = part[i * (PART_ELEMS / 4) + q * OWN_ROWS];
+                r[q * 4] = __float_as_uint(__uint_as_float(r[q * 4]) + u.x);
+                r[q * 4 + 1] = __float_as_uint(__uint_as_float(r[q * 4 + 1]) + u.y);
+                r[q * 4 + 2] = __float_as_uint(__uint_as_float(r[q * 4 + 2]) + u.z);
+                r[q * 4 + 3] = __float_as_uint(__uint_as_float(r[q * 4 + 3]) + u.w);
+              }
+          }
           const bool full = col0 + 32 <= p.N;
           float v[32];
 #pragma unroll
@@ -1370,53 +1431,70 @@ inline bool plan_epilogue(GemmParams& p, OutMaps& maps) {
   }
   return true;
 }
-// Whether the epilogue only writes the bf16 output.  One staging block per warp is enough then, and the operand ring gets the
-// room: its depth covers the latency of weights that come from HBM.
-inline bool plain_epilogue(const GemmParams& p) {
-  return !p.out_fp32 && !p.accumulate && !p.residual && !p.aux_out && p.act != ACT_GELU_BWD && p.act != ACT_RELU_BWD;
+// Whether the epilogue's loads and stores deserve more staging blocks per warp at the price of a stage of the operand ring: an
+// operand does (16384 x 3072 x 768 plus residual 82 us and 93), a saved pre-activation where several rounds of a short K wait for
+// its stores (the same product with GELU 91 and 99).  Elsewhere the deeper ring is worth 2 to 4 %, most where large weights come
+// from HBM.
+inline bool staged_epilogue(const GemmParams& p) {
+  if (p.operand_tma) return true;
+  return p.aux_tma && p.K < 1024 && (long long)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256) >= 2 * st::sm_count();
 }
 
 // Tile width of a product.  A tile's main loop takes about c per K block (c2 from the 33rd on, where the start-up of the ring no
 // longer counts) and its epilogue e, which runs beside the next tile's main loop; what does not overlap is the first main loop and
 // the last epilogue:
 //   time = a + (rounds - 1) max(main, e) + main + e
-// in microseconds, fitted to 1314 products of 64 to 32768 rows, 64 to 50304 columns and K of 128 to 16384 with every epilogue.
-// Narrow tiles lose throughput but fill the chip where wide ones leave SMs without a tile: 777 x 2048 x 8192 takes 39 us with 112
-// tiles of 128 x 128 and 53 with 56 of 128 x 256; their short epilogues matter where K is short: 777 x 256 x 256 5.3 us in tiles of
-// 64 columns, 7.4 of 256, with GELU' 8.2 and 13.5.  128 x 256 and the pair come out within a few percent of one another over much
-// of the range, timed alone; inside a training step, under the power limit, the pair is the faster one (the products of the 85 M
-// byte model's step, K = 768 and 3072: 7.87 ms against 8.10), so it is taken up to 7 % above.
-// Against the fastest form of each, timed alone, the rule takes 0.3 to 0.7 % longer on average with bf16 outputs (1.0 with GELU')
-// and 1.0 to 1.4 % with fp32 ones, at most 16 %.
-enum TileEpilogue : int { EPI_PLAIN, EPI_OPERAND, EPI_GELU, EPI_GELU_BWD, EPI_FP32, EPI_FP32_ADD, EPI_FP32_ATOMIC };
+// in microseconds, fitted to 551 products of 64 to 16384 rows, 64 to 50304 columns and K of 64 to 16384 with every epilogue
+// (large weights not in L2).  Narrow tiles lose throughput but fill the chip where wide ones leave SMs without a tile: 777 x 2048 x
+// 8192 takes 38 us with 112 tiles of 128 x 128 and 50 with 56 of 128 x 256.
+// Where the tiles are so few that two or four CTAs can share each, their K loops are split (launch_parts): the same product takes
+// 31 us with two CTAs on each of 56 tiles; 128 x 2048 x 8192 20 and 39; 777 x 512 x 4608 13 in four parts and 20 in tiles of 64
+// columns; 128 x 768 x 3072 9.8 and 13.8.  The exchange costs about 4 us, so a K of 768 stays whole (777 x 768 x 768: 8.6 and
+// 7.2).  A cluster of four needs four SMs of one graphics processing cluster: 144 such CTAs took two rounds (128 x 4608 x 1536: 19 us
+// against 11), 128 run at once.  Parts are taken when they promise 4 % or more.
+// 128 x 256 and the pair come out within a few percent of one another over much of the range, timed alone; inside a training
+// step, under the power limit, the pair is the faster one (the products of the 85 M byte model's step, K = 768 and 3072: 7.87 ms
+// against 8.10), so it is taken up to 11 % above.
+// Against the fastest form of each, timed alone, the rule takes 0.2 to 0.5 % longer on average, at most 11 %.
+enum TileEpilogue : int { EPI_PLAIN, EPI_OPERAND, EPI_GELU, EPI_GELU_BWD, EPI_FP32, EPI_FP32_ADD };
 struct TileCost {
-  double a, c, c2, e[7];
+  double a, c, c2, e[6];
 };
-constexpr TileCost kTileCost[4] = {
-    //  a    c      c2     plain operand gelu gelu'  fp32  add   atomics
-    {3.37, 0.253, 0.224, {1.04, 1.85, 2.15, 3.75, 2.00, 6.27, 1.26}},       // 128 x 64
-    {2.43, 0.290, 0.248, {2.25, 3.25, 3.75, 5.86, 4.55, 11.56, 3.23}},      // 128 x 128
-    {1.49, 0.376, 0.302, {3.98, 5.77, 6.87, 10.39, 8.14, 20.0, 5.42}},      // 128 x 256
-    {2.18, 0.366, 0.301, {4.30, 6.27, 7.21, 11.06, 8.54, 20.0, 6.45}}};     // 256 x 256 on a pair
+constexpr TileCost kTileCost[8] = {
+    //  a    c      c2     plain operand gelu gelu'  fp32  added
+    {2.86, 0.249, 0.224, {1.32, 2.20, 2.39, 3.38, 1.55, 4.13}},      // 128 x 64
+    {1.67, 0.288, 0.248, {2.73, 3.79, 4.43, 5.53, 3.30, 5.98}},      // 128 x 128
+    {0.00, 0.398, 0.327, {4.62, 7.10, 7.93, 10.70, 5.35, 7.66}},     // 128 x 256
+    {1.00, 0.368, 0.282, {5.07, 6.67, 8.29, 10.52, 6.08, 9.23}},     // 256 x 256 on a pair
+    {5.43, 0.258, 0.263, {1.79, 2.68, 3.30, 4.63, 2.03, 2.03}},      // 128 x 128, two K parts (c, c2 per block of a part)
+    {5.26, 0.287, 1.179, {2.38, 3.27, 3.83, 5.23, 2.75, 2.75}},      // 128 x 128, four
+    {7.34, 0.298, 0.415, {1.60, 3.51, 4.16, 7.52, 2.25, 2.25}},      // 128 x 256, two
+    {7.13, 0.360, 0.402, {2.85, 4.79, 5.46, 8.90, 3.58, 3.58}}};     // 128 x 256, four
 struct TileChoice {
   int bn;
   bool pair;
+  int parts;      // CTAs that share the K blocks of a tile
   double us;      // modelled time
 };
-inline TileChoice choose_tile(long long M, long long N, long long K, long long batch, int ctas, TileEpilogue epi) {
+inline TileChoice choose_tile(long long M, long long N, long long K, long long batch, int ctas, TileEpilogue epi, bool may_split) {
   const double kb = (double)((K + BK - 1) / BK);
-  auto cost = [&](const TileCost& t, int bm, int bn, long long at_once) {
-    const long long tiles = ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch;
-    const double main = t.c * (kb < 32 ? kb : 32) + t.c2 * (kb > 32 ? kb - 32 : 0), e = t.e[epi];
-    return t.a + (double)((tiles + at_once - 1) / at_once - 1) * (main > e ? main : e) + main + e;
+  auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch; };
+  auto cost = [&](const TileCost& t, int bm, int bn, long long at_once, double blocks) {
+    const double main = t.c * (blocks < 32 ? blocks : 32) + t.c2 * (blocks > 32 ? blocks - 32 : 0), e = t.e[epi];
+    return t.a + (double)((tiles(bm, bn) + at_once - 1) / at_once - 1) * (main > e ? main : e) + main + e;
   };
-  TileChoice best{64, false, cost(kTileCost[0], BM, 64, ctas)};
-  auto take = [&](int bn, bool pair, double us) {
-    if (us <= best.us) best = {bn, pair, us};
+  TileChoice best{64, false, 1, cost(kTileCost[0], BM, 64, ctas, kb)};
+  auto take = [&](int bn, bool pair, int parts, double us) {
+    if (us <= best.us) best = {bn, pair, parts, us};
   };
-  if (N > 64) take(128, false, cost(kTileCost[1], BM, 128, ctas));
-  if (N > 128) take(256, false, cost(kTileCost[2], BM, 256, ctas));
-  if (N > 128 && M > BM && ctas >= 2) take(256, true, 0.93 * cost(kTileCost[3], 2 * BM, 256, ctas / 2));
+  if (N > 64) take(128, false, 1, cost(kTileCost[1], BM, 128, ctas, kb));
+  if (N > 128) take(256, false, 1, cost(kTileCost[2], BM, 256, ctas, kb));
+  if (N > 128 && M > BM && ctas >= 2) take(256, true, 1, 0.9 * cost(kTileCost[3], 2 * BM, 256, ctas / 2, kb));
+  if (may_split && N > 64)
+    for (int f = 0; f < 4; ++f) {
+      const int bn = f < 2 ? 128 : 256, parts = f & 1 ? 4 : 2, at_once = parts == 2 ? ctas / 2 : ctas * 7 / 32;
+      if (N > bn / 2 && kb >= 4 * parts && tiles(BM, bn) <= at_once) take(bn, false, parts, 1.04 * cost(kTileCost[4 + f], BM, bn, at_once, kb / parts));
+    }
   return best;
 }
 
@@ -1441,8 +1519,30 @@ int launch_pair_ring(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMa
 
 template <bool A_MN, bool B_MN>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
-  if (plain_epilogue(p)) return launch_pair_ring<A_MN, B_MN, 6>(tmA, tmB, tmC, p, stream);
-  return launch_pair_ring<A_MN, B_MN, 5>(tmA, tmB, tmC, p, stream);
+  if (!A_MN && staged_epilogue(p)) return launch_pair_ring<false, B_MN, 5>(tmA, tmB, tmC, p, stream);
+  return launch_pair_ring<A_MN, B_MN, 6>(tmA, tmB, tmC, p, stream);
+}
+
+// Launch of the K-part form: a cluster of KS CTAs per tile.
+template <int BN, int STAGES, int KS, bool A_MN, bool B_MN>
+int launch_parts_of(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
+  using L = SmemLayout<BN, STAGES>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, COMM_NONE, 1, KS>;
+  static bool configured[st::kMaxDevices] = {false};   // the attribute is per device
+  const int dev = st::current_device();
+  if (!configured[dev]) {
+    ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+    configured[dev] = true;
+  }
+  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
+  GemmComm none{};
+  ST_CUDA_CHECK(st::chained(kern, KS * tiles, NUM_THREADS, L::TOTAL, stream, KS)(tmA, tmB, tmC, tmA, p, none));
+  return ST_OK;
+}
+template <bool A_MN, bool B_MN>
+int launch_parts(int bn, int parts, const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
+  if (bn == 128) return parts == 2 ? launch_parts_of<128, 5, 2, A_MN, B_MN>(tmA, tmB, tmC, p, stream) : launch_parts_of<128, 5, 4, A_MN, B_MN>(tmA, tmB, tmC, p, stream);
+  return parts == 2 ? launch_parts_of<256, 4, 2, A_MN, B_MN>(tmA, tmB, tmC, p, stream) : launch_parts_of<256, 4, 4, A_MN, B_MN>(tmA, tmB, tmC, p, stream);
 }
 
 }  // namespace gemm

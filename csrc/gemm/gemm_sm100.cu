@@ -87,13 +87,13 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
 
   const bool limited = a->max_ctas > 0 && a->max_ctas < st::sm_count();
-  const TileEpilogue epi = a->accumulate == 2 ? EPI_FP32_ATOMIC
-                           : a->out_fp32      ? (a->accumulate ? EPI_FP32_ADD : EPI_FP32)
+  const TileEpilogue epi = a->out_fp32        ? (a->accumulate ? EPI_FP32_ADD : EPI_FP32)
                            : a->act == ACT_GELU_BWD ? EPI_GELU_BWD
                            : a->act == ACT_GELU     ? EPI_GELU
                            : a->residual || a->aux_out || a->aux_in || a->accumulate ? EPI_OPERAND
                                                                                      : EPI_PLAIN;
-  TileChoice tile = choose_tile(a->M, a->N, a->K, a->batch, limited ? a->max_ctas : st::sm_count(), epi);
+  TileChoice tile = choose_tile(a->M, a->N, a->K, a->batch, limited ? a->max_ctas : st::sm_count(), epi,
+                                a->max_ctas <= 0 && !a->a_mn_major);
   if (a->max_ctas > 0) tile.pair = false;      // a limited grid runs beside another kernel: single CTAs find room anywhere
   const int BN = tile.bn;
   const bool pair = tile.pair;
@@ -153,12 +153,12 @@ ST_API int st_gemm_bf16(const StGemmArgs* a, void* stream_v) {
     if (!a->b_mn_major) return launch_pair<true, false>(tmA, tmB, tmC, p, stream);
     return launch_pair<true, true>(tmA, tmB, tmC, p, stream);
   }
-  const bool plain = plain_epilogue(p), a_mn = a->a_mn_major != 0, b_mn = a->b_mn_major != 0;
-  if (BN == 64)
-    return plain ? dispatch_major<64, 8>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas)
-                 : dispatch_major<64, 6>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
+  if (tile.parts > 1) return a->b_mn_major ? launch_parts<false, true>(BN, tile.parts, tmA, tmB, tmC, p, stream)
+                                           : launch_parts<false, false>(BN, tile.parts, tmA, tmB, tmC, p, stream);
+  const bool a_mn = a->a_mn_major != 0, b_mn = a->b_mn_major != 0;
+  if (BN == 64) return dispatch_major<64, 8>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
   if (BN == 128)
-    return plain ? dispatch_major<128, 6>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas)
-                 : dispatch_major<128, 5>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
+    return staged_epilogue(p) ? dispatch_major<128, 5>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas)
+                              : dispatch_major<128, 6>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
   return dispatch_major<256, 4>(a_mn, b_mn, tmA, tmB, tmC, p, stream, a->max_ctas);
 }
