@@ -444,7 +444,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // in the log2 domain and minus infinity wherever a key is masked: 16-byte loads that all lanes share, one packed multiply-
 // add per two logits and no comparisons, except in the tile that holds the length, where a padded key may have given a logit
 // that is not finite and is replaced by comparison.  The single-tile kernel loaded and compared per element: 244 us for 96 contexts of
-// up to 1000 keys, D = 64, where this form takes 95.  A bias per (query, key) stays with the single-tile kernel.
+// up to 1000 keys, D = 64, where this form takes 65 (93 with the
+// bias read from global memory where it is used and the outputs stored by their lanes).  A bias per (query, key) stays with the single-tile kernel.
 // ------------------------------------------------------------------------------------------------------------------
 // Phase clocks of CTA 0 (SM cycles summed over the launch), written when tracing is switched on:
 //   softmax warp 0:  0 steps, 1 wait for S, 2 S load, 3 maximum / rescale, 4 first half of P, 5 second half of P,
@@ -464,8 +465,13 @@ struct PairSmem {
   static constexpr int TILE = BLK * D * 2;
   static constexpr int Q_OFF = 0;                          // two query tiles
   static constexpr int KV_OFF = 2 * TILE;
-  static constexpr int BAR_OFF = KV_OFF + PAIR_STAGES * TILE;
+  // per softmax warp: blocks of 32 rows and 64 bytes of the output on their way out, and the key bias of two tiles
+  static constexpr int STG_SLOTS = D == 64 ? 2 : 1;
+  static constexpr int STG_OFF = KV_OFF + PAIR_STAGES * TILE;
+  static constexpr int BIAS_OFF = STG_OFF + 8 * STG_SLOTS * 2048;
+  static constexpr int BAR_OFF = BIAS_OFF + 8 * 2 * BLK * 4;
   static constexpr int TOTAL = BAR_OFF + 256;
+  static_assert(TOTAL <= 232448, "shared memory");
 };
 
 // out[b, (h,) key] = key_bias * log2(e) for the keys below the valid length, minus infinity from there to the padded end
@@ -484,11 +490,15 @@ __global__ void attn_key_bias_kernel(const float* __restrict__ kb, long long kb_
   }
 }
 
-// FP32: the launch may ask for an fp32 copy of the output; its stores cost the plain form 2 %.
+// FP32: the launch may ask for an fp32 copy of the output.
+// Outputs leave by TMA: a lane that stores its own row touches 32 lines with each instruction.  The key bias of a tile passes
+// through shared memory, fetched by the warp one tile ahead: read from global memory where it is used, its four lines cost
+// about as much as the exponentials.
 template <int D, bool KEYB, bool FP32>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, const AttnFwdParams p) {
+                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
+                     const __grid_constant__ CUtensorMap tmO32, const AttnFwdParams p) {
   using L = PairSmem<D>;
   constexpr int KB = D / 64;
   constexpr uint32_t S_COL = 0;       // S_t at S_COL + 128 t; P_t (bf16 pairs) over its first 64 columns
@@ -736,6 +746,24 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t s_addr = tmem_base + lane_off + S_COL + t * BLK;
     const uint32_t o_addr = tmem_base + lane_off + O_COL + t * D;
     const float sc = p.scale_log2;
+    uint8_t* const stg = smem + L::STG_OFF + warp * (L::STG_SLOTS * 2048);
+    int staged = 0;
+    // 32 rows and 64 bytes (16 fp32 or 32 bf16 columns from `col`) of the output through this warp's staging slots
+    auto stage = [&](const CUtensorMap* map, const uint4 (&u)[4], int col, int row0, int h, int b) {
+      uint8_t* const slot = stg + (staged % L::STG_SLOTS) * 2048;
+      ++staged;
+      if (lane == 0) tma_store_wait_read<L::STG_SLOTS - 1>();
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(slot + sw64_offset(lane, q)) = u[q];
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_4d(map, smem_u32(slot), col, h, row0, b);
+        tma_store_commit();
+      }
+    };
+    float4* const bias_slots = reinterpret_cast<float4*>(smem + L::BIAS_OFF) + warp * (2 * BLK / 4);
     uint32_t steps = 0;   // softmax steps done (phase of s_full)
     int items = 0;        // items this tile took part in (phase of o_full)
     bool ok = true;
@@ -751,14 +779,15 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int q_tile = 2 * qp + t;
       const int row_g = q_tile * BLK + r;
       if (n_kv <= 0) {
-        if (KEYB && row_g < p.Sq) {      // a query tile beyond the valid length, or a context without keys
-          __nv_bfloat16* op = p.O + (long long)b * p.o_sb + (long long)row_g * p.o_ss + (long long)h * p.o_sh;
-          for (int c = 0; c < D / 8; ++c) reinterpret_cast<uint4*>(op)[c] = make_uint4(0, 0, 0, 0);
-          if (FP32 && p.O32) {
-            float4* o32 = reinterpret_cast<float4*>(p.O32 + (((long long)b * p.Sq + row_g) * p.H + h) * D);
-            for (int c = 0; c < D / 4; ++c) o32[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          }
-          p.lse[((long long)b * p.H + h) * p.Sq + row_g] = -INFINITY;
+        const int row0 = q_tile * BLK + quad * 32;
+        if (KEYB && row0 < p.Sq) {       // a query tile beyond the valid length, or a context without keys
+          uint4 none[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) none[q] = make_uint4(0, 0, 0, 0);
+          for (int c = 0; c < D; c += 32) stage(&tmO, none, c, row0, h, b);
+          if (FP32 && p.O32)
+            for (int c = 0; c < D; c += 16) stage(&tmO32, none, c, row0, h, b);
+          if (row_g < p.Sq) p.lse[((long long)b * p.H + h) * p.Sq + row_g] = -INFINITY;
         }
         continue;
       }
@@ -767,7 +796,15 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const bool row_live = !KEYB || !p.lengths || row_g < kv_len;
       const float4* bias_row = KEYB ? reinterpret_cast<const float4*>(p.kb_pad + b * p.kp_sb + h * p.kp_sh) : nullptr;
       float m = -INFINITY, l = 0.0f;
+      float4 bias_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);      // this lane's four keys of the next tile
+      if (KEYB) bias_next = __ldg(bias_row + lane);
       for (int j = 0; j < n_kv; ++j) {
+        const float4* const bias = bias_slots + (j & 1) * (BLK / 4);
+        if (KEYB) {
+          bias_slots[(j & 1) * (BLK / 4) + lane] = bias_next;
+          if (j + 1 < n_kv) bias_next = __ldg(bias_row + (j + 1) * (BLK / 4) + lane);
+          __syncwarp();
+        }
         if (tr) c0 = static_cast<uint32_t>(clock());
         if (!mbar_wait_warp(smem_u32(&s_full[t]), steps & 1u, abort_flag)) { ok = false; break; }
         ++steps;
@@ -790,9 +827,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const float2 sc2 = make_float2(sc, sc);
 #pragma unroll
           for (int c = 0; c < BLK; c += 4) {
-            const float4 bias = __ldg(bias_row + (col0 + c) / 4);
-            const float2 x = fma2(make_float2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, make_float2(bias.x, bias.y));
-            const float2 y = fma2(make_float2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, make_float2(bias.z, bias.w));
+            const float4 v = bias[c / 4];
+            const float2 x = fma2(make_float2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, make_float2(v.x, v.y));
+            const float2 y = fma2(make_float2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, make_float2(v.z, v.w));
             sr[c] = __float_as_uint(x.x); sr[c + 1] = __float_as_uint(x.y);
             sr[c + 2] = __float_as_uint(y.x); sr[c + 3] = __float_as_uint(y.y);
           }
@@ -883,33 +920,35 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       ++items;
       tc_fence_after();
       const float inv = l > 0.0f && row_live ? 1.0f / l : 0.0f;
-      __nv_bfloat16* op = p.O + (long long)b * p.o_sb + (long long)row_g * p.o_ss + (long long)h * p.o_sh;
-      float4* o32 = FP32 && p.O32 ? reinterpret_cast<float4*>(p.O32 + (((long long)b * p.Sq + row_g) * p.H + h) * D) : nullptr;
+      const int row0 = q_tile * BLK + quad * 32;
 #pragma unroll
       for (int ch = 0; ch < D / 32; ++ch) {
         uint32_t v[32];
         tmem_ld_32x32(o_addr + ch * 32, v);
         tmem_ld_wait();
-        if (KEYB && !row_live) {      // zeros by value: what a padded query summed up need not be finite
 #pragma unroll
-          for (int c = 0; c < 32; ++c) v[c] = 0;
-        }
-        if (row_g < p.Sq) {
-          if (o32) {
+        for (int c = 0; c < 32; ++c)      // zeros by value: what a padded query summed up need not be finite
+          v[c] = KEYB && !row_live ? 0 : __float_as_uint(__uint_as_float(v[c]) * inv);
+        if (row0 < p.Sq) {
+          uint4 u[4];
+          if (FP32 && p.O32) {
 #pragma unroll
-            for (int c4 = 0; c4 < 8; ++c4)
-              o32[ch * 8 + c4] = make_float4(__uint_as_float(v[c4 * 4]) * inv, __uint_as_float(v[c4 * 4 + 1]) * inv,
-                                             __uint_as_float(v[c4 * 4 + 2]) * inv, __uint_as_float(v[c4 * 4 + 3]) * inv);
+            for (int piece = 0; piece < 2; ++piece) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const int c = piece * 16 + q * 4;
+                u[q] = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+              }
+              stage(&tmO32, u, ch * 32 + piece * 16, row0, h, b);
+            }
           }
 #pragma unroll
-          for (int c8 = 0; c8 < 4; ++c8) {
-            uint4 u;
-            u.x = pack_bf16x2(__uint_as_float(v[c8 * 8 + 0]) * inv, __uint_as_float(v[c8 * 8 + 1]) * inv);
-            u.y = pack_bf16x2(__uint_as_float(v[c8 * 8 + 2]) * inv, __uint_as_float(v[c8 * 8 + 3]) * inv);
-            u.z = pack_bf16x2(__uint_as_float(v[c8 * 8 + 4]) * inv, __uint_as_float(v[c8 * 8 + 5]) * inv);
-            u.w = pack_bf16x2(__uint_as_float(v[c8 * 8 + 6]) * inv, __uint_as_float(v[c8 * 8 + 7]) * inv);
-            reinterpret_cast<uint4*>(op)[ch * 4 + c8] = u;
+          for (int q = 0; q < 4; ++q) {
+            const int c = q * 8;
+            u[q] = make_uint4(pack_bf16x2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), pack_bf16x2(__uint_as_float(v[c + 2]), __uint_as_float(v[c + 3])),
+                              pack_bf16x2(__uint_as_float(v[c + 4]), __uint_as_float(v[c + 5])), pack_bf16x2(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
           }
+          stage(&tmO, u, ch * 32, row0, h, b);
         }
       }
       if (row_g < p.Sq)
@@ -922,6 +961,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     if (tr)
       for (int i = 0; i < 8; ++i) p.trace[i] += tacc[i];
+    if (lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -941,6 +981,16 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 namespace st {
 // 4-D tensor map over a [B, S, H, D] bf16 view with arbitrary B/S/H strides (D contiguous):
 // dims {D, H, S, B}, box {64, 1, rows, 1}.
+// Boxes of 32 rows and 64 bytes of an output or a gradient, fp32 or bf16; strides in elements
+bool encode_out_tmap(CUtensorMap* out, const void* base, bool f32, int B, int S, int H, int D, long long sb, long long ss, long long sh) {
+  const uint64_t es = f32 ? 4 : 2;
+  const uint64_t dims[4] = {(uint64_t)D, (uint64_t)H, (uint64_t)S, (uint64_t)B};
+  const uint64_t strides[3] = {(uint64_t)sh * es, (uint64_t)ss * es, (uint64_t)sb * es};
+  const uint32_t box[4] = {(uint32_t)(64 / es), 1, 32, 1};
+  return encode_tmap(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box,
+                     CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
 bool encode_bshd_tmap(CUtensorMap* out, const void* base, int B, int S, int H, int D,
                       long long sb, long long ss, long long sh, int box_rows) {
   uint64_t dims[4] = {(uint64_t)D, (uint64_t)H, (uint64_t)S, (uint64_t)B};
@@ -1058,13 +1108,18 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
     if (g_pair_trace_on) ST_CUDA_CHECK(cudaGetSymbolAddress(reinterpret_cast<void**>(&p.trace), g_pair_trace));
     p.n_items = ((p.n_q + 1) / 2) * a->H * a->B;
     const dim3 pgrid(std::min(p.n_items, st::sm_count()));
+    CUtensorMap to, to32;
+    if (!st::encode_out_tmap(&to, a->O, false, a->B, a->Sq, a->H, a->D, a->o_sb, a->o_ss, a->o_sh)) return ST_ERR_CUDA;
+    to32 = to;
+    if (out32 && !st::encode_out_tmap(&to32, out32, true, a->B, a->Sq, a->H, a->D, (long long)a->Sq * a->H * a->D, (long long)a->H * a->D, a->D))
+      return ST_ERR_CUDA;
     const int dev = st::current_device();
     auto plaunch = [&](auto kern, int smem_bytes, bool* cfg) -> int {
       if (!cfg[dev]) {
         ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         cfg[dev] = true;
       }
-      st::chained(kern, pgrid, PAIR_THREADS, smem_bytes, s)(tq, tk, tv, p);
+      st::chained(kern, pgrid, PAIR_THREADS, smem_bytes, s)(tq, tk, tv, to, to32, p);
       return ST_OK;
     };
     static bool pcfg[6][st::kMaxDevices] = {{false}};

@@ -200,6 +200,11 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
 // Untiled bulk copies (both addresses 16-byte aligned, size a multiple of 16 bytes).
 __device__ __forceinline__ void bulk_load_g2s(uint32_t dst_smem, const void* src_gmem, uint32_t bytes,
                                               uint32_t bar) {
@@ -471,6 +476,11 @@ __device__ __forceinline__ void tmem_ld_wait() {
 // tile whose rows are 128 bytes and whose base is 1024-byte aligned.
 __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk16) {
   return row * 128u + (((chunk16 ^ (row & 7u)) & 7u) << 4);
+}
+
+// The same for rows of 64 bytes with the 64-byte swizzle, chunk 0..3 and a 512-byte aligned base.
+__device__ __forceinline__ uint32_t sw64_offset(uint32_t row, uint32_t chunk16) {
+  return row * 64u + (((chunk16 ^ (row >> 1)) & 3u) << 4);
 }
 
 // ---------------------------------------------------------------------------------------
