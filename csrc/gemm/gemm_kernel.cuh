@@ -100,12 +100,12 @@ struct GemmParams {
   int accumulate;
   int batch;
   long long batch_stride_c;
-  int use_tma_store;   // StoreMode: the output goes through shared memory and the copy engine
+  int use_tma_store;   // OutputMode: the output goes through shared memory and the copy engine
   int operand_tma;     // the epilogue's operand (aux_in of a derivative, else the residual) arrives by TMA, OutMaps.m[1]
   int aux_tma;         // aux_out leaves by TMA, OutMaps.m[2]
   unsigned* err;
 };
-enum StoreMode : int { STORE_DIRECT = 0, STORE_BF16 = 1, STORE_FP32 = 2, STORE_FP32_ADD = 3 };
+enum OutputMode : int { STORE_DIRECT = 0, STORE_BF16 = 1, STORE_FP32 = 2, STORE_FP32_ADD = 3 };
 
 // Tensor maps of the output, one per owner rank for GEMM → reduce-scatter.  Plain product: [0] the output, [1] the epilogue's
 // operand, [2] the saved pre-activation.
