@@ -207,7 +207,8 @@ class GPTModel(nn.Module):
         o, lse = attn_ops.attention_forward(qkv5[:, :, 0], qkv5[:, :, 1], qkv5[:, :, 2], True)
         attn_out = tp.gemm_rs(o.view(B * S, hl * D), P[f"h{l}.proj.weight"])
         y2, h2, m2, r2 = self._norm_fwd(attn_out, f"h{l}.norm2", residual=h1, gather_key=(l, "y2"))
-        u = torch.empty((y2.shape[0] * tp.world, self.ffn_local), dtype=y2.dtype, device=y2.device)
+        # the pre-activation is only read by the backward pass
+        u = torch.empty((y2.shape[0] * tp.world, self.ffn_local), dtype=y2.dtype, device=y2.device) if keep else None
         a, y2_full = tp.ag_gemm(y2, P[f"h{l}.fc1.weight"], key=(l, "y2"), act="gelu", aux_out=u)
         mlp_out = tp.gemm_rs(a, P[f"h{l}.fc2.weight"])
         if keep:

@@ -9,6 +9,8 @@ reference layout).  CPU tensors use ``torch.nn.functional.conv2d`` on the same d
 from __future__ import annotations
 
 import ctypes
+import functools
+import struct
 from typing import Optional
 
 import torch
@@ -21,9 +23,8 @@ from .gemm import gemm
 launch_count = 0
 
 
-class _ConvArgs(ctypes.Structure):
-    _fields_ = [("x", ctypes.c_void_p), ("w", ctypes.c_void_p), ("bias", ctypes.c_void_p), ("y", ctypes.c_void_p),
-                ("aux_in", ctypes.c_void_p)] + [(n, ctypes.c_int) for n in ("N", "H", "W", "C", "OC", "act")]
+# StConvArgs of csrc/conv/conv.cu: x, w, bias, y, aux_in; N, H, W, C, OC, act
+_pack_conv = struct.Struct("@5P6i").pack
 
 
 class _WgradArgs(ctypes.Structure):
@@ -56,6 +57,7 @@ def dgrad_weights(w_tap: torch.Tensor, ic: int) -> torch.Tensor:
     return w_tap.reshape(oc, 3, 3, ic).flip(1, 2).permute(3, 1, 2, 0).reshape(ic, 9 * oc).contiguous()
 
 
+@functools.lru_cache(maxsize=1024)
 def implicit_ok(N: int, H: int, W: int, C: int, OC: int, pixels: int = 128) -> bool:
     """Whether the implicit-GEMM kernels take this geometry: channels in 64-blocks, and a pixel block of
     ``pixels`` output positions (128 forward / data gradient, 64 weight gradient) must be W columns x whole rows
@@ -79,9 +81,8 @@ def im2col(x: torch.Tensor, OC: int) -> Optional[torch.Tensor]:
         return None
     kpad = (9 * C + 31) // 32 * 32
     col = torch.empty((N * H * W, kpad), dtype=torch.bfloat16, device=x.device)
-    native.check(native.lib().st_im2col3x3_small(native.ptr(x), native.ptr(col), ctypes.c_int(N), ctypes.c_int(H), ctypes.c_int(W),
-                                                 ctypes.c_int(C), ctypes.c_int(kpad), native.stream_ptr(x.device)),
-                 "st_im2col3x3_small")
+    native.check(native.entry("st_im2col3x3_small", "ppiiiiip")(x.data_ptr(), col.data_ptr(), N, H, W, C, kpad,
+                                                                native.raw_stream(x.get_device())), "st_im2col3x3_small")
     launch_count += 1
     return col
 
@@ -110,7 +111,7 @@ def conv3x3(x: torch.Tensor, w_tap: torch.Tensor, bias: Optional[torch.Tensor] =
     act = 4 if relu_mask_of is not None else (1 if relu else 0)
     if not native.use_native(x):
         return _conv_ref(x, w_tap, bias, act, relu_mask_of)
-    native.require_cuda("conv3x3", x, w_tap, bias, relu_mask_of)
+    device = native.require_cuda("conv3x3", x, w_tap, bias, relu_mask_of)
     assert x.dtype == torch.bfloat16 and x.is_contiguous() and w_tap.dtype == torch.bfloat16 and w_tap.is_contiguous()
     assert w_tap.shape[1] == 9 * C, "weights must be [OC, 9*C] (tap-major)"
     assert relu_mask_of is None or relu_mask_of.shape == (N, H, W, OC)
@@ -127,13 +128,9 @@ def conv3x3(x: torch.Tensor, w_tap: torch.Tensor, bias: Optional[torch.Tensor] =
         else:
             y = gemm(col, wp, bias=bias, act="relu" if relu else None)
         return y.view(N, H, W, OC)
-    y = torch.empty((N, H, W, OC), dtype=torch.bfloat16, device=x.device)
-    a = _ConvArgs()
-    a.x, a.w, a.y = x.data_ptr(), w_tap.data_ptr(), y.data_ptr()
-    a.bias = None if bias is None else bias.data_ptr()
-    a.aux_in = None if relu_mask_of is None else relu_mask_of.data_ptr()
-    a.N, a.H, a.W, a.C, a.OC, a.act = N, H, W, C, OC, act
-    native.check(native.lib().st_conv3x3_fwd(ctypes.byref(a), native.stream_ptr(x.device)), "st_conv3x3_fwd")
+    y = x.new_empty((N, H, W, OC))
+    args = _pack_conv(x.data_ptr(), w_tap.data_ptr(), native.address(bias), y.data_ptr(), native.address(relu_mask_of), N, H, W, C, OC, act)
+    native.check(native.lib().st_conv3x3_fwd(args, ctypes.c_void_p(native.raw_stream(device))), "st_conv3x3_fwd")
     launch_count += 1
     return y
 
@@ -175,11 +172,10 @@ def maxpool2(x: torch.Tensor):
         xv = x.reshape(N, H // 2, 2, W // 2, 2, C).permute(0, 1, 3, 5, 2, 4).reshape(N, H // 2, W // 2, C, 4)
         y, idx = xv.float().max(-1)
         return y.to(x.dtype), idx.to(torch.uint8)
-    y = torch.empty((N, H // 2, W // 2, C), dtype=x.dtype, device=x.device)
-    idx = torch.empty((N, H // 2, W // 2, C), dtype=torch.uint8, device=x.device)
-    st = native.lib().st_maxpool2_fwd(native.ptr(x), native.ptr(y), native.ptr(idx), ctypes.c_int(N), ctypes.c_int(H),
-                                      ctypes.c_int(W), ctypes.c_int(C), native.stream_ptr(x.device))
-    native.check(st, "st_maxpool2_fwd")
+    y = x.new_empty((N, H // 2, W // 2, C))
+    idx = x.new_empty((N, H // 2, W // 2, C), dtype=torch.uint8)
+    native.check(native.entry("st_maxpool2_fwd", "pppiiiip")(x.data_ptr(), y.data_ptr(), idx.data_ptr(), N, H, W, C,
+                                                             native.raw_stream(x.get_device())), "st_maxpool2_fwd")
     launch_count += 1
     return y, idx
 
@@ -231,10 +227,9 @@ def global_avgpool(x: torch.Tensor) -> torch.Tensor:
     N, H, W, C = x.shape
     if not native.use_native(x):
         return x.float().mean((1, 2)).to(x.dtype)
-    y = torch.empty((N, C), dtype=x.dtype, device=x.device)
-    st = native.lib().st_avgpool_fwd(native.ptr(x), native.ptr(y), ctypes.c_int(N), ctypes.c_int(H * W), ctypes.c_int(C),
-                                     native.stream_ptr(x.device))
-    native.check(st, "st_avgpool_fwd")
+    y = x.new_empty((N, C))
+    native.check(native.entry("st_avgpool_fwd", "ppiiip")(x.data_ptr(), y.data_ptr(), N, H * W, C, native.raw_stream(x.get_device())),
+                 "st_avgpool_fwd")
     launch_count += 1
     return y
 

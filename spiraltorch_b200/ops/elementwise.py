@@ -21,7 +21,7 @@ _rope_cache: dict = {}
 
 def rope_tables(seq_len: int, head_dim: int, base: float, device) -> tuple[torch.Tensor, torch.Tensor]:
     """cos/sin tables ``[seq_len, head_dim/2]`` fp32 (cached per device)."""
-    key = (seq_len, head_dim, float(base), str(device))
+    key = (seq_len, head_dim, float(base), device)
     hit = _rope_cache.get(key)
     if hit is None:
         inv = 1.0 / (base ** (torch.arange(0, head_dim, 2, dtype=torch.float64) / head_dim))
@@ -52,11 +52,10 @@ def rope_(x: torch.Tensor, heads: int, head_dim: int, seq_len: int, base: float 
         view = x[:, : heads * head_dim].reshape(T, heads, head_dim)
         view.copy_(rope_reference(view, cos, sin, seq_len, backward))
         return x
-    assert x.dtype == torch.bfloat16 and x.stride(-1) == 1
-    st = native.lib().st_rope(native.ptr(x), native.ptr(cos), native.ptr(sin), ctypes.c_longlong(T),
-                              ctypes.c_int(heads), ctypes.c_int(head_dim), ctypes.c_longlong(x.stride(0)),
-                              ctypes.c_int(seq_len), ctypes.c_int(0), ctypes.c_int(int(backward)),
-                              native.stream_ptr(x.device))
+    ld, unit = x.stride()
+    assert x.dtype == torch.bfloat16 and unit == 1
+    st = native.entry("st_rope", "pppqiiqiiip")(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, heads, head_dim, ld, seq_len, 0,
+                                                backward, native.raw_stream(x.get_device()))
     native.check(st, "st_rope")
     launch_count += 1
     return x
@@ -120,8 +119,8 @@ def colsum(x2: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: boo
     if out is None and 0 < rows <= 1024 and rows * cols <= 1 << 25 and cols % 8 == 0 and cols > 0 and native.use_native(x2) and x2.dtype == torch.bfloat16 \
             and x2.stride(-1) == 1 and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0:
         out = torch.empty(cols, dtype=torch.float32, device=x2.device)
-        native.check(native.lib().st_colsum_short(native.ptr(x2), native.ptr(out), ctypes.c_longlong(rows), ctypes.c_int(cols),
-                                                  ctypes.c_longlong(x2.stride(0)), native.stream_ptr(x2.device)), "st_colsum_short")
+        native.check(native.entry("st_colsum_short", "ppqiqp")(x2.data_ptr(), out.data_ptr(), rows, cols, x2.stride(0),
+                                                               native.raw_stream(x2.get_device())), "st_colsum_short")
         launch_count += 1
         return out
     if out is None:

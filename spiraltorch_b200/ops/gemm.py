@@ -194,22 +194,22 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     """
     global launch_count
     act_id = _ACT_NAMES[act] if not isinstance(act, int) else act
+    on_cuda = native.use_native(a)
     if out is not None:
         out_dtype = out.dtype
-    if out_dtype is None:
-        out_dtype = torch.bfloat16 if a.is_cuda else a.dtype
-    if not native.use_native(a):
+    elif out_dtype is None:
+        out_dtype = torch.bfloat16 if on_cuda else a.dtype
+    if not on_cuda:
         return _reference(a, b, a_mn, b_mn, out, out_dtype, bias, act_id, residual, aux_out, aux_in,
                           alpha, accumulate)
 
-    native.require_cuda("gemm", a, b, out, bias, residual, aux_out, aux_in)
-    batched = a.dim() == 3
+    device = native.require_cuda("gemm", a, b, out, bias, residual, aux_out, aux_in)
+    shape_a, shape_b = a.shape, b.shape
+    batched = len(shape_a) == 3
     if batched:
-        assert b.dim() == 3 and a.shape[0] == b.shape[0]
-    M = a.shape[-1] if a_mn else a.shape[-2]
-    K = a.shape[-2] if a_mn else a.shape[-1]
-    N = b.shape[-1] if b_mn else b.shape[-2]
-    Kb = b.shape[-2] if b_mn else b.shape[-1]
+        assert len(shape_b) == 3 and shape_a[0] == shape_b[0]
+    K, M = (shape_a[-2], shape_a[-1]) if a_mn else (shape_a[-1], shape_a[-2])
+    Kb, N = (shape_b[-2], shape_b[-1]) if b_mn else (shape_b[-1], shape_b[-2])
     if K != Kb:
         raise ValueError(f"gemm: inner dimensions differ ({K} vs {Kb})")
     if a.dtype != torch.bfloat16:
@@ -217,46 +217,49 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if b.dtype != torch.bfloat16:
         b = b.to(torch.bfloat16)
     a, b = _tma_ready(a), _tma_ready(b)
-    batch = a.shape[0] if batched else 1
+    batch = shape_a[0] if batched else 1
     if out is None:
         shape = (batch, M, N) if batched else (M, N)
-        out = torch.empty(shape, dtype=out_dtype, device=a.device)
+        out = a.new_empty(shape) if out_dtype == torch.bfloat16 else a.new_empty(shape, dtype=out_dtype)
     else:
         assert out.stride(-1) == 1 and out.shape[-2] == M and out.shape[-1] == N
-        assert out.dtype in (torch.bfloat16, torch.float32)
-    for t in (bias, residual, aux_out, aux_in):
+        assert out_dtype in (torch.bfloat16, torch.float32)
+    operands = [0, 0, 0, 0, 0, 0, 0]           # addresses of the epilogue's operands, then the leading dimensions of the matrices
+    for i, t in enumerate((bias, residual, aux_out, aux_in)):
         if t is not None:
-            assert t.dtype == torch.bfloat16 and t.stride(-1) == 1, "epilogue operands must be bf16"
-    lib, stream = native.lib(), native.stream_ptr(a.device)
-    fp32 = out.dtype == torch.float32
-    target, ldc, k_part, parts, acc, max_ctas = out, out.stride(-2), K, batch, int(accumulate), int(max_ctas)
-    strides = (a.stride(0), b.stride(0), out.stride(0)) if batched else (0, 0, 0)
+            ld = t.stride()
+            assert t.dtype == torch.bfloat16 and ld[-1] == 1, "epilogue operands must be bf16"
+            operands[i] = t.data_ptr()
+            if i:
+                operands[3 + i] = ld[-2]
+    lib, stream = native.lib(), native.raw_stream(device)
+    stride_a, stride_b, stride_c = a.stride(), b.stride(), out.stride()
+    fp32 = out_dtype == torch.float32
+    target, ldc, k_part, parts, acc, max_ctas = out, stride_c[-2], K, batch, int(accumulate), int(max_ctas)
+    strides = (stride_a[0], stride_b[0], stride_c[0]) if batched else (0, 0, 0)
     in_parts = False
     if SPLIT_K and a_mn and b_mn and fp32 and not batched and bias is None and residual is None and act_id == 0:
         n = _partial_splits(M, N, K) if aux_out is None and max_ctas == 0 and out.is_contiguous() else 1
         if n > 1:
             in_parts = True
             target, ldc, acc = torch.empty((n, M, N), dtype=torch.float32, device=a.device), N, 0
-        elif accumulate and N % 32 == 0 and out.stride(0) % 4 == 0 and not native.deterministic_reduction():
+        elif accumulate and N % 32 == 0 and stride_c[0] % 4 == 0 and not native.deterministic_reduction():
             # weight-gradient shape with a poor tile count: split the long reduction over CTAs of the same tile
             # (expressed as a batch over K) and add the partials with fp32 atomics
             n = _split_k(M, N, K)
             acc = 2 if n > 1 else acc
         if n > 1:
             k_part, parts = K // n, n
-            strides = (k_part * a.stride(0), k_part * b.stride(0), M * N if in_parts else 0)
-    args = _pack_args(
-        a.data_ptr(), b.data_ptr(), target.data_ptr(), 0 if bias is None else bias.data_ptr(),
-        0 if residual is None else residual.data_ptr(), 0 if aux_out is None else aux_out.data_ptr(),
-        0 if aux_in is None else aux_in.data_ptr(), a.stride(-2), b.stride(-2), ldc,
-        0 if residual is None else residual.stride(-2), 0 if aux_out is None else aux_out.stride(-2),
-        0 if aux_in is None else aux_in.stride(-2), *strides, M, N, k_part, parts, int(a_mn), int(b_mn), int(fp32), acc,
-        act_id, float(alpha), max_ctas)
-    native.check(lib.st_gemm_bf16(args, stream), "st_gemm_bf16")
+            strides = (k_part * stride_a[0], k_part * stride_b[0], M * N if in_parts else 0)
+    args = _pack_args(a.data_ptr(), b.data_ptr(), target.data_ptr(), *operands[:4], stride_a[-2], stride_b[-2], ldc, *operands[4:],
+                      *strides, M, N, k_part, parts, a_mn, b_mn, fp32, acc, act_id, alpha, max_ctas)
+    status = lib.st_gemm_bf16(args, ctypes.c_void_p(stream))
+    if status:
+        native.check(status, "st_gemm_bf16")
     launch_count += 1
     if in_parts:
-        native.check(lib.st_reduce_partials(native.ptr(target), native.ptr(out), ctypes.c_int(n), ctypes.c_int(M * N),
-                                            ctypes.c_int(int(accumulate)), stream), "st_reduce_partials")
+        native.check(native.entry("st_reduce_partials", "ppiiip")(target.data_ptr(), out.data_ptr(), n, M * N, int(accumulate), stream),
+                     "st_reduce_partials")
         launch_count += 1
     return out
 

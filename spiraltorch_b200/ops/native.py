@@ -7,6 +7,7 @@ be built, every CUDA op raises instead of silently running a PyTorch fallback.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from typing import Optional
@@ -150,20 +151,44 @@ def same_device(op: str, *tensors: Optional[torch.Tensor]) -> None:
             raise ValueError(f"{op}: operands live on different devices ({dev} and {t.device})")
 
 
-def require_cuda(op: str, *tensors: Optional[torch.Tensor]) -> None:
-    """Refuse a launch unless every operand is a CUDA tensor on one device.  Launchers receive raw addresses:
-    a host tensor's address would be encoded into a TMA tensor map or dereferenced by the kernel and fault the
+def require_cuda(op: str, *tensors: Optional[torch.Tensor]) -> int:
+    """Refuse a launch unless every operand is a CUDA tensor on one device, whose index is returned.  Launchers receive raw
+    addresses: a host tensor's address would be encoded into a TMA tensor map or dereferenced by the kernel and fault the
     context, so the check comes before any pointer is taken."""
-    dev = None
+    first, index = None, -1
     for t in tensors:
         if t is None:
             continue
         if not t.is_cuda:
             raise ValueError(f"{op}: operand of shape {tuple(t.shape)} is a host tensor; move it to the GPU first")
-        if dev is None:
-            dev = t.device
-        elif t.device != dev:
-            raise ValueError(f"{op}: operands live on different devices ({dev} and {t.device})")
+        i = t.get_device()
+        if i != index:
+            if first is not None:
+                raise ValueError(f"{op}: operands live on different devices ({first.device} and {t.device})")
+            first, index = t, i
+    return index
+
+
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "q": ctypes.c_longlong, "f": ctypes.c_float}
+
+
+@functools.cache
+def entry(name: str, types: str):
+    """The launcher ``name`` with its argument types (p address, i int, q long long, f float) set: it then takes plain numbers.
+    A ctypes object built for each of a dozen arguments costs as much as the launch itself."""
+    fn = getattr(lib(), name)
+    fn.argtypes = [_CTYPES[t] for t in types]
+    return fn
+
+
+def address(t: Optional[torch.Tensor]) -> int:
+    """Address of a tensor that :func:`require_cuda` has seen, 0 for none."""
+    return 0 if t is None else t.data_ptr()
+
+
+def raw_stream(index: int) -> int:
+    """Handle of the current stream of device ``index``."""
+    return _raw_stream(index) if _raw_stream is not None else torch.cuda.current_stream(index).cuda_stream
 
 
 def deterministic_reduction() -> bool:

@@ -25,8 +25,7 @@ def _scratch(lib, x2: torch.Tensor) -> torch.Tensor:
     """Partial parameter gradients of one backward call.  A tensor per call: a buffer kept for a device would be shared by its
     streams and threads, and a captured step would go on writing to it after a larger call had replaced it."""
     lib.st_norm_bwd_scratch_elems.restype = ctypes.c_longlong
-    elems = lib.st_norm_bwd_scratch_elems(ctypes.c_int(x2.shape[0]), ctypes.c_int(x2.shape[1]))
-    return torch.empty(elems, dtype=torch.float32, device=x2.device)
+    return x2.new_empty(native.entry("st_norm_bwd_scratch_elems", "ii")(*x2.shape), dtype=torch.float32)
 
 
 @functools.cache
@@ -46,8 +45,8 @@ def takes_f32(d: int, *tensors: Optional[torch.Tensor]) -> bool:
         and d <= _limit("st_norm_f32_max_features")
 
 
-def _form(lib, entry: str, x2: torch.Tensor, rounded: bool):
-    return getattr(lib, entry if x2.dtype != torch.float32 else entry + ("_f32_rounded" if rounded else "_f32"))
+def _form(entry: str, types: str, x2: torch.Tensor, rounded: bool):
+    return native.entry(entry if x2.dtype != torch.float32 else entry + ("_f32_rounded" if rounded else "_f32"), types)
 
 
 def norm_reference(x, gamma, beta, eps, rms, residual=None):
@@ -83,15 +82,16 @@ def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=
         if out is not None:
             y = out.copy_(y)
         return y, (xs.to(x2.dtype) if residual is not None else None), mean, rstd
+    device = native.require_cuda("norm_forward", x2, residual, gamma, beta)
     y = torch.empty_like(x2) if out is None else out
     s = torch.empty_like(x2) if residual is not None or (copy_input and x2.dtype == torch.float32) else None
-    mean = torch.empty(rows, dtype=torch.float32, device=x2.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
-    st = _form(native.lib(), "st_norm_fwd", x2, rounded)(
-        ctypes.c_int(int(rms)), native.ptr(x2), native.ptr(residual), native.ptr(gamma), native.ptr(beta),
-        native.ptr(y), native.ptr(s), native.ptr(mean), native.ptr(rstd), ctypes.c_int(rows),
-        ctypes.c_int(d), ctypes.c_float(eps), native.stream_ptr(x2.device))
-    native.check(st, "st_norm_fwd")
+    mean = x2.new_empty(rows, dtype=torch.float32)
+    rstd = torch.empty_like(mean)
+    status = _form("st_norm_fwd", "ippppppppiifp", x2, rounded)(
+        rms, x2.data_ptr(), native.address(residual), native.address(gamma), native.address(beta), y.data_ptr(), native.address(s),
+        mean.data_ptr(), rstd.data_ptr(), rows, d, eps, native.raw_stream(device))
+    if status:
+        native.check(status, "st_norm_fwd")
     launch_count += 1
     return y, s, mean, rstd
 
@@ -120,15 +120,14 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
             dbeta.copy_(dbeta + db if accumulate else db)
         dx = dx.to(x2.dtype)
         return dx if out is None else out.copy_(dx)
+    device = native.require_cuda("norm_backward", dy2, x2, gamma, mean, rstd, dres, dgamma, dbeta)
     dx = torch.empty_like(x2) if out is None else out
-    lib = native.lib()
-    scratch = _scratch(lib, x2)
-    st = _form(lib, "st_norm_bwd", x2, rounded)(
-        ctypes.c_int(int(rms)), native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(mean),
-        native.ptr(rstd), native.ptr(dres), native.ptr(dx), native.ptr(dgamma), native.ptr(dbeta),
-        ctypes.c_int(int(accumulate)), native.ptr(scratch), ctypes.c_int(rows), ctypes.c_int(d),
-        native.stream_ptr(x2.device))
-    native.check(st, "st_norm_bwd")
+    scratch = _scratch(native.lib(), x2)
+    status = _form("st_norm_bwd", "ipppppppppipiip", x2, rounded)(
+        rms, dy2.data_ptr(), x2.data_ptr(), gamma.data_ptr(), native.address(mean), rstd.data_ptr(), native.address(dres),
+        dx.data_ptr(), dgamma.data_ptr(), native.address(dbeta), accumulate, scratch.data_ptr(), rows, d, native.raw_stream(device))
+    if status:
+        native.check(status, "st_norm_bwd")
     launch_count += 2
     return dx
 
@@ -136,13 +135,14 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
 def norm_gelu_forward(x2: torch.Tensor, gamma, beta, eps: float):
     """``gelu(layer_norm(x2))`` of contiguous bf16 rows of at most :func:`gelu_max_features` on CUDA: ``(y, mean, rstd)``."""
     global launch_count
-    native.require_cuda("norm_gelu_forward", x2, gamma, beta)
+    device = native.require_cuda("norm_gelu_forward", x2, gamma, beta)
     rows, d = x2.shape
     y = torch.empty_like(x2)
-    mean, rstd = (torch.empty(rows, dtype=torch.float32, device=x2.device) for _ in range(2))
-    native.check(native.lib().st_norm_gelu_fwd(
-        native.ptr(x2), native.ptr(gamma), native.ptr(beta), native.ptr(y), native.ptr(mean), native.ptr(rstd), ctypes.c_int(rows),
-        ctypes.c_int(d), ctypes.c_float(eps), native.stream_ptr(x2.device)), "st_norm_gelu_fwd")
+    mean = x2.new_empty(rows, dtype=torch.float32)
+    rstd = torch.empty_like(mean)
+    native.check(native.entry("st_norm_gelu_fwd", "ppppppiifp")(
+        x2.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), rows, d, eps,
+        native.raw_stream(device)), "st_norm_gelu_fwd")
     launch_count += 1
     return y, mean, rstd
 
@@ -150,15 +150,13 @@ def norm_gelu_forward(x2: torch.Tensor, gamma, beta, eps: float):
 def norm_gelu_backward(dy2, x2, gamma, beta, mean, rstd, dgamma: torch.Tensor, dbeta: torch.Tensor) -> torch.Tensor:
     """Backward of :func:`norm_gelu_forward`: returns dx, writes the fp32 ``dgamma`` and ``dbeta``."""
     global launch_count
-    native.require_cuda("norm_gelu_backward", dy2, x2, gamma, beta, mean, rstd, dgamma, dbeta)
+    device = native.require_cuda("norm_gelu_backward", dy2, x2, gamma, beta, mean, rstd, dgamma, dbeta)
     rows, d = x2.shape
-    lib = native.lib()
-    scratch = _scratch(lib, x2)
+    scratch = _scratch(native.lib(), x2)
     dx = torch.empty_like(x2)
-    native.check(lib.st_norm_gelu_bwd(
-        native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(beta), native.ptr(mean), native.ptr(rstd), native.ptr(dx),
-        native.ptr(dgamma), native.ptr(dbeta), ctypes.c_int(0), native.ptr(scratch), ctypes.c_int(rows), ctypes.c_int(d),
-        native.stream_ptr(x2.device)), "st_norm_gelu_bwd")
+    native.check(native.entry("st_norm_gelu_bwd", "pppppppppipiip")(
+        dy2.data_ptr(), x2.data_ptr(), gamma.data_ptr(), beta.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
+        dgamma.data_ptr(), dbeta.data_ptr(), 0, scratch.data_ptr(), rows, d, native.raw_stream(device)), "st_norm_gelu_bwd")
     launch_count += 2
     return dx
 
