@@ -1,0 +1,53 @@
+"""Backward attention in one pass over the tile pairs (head_dim 64, up to eight key tiles) against 64 bits, at its edges: one, two
+and three key tiles (one sum of dQ, one of two tiles, two sums), the last count it takes and the first it leaves to two passes,
+other query than key lengths, contexts without keys; the same bits on every run."""
+import math
+
+import pytest
+import torch
+
+from spiraltorch_b200.ops import attention as A
+from spiraltorch_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(q, k, v, g, causal, bias, lengths):
+    q, k, v = (t.double().transpose(1, 2).requires_grad_(True) for t in (q, k, v))
+    s = q @ k.transpose(-1, -2) / math.sqrt(q.shape[-1])
+    keys, rows = torch.arange(k.shape[2], device=q.device), torch.arange(q.shape[2], device=q.device)
+    if bias is not None:
+        s = s + bias.double()[:, None, None, :]
+    if causal:
+        s = s.masked_fill(keys > rows[:, None], -1e30)
+    if lengths is not None:
+        s = s.masked_fill(keys >= lengths[:, None, None, None], -1e30)
+    o = torch.softmax(s, -1) @ v
+    if lengths is not None:
+        o = o * (rows[:, None] < lengths[:, None, None, None])
+    return [t.transpose(1, 2) for t in torch.autograd.grad(o, (q, k, v), g.double().transpose(1, 2))]
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("B,Sq,Sk,H,causal,extras", [(2, 128, 128, 3, True, False), (3, 200, 256, 2, False, True),
+                                                     (2, 385, 385, 2, True, True), (150, 300, 257, 1, False, True),
+                                                     (1, 1024, 1024, 2, True, False), (2, 100, 1025, 1, False, True)])
+def test_gradients(B, Sq, Sk, H, causal, extras, f32):
+    torch.manual_seed(Sq + Sk)
+    q, g = (torch.randn(B, Sq, H, 64, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Sk, H, 64, device="cuda").bfloat16() for _ in range(2))
+    bias = torch.randn(B, Sk, device="cuda") if extras else None
+    lengths = torch.randint(0, min(Sq, Sk) + 1, (B,), device="cuda", dtype=torch.int32) if extras else None
+    o, lse = A.attention_forward(q, k, v, causal, key_bias=bias, lengths=lengths)
+
+    def run():
+        dtype = torch.float32 if f32 else torch.bfloat16
+        out = [torch.full(t.shape, 7.0, dtype=dtype, device="cuda") for t in (q, k, v)]
+        return A.attention_backward(q, k, v, o, lse, g, causal, None, *out, key_bias=bias, lengths=lengths)
+
+    got, again = run(), run()
+    for x, y, ref in zip(got, again, _exact(q, k, v, g, causal, bias, lengths)):
+        assert torch.equal(x, y)
+        # P, dS, the output in delta and the result are rounded to bf16, 2^-9 each
+        assert (x.double() - ref).norm() <= 4 * 2.0 ** -9 * ref.norm()
+    native.raise_on_device_error()
