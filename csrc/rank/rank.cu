@@ -142,8 +142,8 @@ __global__ void rank_k1_kernel(const float* __restrict__ in, float* __restrict__
 // ---- top / bottom with k <= 128: warp-resident candidate lists ------------------------------------------------------
 // A row is read once, so the bound is its bytes.  What made the full sort slow was shared memory: 78 exchange stages
 // over 4096 keys per row.  Here an element costs one comparison with a bound on the k-th best value; the few that pass
-// go to a small queue, and a full queue is sorted in registers and merged into the list.  4096 x 4096, k = 32: 22 us
-// (the bytes take 10) with half of the issue slots busy and the rest waiting for loads; two sorts of row halves and the merge of
+// go to a small queue, and a full queue is sorted in registers and merged into the list.  4096 x 4096, k = 32: 19.4 us
+// (the bytes take 10), bound by the latency of two passes over a row; two sorts of row halves and the merge of
 // their lists took 669.
 using u64 = unsigned long long;
 constexpr int TOPK_MAX_K = 128;
@@ -151,6 +151,10 @@ constexpr int TOPK_GROUP = 128;             // columns of a warp-wide load: four
 constexpr int TOPK_STEP = 4 * TOPK_GROUP;   // columns per step of a warp: 2 KB of loads in flight
 constexpr int topk_capacity(int R) { return 32 * R + TOPK_STEP; }
 constexpr int TOPK_MAX_WARPS = 16;          // warps of one CTA on one row
+constexpr int TOPK_BOUND_SHARE = 512;       // columns of a share per list register from which a bound is looked for first
+__host__ __device__ inline int topk_share(int cols, int split) {
+  return ((cols + split - 1) / split + TOPK_GROUP - 1) / TOPK_GROUP * TOPK_GROUP;
+}
 
 __device__ __forceinline__ u64 min64(u64 a, u64 b) { return a < b ? a : b; }
 __device__ __forceinline__ u64 max64(u64 a, u64 b) { return a < b ? b : a; }
@@ -237,11 +241,12 @@ __device__ __forceinline__ void write_best(const u64 (&best)[R], float* out_v, i
 
 // `warps` warps (a power of two) share a row, each with a contiguous share of its columns; a CTA holds
 // blockDim / (32 warps) rows.  With parts > 1 a row is also split over `parts` CTAs, whose lists go to `lists`
-// [rows][parts][N].  VEC: rows start at 16-byte boundaries and are read as float4.
-template <int R, bool VEC, bool TOP_MODE>
+// [rows][parts][N].  VEC: rows start at 16-byte boundaries and are read as float4.  BOUNDED: shares are long enough for a bound.
+template <int R, bool VEC, bool TOP_MODE, bool BOUNDED>
 __global__ void __launch_bounds__(TOPK_MAX_WARPS * 32)
 rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* __restrict__ out_i, int rows, int cols,
                  int k, int warps, int parts, u64* __restrict__ lists) {
+  chain_begin(in);
   constexpr int N = 32 * R, CAP = topk_capacity(R);
   extern __shared__ u64 queues[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -257,7 +262,7 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
   int qn = 0;
   if (row < rows) {
     const float* x = in + row * cols;
-    const int share = (((cols + warps * parts - 1) / (warps * parts)) + TOPK_GROUP - 1) / TOPK_GROUP * TOPK_GROUP;
+    const int share = topk_share(cols, warps * parts);
     const int c_begin = (int)min((long long)cols, (long long)(part * warps + wr) * share), c_end = min(cols, c_begin + share);
     // element j of a group sits at column 4 lane + j (VEC) or lane + 32 j; columns past the share read as NaN, which
     // fails every comparison
@@ -278,18 +283,22 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
     // the share; k of the warp's 64 R parts hold a value at least as good as the k-th best of these, so the k-th best of
     // the row does too.  With 64 parts and k = 32 about 45 of 4096 elements then pass, instead of some 300 with a list
     // that starts empty, whose sorts were most of the time.  The second read of the share comes from L2.
-    if (c_end - c_begin >= 512 * R) {
+    if (BOUNDED && c_end - c_begin >= TOPK_BOUND_SHARE * R) {
       constexpr int PARTS = 2 * R;
       float ext[PARTS];
 #pragma unroll
       for (int g = 0; g < PARTS; ++g) ext[g] = TOP_MODE ? -INFINITY : INFINITY;
+      constexpr int AHEAD = 8;                      // loads in flight per lane
 #pragma unroll 1
-      for (int c0 = c_begin; c0 < c_end; c0 += TOPK_GROUP * PARTS * (R == 1 ? 2 : 1)) {
+      for (int c0 = c_begin; c0 < c_end; c0 += TOPK_GROUP * AHEAD) {
+        float4 f[AHEAD];
 #pragma unroll
-        for (int g = 0; g < PARTS * (R == 1 ? 2 : 1); ++g) {
-          const float4 f = load(c0 + g * TOPK_GROUP);
+        for (int g = 0; g < AHEAD; ++g) f[g] = load(c0 + g * TOPK_GROUP);
+#pragma unroll
+        for (int g = 0; g < AHEAD; ++g) {
           float& e = ext[g % PARTS];
-          e = TOP_MODE ? fmaxf(fmaxf(fmaxf(e, f.x), fmaxf(f.y, f.z)), f.w) : fminf(fminf(fminf(e, f.x), fminf(f.y, f.z)), f.w);
+          e = TOP_MODE ? fmaxf(fmaxf(fmaxf(e, f[g].x), fmaxf(f[g].y, f[g].z)), f[g].w)
+                       : fminf(fminf(fminf(e, f[g].x), fminf(f[g].y, f[g].z)), f[g].w);
         }
       }
       unsigned better[PARTS];                       // larger is better; 0 for a part whose extreme is not finite
@@ -307,31 +316,61 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
       if (bound >= 0x00800000u) thr_v = from_orderable(TOP_MODE ? bound : ~bound);
     }
     // The queue and merge code sits once in a rolled loop: unrolled per element it outgrew the instruction cache.
+    // With a bound few elements pass: a step's loads are under way while the step before it is examined, and a lane marks its
+    // elements that pass and hands over one mark at a time, so that a step takes as many rounds as the lane with the most marks
+    // has.  Without one most of the first steps pass, and the sixteen elements are voted on in turn.
+    // us, votes and marks: 4096 x 4096, k = 32, 24.0 and 20.6 (from DRAM 31 and 27); 335 x 50000 35.3 and 26.4; 3000 x 4100, k = 128,
+    // 43.3 and 38.9; without a bound 16 x 50000 23.4 and 25.7, 8192 x 512, k = 64, 61 and 67.
+    float4 next[4];
+    if constexpr (BOUNDED) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) next[g] = load(c_begin + g * TOPK_GROUP);
+    }
 #pragma unroll 1
     for (int c0 = c_begin; c0 < c_end; c0 += TOPK_STEP) {
       float v[16];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const float4 f = load(c0 + g * TOPK_GROUP);
+        const float4 f = BOUNDED ? next[g] : load(c0 + g * TOPK_GROUP);
         v[4 * g] = f.x; v[4 * g + 1] = f.y; v[4 * g + 2] = f.z; v[4 * g + 3] = f.w;
+        if constexpr (BOUNDED) next[g] = load(c0 + TOPK_STEP + g * TOPK_GROUP);
       }
-      bool any = false;
+      // equal values are decided by the whole key: the lower column wins
+      auto enqueue = [&](float e, int j, bool near) {
+        const int c = c0 + (j >> 2) * TOPK_GROUP + (VEC ? lane * 4 + (j & 3) : lane + 32 * (j & 3));
+        unsigned o = orderable(e);
+        if (TOP_MODE) o = ~o;
+        const u64 key = (static_cast<u64>(o) << 32) | static_cast<unsigned>(c);
+        const bool pass = near && isfinite(e) && key < thr;
+        const unsigned m = __ballot_sync(0xffffffffu, pass);
+        if (pass) queue[qn + __popc(m & ((1u << lane) - 1u))] = key;
+        qn += __popc(m);
+      };
+      auto near = [&](float e) { return TOP_MODE ? e >= thr_v : e <= thr_v; };
+      if constexpr (BOUNDED) {
+        unsigned marks = 0;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) any |= TOP_MODE ? v[j] >= thr_v : v[j] <= thr_v;
-      if (__any_sync(0xffffffffu, any)) {
+        for (int j = 0; j < 16; ++j) marks |= near(v[j]) ? 1u << j : 0u;
+        while (__any_sync(0xffffffffu, marks != 0)) {
+          const int j = marks ? __ffs(marks) - 1 : 0;
+          float e8[8], e4[4], e2[2];                      // v[j]
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const bool near = TOP_MODE ? v[j] >= thr_v : v[j] <= thr_v;
-          if (!__any_sync(0xffffffffu, near)) continue;
-          const int c = c0 + (j >> 2) * TOPK_GROUP + (VEC ? lane * 4 + (j & 3) : lane + 32 * (j & 3));
-          unsigned o = orderable(v[j]);
-          if (TOP_MODE) o = ~o;
-          const u64 key = (static_cast<u64>(o) << 32) | static_cast<unsigned>(c);
-          // equal values are decided by the whole key: the lower column wins
-          const bool pass = near && isfinite(v[j]) && key < thr;
-          const unsigned m = __ballot_sync(0xffffffffu, pass);
-          if (pass) queue[qn + __popc(m & ((1u << lane) - 1u))] = key;
-          qn += __popc(m);
+          for (int i = 0; i < 8; ++i) e8[i] = j & 1 ? v[2 * i + 1] : v[2 * i];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) e4[i] = j & 2 ? e8[2 * i + 1] : e8[2 * i];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) e2[i] = j & 4 ? e4[2 * i + 1] : e4[2 * i];
+          enqueue(j & 8 ? e2[1] : e2[0], j, marks != 0);
+          marks &= marks - 1;
+        }
+      } else {
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) any |= near(v[j]);
+        if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (__any_sync(0xffffffffu, near(v[j]))) enqueue(v[j], j, near(v[j]));
         }
       }
       // full queue, or the end of the share: sort it and merge it into the list
@@ -372,6 +411,7 @@ constexpr int MERGE_WARPS = 8;
 template <int R>
 __global__ void __launch_bounds__(MERGE_WARPS * 32)
 rank_merge_kernel(const u64* __restrict__ lists, float* __restrict__ out_v, int* __restrict__ out_i, int k, int parts, int top) {
+  chain_begin(lists);
   constexpr int N = 32 * R, CAP = topk_capacity(R);
   __shared__ u64 queues[MERGE_WARPS * CAP];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -413,22 +453,23 @@ int launch_topk(const float* in, float* out_v, int* out_i, int rows, int cols, i
   const int per_cta = (threads / 32) / warps;
   const int grid = ((rows + per_cta - 1) / per_cta) * parts;
   const size_t smem = (size_t)(threads / 32) * topk_capacity(R) * sizeof(u64);
-  static bool cfg[st::kMaxDevices] = {false};      // the attribute is per device
-  const int dev = st::current_device();
-  if (!cfg[dev]) {
-    const int most = TOPK_MAX_WARPS * topk_capacity(R) * (int)sizeof(u64);       // at most 80 KB
-    ST_CUDA_CHECK(cudaFuncSetAttribute(rank_topk_kernel<R, VEC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    ST_CUDA_CHECK(cudaFuncSetAttribute(rank_topk_kernel<R, VEC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    cfg[dev] = true;
-  }
-  if (mode == TOP)
-    rank_topk_kernel<R, VEC, true><<<grid, threads, smem, s>>>(in, out_v, out_i, rows, cols, k, warps, parts, lists);
-  else
-    rank_topk_kernel<R, VEC, false><<<grid, threads, smem, s>>>(in, out_v, out_i, rows, cols, k, warps, parts, lists);
-  ST_CUDA_CHECK(cudaGetLastError());
+  auto run = [&](auto kernel, bool* cfg) -> int {
+    const int dev = st::current_device();      // the attribute is per device
+    if (!cfg[dev]) {
+      const int most = TOPK_MAX_WARPS * topk_capacity(R) * (int)sizeof(u64);       // at most 80 KB
+      ST_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      cfg[dev] = true;
+    }
+    ST_CUDA_CHECK(st::chained(kernel, grid, threads, smem, s)(in, out_v, out_i, rows, cols, k, warps, parts, lists));
+    return ST_OK;
+  };
+  static bool cfg[4][st::kMaxDevices] = {{false}};
+  const bool bounded = topk_share(cols, warps * parts) >= TOPK_BOUND_SHARE * R;
+  const int rc = mode == TOP ? (bounded ? run(rank_topk_kernel<R, VEC, true, true>, cfg[0]) : run(rank_topk_kernel<R, VEC, true, false>, cfg[1]))
+                             : (bounded ? run(rank_topk_kernel<R, VEC, false, true>, cfg[2]) : run(rank_topk_kernel<R, VEC, false, false>, cfg[3]));
+  if (rc != ST_OK) return rc;
   if (parts > 1) {
-    rank_merge_kernel<R><<<rows, MERGE_WARPS * 32, 0, s>>>(lists, out_v, out_i, k, parts, mode == TOP);
-    ST_CUDA_CHECK(cudaGetLastError());
+    ST_CUDA_CHECK(st::chained(rank_merge_kernel<R>, rows, MERGE_WARPS * 32, 0, s)(lists, out_v, out_i, k, parts, mode == TOP));
   }
   return ST_OK;
 }
