@@ -31,7 +31,8 @@ namespace gemm {
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int NUM_THREADS = 320;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-9: epilogue, two per 32 lanes
+constexpr int num_threads(int sets) { return 64 + 128 * sets; }      // warp 0: TMA, warp 1: MMA + TMEM owner, then the epilogue's warps
+constexpr int NUM_THREADS = num_threads(2);
 constexpr int NUM_THREADS_RS = 192;  // reduce-scatter variant: one epilogue warp per 32 lanes
 constexpr int NUM_THREADS_AG = 256;  // all-gather variant: + warp 6 (shard push) and warp 7 (arrival publisher)
 constexpr int AG_RING_CHUNK = 16384;  // bytes per bulk copy of the push ring
@@ -113,21 +114,21 @@ struct OutMaps {
   CUtensorMap m[kMaxRanks];
 };
 
-// CBUF: 4 KiB staging blocks per epilogue warp of the plain product (eight warps), as many as fit beside the operand ring; the
-// tensor-parallel variants have four warps with two blocks each, which is the room of CBUF = 1.
+// CBUF: 4 KiB staging blocks per epilogue warp of the plain product (four times SETS warps), as many as fit beside the operand
+// ring; the tensor-parallel variants have four warps with two blocks each, which is the room of CBUF = 1 of eight.
 constexpr int kSmemMax = 232448;      // 227 KiB
-template <int BN, int STAGES, int CB = 0>
+template <int BN, int STAGES, int CB = 0, int SETS = 2>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int BAR_BYTES = 512;                            // barriers
   static constexpr int SLACK = BAR_BYTES + 1024;                   // and alignment
-  static constexpr int ROOM = (kSmemMax - SLACK - STAGES * STAGE_BYTES) / (8 * 4096);
+  static constexpr int ROOM = (kSmemMax - SLACK - STAGES * STAGE_BYTES) / (4 * SETS * 4096);
   static constexpr int CBUF = CB ? CB : ROOM < 4 ? ROOM : 4;
   static_assert(CBUF >= 1, "no room for the staged output");
   static constexpr int CSTAGE_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int CSTAGE_BYTES = 8 * CBUF * 4096;
+  static constexpr int CSTAGE_BYTES = 4 * SETS * CBUF * 4096;
   static constexpr int BAR_OFFSET = CSTAGE_OFFSET + CSTAGE_BYTES;
   static constexpr int OPBAR_OFFSET = BAR_OFFSET + 256;            // one barrier per epilogue warp and staging block (at most 32)
   static constexpr int TOTAL = BAR_OFFSET + SLACK;
@@ -304,17 +305,17 @@ __device__ __forceinline__ void load32_bf16(uint4 (&x)[4], const __nv_bfloat16* 
 // CG = 2 (COMM_NONE only): a cluster of two CTAs works on one tile of 256 x BN.  Each CTA brings its 128 rows of A and its half
 // of B into its own shared memory, the even CTA's MMA warp issues for both, and each CTA's epilogue stores its own 128 rows.
 // A K block then costs an SM 32 KB of loads instead of 48 (BN = 256), and the ring holds six stages instead of four.
-template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM, int CG = 1, int KS = 1>
-__global__ void __launch_bounds__(COMM == COMM_AG ? NUM_THREADS_AG : COMM == COMM_RS ? NUM_THREADS_RS : NUM_THREADS, 1)
+template <int BN, int STAGES, bool A_MN, bool B_MN, int COMM, int CG = 1, int KS = 1, int SETS_ = 2>
+__global__ void __launch_bounds__(COMM == COMM_AG ? NUM_THREADS_AG : COMM == COMM_RS ? NUM_THREADS_RS : num_threads(SETS_), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ OutMaps tmC, const __grid_constant__ CUtensorMap tmA_local,
                  const GemmParams p, const GemmComm cm) {
   static_assert((CG == 1 && KS == 1) || (COMM == COMM_NONE && (CG == 1 || KS == 1)), "CTA pairs and K parts run the plain product only");
-  using L = SmemLayout<BN / CG, STAGES, COMM == COMM_NONE ? 0 : 1>;
-  // Epilogue warps per 32 lanes of the accumulator.  Two of them take 64-column groups in turn, or, where a tile has only one
-  // group, whole tiles in turn: one warp's loads, arithmetic and stores for a tile are longer than the main loop of a short K.
-  constexpr int SETS = COMM == COMM_NONE ? 2 : 1;
-  constexpr bool SPLIT = SETS == 2 && BN > 64;
+  using L = SmemLayout<BN / CG, STAGES, COMM == COMM_NONE ? 0 : 1, SETS_>;
+  // Epilogue warps per 32 lanes of the accumulator.  Two or three of them take 64-column groups in turn, or, where a tile has only
+  // one group, whole tiles in turn: one warp's loads, arithmetic and stores for a tile are longer than the main loop of a short K.
+  constexpr int SETS = COMM == COMM_NONE ? SETS_ : 1, GROUPS = BN / 64;
+  constexpr bool SPLIT = SETS >= 2 && BN > 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -351,10 +352,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tfull_bar[a]), 1);
-      mbar_init(smem_u32(&tempty_bar[a]), (SPLIT ? 8 : 4) * CG);
+      mbar_init(smem_u32(&tempty_bar[a]), (SPLIT ? 4 * SETS : 4) * CG);
     }
     if constexpr (COMM == COMM_NONE)
-      for (int i = 0; i < 8 * L::CBUF; ++i) mbar_init(smem_u32(smem + L::OPBAR_OFFSET) + i * 8, 1);
+      for (int i = 0; i < 4 * SETS * L::CBUF; ++i) mbar_init(smem_u32(smem + L::OPBAR_OFFSET) + i * 8, 1);
     *abort_flag = 0;
     if constexpr (COMM == COMM_AG) {
       tmem_slot[2] = 0;   // items whose stores are complete (push warp → publisher warp)
@@ -626,14 +627,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const bool tma_op = CBUF >= 2 && p.operand_tma, tma_aux = CBUF >= 2 && p.aux_tma;
     const bool bwd = p.act == ACT_GELU_BWD || p.act == ACT_RELU_BWD;
     int iter = 0, blocks = 0;       // blocks staged by this warp
-    // the warp's 64-column groups of tile t: set, set + 2, ... (SPLIT), or the only one of every second tile
+    // the warp's 64-column groups: every SETS-th, counted over its CTA's tiles (SPLIT), or the only one of every SETS-th tile
+    auto first_group = [&](int iter) { return SPLIT ? (set + SETS * GROUPS - iter * GROUPS % SETS) % SETS : 0; };
     auto groups_of = [&](int t, int& m0, int& n0, int& b) {
       int tm, tn;
       map_tile<COMM>(t, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
       m0 = tm * BM * CG + cta * BM + quad * 32;
       n0 = tn * BN;
       if (KS > 1 && quad / (4 / KS) != kpart) return 0;
-      return m0 < p.M ? min(BN / 64, (p.N - n0 + 63) >> 6) : 0;
+      return m0 < p.M ? min(GROUPS, (p.N - n0 + 63) >> 6) : 0;
     };
     // K parts: CTA i of the cluster finishes rows [i, i + 1) * 128 / KS of the tile.  Once every CTA's products are complete the
     // operand ring is idle and takes the others' partial sums of those rows, [source][column / 4][row] in 16-byte pieces.
@@ -649,7 +651,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         map_tile<COMM>(gemm_bid, tiles_m, tiles_n, tiles_per_batch, cm, b, tm, tn);
         const int slot = kpart < owner ? kpart : kpart - 1;
         const uint32_t dst = cluster_map(smem_u32(smem), owner) + (slot * PART_ELEMS + ((quad % (4 / KS)) * 32 + lane) * 4) * 4;
-        for (int c = set; c < BN / 32 && tn * BN + c * 32 < p.N; c += 2) {
+        for (int c = set; c < BN / 32 && tn * BN + c * 32 < p.N; c += SETS) {
           uint32_t r[32];
           tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + c * 32, r);
           tmem_ld_wait();
@@ -660,12 +662,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       cluster_sync();
     }
     // operand requests run up to CBUF - 1 blocks ahead of the arithmetic
-    int req_t = SPLIT ? gemm_bid : gemm_bid + set * grid_stride, req_g = SPLIT ? set : 0, requested = 0;
+    int req_t = SPLIT ? gemm_bid : gemm_bid + set * grid_stride, req_iter = 0, req_g = first_group(0), requested = 0;
     auto request = [&]() {
       int m0, n0, b;
       while (req_t < total_tiles && req_g >= groups_of(req_t, m0, n0, b)) {
-        req_t += SPLIT ? grid_stride : 2 * grid_stride;
-        req_g = SPLIT ? set : 0;
+        req_t += SPLIT ? grid_stride : SETS * grid_stride;
+        req_g = first_group(++req_iter);
       }
       if (req_t >= total_tiles) return;
       if (lane == 0) {
@@ -674,12 +676,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tma_load_3d(smem_u32(bufs + (requested % CBUF) * 4096), &tmC.m[1], bar, n0 + req_g * 64, m0, 0);
       }
       ++requested;
-      req_g += SPLIT ? 2 : BN / 64;
+      req_g += SPLIT ? SETS : GROUPS;
     };
     if (tma_op)
       for (int i = 1; i < CBUF; ++i) request();
     for (int t = gemm_bid; t < total_tiles; t += grid_stride, ++iter) {
-      if (!SPLIT && (iter & 1) != set) continue;
+      if (!SPLIT && iter % SETS != set) continue;
       int m0, n0, b;
       const int groups = groups_of(t, m0, n0, b);
       const int acc = iter & 1;
@@ -698,7 +700,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         held = false;
       };
 #pragma unroll 1
-      for (int g = SPLIT ? set : 0; g < groups; g += SPLIT ? 2 : 1) {
+      for (int g = first_group(iter); g < groups; g += SPLIT ? SETS : 1) {
         // saved pre-activation and result take turns
         const int at = tma_aux ? (2 * blocks) % (CBUF & ~1) : blocks % CBUF;
         uint8_t* const cs = bufs + (tma_aux ? at + 1 : at) * 4096;
@@ -711,13 +713,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int half = 0; half < 2; ++half) {
           const int col0 = n0 + g * 64 + half * 32;
           if (col0 >= p.N) {
-            if (held && g + (SPLIT ? 2 : 1) >= groups) release();
+            if (held && g + (SPLIT ? SETS : 1) >= groups) release();
             break;  // uniform across the warp
           }
           uint32_t r[32];
           tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + g * 64 + half * 32, r);
           tmem_ld_wait();
-          if (half == 1 && g + (SPLIT ? 2 : 1) >= groups) release();
+          if (half == 1 && g + (SPLIT ? SETS : 1) >= groups) release();
           if constexpr (KS > 1) {
             const float4* part = reinterpret_cast<const float4*>(smem) + (g * 64 + half * 32) / 4 * OWN_ROWS + (quad % (4 / KS)) * 32 + lane;
 #pragma unroll
@@ -1431,14 +1433,10 @@ inline bool plan_epilogue(GemmParams& p, OutMaps& maps) {
   }
   return true;
 }
-// Whether the epilogue's loads and stores deserve more staging blocks per warp at the price of a stage of the operand ring: an
-// operand does (16384 x 3072 x 768 plus residual 82 us and 93), a saved pre-activation where several rounds of a short K wait for
-// its stores (the same product with GELU 91 and 99).  Elsewhere the deeper ring is worth 2 to 4 %, most where large weights come
-// from HBM.
-inline bool staged_epilogue(const GemmParams& p) {
-  if (p.operand_tma) return true;
-  return p.aux_tma && p.K < 1024 && (long long)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256) >= 2 * st::sm_count();
-}
+// Whether an operand of the epilogue arrives by TMA: it deserves more staging blocks per warp at the price of a stage of the
+// operand ring (16384 x 3072 x 768 plus residual 82 us and 93).  Elsewhere the deeper ring is worth 2 to 4 %, most where large
+// weights come from HBM.
+inline bool staged_epilogue(const GemmParams& p) { return p.operand_tma != 0; }
 
 // Tile width of a product.  A tile's main loop takes about c per K block (c2 from the 33rd on, where the start-up of the ring no
 // longer counts) and its epilogue e, which runs beside the next tile's main loop; what does not overlap is the first main loop and
@@ -1499,11 +1497,11 @@ inline TileChoice choose_tile(long long M, long long N, long long K, long long b
 }
 
 // Launch of the CTA-pair form: an even grid of at most one CTA per SM, in clusters of two.
-template <bool A_MN, bool B_MN, int STAGES>
+template <bool A_MN, bool B_MN, int STAGES, int SETS = 2>
 int launch_pair_ring(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
   constexpr int BN = 256;
-  using L = SmemLayout<BN / 2, STAGES>;
-  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, COMM_NONE, 2>;
+  using L = SmemLayout<BN / 2, STAGES, 0, SETS>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, COMM_NONE, 2, 1, SETS>;
   static bool configured[st::kMaxDevices] = {false};   // the attribute is per device
   const int dev = st::current_device();
   if (!configured[dev]) {
@@ -1513,13 +1511,23 @@ int launch_pair_ring(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMa
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.batch;
   const int pairs = st::sm_count() / 2;
   GemmComm none{};
-  ST_CUDA_CHECK(st::chained(kern, 2 * (tiles < pairs ? tiles : pairs), NUM_THREADS, L::TOTAL, stream, 2)(tmA, tmB, tmC, tmA, p, none));
+  ST_CUDA_CHECK(st::chained(kern, 2 * (tiles < pairs ? tiles : pairs), num_threads(SETS), L::TOTAL, stream, 2)(tmA, tmB, tmC, tmA, p, none));
   return ST_OK;
 }
 
 template <bool A_MN, bool B_MN>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
-  if (!A_MN && staged_epilogue(p)) return launch_pair_ring<false, B_MN, 5>(tmA, tmB, tmC, p, stream);
+  // With operands, a saved pre-activation or GELU the epilogue of a tile is longer than the main loop of a short K.  A third set of
+  // warps shares it then, with four ring stages and two staging blocks per warp where anything is staged beside the output.  us, two
+  // sets and three: 16384 x 3072 x 768 with GELU' 126 and 108, GELU and its saved input 100 and 88, GELU alone 80 and 73, plus
+  // residual 86 and 79; 8192 x 4096 x 1024 with GELU' 92 and 81; from K = 2048 on the ring matters more (4096 x 8192 x 2048 with
+  // GELU' 113 and 123), and a bare output gains nothing (58.2 and 58.2).
+  if constexpr (!A_MN) {
+    const bool staged = p.operand_tma || p.aux_tma;
+    if (p.K <= 1536 && staged) return launch_pair_ring<false, B_MN, 4, 3>(tmA, tmB, tmC, p, stream);
+    if (p.K <= 1536 && p.act == ACT_GELU) return launch_pair_ring<false, B_MN, 5, 3>(tmA, tmB, tmC, p, stream);
+    if (staged_epilogue(p)) return launch_pair_ring<false, B_MN, 5>(tmA, tmB, tmC, p, stream);
+  }
   return launch_pair_ring<A_MN, B_MN, 6>(tmA, tmB, tmC, p, stream);
 }
 
