@@ -107,13 +107,23 @@ im2col3x3_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __res
 // pixel and no division per entry, which bounded the kernel above (55 us for 256 images of 64 x 64 x 3).  The row goes
 // through shared memory, as 16-byte units in an order without bank conflicts, so that neighbouring threads store
 // neighbouring units; what is left is the store of 67 MB.
-template <int C>
+// PLANES: the images are [N][C][H][W] instead of [N][H][W][C] (a pass that only reorders them takes 7 us for the same batch), and
+// the weights [OC][9 C], if given, are padded to the matrix's width in the same launch.
+template <int C, bool PLANES>
 __global__ void __launch_bounds__(256)
-im2col3x3_image_kernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ col, long long pixels, int H, int W) {
-  chain_begin(x);
+im2col3x3_image_kernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ col, long long pixels, int H, int W,
+                       const __nv_bfloat16* __restrict__ weights, __nv_bfloat16* __restrict__ padded, int OC) {
+  chain_begin(x, weights);
   constexpr int K8 = (9 * C + 31) / 32 * 4;
   __shared__ uint4 rows[256 * K8];
   const __nv_bfloat16 zero = __float2bfloat16(0.0f);
+  if (PLANES && weights) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < OC * K8 * 8; i += gridDim.x * 256) {
+      const int oc = i / (K8 * 8), k = i - oc * (K8 * 8);
+      padded[i] = k < 9 * C ? weights[oc * (9 * C) + k] : zero;
+    }
+  }
+  const long long plane = (long long)H * W;
   for (long long base = (long long)blockIdx.x * 256; base < pixels; base += (long long)gridDim.x * 256) {
     const long long pix = base + threadIdx.x;
     uint32_t v[K8 * 4];
@@ -124,12 +134,13 @@ im2col3x3_image_kernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ 
 #pragma unroll
       for (int dh = -1; dh <= 1; ++dh) {
         const bool row_in = h + dh >= 0 && h + dh < H;
-        const __nv_bfloat16* src = x + (pix + (long long)dh * W - 1) * C;
+        const __nv_bfloat16* src = PLANES ? x + pix + pix / plane * (C - 1) * plane + (long long)dh * W - 1
+                                          : x + (pix + (long long)dh * W - 1) * C;
 #pragma unroll
         for (int e = 0; e < 3 * C; ++e) {
           const int dw = e / C - 1, k = (dh + 1) * 3 * C + e;
           const bool in = row_in && (dw < 0 ? w > 0 : dw > 0 ? w + 1 < W : true);
-          const uint32_t u = __bfloat16_as_ushort(in ? src[e] : zero);
+          const uint32_t u = __bfloat16_as_ushort(in ? src[PLANES ? e % C * plane + e / C : e] : zero);
           v[k / 2] |= (k & 1) ? u << 16 : u;
         }
       }
@@ -220,7 +231,7 @@ maxpool2_fwd8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
     uint2 a;
     a.x = arg[0] | (arg[1] << 8) | (arg[2] << 16) | (arg[3] << 24);
     a.y = arg[4] | (arg[5] << 8) | (arg[6] << 16) | (arg[7] << 24);
-    *reinterpret_cast<uint2*>(idx + (p * C + c8 * 8)) = a;
+    if (idx) *reinterpret_cast<uint2*>(idx + (p * C + c8 * 8)) = a;
   }
 }
 
@@ -248,8 +259,10 @@ __global__ void maxpool2_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bf
       if (f.y > best.y) { best.y = f.y; iy = t; }
     }
     *reinterpret_cast<__nv_bfloat162*>(y + (p * C + c2 * 2)) = __floats2bfloat162_rn(best.x, best.y);
-    idx[p * C + c2 * 2] = (unsigned char)ix;
-    idx[p * C + c2 * 2 + 1] = (unsigned char)iy;
+    if (idx) {
+      idx[p * C + c2 * 2] = (unsigned char)ix;
+      idx[p * C + c2 * 2 + 1] = (unsigned char)iy;
+    }
   }
 }
 
@@ -553,8 +566,9 @@ ST_API int st_im2col3x3_small(const void* x, void* col, int N, int H, int W, int
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_v);
   if (aligned && C >= 1 && C <= 4 && Kpad == (9 * C + 31) / 32 * 32) {
     const long long pixels = (long long)N * H * W;
-    auto kern = C == 1 ? im2col3x3_image_kernel<1> : C == 2 ? im2col3x3_image_kernel<2> : C == 3 ? im2col3x3_image_kernel<3> : im2col3x3_image_kernel<4>;
-    st::chained(kern, grid_for(pixels, 256), 256, 0, s)(static_cast<const __nv_bfloat16*>(x), static_cast<uint4*>(col), pixels, H, W);
+    auto kern = C == 1 ? im2col3x3_image_kernel<1, false> : C == 2 ? im2col3x3_image_kernel<2, false>
+                : C == 3 ? im2col3x3_image_kernel<3, false> : im2col3x3_image_kernel<4, false>;
+    st::chained(kern, grid_for(pixels, 256), 256, 0, s)(static_cast<const __nv_bfloat16*>(x), static_cast<uint4*>(col), pixels, H, W, nullptr, nullptr, 0);
   } else if (aligned && (C & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     auto kern = narrow ? im2col3x3_c8_kernel<unsigned> : im2col3x3_c8_kernel<long long>;
     st::chained(kern, grid, 256, 0, s)(static_cast<const uint4*>(x), static_cast<uint4*>(col), N, H, W, C / 8, Kpad / 8);
@@ -566,6 +580,22 @@ ST_API int st_im2col3x3_small(const void* x, void* col, int N, int H, int W, int
   return ST_OK;
 }
 
+// Columns of 3x3 patches straight from images [N][C][H][W] of 1 to 4 channels, rows of K = 9 C rounded up to 32, and the weights
+// [OC][9 C] padded to K (padded: [OC][K]).
+ST_API int st_im2col3x3_planes(const void* x, void* col, const void* weights, void* padded, int N, int H, int W, int C, int OC, void* stream_v) {
+  if (!x || !col || !weights || !padded || N <= 0 || H <= 0 || W <= 0 || OC <= 0) return st::fail(ST_ERR_INVALID, "im2col planes: bad arguments");
+  if (C < 1 || C > 4 || (reinterpret_cast<uintptr_t>(col) & 15) != 0)
+    return st::fail(ST_ERR_INVALID, "im2col planes: 1 to 4 channels and a 16-byte aligned matrix");
+  const long long pixels = (long long)N * H * W;
+  auto kern = C == 1 ? im2col3x3_image_kernel<1, true> : C == 2 ? im2col3x3_image_kernel<2, true>
+              : C == 3 ? im2col3x3_image_kernel<3, true> : im2col3x3_image_kernel<4, true>;
+  ST_CUDA_CHECK(st::chained(kern, grid_for(pixels, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_v))(
+      static_cast<const __nv_bfloat16*>(x), static_cast<uint4*>(col), pixels, H, W, static_cast<const __nv_bfloat16*>(weights),
+      static_cast<__nv_bfloat16*>(padded), OC));
+  return ST_OK;
+}
+
+// idx may be null: no backward pass follows.
 ST_API int st_maxpool2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream_v) {
   if ((H & 1) || (W & 1) || (C & 1)) return st::fail(ST_ERR_INVALID, "maxpool2: H, W and C must be even");
   if ((C & 7) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&

@@ -269,6 +269,7 @@ int st_gemm_rs(const StGemmRsArgs* a, void* stream_v);   /* csrc/comm/tp_gemm.cu
 int st_gemm_rs_arrivals_per_launch(int world, int N);   /* csrc/comm/tp_gemm.cu */
 int st_hyper_accumulate(float* g, const float* v, long long n, float curvature, float tol, float saturation, float porosity, int conformal, float scale, void* stream_v);   /* csrc/optim/optim.cu */
 int st_hyper_apply(float* w, float* g, float* g_real, int rows, int cols, float curvature, float lr, float lr_real, float tol, float saturation, float porosity, void* stream_v);   /* csrc/optim/optim.cu */
+int st_im2col3x3_planes(const void* x, void* col, const void* weights, void* padded, int N, int H, int W, int C, int OC, void* stream_v);   /* csrc/conv/conv.cu */
 int st_im2col3x3_small(const void* x, void* col, int N, int H, int W, int C, int Kpad, void* stream_v);   /* csrc/conv/conv.cu */
 int st_info_nce_fwd(const StInfoNceArgs* a, void* stream_v);   /* csrc/comm/contrastive.cu */
 int st_info_nce_grad(const float* logits, const float* row_lse, const float* coef, void* dl, void* dl_t, int R, int C, int target_offset, void* stream_v);   /* csrc/comm/contrastive.cu */

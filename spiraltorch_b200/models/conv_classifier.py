@@ -79,14 +79,22 @@ class ConvClassifier(nn.Module):
         into ``main_grad``), or the logits when ``labels`` is None.  ``layer_done(name)`` is called as
         soon as the gradient of a parameter tensor is final (hook for overlapping the all-reduce)."""
         P = self.p
-        x = images.to(self.flat_w.device, self.dtype).permute(0, 2, 3, 1).contiguous()
+        x = images.to(self.flat_w.device, self.dtype)
+        stem = C.stem_columns(x, P["conv0_0.weight"])
+        x = x.permute(0, 2, 3, 1)
+        if stem is None:
+            x = x.contiguous()
         acts, pools = [x], []
-        col = C.im2col(x, STAGES[0])                # the stem's column matrix, kept for its weight gradient
+        col = C.im2col(x, STAGES[0]) if stem is None else stem[0]      # the stem's column matrix, kept for its weight gradient
+        keep = labels is not None and backward
         for s in range(4):
             for i in range(2):
-                x = C.conv3x3(x, P[f"conv{s}_{i}.weight"], P[f"conv{s}_{i}.bias"], relu=True, col=col if s + i == 0 else None)
+                if s + i == 0 and stem is not None:
+                    x = gemm_ops.gemm(col, stem[1], bias=P["conv0_0.bias"], act="relu").view(*x.shape[:3], STAGES[0])
+                else:
+                    x = C.conv3x3(x, P[f"conv{s}_{i}.weight"], P[f"conv{s}_{i}.bias"], relu=True, col=col if s + i == 0 else None)
                 acts.append(x)
-            x, idx = C.maxpool2(x)
+            x, idx = C.maxpool2(x, argmax=keep)
             pools.append((idx, acts[-1].shape[1], acts[-1].shape[2]))
             acts.append(x)
         N, H, W, Cc = x.shape

@@ -87,6 +87,25 @@ def im2col(x: torch.Tensor, OC: int) -> Optional[torch.Tensor]:
     return col
 
 
+def stem_columns(images: torch.Tensor, w_tap: torch.Tensor):
+    """For a first convolution over ``images`` NCHW (contiguous bf16 on CUDA, at most four channels): its column matrix, as
+    :func:`im2col` builds it from NHWC, and ``w_tap`` padded to the matrix's width; None elsewhere."""
+    global launch_count
+    if not (native.use_native(images) and images.dtype == w_tap.dtype == torch.bfloat16 and images.dim() == 4 and images.shape[1] <= 4
+            and images.is_contiguous() and images.numel() > 0 and w_tap.is_contiguous()):
+        return None
+    device = native.require_cuda("stem_columns", images, w_tap)
+    N, C, H, W = images.shape
+    assert w_tap.shape[1] == 9 * C, "weights must be [OC, 9*C] (tap-major)"
+    kpad = (9 * C + 31) // 32 * 32
+    col, padded = images.new_empty((N * H * W, kpad)), images.new_empty((w_tap.shape[0], kpad))
+    native.check(native.entry("st_im2col3x3_planes", "ppppiiiiip")(images.data_ptr(), col.data_ptr(), w_tap.data_ptr(), padded.data_ptr(),
+                                                                   N, H, W, C, w_tap.shape[0], native.raw_stream(device)),
+                 "st_im2col3x3_planes")
+    launch_count += 1
+    return col, padded
+
+
 def _conv_ref(x, w_tap, bias, act, aux_in):
     N, H, W, C = x.shape
     oc = w_tap.shape[0]
@@ -148,7 +167,7 @@ def conv3x3_wgrad(dy: torch.Tensor, x: torch.Tensor, dw_tap: torch.Tensor, col: 
         return
     native.require_cuda("conv3x3_wgrad", dy, x, dw_tap)
     assert dw_tap.dtype == torch.float32 and dw_tap.is_contiguous() and dw_tap.numel() == OC * 9 * C
-    assert dy.shape[:3] == x.shape[:3] and dy.is_contiguous() and x.is_contiguous()
+    assert dy.shape[:3] == x.shape[:3] and dy.is_contiguous() and (x.is_contiguous() or col is not None)
     if not implicit_ok(N, H, W, C, OC, 64):
         if col is None:
             col = im2col(x, OC)
@@ -164,17 +183,17 @@ def conv3x3_wgrad(dy: torch.Tensor, x: torch.Tensor, dw_tap: torch.Tensor, col: 
     launch_count += 1
 
 
-def maxpool2(x: torch.Tensor):
-    """2x2 max pool on NHWC; returns ``(y, argmax)``."""
+def maxpool2(x: torch.Tensor, argmax: bool = True):
+    """2x2 max pool on NHWC; returns ``(y, argmax)``, the latter None if not asked for."""
     global launch_count
     N, H, W, C = x.shape
     if not native.use_native(x):
         xv = x.reshape(N, H // 2, 2, W // 2, 2, C).permute(0, 1, 3, 5, 2, 4).reshape(N, H // 2, W // 2, C, 4)
         y, idx = xv.float().max(-1)
-        return y.to(x.dtype), idx.to(torch.uint8)
+        return y.to(x.dtype), idx.to(torch.uint8) if argmax else None
     y = x.new_empty((N, H // 2, W // 2, C))
-    idx = x.new_empty((N, H // 2, W // 2, C), dtype=torch.uint8)
-    native.check(native.entry("st_maxpool2_fwd", "pppiiiip")(x.data_ptr(), y.data_ptr(), idx.data_ptr(), N, H, W, C,
+    idx = x.new_empty((N, H // 2, W // 2, C), dtype=torch.uint8) if argmax else None
+    native.check(native.entry("st_maxpool2_fwd", "pppiiiip")(x.data_ptr(), y.data_ptr(), native.address(idx), N, H, W, C,
                                                              native.raw_stream(x.get_device())), "st_maxpool2_fwd")
     launch_count += 1
     return y, idx

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 # rows and columns below, at and past 32-, 64-, 128- and 256-wide blocks; several tiles per CTA; few tiles with a long K, whose K
 # blocks two or four CTAs share (uneven shares, a last block that is not whole)
 SHAPES = [(1, 8, 64), (31, 72, 40), (129, 136, 200), (257, 264, 520), (300, 1000, 136), (5000, 712, 72), (100, 136, 1096),
-          (97, 520, 4104), (777, 1032, 2888), (1000, 264, 4616)]
+          (97, 520, 4104), (777, 1032, 2888), (1000, 264, 4616), (9000, 1288, 136)]
 
 
 def _error(y, ref):
