@@ -11,7 +11,6 @@ selfsup.rs:591-706) and docs/benchmarks/selfsup.md for the expected metric range
 """
 from __future__ import annotations
 
-import ctypes
 import math
 from typing import Optional
 
@@ -79,6 +78,14 @@ def _parts(encoder):
     return [list(part._parameters.values()) for part in (encoder.weights, encoder.biases, encoder.gammas, encoder.betas)]
 
 
+def _modules(root):
+    """Every module below ``root`` and itself; ``Module.modules()`` spends 20 us on names and a set."""
+    found = [root]
+    for m in found:
+        found.extend(child for child in m._modules.values() if child is not None)
+    return found
+
+
 def _accumulation_held(leaves) -> bool:
     """Whether anything outside holds an accumulation node of these leaves, and may have hooks on it that only a backward pass
     runs.  A node that nobody holds ends with its graph, so a mark on it is gone in the next one."""
@@ -111,7 +118,7 @@ def _schedulable(encoder, base: torch.Tensor, temperature: float) -> bool:
             and not base.requires_grad and 0 < base.shape[0] <= 12000 and [len(part) for part in parts] == [3, 3, 2, 2]
             and len(set(map(id, params))) == 10):
         return False
-    for m in encoder.modules():
+    for m in _modules(encoder):
         if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m.__dict__.get("forward"):
             return False
     module_hooks = torch.nn.modules.module
@@ -133,8 +140,8 @@ def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: floa
     """Loss and gradients of one batch with forward and backward written out: both views go through the encoder as one
     batch, LayerNorm and GELU are one pass in each direction, and the softmax rows of the similarities turn into their
     gradient in place.  163 launches become about 35; the similarity products stay in fp32."""
-    lib, dev, g = native.lib(), base.device, None
-    stream = native.stream_ptr(dev)
+    dev, g = base.device, None
+    stream = native.raw_stream(base.get_device())
     B, width = base.shape
     if seed is not None:
         g = torch.Generator(device=dev).manual_seed(seed)
@@ -142,8 +149,8 @@ def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: floa
     n2 = torch.randn(base.shape, generator=g, device=dev, dtype=base.dtype)
     w, b, gamma, beta = _parts(encoder)
     x = torch.empty((2 * B, width), dtype=torch.bfloat16, device=dev)
-    native.check(lib.st_contrastive_views(native.ptr(base), native.ptr(n1), native.ptr(n2), ctypes.c_float(noise), native.ptr(x),
-                                          ctypes.c_longlong(B * width), stream), "st_contrastive_views")
+    native.check(native.entry("st_contrastive_views", "pppfpqp")(base.data_ptr(), n1.data_ptr(), n2.data_ptr(), noise, x.data_ptr(),
+                                                                 B * width, stream), "st_contrastive_views")
     inputs, pre, stats = [x], [], []
     for i in range(2):
         h = gemm_ops.gemm(inputs[-1], w[i], bias=b[i])
@@ -155,19 +162,19 @@ def _scheduled_step(encoder, base: torch.Tensor, temperature: float, noise: floa
     out = z.shape[1]
     unit = torch.empty((2 * B, out), dtype=torch.float32, device=dev)
     norms = torch.empty(2 * B, dtype=torch.float32, device=dev)
-    native.check(lib.st_row_normalize(native.ptr(z), native.ptr(unit), native.ptr(norms), ctypes.c_int(2 * B), ctypes.c_int(out),
-                                      stream), "st_row_normalize")
+    native.check(native.entry("st_row_normalize", "pppiip")(z.data_ptr(), unit.data_ptr(), norms.data_ptr(), 2 * B, out, stream),
+                 "st_row_normalize")
     anchors, positives = unit[:B], unit[B:]
     sim = anchors @ positives.t()
     rows = torch.empty(B, dtype=torch.float32, device=dev)
-    native.check(lib.st_nce_rows(native.ptr(sim), native.ptr(rows), ctypes.c_int(B), ctypes.c_float(temperature), stream), "st_nce_rows")
+    native.check(native.entry("st_nce_rows", "ppifp")(sim.data_ptr(), rows.data_ptr(), B, temperature, stream), "st_nce_rows")
     loss = rows.mean()
     d_unit = torch.empty_like(unit)
     torch.mm(sim, positives, out=d_unit[:B])
     torch.mm(sim.t(), anchors, out=d_unit[B:])
     d = torch.empty_like(z)
-    native.check(lib.st_row_normalize_bwd(native.ptr(d_unit), native.ptr(unit), native.ptr(norms), native.ptr(d), ctypes.c_int(2 * B),
-                                          ctypes.c_int(out), stream), "st_row_normalize_bwd")
+    native.check(native.entry("st_row_normalize_bwd", "ppppiip")(d_unit.data_ptr(), unit.data_ptr(), norms.data_ptr(), d.data_ptr(), 2 * B,
+                                                                 out, stream), "st_row_normalize_bwd")
     # vector gradients: fp32 sums side by side, rounded to bf16 in one launch
     vectors = [*b, *gamma, *beta]
     flat = torch.zeros(sum(v.numel() for v in vectors), dtype=torch.float32, device=dev)

@@ -41,24 +41,22 @@ def _most() -> int:
 def _run(op: int, src, dst, value: float) -> Optional[int]:
     """Index of the first tensor of ``src`` with a value that is not finite, or None."""
     global launch_count
-    lib, stream = native.lib(), torch.cuda.current_stream()
+    stream = torch.cuda.current_stream()
+    launch, blocks_of = native.entry("st_multi", "iipppfpp"), native.entry("st_multi_blocks", "q")
     first = None
     for at in range(0, len(src), _most()):
         s = src[at:at + _most()]
         n = len(s)
         counts = [t.numel() for t in s]
-        blocks = lib.st_multi_blocks(ctypes.c_longlong(max(counts)))
+        blocks = blocks_of(max(counts))
         bad = torch.empty(n * blocks, dtype=torch.int32, pin_memory=True)
         ptrs = (ctypes.c_void_p * n)(*[t.data_ptr() for t in s])
         outs = None if dst is None else (ctypes.c_void_p * n)(*[t.data_ptr() for t in dst[at:at + _most()]])
-        native.check(lib.st_multi(ctypes.c_int(op), ctypes.c_int(n), ptrs, outs, (ctypes.c_longlong * n)(*counts),
-                                  ctypes.c_float(value), ctypes.c_void_p(bad.data_ptr()),
-                                  ctypes.c_void_p(stream.cuda_stream)), "st_multi")
+        native.check(launch(op, n, ptrs, outs, (ctypes.c_longlong * n)(*counts), value, bad.data_ptr(), stream.cuda_stream), "st_multi")
         launch_count += 1
         stream.synchronize()
-        hits = bad.nonzero()
-        if first is None and hits.numel():
-            first = at + int(hits[0]) // blocks
+        if first is None and bad.any():
+            first = at + int(bad.nonzero()[0]) // blocks
     return first
 
 
@@ -110,12 +108,12 @@ def descend_(values: Sequence[torch.Tensor], grads: Sequence[torch.Tensor], lr: 
 def to_bf16(tensors: Sequence[torch.Tensor]):
     """bf16 copies of dense 16-byte aligned fp32 CUDA tensors."""
     global launch_count
-    out = [torch.empty(t.shape, dtype=torch.bfloat16, device=t.device) for t in tensors]
+    device = native.require_cuda("to_bf16", *tensors)
+    out = [torch.empty_like(t, dtype=torch.bfloat16, memory_format=torch.contiguous_format) for t in tensors]
     n = len(out)
-    native.require_cuda("to_bf16", *tensors)
-    native.check(native.lib().st_multi_cast_bf16(
-        ctypes.c_int(n), (ctypes.c_void_p * n)(*[t.data_ptr() for t in tensors]), (ctypes.c_void_p * n)(*[t.data_ptr() for t in out]),
-        (ctypes.c_longlong * n)(*[t.numel() for t in out]), native.stream_ptr(out[0].device)), "st_multi_cast_bf16")
+    native.check(native.entry("st_multi_cast_bf16", "ipppp")(
+        n, (ctypes.c_void_p * n)(*[t.data_ptr() for t in tensors]), (ctypes.c_void_p * n)(*[t.data_ptr() for t in out]),
+        (ctypes.c_longlong * n)(*[t.numel() for t in out]), native.raw_stream(device)), "st_multi_cast_bf16")
     launch_count += 1
     return out
 
@@ -123,12 +121,13 @@ def to_bf16(tensors: Sequence[torch.Tensor]):
 def mse_forward(p: torch.Tensor, t: torch.Tensor):
     """``(mean((p - t)^2) of shape (1, 1), all inputs are finite)``."""
     global launch_count
+    native.require_cuda("mse_forward", p, t)
     lib, stream, n = native.lib(), torch.cuda.current_stream(), p.numel()
-    value = torch.empty((1, 1), dtype=torch.float32, device=p.device)
-    work = torch.empty(lib.st_mse_workspace(), dtype=torch.float32, device=p.device)
-    bad = torch.empty(lib.st_mse_blocks(ctypes.c_longlong(n)), dtype=torch.int32, pin_memory=True)
-    native.check(lib.st_mse_forward(native.ptr(p), native.ptr(t), ctypes.c_longlong(n), native.ptr(value), native.ptr(work),
-                                    ctypes.c_void_p(bad.data_ptr()), ctypes.c_void_p(stream.cuda_stream)), "st_mse_forward")
+    value = p.new_empty((1, 1), dtype=torch.float32)
+    work = p.new_empty(lib.st_mse_workspace(), dtype=torch.float32)
+    bad = torch.empty(native.entry("st_mse_blocks", "q")(n), dtype=torch.int32, pin_memory=True)
+    native.check(native.entry("st_mse_forward", "ppqpppp")(p.data_ptr(), t.data_ptr(), n, value.data_ptr(), work.data_ptr(),
+                                                           bad.data_ptr(), stream.cuda_stream), "st_mse_forward")
     launch_count += 1
     stream.synchronize()
     return value, not bool(bad.any())
@@ -137,11 +136,12 @@ def mse_forward(p: torch.Tensor, t: torch.Tensor):
 def mse_backward(p: torch.Tensor, t: torch.Tensor):
     """``(2 (p - t) / n, all inputs are finite)``."""
     global launch_count
-    lib, stream, n = native.lib(), torch.cuda.current_stream(), p.numel()
+    native.require_cuda("mse_backward", p, t)
+    stream, n = torch.cuda.current_stream(), p.numel()
     g = torch.empty_like(p)
-    bad = torch.empty(lib.st_mse_blocks(ctypes.c_longlong(n)), dtype=torch.int32, pin_memory=True)
-    native.check(lib.st_mse_backward(native.ptr(p), native.ptr(t), ctypes.c_longlong(n), native.ptr(g),
-                                     ctypes.c_void_p(bad.data_ptr()), ctypes.c_void_p(stream.cuda_stream)), "st_mse_backward")
+    bad = torch.empty(native.entry("st_mse_blocks", "q")(n), dtype=torch.int32, pin_memory=True)
+    native.check(native.entry("st_mse_backward", "ppqppp")(p.data_ptr(), t.data_ptr(), n, g.data_ptr(), bad.data_ptr(),
+                                                           stream.cuda_stream), "st_mse_backward")
     launch_count += 1
     stream.synchronize()
     return g, not bool(bad.any())
