@@ -851,7 +851,7 @@ struct StAttnBwdArgs {
 };
 
 namespace {
-int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_ws, void* stream_v) {
+int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_ws, float* dq_sums, void* stream_v) {
   if (!a || !a->Q || !a->K || !a->V || !a->O || !a->dO || !a->lse || !a->delta ||
       !a->dQ || !a->dK || !a->dV)
     return st::fail(ST_ERR_INVALID, "attn_bwd: null pointer");
@@ -871,13 +871,13 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
   const bool biased = a->key_bias || a->attn_bias || a->lengths;
   const bool keyb = biased && !a->attn_bias && bias_ws;
   const int n_kv = (a->Sk + BLK - 1) / BLK;
-  const bool one = a->dQ_acc && a->D == 64 && n_kv <= kOnePassTiles && (!biased || keyb);
-  if (one && (reinterpret_cast<uintptr_t>(a->dQ_acc) & 15)) return st::fail(ST_ERR_INVALID, "attn_bwd: dQ_acc must be 16-byte aligned");
+  const bool one = dq_sums && a->D == 64 && n_kv <= kOnePassTiles && (!biased || keyb);
+  if (one && (reinterpret_cast<uintptr_t>(dq_sums) & 15)) return st::fail(ST_ERR_INVALID, "attn_bwd: the dQ workspace must be 16-byte aligned");
   const bool in_place = one && grad_f32 && n_kv <= 2;
-  float* const acc = !one ? nullptr : in_place ? static_cast<float*>(a->dQ) : a->dQ_acc;
+  float* const acc = !one ? nullptr : in_place ? static_cast<float*>(a->dQ) : dq_sums;
   const long long acc_sb = in_place ? a->dq_sb : (long long)a->Sq * a->H * a->D, acc_ss = in_place ? a->dq_ss : (long long)a->H * a->D,
                   acc_sh = in_place ? a->dq_sh : a->D, acc_buffer = (long long)a->B * a->Sq * a->H * a->D;
-  unsigned* const queue = one ? reinterpret_cast<unsigned*>(a->dQ_acc + acc_buffer * ((n_kv + 1) / 2)) : nullptr;
+  unsigned* const queue = one ? reinterpret_cast<unsigned*>(dq_sums + acc_buffer * ((n_kv + 1) / 2)) : nullptr;
 
   {
     const long long rows = (long long)a->B * a->Sq * a->H;
@@ -972,19 +972,25 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
 }
 }  // namespace
 
-// Floats of workspace (16-byte aligned) for the one-pass form; 0 where it does not apply.
-ST_API long long st_attn_bwd_workspace(int B, int H, int Sq, int Sk, int D) {
-  const int n_kv = (Sk + BLK - 1) / BLK;
-  return D == 64 && n_kv <= kOnePassTiles ? (long long)B * Sq * H * D * ((n_kv + 1) / 2) + 4 : 0;
-}
-
-// delta: fp32 [B,H,Sq] workspace.  dQ_acc: null, or st_attn_bwd_workspace floats for the one-pass form (ignored with a bias per
-// query and key, and with a key bias or lengths without their workspace).
-ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) { return attn_bwd_run(a, nullptr, 0, nullptr, stream_v); }
+// delta: fp32 [B,H,Sq] workspace.  dQ_acc is unused (kept in the argument block for ABI stability).
+ST_API int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v) { return attn_bwd_run(a, nullptr, 0, nullptr, nullptr, stream_v); }
 
 // The same with, all optional: the output's gradient in fp32 (dO32, contiguous [B, Sq, H, D]; a->dO then receives its bf16
 // form), gradients in fp32 (grad_f32: dQ, dK, dV are float*, strides in elements), and a workspace of
 // st_attn_bias_workspace floats for a key bias or lengths.
 ST_API int st_attn_bwd_f32(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, void* stream_v) {
-  return attn_bwd_run(a, dO32, grad_f32, bias_workspace, stream_v);
+  return attn_bwd_run(a, dO32, grad_f32, bias_workspace, nullptr, stream_v);
+}
+
+// Floats of workspace (16-byte aligned) for the sums of dQ in the one-pass form; 0 where it does not apply.
+ST_API long long st_attn_bwd_workspace(int B, int H, int Sq, int Sk, int D) {
+  const int n_kv = (Sk + BLK - 1) / BLK;
+  return D == 64 && n_kv <= kOnePassTiles ? (long long)B * Sq * H * D * ((n_kv + 1) / 2) + 4 : 0;
+}
+
+// st_attn_bwd_f32 in one pass over the tile pairs where dq_workspace (st_attn_bwd_workspace floats) is given; in two with null, with
+// a bias per query and key, and with a key bias or lengths without their workspace.
+ST_API int st_attn_bwd_one_pass(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, float* dq_workspace,
+                                void* stream_v) {
+  return attn_bwd_run(a, dO32, grad_f32, bias_workspace, dq_workspace, stream_v);
 }

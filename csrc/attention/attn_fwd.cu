@@ -979,8 +979,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }  // namespace
 
 namespace st {
-// 4-D tensor map over a [B, S, H, D] bf16 view with arbitrary B/S/H strides (D contiguous):
-// dims {D, H, S, B}, box {64, 1, rows, 1}.
 // Boxes of 32 rows and 64 bytes of an output or a gradient, fp32 or bf16; strides in elements
 bool encode_out_tmap(CUtensorMap* out, const void* base, bool f32, int B, int S, int H, int D, long long sb, long long ss, long long sh) {
   const uint64_t es = f32 ? 4 : 2;
@@ -991,6 +989,8 @@ bool encode_out_tmap(CUtensorMap* out, const void* base, bool f32, int B, int S,
                      CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
+// 4-D tensor map over a [B, S, H, D] bf16 view with arbitrary B/S/H strides (D contiguous):
+// dims {D, H, S, B}, box {64, 1, rows, 1}.
 bool encode_bshd_tmap(CUtensorMap* out, const void* base, int B, int S, int H, int D,
                       long long sb, long long ss, long long sh, int box_rows) {
   uint64_t dims[4] = {(uint64_t)D, (uint64_t)H, (uint64_t)S, (uint64_t)B};

@@ -233,7 +233,7 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
     delta = torch.empty((B, H, Sq), dtype=torch.float32, device=dev)
     a = _BwdArgs()
     a.Q, a.K, a.V, a.O, a.dO = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr()
-    a.lse, a.delta, a.dQ_acc = lse.data_ptr(), delta.data_ptr(), None
+    a.lse, a.delta, a.dQ_acc = lse.data_ptr(), delta.data_ptr(), None      # dQ accumulates elsewhere
     a.dQ, a.dK, a.dV = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
     for pre, t in (("q", q), ("k", k), ("v", v), ("o", o), ("do", do), ("dq", dq), ("dk", dk), ("dv", dv)):
         setattr(a, pre + "_sb", t.stride(0))
@@ -248,19 +248,21 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
     for t, n in ((dq, "dq"), (dk, "dk"), (dv, "dv")):
         if t.dtype != (torch.float32 if f32 else torch.bfloat16) or t.stride(-1) != 1:
             raise ValueError(f"attention_backward: {n} must be a view with contiguous D, and all gradients bf16 or all fp32")
+    sums = None
     if D == 64 and attn_bias is None:      # one pass over the tile pairs instead of two, where the kernel takes it
         lib = native.lib()
         lib.st_attn_bwd_workspace.restype = ctypes.c_longlong
         room = lib.st_attn_bwd_workspace(*(ctypes.c_int(n) for n in (B, H, Sq, Sk, D)))
         if room:
-            acc = torch.empty(room, dtype=torch.float32, device=dev)
-            keep.append(acc)
-            a.dQ_acc = acc.data_ptr()
+            try:
+                sums = torch.empty(room, dtype=torch.float32, device=dev)
+            except torch.cuda.OutOfMemoryError:      # two passes need no such room
+                pass
     if do32 is not None:
         assert do32.shape == do.shape and do32.dtype == torch.float32 and do32.is_contiguous() and do32.device == dev
         assert do32.data_ptr() % 16 == 0
-    native.check(native.lib().st_attn_bwd_f32(ctypes.byref(a), native.ptr(do32), ctypes.c_int(int(f32)), native.ptr(work),
-                                              native.stream_ptr(dev)), "st_attn_bwd")
+    native.check(native.lib().st_attn_bwd_one_pass(ctypes.byref(a), native.ptr(do32), ctypes.c_int(int(f32)), native.ptr(work),
+                                                   native.ptr(sums), native.stream_ptr(dev)), "st_attn_bwd")
     launch_count += 3
     return dq, dk, dv
 

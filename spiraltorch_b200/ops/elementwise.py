@@ -52,9 +52,9 @@ def rope_(x: torch.Tensor, heads: int, head_dim: int, seq_len: int, base: float 
         view = x[:, : heads * head_dim].reshape(T, heads, head_dim)
         view.copy_(rope_reference(view, cos, sin, seq_len, backward))
         return x
-    ld, unit = x.stride()
-    assert x.dtype == torch.bfloat16 and unit == 1
-    st = native.entry("st_rope", "pppqiiqiiip")(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, heads, head_dim, ld, seq_len, 0,
+    strides = x.stride()
+    assert x.dtype == torch.bfloat16 and strides[-1] == 1
+    st = native.entry("st_rope", "pppqiiqiiip")(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, heads, head_dim, strides[0], seq_len, 0,
                                                 backward, native.raw_stream(x.get_device()))
     native.check(st, "st_rope")
     launch_count += 1
