@@ -443,9 +443,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // With a key bias or valid lengths (KEYB) the logits take them from a padded fp32 row per batch entry (and head), already
 // in the log2 domain and minus infinity wherever a key is masked: 16-byte loads that all lanes share, one packed multiply-
 // add per two logits and no comparisons, except in the tile that holds the length, where a padded key may have given a logit
-// that is not finite and is replaced by comparison.  The single-tile kernel loaded and compared per element: 244 us for 96 contexts of
-// up to 1000 keys, D = 64, where this form takes 65 (93 with the
-// bias read from global memory where it is used and the outputs stored by their lanes).  A bias per (query, key) stays with the single-tile kernel.
+// that is not finite and is replaced by comparison.  The single-tile kernel loaded and compared per element: 244 us for 96
+// contexts of up to 1000 keys, D = 64, where this form takes 65 (93 with the bias read from global memory where it is used and the
+// outputs stored by their lanes).  A bias per (query, key) stays with the single-tile kernel.
 // ------------------------------------------------------------------------------------------------------------------
 // Phase clocks of CTA 0 (SM cycles summed over the launch), written when tracing is switched on:
 //   softmax warp 0:  0 steps, 1 wait for S, 2 S load, 3 maximum / rescale, 4 first half of P, 5 second half of P,
