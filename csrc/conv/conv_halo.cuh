@@ -67,7 +67,6 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     tma_prefetch_desc(&tmX);
     tma_prefetch_desc(&tmW);
   }
-  if (threadIdx.x < BN) s_bias[threadIdx.x] = p.bias && static_cast<int>(threadIdx.x) < p.OC ? __bfloat162float(p.bias[threadIdx.x]) : 0.0f;
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
     tmem_relinquish();
@@ -155,6 +154,10 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     // ------------------------------- epilogue: one warp per 32 lanes and half -------------------------------
     const int quad = warp & 3, half = (warp - 2) >> 2;
     uint8_t* cs = cstage + (warp - 2) * 4096;
+    // only these warps read the bias; it is fetched behind chain_begin(), as the kernel before this one may have written it
+    const int oc = threadIdx.x - 64;
+    if (oc < BN) s_bias[oc] = p.bias && oc < p.OC ? __bfloat162float(p.bias[oc]) : 0.0f;
+    asm volatile("bar.sync 1, %0;" ::"n"(kHaloThreads - 64) : "memory");
     int iter = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x, ++iter) {

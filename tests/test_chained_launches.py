@@ -1,0 +1,78 @@
+"""Kernels whose start-up overlaps the end of the kernel before them: none touches global memory before it has waited for that
+kernel (read from the sources), and what one kernel writes the next one reads, whatever stands between them in the stream."""
+import re
+from pathlib import Path
+
+import pytest
+import torch
+
+from spiraltorch_b200.ops import conv as C
+from spiraltorch_b200.ops import gemm as G
+from spiraltorch_b200.ops import native
+
+CSRC = Path(__file__).resolve().parents[1] / "csrc"
+
+
+def _block(text, start):
+    """The text between the brace at or after ``start`` and its partner."""
+    at, depth = text.index("{", start), 0
+    for i in range(at, len(text)):
+        depth += (text[i] == "{") - (text[i] == "}")
+        if depth == 0:
+            return text[at + 1:i]
+    raise AssertionError("unbalanced braces")
+
+
+def _chained_kernels():
+    """(file and name, parameters, body) of every kernel that waits for the one before it."""
+    found = []
+    for path in sorted(CSRC.rglob("*.cu*")):
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", path.read_text(), flags=re.S)
+        for m in re.finditer(r"__global__", text):
+            body = _block(text, m.start())
+            if "chain_begin(" in body:
+                head = text[m.start():text.index("{", m.start())]
+                name = [n for n in re.findall(r"(\w+)\s*\(", head) if n not in ("__launch_bounds__", "num_threads")][0]
+                found.append((f"{path.name}:{name}", head, body))
+    return found
+
+
+def _without_lambdas(code):
+    """What runs where it stands: the bodies of lambdas are left out."""
+    while (m := re.search(r"=\s*\[&\]", code)) is not None:
+        code = code[:m.start()] + code[m.start():].replace(_block(code, m.start()), "", 1).replace("[&]", "[]", 1)
+    return code
+
+
+def test_nothing_reads_global_memory_before_the_wait():
+    kernels = _chained_kernels()
+    assert len(kernels) > 40
+    early = []
+    for name, head, body in kernels:
+        before = _without_lambdas(body[:body.index("chain_begin(")])
+        pointers = re.findall(r"\*\s*(?:__restrict__\s+)?(\w+)\s*[,)]", head)
+        access = r"\b(?:p|cm)\.\w+\s*\[|__ldg|[=(,?:]\s*\*\s*(?:p|cm)\.\w+|tma_load|bulk_load|atomic\w+\(" + "".join(rf"|\b{x}\s*\[" for x in pointers)
+        if (hit := re.search(access, before)) is not None:
+            early.append((name, hit.group(0)))
+    assert not early
+
+
+@pytest.mark.gpu
+def test_convolution_reads_the_bias_that_was_just_written():
+    """64 channels at 64 x 64 run the shared-row kernel; its bias is the last row of a product launched right before it."""
+    torch.manual_seed(0)
+    x = torch.randn(16, 64, 64, 64, device="cuda").bfloat16()
+    w = (torch.randn(64, 9 * 64, device="cuda") / 24).bfloat16()
+    b = torch.randn(64, 4096, device="cuda").bfloat16()
+    products = [torch.randn(4096, 4096, device="cuda").bfloat16() for _ in range(6)]
+    out = torch.zeros(4096, 64, device="cuda", dtype=torch.bfloat16)
+    got = []
+    for a in products:
+        G.gemm(a, b, out=out)
+        got.append(C.conv3x3(x, w, out[-1]))
+    torch.cuda.synchronize()
+    for a, y in zip(products, got):
+        G.gemm(a, b, out=out)
+        torch.cuda.synchronize()
+        assert torch.equal(y, C.conv3x3(x, w, out[-1]))
+    native.raise_on_device_error()
