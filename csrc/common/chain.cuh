@@ -21,6 +21,9 @@ __device__ __forceinline__ void chain_begin(P&... pointers) {
 // last ones drain, and chain_begin(), which every such kernel calls before it touches global memory, waits for its completion.
 // Between two kernels of a forward pass this saves the 1 to 2 us of launch latency and ramp-up.  A captured launch is an
 // ordinary one: a graph's edges to copies, fills and other streams' nodes only exist in that form.
+// in_order: the launch of such a kernel that leaves SMs to another stream.  Early blocks would hold SMs of that stream for as long
+// as the kernel before them runs, beyond the number left to this one: of two products of 40 blocks, 330 us each, the second's
+// blocks were there 50 to 80 us after the first's.
 template <typename... P>
 struct ChainedLaunch {
   void (*kernel)(P...);
@@ -28,10 +31,11 @@ struct ChainedLaunch {
   size_t smem;
   cudaStream_t stream;
   int cluster;
+  bool early;
   template <typename... A>
   cudaError_t operator()(A&&... args) const {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
-    const bool chain = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    const bool chain = early && cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
     cudaLaunchAttribute attr[2]{};
     unsigned n = 0;
     if (chain) {
@@ -56,7 +60,11 @@ struct ChainedLaunch {
 };
 template <typename... P>
 ChainedLaunch<P...> chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster = 1) {
-  return {kernel, grid, block, smem, stream, cluster};
+  return {kernel, grid, block, smem, stream, cluster, true};
+}
+template <typename... P>
+ChainedLaunch<P...> in_order(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
+  return {kernel, grid, block, smem, stream, 1, false};
 }
 
 }  // namespace st

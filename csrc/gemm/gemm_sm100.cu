@@ -39,7 +39,9 @@ int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps
   int grid = tiles < st::sm_count() ? tiles : st::sm_count();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   GemmComm none{};
-  ST_CUDA_CHECK(st::chained(kern, grid, NUM_THREADS, L::TOTAL, stream)(tmA, tmB, tmC, tmA, p, none));
+  // a limited grid runs beside another stream's kernels and takes no more SMs than its limit
+  const auto launch = max_ctas > 0 ? st::in_order(kern, grid, NUM_THREADS, L::TOTAL, stream) : st::chained(kern, grid, NUM_THREADS, L::TOTAL, stream);
+  ST_CUDA_CHECK(launch(tmA, tmB, tmC, tmA, p, none));
   return ST_OK;
 }
 

@@ -76,3 +76,23 @@ def test_convolution_reads_the_bias_that_was_just_written():
         torch.cuda.synchronize()
         assert torch.equal(y, C.conv3x3(x, w, out[-1]))
     native.raise_on_device_error()
+
+
+@pytest.mark.gpu
+def test_products_with_a_block_limit_wait_for_their_turn():
+    """A limited product leaves the other SMs to another stream; the next one's blocks must not sit beside it while it runs."""
+    a, b = (torch.randn(4096, 4096, device="cuda").bfloat16() for _ in range(2))
+    outs = [torch.zeros(4096, 4096, device="cuda") for _ in range(2)]
+
+    def products():
+        for out in outs:
+            G.gemm(a, b, a_mn=True, b_mn=True, out=out, accumulate=True, max_ctas=40)
+        torch.cuda.synchronize()
+
+    products()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as trace:
+        products()
+    times = sorted((e.time_range.start, e.time_range.end) for e in trace.events() if "gemm_bf16_kernel" in e.name)
+    if len(times) != 2:
+        pytest.skip("kernels are not traced here")
+    assert times[1][0] >= times[0][1]
