@@ -739,7 +739,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 __device__ __forceinline__ int dq_buffers(int s, int n_kv, int causal, const int* lengths, int b) {
   const int tile = s / BLK;
   if (lengths) {
-    n_kv = min(n_kv, (max(0, lengths[b]) + BLK - 1) / BLK);
+    n_kv = (max(0, min(n_kv * BLK, lengths[b])) + BLK - 1) / BLK;      // clamped first: a length may be the largest int
     if (tile >= n_kv) return 0;
   }
   return ((causal ? min(n_kv, tile + 1) : n_kv) + 1) >> 1;
