@@ -79,10 +79,13 @@ def _parts(encoder):
 
 
 def _modules(root):
-    """Every module below ``root`` and itself; ``Module.modules()`` spends 20 us on names and a set."""
-    found = [root]
+    """Every module below ``root`` and itself, once; ``Module.modules()`` spends 20 us on names."""
+    found, seen = [root], {id(root)}
     for m in found:
-        found.extend(child for child in m._modules.values() if child is not None)
+        for child in m._modules.values():
+            if child is not None and id(child) not in seen:
+                seen.add(id(child))
+                found.append(child)
     return found
 
 
