@@ -55,7 +55,7 @@ def rope_(x: torch.Tensor, heads: int, head_dim: int, seq_len: int, base: float 
     strides = x.stride()
     assert x.dtype == torch.bfloat16 and strides[-1] == 1
     st = native.entry("st_rope", "pppqiiqiiip")(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, heads, head_dim, strides[0], seq_len, 0,
-                                                backward, native.raw_stream(x.get_device()))
+                                                int(backward), native.raw_stream(x.get_device()))
     native.check(st, "st_rope")
     launch_count += 1
     return x

@@ -252,7 +252,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             k_part, parts = K // n, n
             strides = (k_part * stride_a[0], k_part * stride_b[0], M * N if in_parts else 0)
     args = _pack_args(a.data_ptr(), b.data_ptr(), target.data_ptr(), *operands[:4], stride_a[-2], stride_b[-2], ldc, *operands[4:],
-                      *strides, M, N, k_part, parts, a_mn, b_mn, fp32, acc, act_id, alpha, max_ctas)
+                      *strides, M, N, k_part, parts, int(a_mn), int(b_mn), fp32, acc, act_id, float(alpha), max_ctas)
     status = lib.st_gemm_bf16(args, ctypes.c_void_p(stream))
     if status:
         native.check(status, "st_gemm_bf16")

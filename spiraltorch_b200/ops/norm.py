@@ -88,7 +88,7 @@ def norm_forward(x2: torch.Tensor, gamma, beta, eps: float, rms: bool, residual=
     mean = x2.new_empty(rows, dtype=torch.float32)
     rstd = torch.empty_like(mean)
     status = _form("st_norm_fwd", "ippppppppiifp", x2, rounded)(
-        rms, x2.data_ptr(), native.address(residual), native.address(gamma), native.address(beta), y.data_ptr(), native.address(s),
+        int(rms), x2.data_ptr(), native.address(residual), native.address(gamma), native.address(beta), y.data_ptr(), native.address(s),
         mean.data_ptr(), rstd.data_ptr(), rows, d, eps, native.raw_stream(device))
     if status:
         native.check(status, "st_norm_fwd")
@@ -124,8 +124,8 @@ def norm_backward(dy2, x2, gamma, mean, rstd, rms: bool, dgamma: torch.Tensor,
     dx = torch.empty_like(x2) if out is None else out
     scratch = _scratch(native.lib(), x2)
     status = _form("st_norm_bwd", "ipppppppppipiip", x2, rounded)(
-        rms, dy2.data_ptr(), x2.data_ptr(), gamma.data_ptr(), native.address(mean), rstd.data_ptr(), native.address(dres),
-        dx.data_ptr(), dgamma.data_ptr(), native.address(dbeta), accumulate, scratch.data_ptr(), rows, d, native.raw_stream(device))
+        int(rms), dy2.data_ptr(), x2.data_ptr(), gamma.data_ptr(), native.address(mean), rstd.data_ptr(), native.address(dres),
+        dx.data_ptr(), dgamma.data_ptr(), native.address(dbeta), int(accumulate), scratch.data_ptr(), rows, d, native.raw_stream(device))
     if status:
         native.check(status, "st_norm_bwd")
     launch_count += 2
