@@ -31,13 +31,13 @@ enum MultiOp : int { MULTI_CHECK = 0, MULTI_DIV = 1, MULTI_STEP = 2 };
 template <int OP>
 __global__ void __launch_bounds__(kMultiThreads)
 multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict__ bad, int slots) {
-  st::chain_begin();
   int which = 0;
 #pragma unroll
   for (int step = 32; step > 0; step >>= 1)
     if (which + step < kMultiMax && t.first[which + step] <= static_cast<int>(blockIdx.x)) which += step;
   const int block = blockIdx.x - t.first[which], blocks = t.first[which + 1] - t.first[which];
-  const float* __restrict__ src = t.src[which];
+  const float* __restrict__ src = t.src[which];      // the table is part of the arguments: no access to global memory yet
+  st::chain_begin(src);
   float* dst = t.dst[which];
   __nv_bfloat16* half = OP == MULTI_STEP ? t.half[which] : nullptr;
   const long long n = t.n[which], stride = (long long)blocks * kMultiThreads;
@@ -71,8 +71,8 @@ multi_kernel(const __grid_constant__ MultiTable t, float value, int* __restrict_
 // dst (bf16) = src (fp32) for a list of tensors, eight elements per thread and step; the tail element by element
 __global__ void __launch_bounds__(kMultiThreads)
 multi_cast_kernel(const __grid_constant__ MultiTable t) {
-  st::chain_begin();
   const float* __restrict__ src = t.src[blockIdx.y];
+  st::chain_begin(src);
   __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(t.dst[blockIdx.y]);
   const long long n = t.n[blockIdx.y], n8 = n / 8;
   for (long long i = blockIdx.x * (long long)kMultiThreads + threadIdx.x; i < n8; i += (long long)gridDim.x * kMultiThreads) {

@@ -57,6 +57,18 @@ def test_nothing_reads_global_memory_before_the_wait():
     assert not early
 
 
+def test_addresses_of_constant_memory_depend_on_the_wait():
+    """Loads through ``const __restrict__`` pointers may be moved across the wait unless their addresses depend on it; for
+    pointers among the parameters and for local ones."""
+    free = []
+    for name, head, body in _chained_kernels():
+        at = body.index("chain_begin(")
+        behind = body[at + len("chain_begin("):body.index(")", at)].split(",")
+        constant = re.findall(r"\bconst\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", head + body)
+        free += [(name, x) for x in constant if x not in [b.strip() for b in behind]]
+    assert not free
+
+
 @pytest.mark.gpu
 def test_convolution_reads_the_bias_that_was_just_written():
     """64 channels at 64 x 64 run the shared-row kernel; its bias is the last row of a product launched right before it."""
