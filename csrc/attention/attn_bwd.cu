@@ -50,6 +50,7 @@ constexpr int NUM_THREADS = EW_THREADS + 64;       // + TMA producer warp + MMA 
 constexpr int MODE_KV = 0, MODE_Q = 1, MODE_ONE = 2;
 // KV tiles up to which the one-pass form is taken: its sums of dQ take half as many times the size of dQ in fp32.
 constexpr int kOnePassTiles = 8;
+constexpr int kQueueFloats = 32;      // the workspace starts with the work queue, the sums follow on the next 128-byte line
 // Biases: none; a bias per (query, key) among them, read and compared per element; key bias and length only, as padded rows
 // in the log2 domain (minus infinity where masked): 16-byte loads, no comparisons.
 constexpr int BIAS_NONE = 0, BIAS_FULL = 1, BIAS_KEYS = 2;
@@ -874,10 +875,10 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
   const bool one = dq_sums && a->D == 64 && n_kv <= kOnePassTiles && (!biased || keyb);
   if (one && (reinterpret_cast<uintptr_t>(dq_sums) & 15)) return st::fail(ST_ERR_INVALID, "attn_bwd: the dQ workspace must be 16-byte aligned");
   const bool in_place = one && grad_f32 && n_kv <= 2;
-  float* const acc = !one ? nullptr : in_place ? static_cast<float*>(a->dQ) : dq_sums;
+  float* const acc = !one ? nullptr : in_place ? static_cast<float*>(a->dQ) : dq_sums + kQueueFloats;
   const long long acc_sb = in_place ? a->dq_sb : (long long)a->Sq * a->H * a->D, acc_ss = in_place ? a->dq_ss : (long long)a->H * a->D,
                   acc_sh = in_place ? a->dq_sh : a->D, acc_buffer = (long long)a->B * a->Sq * a->H * a->D;
-  unsigned* const queue = one ? reinterpret_cast<unsigned*>(dq_sums + acc_buffer * ((n_kv + 1) / 2)) : nullptr;
+  unsigned* const queue = one ? reinterpret_cast<unsigned*>(dq_sums) : nullptr;
 
   {
     const long long rows = (long long)a->B * a->Sq * a->H;
@@ -982,13 +983,18 @@ ST_API int st_attn_bwd_f32(const StAttnBwdArgs* a, const float* dO32, int grad_f
   return attn_bwd_run(a, dO32, grad_f32, bias_workspace, nullptr, stream_v);
 }
 
-// Floats of workspace (16-byte aligned) for the sums of dQ in the one-pass form; 0 where it does not apply.
+// Floats of workspace (16-byte aligned) of the one-pass form, whatever the gradients' type; 0 where it does not apply.
 ST_API long long st_attn_bwd_workspace(int B, int H, int Sq, int Sk, int D) {
   const int n_kv = (Sk + BLK - 1) / BLK;
-  return D == 64 && n_kv <= kOnePassTiles ? (long long)B * Sq * H * D * ((n_kv + 1) / 2) + 4 : 0;
+  return D == 64 && n_kv <= kOnePassTiles ? (long long)B * Sq * H * D * ((n_kv + 1) / 2) + kQueueFloats : 0;
 }
 
-// st_attn_bwd_f32 in one pass over the tile pairs where dq_workspace (st_attn_bwd_workspace floats) is given; in two with null, with
+// What fp32 gradients need of it: with one sum, which is dQ itself, only the work queue.
+ST_API long long st_attn_bwd_workspace_f32(int B, int H, int Sq, int Sk, int D) {
+  return D == 64 && Sk <= 2 * BLK ? kQueueFloats : st_attn_bwd_workspace(B, H, Sq, Sk, D);
+}
+
+// st_attn_bwd_f32 in one pass over the tile pairs where dq_workspace (as above) is given; in two with null, with
 // a bias per query and key, and with a key bias or lengths without their workspace.
 ST_API int st_attn_bwd_one_pass(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, float* dq_workspace,
                                 void* stream_v) {

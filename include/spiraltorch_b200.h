@@ -237,6 +237,7 @@ int st_attn_bwd(const StAttnBwdArgs* a, void* stream_v);   /* csrc/attention/att
 int st_attn_bwd_f32(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, void* stream_v);   /* csrc/attention/attn_bwd.cu */
 int st_attn_bwd_one_pass(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float* bias_workspace, float* dq_workspace, void* stream_v);   /* csrc/attention/attn_bwd.cu */
 long long st_attn_bwd_workspace(int B, int H, int Sq, int Sk, int D);   /* csrc/attention/attn_bwd.cu */
+long long st_attn_bwd_workspace_f32(int B, int H, int Sq, int Sk, int D);   /* csrc/attention/attn_bwd.cu */
 int st_attn_fwd(const StAttnFwdArgs* a, void* stream_v);   /* csrc/attention/attn_fwd.cu */
 int st_attn_fwd_f32(const StAttnFwdArgs* a, float* out32, float* bias_workspace, void* stream_v);   /* csrc/attention/attn_fwd.cu */
 int st_attn_fwd_get_pair_kernel();   /* csrc/attention/attn_fwd.cu */

@@ -250,9 +250,9 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
             raise ValueError(f"attention_backward: {n} must be a view with contiguous D, and all gradients bf16 or all fp32")
     sums = None
     if D == 64 and attn_bias is None:      # one pass over the tile pairs instead of two, where the kernel takes it
-        lib = native.lib()
-        lib.st_attn_bwd_workspace.restype = ctypes.c_longlong
-        room = lib.st_attn_bwd_workspace(*(ctypes.c_int(n) for n in (B, H, Sq, Sk, D)))
+        size = native.lib().st_attn_bwd_workspace_f32 if f32 else native.lib().st_attn_bwd_workspace
+        size.restype = ctypes.c_longlong
+        room = size(*(ctypes.c_int(n) for n in (B, H, Sq, Sk, D)))
         if room:
             try:
                 sums = torch.empty(room, dtype=torch.float32, device=dev)

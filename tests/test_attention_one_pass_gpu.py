@@ -1,6 +1,7 @@
 """Backward attention in one pass over the tile pairs (head_dim 64, up to eight key tiles) against 64 bits, at its edges: one, two
 and three key tiles (one sum of dQ, one of two tiles, two sums), the last count it takes and the first it leaves to two passes,
 other query than key lengths, contexts without keys; the same bits on every run."""
+import ctypes
 import math
 
 import pytest
@@ -59,14 +60,39 @@ def test_without_room_for_the_sums(monkeypatch):
     q, k, v, g = (torch.randn(2, 300, 2, 64, device="cuda").bfloat16() for _ in range(4))
     o, lse = A.attention_forward(q, k, v, True)
     one = A.attention_backward(q, k, v, o, lse, g, True)
-    empty = torch.empty
+    empty, refused = torch.empty, []
+    workspace = native.lib().st_attn_bwd_workspace
+    workspace.restype = ctypes.c_longlong
+    room = workspace(*(ctypes.c_int(n) for n in (2, 2, 300, 300, 64)))
+    assert room > 2 * q.numel()
 
     def refuse(*size, **kw):
-        if size[0] == q.numel() * 2 + 4:
+        if size[0] == room:
+            refused.append(room)
             raise torch.cuda.OutOfMemoryError("no room")
         return empty(*size, **kw)
 
     monkeypatch.setattr(A.torch, "empty", refuse)
-    for x, y in zip(one, A.attention_backward(q, k, v, o, lse, g, True)):
+    two = A.attention_backward(q, k, v, o, lse, g, True)
+    assert refused == [room]
+    for x, y in zip(one, two):
         assert (x.float() - y.float()).abs().max() <= 2 * 2.0 ** -8 * y.float().abs().max()     # one rounding to bf16 each
+    native.raise_on_device_error()
+
+
+@pytest.mark.parametrize("seq,room", [(256, 0), (257, 2)])
+def test_room_for_fp32_gradients(seq, room):
+    """Up to two key tiles fp32 gradients of the queries are the only sum, added to where they are; beyond, one per two tiles."""
+    torch.manual_seed(0)
+    q, k, v, g = (torch.randn(8, seq, 2, 64, device="cuda").bfloat16() for _ in range(4))
+    o, lse = A.attention_forward(q, k, v, False)
+    out = [torch.empty(t.shape, device="cuda") for t in (q, k, v)]
+    got = [x.clone() for x in A.attention_backward(q, k, v, o, lse, g, False, None, *out)]
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    A.attention_backward(q, k, v, o, lse, g, False, None, *out)
+    # beside the sums: one fp32 number per row, and blocks that are multiples of 512 bytes
+    assert torch.cuda.max_memory_allocated() - before <= room * q.numel() * 4 + lse.numel() * 4 + 4096
+    for x, ref in zip(got, _exact(q, k, v, g, False, None, None)):
+        assert (x.double() - ref).norm() <= 4 * 2.0 ** -9 * ref.norm()
     native.raise_on_device_error()
