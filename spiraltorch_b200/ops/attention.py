@@ -249,7 +249,9 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
         if t.dtype != (torch.float32 if f32 else torch.bfloat16) or t.stride(-1) != 1:
             raise ValueError(f"attention_backward: {n} must be a view with contiguous D, and all gradients bf16 or all fp32")
     sums = None
-    if D == 64 and attn_bias is None:      # one pass over the tile pairs instead of two, where the kernel takes it
+    # One pass over the tile pairs instead of two, where the kernel takes it.  The passes add the parts of dQ in different orders,
+    # so where bits must repeat the form does not depend on the memory left.
+    if D == 64 and attn_bias is None and not native.deterministic_reduction():
         size = native.lib().st_attn_bwd_workspace_f32 if f32 else native.lib().st_attn_bwd_workspace
         size.restype = ctypes.c_longlong
         room = size(*(ctypes.c_int(n) for n in (B, H, Sq, Sk, D)))

@@ -193,8 +193,8 @@ def raw_stream(index: int) -> int:
 
 def deterministic_reduction() -> bool:
     """``SPIRAL_DETERMINISTIC_REDUCTION`` (or the master switch ``SPIRAL_DETERMINISTIC``): reductions whose order
-    would depend on scheduling - split-K weight gradients that meet in fp32 atomics, the embedding scatter-add -
-    take their fixed-order form, so two runs give bit-identical gradients."""
+    would depend on scheduling - split-K weight gradients that meet in fp32 atomics, the embedding scatter-add - or on the
+    memory left - attention backward at head_dim 64 - take their fixed-order form, so two runs give bit-identical gradients."""
     def on(name: str) -> bool:
         return os.environ.get(name, "0").strip().lower() not in ("0", "", "false", "off", "no")
     return on("SPIRAL_DETERMINISTIC_REDUCTION") or on("SPIRAL_DETERMINISTIC")

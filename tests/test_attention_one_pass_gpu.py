@@ -80,6 +80,25 @@ def test_without_room_for_the_sums(monkeypatch):
     native.raise_on_device_error()
 
 
+def test_bits_do_not_depend_on_the_room_where_they_must_repeat(monkeypatch):
+    monkeypatch.setenv("SPIRAL_DETERMINISTIC_REDUCTION", "1")
+    torch.manual_seed(0)
+    q, k, v, g = (torch.randn(2, 700, 2, 64, device="cuda").bfloat16() for _ in range(4))
+    o, lse = A.attention_forward(q, k, v, True)
+    want = A.attention_backward(q, k, v, o, lse, g, True)
+    empty = torch.empty
+
+    def refuse(*size, **kw):
+        if kw.get("dtype") is torch.float32 and size[0] != tuple(lse.shape):
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(A.torch, "empty", refuse)
+    for x, y in zip(A.attention_backward(q, k, v, o, lse, g, True), want):
+        assert torch.equal(x, y)
+    native.raise_on_device_error()
+
+
 @pytest.mark.parametrize("seq,room", [(256, 0), (257, 2)])
 def test_room_for_fp32_gradients(seq, room):
     """Up to two key tiles fp32 gradients of the queries are the only sum, added to where they are; beyond, one per two tiles."""
