@@ -8,7 +8,7 @@ import torch
 
 from spiraltorch_b200.ops import conv as C
 from spiraltorch_b200.ops import gemm as G
-from spiraltorch_b200.ops import native
+from spiraltorch_b200.ops import multi, native
 
 CSRC = Path(__file__).resolve().parents[1] / "csrc"
 
@@ -108,3 +108,91 @@ def test_products_with_a_block_limit_wait_for_their_turn():
     if len(times) != 2:
         pytest.skip("kernels are not traced here")
     assert times[1][0] >= times[0][1]
+
+
+def _chain(a, b, steps=6):
+    """Products that each read what the one before wrote, followed by the loss over the last two: two fp32 matrices and a number."""
+    outs, x = [], a
+    for _ in range(steps):
+        x = G.gemm(x, b, alpha=1.0 / 32)
+        outs.append(x)
+    p, t = outs[-1].float(), outs[-2].float()
+    return [*outs, multi.mse_forward(p, t)[0]]
+
+
+def _synchronised(a, b, steps=6):
+    """The same with a synchronisation behind every kernel."""
+    outs, x = [], a
+    for _ in range(steps):
+        x = G.gemm(x, b, alpha=1.0 / 32)
+        torch.cuda.synchronize()
+        outs.append(x)
+    p, t = outs[-1].float(), outs[-2].float()
+    torch.cuda.synchronize()
+    return [*outs, multi.mse_forward(p, t)[0]]
+
+
+def _operands(seed):
+    torch.manual_seed(seed)
+    return torch.randn(2048, 1024, device="cuda").bfloat16(), torch.randn(1024, 1024, device="cuda").bfloat16()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("stream", ["legacy", "own"])
+def test_one_stream(stream):
+    """Chained kernels one after the other, and behind the fill of a counter that the loss kernel's blocks count on (mse_forward)."""
+    s = torch.cuda.default_stream() if stream == "legacy" else torch.cuda.Stream()
+    for seed in range(4):
+        a, b = _operands(seed)
+        want = _synchronised(a, b)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            got = _chain(a, b)
+        s.synchronize()
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+    native.raise_on_device_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["wait_event", "wait_stream"])
+def test_two_streams_hand_a_buffer_back_and_forth(how):
+    """Each product reads, on its stream, what the one before wrote on the other, into buffers that are used again."""
+    a, b = _operands(0)
+    streams, buffers = [torch.cuda.Stream() for _ in range(2)], [torch.empty_like(a) for _ in range(2)]
+    x, want = a, []
+    for _ in range(12):
+        x = G.gemm(x, b, alpha=1.0 / 32)
+        torch.cuda.synchronize()
+        want.append(x.clone())
+    torch.cuda.synchronize()
+    x, got = a, []
+    for i in range(12):
+        here, other = streams[i & 1], streams[1 - (i & 1)]
+        if how == "wait_event":
+            here.wait_event(other.record_event())
+        else:
+            here.wait_stream(other)
+        with torch.cuda.stream(here):
+            G.gemm(x, b, alpha=1.0 / 32, out=buffers[i & 1])
+            x = buffers[i & 1]
+            got.append(x.clone())
+            G.gemm(x, b, alpha=2.0)                 # one more chained kernel behind the copy
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+    native.raise_on_device_error()
+
+
+@pytest.mark.gpu
+def test_fill_between_chained_kernels():
+    """A fill of the accumulated output stands between two products that add to it."""
+    a, b = _operands(1)
+    out = torch.empty(2048, 1024, device="cuda")
+    want = G.gemm(a, b, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        G.gemm(a, b, out=out, accumulate=True)
+        out.zero_()
+        G.gemm(a, b, out=out, accumulate=True)
+        got = out.clone()
+        assert torch.equal(got, want)
+    native.raise_on_device_error()

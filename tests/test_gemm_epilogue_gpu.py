@@ -61,3 +61,16 @@ def test_fp32_outputs(m, n, k, aligned):
     G.gemm(a.expand(3, m, k).contiguous(), b.expand(3, n, k).contiguous(), out=batched, accumulate=True)
     assert _error(batched, whole.double() + ref) < tol + 2.0 ** -24
     native.raise_on_device_error()
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+def test_added_results_keep_subnormal_numbers(aligned):
+    """fp32 outputs that are added to, by the copy engine and element by element: no sum is flushed to zero."""
+    a = torch.ones(256, 64, device="cuda").bfloat16()
+    out = torch.full((256, 256 if aligned else 257), 1e-40, device="cuda")[:, :256]
+    G.gemm(a, a, alpha=1e-41 / 64, out=out, accumulate=True)
+    want = torch.full((), 1e-40) + torch.full((), 64.0) * torch.tensor(1e-41 / 64)
+    # numbers are multiples of 2^-149 here; the scale, its product and the sum are off by half of one each, the scale's 64-fold
+    assert (out.cpu().double() - want.double()).abs().max() <= 34 * 2.0 ** -149
+    assert out.min() > 1.05e-40
+    native.raise_on_device_error()
