@@ -15,7 +15,9 @@
 // Recomputing S and dP in the dQ pass costs two extra GEMMs per tile pair, but no pass needs more than 512 TMEM columns minus
 // one operand, which lets both software-pipeline: the element-wise phase is split in two (P from S, then dS from dP), S of the
 // next tile is issued as soon as this tile's S has been read, and dP of the next tile right after this tile's accumulate GEMMs,
-// so the tensor pipe works while the element-wise warps do.
+// so the tensor pipe works while the element-wise warps do.  At head_dim 128 S, dP, dV and dK take all 512 columns; dQ of a pair could
+// only have dP's between the read of dP and dP of the next tile, with its drain between two tiles and eight fp32 sums for sixteen
+// KV tiles.  That form has not been built, so how it compares is not known.
 // At head_dim 64 with up to eight KV tiles, one pass does it all (MODE_ONE, launches 2 and 3 in one): dV, dK and two tiles of
 // dQ fit the tensor memory, dQ[q, d] = dS·K of a pair is drained while the next pair's GEMMs run and added by TMA to fp32 sums in
 // memory, and a last pass rounds them.  A sum receives the parts of two KV tiles only, in whatever order they come, so that the

@@ -1029,8 +1029,8 @@ struct StAttnFwdArgs {
   const int* lengths;
 };
 
-// 1 (default): plain attention runs the pair kernel (two query tiles per CTA, P and O in TMEM); 0: the single-tile
-// kernel for every case.  The biased / variable-length instantiation always uses the single-tile kernel.
+// 1 (default): the pair kernel (two query tiles per CTA, P and O in TMEM) runs where its pairs fill the chip, with a key bias or
+// lengths too; 0: the single-tile kernel for every case.  A bias per (query, key) always uses the single-tile kernel.
 static int g_pair_kernel = 1;
 static int g_pair_trace_on = 0;
 // Phase tracing of the pair kernel (CTA 0 only; slots listed at g_pair_trace): on = 1 zeroes the sums and makes

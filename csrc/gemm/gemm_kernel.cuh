@@ -1448,12 +1448,18 @@ inline bool staged_epilogue(const GemmParams& p) { return p.operand_tma != 0; }
 // Where the tiles are so few that two or four CTAs can share each, their K loops are split (launch_parts): the same product takes
 // 31 us with two CTAs on each of 56 tiles; 128 x 2048 x 8192 20 and 39; 777 x 512 x 4608 13 in four parts and 20 in tiles of 64
 // columns; 128 x 768 x 3072 9.8 and 13.8.  The exchange costs about 4 us, so a K of 768 stays whole (777 x 768 x 768: 8.6 and
-// 7.2).  A cluster of four needs four SMs of one graphics processing cluster: 144 such CTAs took two rounds (128 x 4608 x 1536: 19 us
-// against 11), 128 run at once.  Parts are taken when they promise 4 % or more.
+// 7.2).  A cluster of four needs four SMs of one graphics processing cluster, and 33 such clusters are resident at once (a query of the
+// occupancy; 74 of two): the rule takes 32 of 148 SMs / 4 = 37, as 36 took two rounds (128 x 4608 x 1536: 19 us against 11).  Parts
+// are taken when they promise 4 % or more.  Their sums are added in a fixed order, and shorter chains are no further from 64 bits
+// (relative error of fp32 outputs, whole and in parts: 128 x 2048 x 8192 9.1e-6 and 2.1e-6, 777 x 2048 x 8192 9.1e-6 and 4.4e-6, 128 x
+// 768 x 3072 3.2e-6 and 0.7e-6).
 // 128 x 256 and the pair come out within a few percent of one another over much of the range, timed alone; inside a training
 // step, under the power limit, the pair is the faster one (the products of the 85 M byte model's step, K = 768 and 3072: 7.87 ms
-// against 8.10), so it is taken up to 11 % above.
-// Against the fastest form of each, timed alone, the rule takes 0.2 to 0.5 % longer on average, at most 11 %.
+// against 8.10), so it is taken where the model has it up to 11 % above.  Timed alone that preference changes little (plain outputs
+// 0.3 % above the fastest form of each product on average with it and 0.5 without, GELU with its saved input 0.9 and 0.8).
+// Over 528 products, captured and with K-major operands, the rule is above the fastest form by 0.3 % on average with plain outputs, 0.6
+// with a residual, 0.9 with GELU and its saved input, nothing with GELU' and 0.1 with fp32 outputs, and by 4 % where fp32 outputs are
+// added to; for single products by up to 29 % (306 x 1024 x 512, added: 8.6 us against 6.7).
 enum TileEpilogue : int { EPI_PLAIN, EPI_OPERAND, EPI_GELU, EPI_GELU_BWD, EPI_FP32, EPI_FP32_ADD };
 struct TileCost {
   double a, c, c2, e[6];
@@ -1519,9 +1525,11 @@ template <bool A_MN, bool B_MN>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const OutMaps& tmC, const GemmParams& p, cudaStream_t stream) {
   // With operands, a saved pre-activation or GELU the epilogue of a tile is longer than the main loop of a short K.  A third set of
   // warps shares it then, with four ring stages and two staging blocks per warp where anything is staged beside the output.  us, two
-  // sets and three: 16384 x 3072 x 768 with GELU' 126 and 108, GELU and its saved input 100 and 88, GELU alone 80 and 73, plus
-  // residual 86 and 79; 8192 x 4096 x 1024 with GELU' 92 and 81; from K = 2048 on the ring matters more (4096 x 8192 x 2048 with
-  // GELU' 113 and 123), and a bare output gains nothing (58.2 and 58.2).
+  // sets and three (captured): 16384 x 3072 x 768 with GELU' 135 and 111, GELU and its saved input 123 and 101, GELU alone 83 and 76,
+  // plus residual 80 and 78.  Where the longer main loop makes the ring matter more depends on the epilogue: GELU' 141 and 135 at K =
+  // 1536, 164 and 164 at 2048, 226 and 231 at 3072; GELU and its saved input 132 and 130, 158 and 163; GELU alone equal from 1280 on;
+  // a residual 92 and 90 at 1024, but 103 and 106 at 1280 and 118 and 122 at 1536.  One line for all of them lies where GELU', the
+  // longest, still gains.  A bare output gains nothing (58.2 and 58.2).
   if constexpr (!A_MN) {
     const bool staged = p.operand_tma || p.aux_tma;
     if (p.K <= 1536 && staged) return launch_pair_ring<false, B_MN, 4, 3>(tmA, tmB, tmC, p, stream);

@@ -4,10 +4,11 @@
 //   * one elected thread issues tcgen05.mma (128 x BN x 16, or 256 x 256 x 16 over a CTA pair) with fp32
 //     accumulators in TMEM; two accumulator buffers let the epilogue of tile i overlap the
 //     main loop of tile i+1;
-//   * eight epilogue warps read TMEM with tcgen05.ld and apply the fused epilogue:
+//   * eight epilogue warps (twelve under a short K with operands or GELU) read TMEM with tcgen05.ld and apply the fused epilogue:
 //     +bias, ReLU / GELU(tanh), store of the pre-activation, multiply by GELU'/ReLU' of a
 //     saved pre-activation (backward), +residual, C += (gradient accumulation), bf16 or
-//     fp32 output.
+//     fp32 output;
+//   * where tiles are few, a cluster of two or four CTAs shares a tile's K loop and adds its sums through shared memory.
 //
 // Operand layouts.  "K-major" A is a row-major [M,K] matrix, "MN-major" A is a row-major
 // [K,M] matrix (i.e. Aᵀ is what is stored).  Same for B with N in place of M.  This covers
