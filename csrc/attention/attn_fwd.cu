@@ -460,16 +460,21 @@ constexpr int PAIR_THREADS = 384;   // two softmax warpgroups + one warpgroup ho
 constexpr int PAIR_REGS_AUX = 88, PAIR_REGS_SOFTMAX = 208;
 constexpr int PAIR_STAGES = 4;      // ring of K / V tiles in the order K_j, V_j, K_j+1, V_j+1
 
-template <int D>
+// Outputs, and a key bias, pass through shared memory, but not at head_dim 128 with a bias: the tiles alone take 192 KB there, and with
+// any more the carve-out grows from 196 to 228 KB and leaves 28 KB of L1 instead of 60, which the registers that this form spills and
+// the bias no longer fit.  us with both staged, with outputs alone and with neither, 8 heads: 200 contexts of 64 keys 76, 91 and 61; 20 of
+// 500 62, 84 and 58.  Without a bias staging gains: 200 of 128 keys 59 with lane stores and 40, 20 of 500 39 and 34.
+template <int D, bool KEYB>
 struct PairSmem {
   static constexpr int TILE = BLK * D * 2;
   static constexpr int Q_OFF = 0;                          // two query tiles
   static constexpr int KV_OFF = 2 * TILE;
   // per softmax warp: blocks of 32 rows and 64 bytes of the output on their way out, and the key bias of two tiles
+  static constexpr bool STAGED = D == 64 || !KEYB;
   static constexpr int STG_SLOTS = D == 64 ? 2 : 1;
   static constexpr int STG_OFF = KV_OFF + PAIR_STAGES * TILE;
-  static constexpr int BIAS_OFF = STG_OFF + 8 * STG_SLOTS * 2048;
-  static constexpr int BAR_OFF = BIAS_OFF + 8 * 2 * BLK * 4;
+  static constexpr int BIAS_OFF = STG_OFF + (STAGED ? 8 * STG_SLOTS * 2048 : 0);
+  static constexpr int BAR_OFF = BIAS_OFF + (STAGED && KEYB ? 8 * 2 * BLK * 4 : 0);
   static constexpr int TOTAL = BAR_OFF + 256;
   static_assert(TOTAL <= 232448, "shared memory");
 };
@@ -499,7 +504,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                      const __grid_constant__ CUtensorMap tmO32, const AttnFwdParams p) {
-  using L = PairSmem<D>;
+  using L = PairSmem<D, KEYB>;
+  constexpr bool STAGED = L::STAGED;
   constexpr int KB = D / 64;
   constexpr uint32_t S_COL = 0;       // S_t at S_COL + 128 t; P_t (bf16 pairs) over its first 64 columns
   constexpr uint32_t O_COL = 256;     // O_t at O_COL + D t
@@ -763,6 +769,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tma_store_commit();
       }
     };
+    // a row of the output, for the lane that stores its own
+    auto out_row = [&](int row_g, int h, int b) {
+      return reinterpret_cast<uint4*>(p.O + (long long)b * p.o_sb + (long long)row_g * p.o_ss + (long long)h * p.o_sh);
+    };
+    auto out32_row = [&](int row_g, int h, int b) { return reinterpret_cast<float4*>(p.O32 + (((long long)b * p.Sq + row_g) * p.H + h) * D); };
     float4* const bias_slots = reinterpret_cast<float4*>(smem + L::BIAS_OFF) + warp * (2 * BLK / 4);
     uint32_t steps = 0;   // softmax steps done (phase of s_full)
     int items = 0;        // items this tile took part in (phase of o_full)
@@ -781,12 +792,18 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (n_kv <= 0) {
         const int row0 = q_tile * BLK + quad * 32;
         if (KEYB && row0 < p.Sq) {       // a query tile beyond the valid length, or a context without keys
-          uint4 none[4];
+          if constexpr (STAGED) {
+            uint4 none[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) none[q] = make_uint4(0, 0, 0, 0);
-          for (int c = 0; c < D; c += 32) stage(&tmO, none, c, row0, h, b);
-          if (FP32 && p.O32)
-            for (int c = 0; c < D; c += 16) stage(&tmO32, none, c, row0, h, b);
+            for (int q = 0; q < 4; ++q) none[q] = make_uint4(0, 0, 0, 0);
+            for (int c = 0; c < D; c += 32) stage(&tmO, none, c, row0, h, b);
+            if (FP32 && p.O32)
+              for (int c = 0; c < D; c += 16) stage(&tmO32, none, c, row0, h, b);
+          } else if (row_g < p.Sq) {
+            for (int c = 0; c < D / 8; ++c) out_row(row_g, h, b)[c] = make_uint4(0, 0, 0, 0);
+            if (FP32 && p.O32)
+              for (int c = 0; c < D / 4; ++c) out32_row(row_g, h, b)[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          }
           if (row_g < p.Sq) p.lse[((long long)b * p.H + h) * p.Sq + row_g] = -INFINITY;
         }
         continue;
@@ -797,10 +814,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const float4* bias_row = KEYB ? reinterpret_cast<const float4*>(p.kb_pad + b * p.kp_sb + h * p.kp_sh) : nullptr;
       float m = -INFINITY, l = 0.0f;
       float4 bias_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);      // this lane's four keys of the next tile
-      if (KEYB) bias_next = __ldg(bias_row + lane);
+      if (KEYB && STAGED) bias_next = __ldg(bias_row + lane);
       for (int j = 0; j < n_kv; ++j) {
         const float4* const bias = bias_slots + (j & 1) * (BLK / 4);
-        if (KEYB) {
+        if (KEYB && STAGED) {
           bias_slots[(j & 1) * (BLK / 4) + lane] = bias_next;
           if (j + 1 < n_kv) bias_next = __ldg(bias_row + (j + 1) * (BLK / 4) + lane);
           __syncwarp();
@@ -827,7 +844,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const float2 sc2 = make_float2(sc, sc);
 #pragma unroll
           for (int c = 0; c < BLK; c += 4) {
-            const float4 v = bias[c / 4];
+            const float4 v = STAGED ? bias[c / 4] : __ldg(bias_row + (col0 + c) / 4);
             const float2 x = fma2(make_float2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, make_float2(v.x, v.y));
             const float2 y = fma2(make_float2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, make_float2(v.z, v.w));
             sr[c] = __float_as_uint(x.x); sr[c + 1] = __float_as_uint(x.y);
@@ -926,29 +943,34 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         uint32_t v[32];
         tmem_ld_32x32(o_addr + ch * 32, v);
         tmem_ld_wait();
+        if (KEYB && !row_live) {      // zeros by value: what a padded query summed up need not be finite
 #pragma unroll
-        for (int c = 0; c < 32; ++c)      // zeros by value: what a padded query summed up need not be finite
-          v[c] = KEYB && !row_live ? 0 : __float_as_uint(__uint_as_float(v[c]) * inv);
-        if (row0 < p.Sq) {
-          uint4 u[4];
+          for (int c = 0; c < 32; ++c) v[c] = 0;
+        }
+        auto at = [&](int c) { return __uint_as_float(v[c]) * inv; };
+        if (STAGED ? row0 < p.Sq : row_g < p.Sq) {
           if (FP32 && p.O32) {
 #pragma unroll
             for (int piece = 0; piece < 2; ++piece) {
+              uint4 u[4];
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
                 const int c = piece * 16 + q * 4;
-                u[q] = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                const float4 f = make_float4(at(c), at(c + 1), at(c + 2), at(c + 3));
+                if constexpr (STAGED) u[q] = make_uint4(__float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z), __float_as_uint(f.w));
+                else out32_row(row_g, h, b)[ch * 8 + piece * 4 + q] = f;
               }
-              stage(&tmO32, u, ch * 32 + piece * 16, row0, h, b);
+              if constexpr (STAGED) stage(&tmO32, u, ch * 32 + piece * 16, row0, h, b);
             }
           }
+          uint4 u[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int c = q * 8;
-            u[q] = make_uint4(pack_bf16x2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), pack_bf16x2(__uint_as_float(v[c + 2]), __uint_as_float(v[c + 3])),
-                              pack_bf16x2(__uint_as_float(v[c + 4]), __uint_as_float(v[c + 5])), pack_bf16x2(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
+            u[q] = make_uint4(pack_bf16x2(at(c), at(c + 1)), pack_bf16x2(at(c + 2), at(c + 3)), pack_bf16x2(at(c + 4), at(c + 5)), pack_bf16x2(at(c + 6), at(c + 7)));
+            if constexpr (!STAGED) out_row(row_g, h, b)[ch * 4 + q] = u[q];
           }
-          stage(&tmO, u, ch * 32, row0, h, b);
+          if constexpr (STAGED) stage(&tmO, u, ch * 32, row0, h, b);
         }
       }
       if (row_g < p.Sq)
@@ -1125,14 +1147,14 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
     static bool pcfg[6][st::kMaxDevices] = {{false}};
     int prc;
     if (keyb)
-      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, true, true>, PairSmem<128>::TOTAL, pcfg[2])
-                        : plaunch(attn_fwd_pair_kernel<64, true, true>, PairSmem<64>::TOTAL, pcfg[3]);
+      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, true, true>, PairSmem<128, true>::TOTAL, pcfg[2])
+                        : plaunch(attn_fwd_pair_kernel<64, true, true>, PairSmem<64, true>::TOTAL, pcfg[3]);
     else if (out32)
-      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, false, true>, PairSmem<128>::TOTAL, pcfg[4])
-                        : plaunch(attn_fwd_pair_kernel<64, false, true>, PairSmem<64>::TOTAL, pcfg[5]);
+      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, false, true>, PairSmem<128, false>::TOTAL, pcfg[4])
+                        : plaunch(attn_fwd_pair_kernel<64, false, true>, PairSmem<64, false>::TOTAL, pcfg[5]);
     else
-      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, false, false>, PairSmem<128>::TOTAL, pcfg[0])
-                        : plaunch(attn_fwd_pair_kernel<64, false, false>, PairSmem<64>::TOTAL, pcfg[1]);
+      prc = a->D == 128 ? plaunch(attn_fwd_pair_kernel<128, false, false>, PairSmem<128, false>::TOTAL, pcfg[0])
+                        : plaunch(attn_fwd_pair_kernel<64, false, false>, PairSmem<64, false>::TOTAL, pcfg[1]);
     if (prc != ST_OK) return prc;
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
