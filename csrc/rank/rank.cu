@@ -22,6 +22,7 @@
 // zero the padding and return the per-row counts.
 #include "../common/host.h"
 #include "../common/ptx.cuh"
+#include <cfloat>
 
 namespace {
 using namespace st;
@@ -258,7 +259,7 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
 #pragma unroll
   for (int r = 0; r < R; ++r) best[r] = KEY_INVALID;
   u64 thr = KEY_INVALID;                               // k-th best key so far
-  float thr_v = TOP_MODE ? -INFINITY : INFINITY;       // a bound: an element beyond it cannot be among the k best
+  float thr_v = TOP_MODE ? -FLT_MAX : FLT_MAX;         // a bound: an element beyond it cannot be among the k best, nor can infinities
   int qn = 0;
   if (row < rows) {
     const float* x = in + row * cols;
@@ -390,8 +391,10 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
           if (r == (k - 1) >> 5) t = best[r];
         thr = __shfl_sync(0xffffffffu, t, (k - 1) & 31);
         if (thr != KEY_INVALID) {
+          // the next better value: in the columns to come an equal one loses against the k-th best, which stands further left.
+          // With the value itself rows of few values passed whole: 859 x 17693 equal ones, k = 1, 71 us and 44.
           const unsigned o = static_cast<unsigned>(thr >> 32);
-          thr_v = from_orderable(TOP_MODE ? ~o : o);
+          thr_v = from_orderable(TOP_MODE ? ~o + 1u : o - 1u);
         }
       }
     }
