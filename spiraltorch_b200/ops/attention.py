@@ -12,6 +12,7 @@ the reference (its attention is forward-only).
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from typing import Optional
@@ -198,6 +199,14 @@ def attention_forward(q, k, v, causal: bool = True, scale: Optional[float] = Non
     return o, lse
 
 
+@functools.cache
+def _one_pass_room(f32: bool):
+    """The library's function for the floats of workspace that the one-pass form takes."""
+    size = native.entry("st_attn_bwd_workspace_f32" if f32 else "st_attn_bwd_workspace", "iiiii")
+    size.restype = ctypes.c_longlong
+    return size
+
+
 def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional[float] = None,
                        dq=None, dk=None, dv=None, *, key_bias=None, attn_bias=None, lengths=None, do32=None):
     """Returns ``(dq, dk, dv)`` (bf16, ``[B,S,H,D]``); outputs may be preallocated strided views, all bf16 or all fp32.
@@ -231,16 +240,10 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
     dk = torch.empty((B, Sk, H, D), dtype=torch.bfloat16, device=dev) if dk is None else dk
     dv = torch.empty((B, Sk, H, D), dtype=torch.bfloat16, device=dev) if dv is None else dv
     delta = torch.empty((B, H, Sq), dtype=torch.float32, device=dev)
-    a = _BwdArgs()
-    a.Q, a.K, a.V, a.O, a.dO = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr()
-    a.lse, a.delta, a.dQ_acc = lse.data_ptr(), delta.data_ptr(), None      # dQ accumulates elsewhere
-    a.dQ, a.dK, a.dV = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    for pre, t in (("q", q), ("k", k), ("v", v), ("o", o), ("do", do), ("dq", dq), ("dk", dk), ("dv", dv)):
-        setattr(a, pre + "_sb", t.stride(0))
-        setattr(a, pre + "_ss", t.stride(1))
-        setattr(a, pre + "_sh", t.stride(2))
-    a.B, a.H, a.Sq, a.Sk, a.D = B, H, Sq, Sk, D
-    a.scale, a.causal = float(scale), int(causal)
+    # all fields before the biases at once: one by one they take 8 us, as long as a launch
+    strides = [n for t in (q, k, v, o, do, dq, dk, dv) for n in t.stride()[:3]]
+    a = _BwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
+                 None, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *strides, B, H, Sq, Sk, D, float(scale), int(causal))
     keep: list = []
     _bias_args(a, q, k, key_bias, attn_bias, lengths, keep)
     work = _bias_workspace(q, k, key_bias, attn_bias, lengths)
@@ -252,9 +255,7 @@ def attention_backward(q, k, v, o, lse, do, causal: bool = True, scale: Optional
     # One pass over the tile pairs instead of two, where the kernel takes it.  The passes add the parts of dQ in different orders,
     # so where bits must repeat the form does not depend on the memory left.
     if D == 64 and attn_bias is None and not native.deterministic_reduction():
-        size = native.lib().st_attn_bwd_workspace_f32 if f32 else native.lib().st_attn_bwd_workspace
-        size.restype = ctypes.c_longlong
-        room = size(*(ctypes.c_int(n) for n in (B, H, Sq, Sk, D)))
+        room = _one_pass_room(f32)(B, H, Sq, Sk, D)
         if room:
             try:
                 sums = torch.empty(room, dtype=torch.float32, device=dev)
