@@ -52,7 +52,7 @@ constexpr int NUM_THREADS = EW_THREADS + 64;       // + TMA producer warp + MMA 
 constexpr int MODE_KV = 0, MODE_Q = 1, MODE_ONE = 2;
 // KV tiles up to which the one-pass form is taken: its sums of dQ take half as many times the size of dQ in fp32.
 constexpr int kOnePassTiles = 8;
-constexpr int kQueueFloats = 32;      // the workspace starts with the work queue, the sums follow on the next 128-byte line
+constexpr int kQueueFloats = 4;      // the work queue, behind the sums: before them it would move them off their 512-byte blocks (1 % slower)
 // Biases: none; a bias per (query, key) among them, read and compared per element; key bias and length only, as padded rows
 // in the log2 domain (minus infinity where masked): 16-byte loads, no comparisons.
 constexpr int BIAS_NONE = 0, BIAS_FULL = 1, BIAS_KEYS = 2;
@@ -877,10 +877,10 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
   const bool one = dq_sums && a->D == 64 && n_kv <= kOnePassTiles && (!biased || keyb);
   if (one && (reinterpret_cast<uintptr_t>(dq_sums) & 15)) return st::fail(ST_ERR_INVALID, "attn_bwd: the dQ workspace must be 16-byte aligned");
   const bool in_place = one && grad_f32 && n_kv <= 2;
-  float* const acc = !one ? nullptr : in_place ? static_cast<float*>(a->dQ) : dq_sums + kQueueFloats;
+  float* const acc = !one ? nullptr : in_place ? static_cast<float*>(a->dQ) : dq_sums;
   const long long acc_sb = in_place ? a->dq_sb : (long long)a->Sq * a->H * a->D, acc_ss = in_place ? a->dq_ss : (long long)a->H * a->D,
                   acc_sh = in_place ? a->dq_sh : a->D, acc_buffer = (long long)a->B * a->Sq * a->H * a->D;
-  unsigned* const queue = one ? reinterpret_cast<unsigned*>(dq_sums) : nullptr;
+  unsigned* const queue = one ? reinterpret_cast<unsigned*>(dq_sums + (in_place ? 0 : acc_buffer * ((n_kv + 1) / 2))) : nullptr;
 
   {
     const long long rows = (long long)a->B * a->Sq * a->H;
