@@ -72,6 +72,10 @@ struct AttnBwdParams {
   const float* kb_pad;          // BIAS_KEYS
   long long kp_sb, kp_sh;
   int grad_f32;                 // dQ, dK and dV are fp32
+  struct Grad {
+    void* p;
+    long long sb, ss, sh;       // in elements
+  } dq, dk, dv;                 // where the lanes store their own rows
   unsigned* queue;              // items drawn beyond the first of every CTA, or null
 };
 
@@ -86,7 +90,7 @@ struct GradMaps {
   CUtensorMap dq, dk, dv;
 };
 
-template <int D, int MODE>
+template <int D, int MODE, int BIAS>
 struct BwdSmem {
   static_assert(MODE != MODE_ONE || D == 64, "dV, dK and two dQ tiles fit the tensor memory at head_dim 64 only");
   static constexpr int TILE = BLK * D * 2;
@@ -106,9 +110,13 @@ struct BwdSmem {
   static constexpr int B_OFF = A_OFF + NA * TILE;
   static constexpr int DS_OFF = B_OFF + NB * TILE;
   static constexpr int P_OFF = DS_OFF + P_TILE;        // not in MODE_Q
-  // gradients leave by TMA, 2 KB per warp at a time; at head_dim 128 they are staged in the dS tile, which is idle then
+  // Gradients leave by TMA, 2 KB per warp at a time; at head_dim 128 they are staged in the dS tile, which is idle then.  With a bias per
+  // (query, key) at head_dim 64 the lanes store their own rows: 32 KB for staging would leave half as much L1, through which they read
+  // the bias (us, 22 contexts of 504, 16 heads, causal: 450 staged, 344 from the lanes; 2 of 1738, 8 heads, 353 and 262), and staged in
+  // the dS tile contexts of up to 32 queries wait for it, 13 % of their time.
   static constexpr int STG = 2048;
-  static constexpr bool OWN_STG = D == 64;
+  static constexpr bool LANES = D == 64 && BIAS == BIAS_FULL;
+  static constexpr bool OWN_STG = D == 64 && !LANES;
   static constexpr int STG_OFF = OWN_STG ? P_OFF + (MODE == MODE_Q ? 0 : P_TILE) : DS_OFF;
   static constexpr int BAR_OFF = P_OFF + (MODE == MODE_Q ? 0 : P_TILE) + (OWN_STG ? EW_WARPS * STG : 0);
   static constexpr int TOTAL = BAR_OFF + 320;
@@ -128,7 +136,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ GradMaps tmG, const AttnBwdParams p) {
-  using L = BwdSmem<D, MODE>;
+  using L = BwdSmem<D, MODE, BIAS>;
   constexpr int KB = D / 64;
   constexpr int NA = L::NA, NB = L::NB;
   // TMEM columns.  MODE_KV: S, dP, dV, dK.  MODE_Q: S, dP (even tiles), dQ, dP (odd tiles).
@@ -472,6 +480,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             make_float4(__uint_as_float(t[4 * q]) * scale, __uint_as_float(t[4 * q + 1]) * scale,
                         __uint_as_float(t[4 * q + 2]) * scale, __uint_as_float(t[4 * q + 3]) * scale);
     };
+    // 32 columns of an accumulator, by the lane whose row it is
+    auto store_row = [&](const AttnBwdParams::Grad& to, int rows, const uint32_t (&t)[32], float scale, int col, int row0, int h, int b) {
+      if (row0 + lane >= rows) return;
+      const long long at = b * to.sb + (row0 + lane) * to.ss + h * to.sh + col;
+      auto v = [&](int i) { return __uint_as_float(t[i]) * scale; };
+      if (p.grad_f32) {
+        float4* const o = reinterpret_cast<float4*>(static_cast<float*>(to.p) + at);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) o[q] = make_float4(v(4 * q), v(4 * q + 1), v(4 * q + 2), v(4 * q + 3));
+      } else {
+        uint4* const o = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(to.p) + at);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          o[q] = make_uint4(pack_bf16x2(v(8 * q), v(8 * q + 1)), pack_bf16x2(v(8 * q + 2), v(8 * q + 3)),
+                            pack_bf16x2(v(8 * q + 4), v(8 * q + 5)), pack_bf16x2(v(8 * q + 6), v(8 * q + 7)));
+      }
+    };
     // 32 columns of an accumulator
     auto store_grad = [&](const CUtensorMap* map, const uint32_t (&t)[32], float scale, int col, int row0, int h, int b) {
       if (p.grad_f32) {
@@ -655,7 +680,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // the previous tile's GEMM that reads the dS buffer must be done: in the dK/dV pass dP(n) was
       // issued after it; the dQ pass issues dP early and signals the buffer separately
       if (MODE == MODE_Q && g > 0 && !mbar_wait_warp(smem_u32(ds_free), (g - 1) & 1, abort_flag)) { ok = false; break; }
-      if (!L::OWN_STG && n == 0 && w != blockIdx.x) {
+      if (!L::OWN_STG && !L::LANES && n == 0 && w != blockIdx.x) {
         // the dS tile still held gradients of the items before: every warp's have been read
         if (lane == 0) {
           tma_store_wait_read<0>();
@@ -711,7 +736,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       };
       read(KV && !first ? ACC1_COL : ACC0_COL, !BOTH);
-      if (!KV) {
+      if constexpr (L::LANES) {
+        if (!KV) {
+          if (first) store_row(p.dq, p.Sq, acc_r, p.scale, ch * 32, row0, h, b);
+        } else {
+          store_row(first ? p.dv : p.dk, p.Sk, acc_r, first ? 1.0f : p.scale, ch * 32, row0, h, b);
+        }
+      } else if (!KV) {
         if (first) store_grad(&tmG.dq, acc_r, p.scale, ch * 32, row0, h, b);
       } else {
         store_grad(first ? &tmG.dv : &tmG.dk, acc_r, first ? 1.0f : p.scale, ch * 32, row0, h, b);
@@ -927,6 +958,9 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
   p.attn_bias = a->attn_bias; p.ab_sb = a->ab_sb; p.ab_sh = a->ab_sh; p.ab_sq = a->ab_sq;
   p.lengths = a->lengths;
   p.grad_f32 = grad_f32;
+  p.dq = {a->dQ, a->dq_sb, a->dq_ss, a->dq_sh};
+  p.dk = {a->dK, a->dk_sb, a->dk_ss, a->dk_sh};
+  p.dv = {a->dV, a->dv_sb, a->dv_ss, a->dv_sh};
   p.queue = queue;
   p.kb_pad = nullptr; p.kp_sb = p.kp_sh = 0;
   if (keyb) {
@@ -945,7 +979,11 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
   const dim3 grid_q(items_q < num_sms ? items_q : num_sms);
   auto launch = [&](auto kernel, int smem_bytes, dim3 grid) -> int {
     ST_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    st::chained(kernel, grid, NUM_THREADS, smem_bytes, s)(tq, tk, tv, tdo, tg, p);
+    // A kernel that starts early finds the L1 that the one before it left: 28 KB behind a product.  The bias per (query, key) needs more:
+    // us with a product of 2048 x 4096 x 1024 before it, early and in order: 13 contexts of 602, 12 heads, causal, 645 and 358; 13 of
+    // 212 200 and 108.
+    const bool own_l1 = a->attn_bias && a->D == 64;
+    (own_l1 ? st::in_order(kernel, grid, NUM_THREADS, smem_bytes, s) : st::chained(kernel, grid, NUM_THREADS, smem_bytes, s))(tq, tk, tv, tdo, tg, p);
     ST_CUDA_CHECK(cudaGetLastError());
     return ST_OK;
   };
@@ -955,8 +993,8 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
     return launch(q, q_smem, grid_q);
   };
   if (one) {
-    const int e = keyb ? launch(attn_bwd_kernel<64, MODE_ONE, BIAS_KEYS>, BwdSmem<64, MODE_ONE>::TOTAL, grid_kv)
-                       : launch(attn_bwd_kernel<64, MODE_ONE, BIAS_NONE>, BwdSmem<64, MODE_ONE>::TOTAL, grid_kv);
+    const int e = keyb ? launch(attn_bwd_kernel<64, MODE_ONE, BIAS_KEYS>, BwdSmem<64, MODE_ONE, BIAS_KEYS>::TOTAL, grid_kv)
+                       : launch(attn_bwd_kernel<64, MODE_ONE, BIAS_NONE>, BwdSmem<64, MODE_ONE, BIAS_NONE>::TOTAL, grid_kv);
     if (e || in_place) return e;
     const long long rows = (long long)a->B * a->Sq * a->H;
     const long long blocks = (rows + 31) / 32, most = 16ll * st::sm_count();
@@ -968,7 +1006,7 @@ int attn_bwd_run(const StAttnBwdArgs* a, const float* dO32, int grad_f32, float*
     return ST_OK;
   }
 #define ST_BWD_BOTH(DV, BV) \
-  both(attn_bwd_kernel<DV, MODE_KV, BV>, BwdSmem<DV, MODE_KV>::TOTAL, attn_bwd_kernel<DV, MODE_Q, BV>, BwdSmem<DV, MODE_Q>::TOTAL)
+  both(attn_bwd_kernel<DV, MODE_KV, BV>, BwdSmem<DV, MODE_KV, BV>::TOTAL, attn_bwd_kernel<DV, MODE_Q, BV>, BwdSmem<DV, MODE_Q, BV>::TOTAL)
   if (a->D == 128) return keyb ? ST_BWD_BOTH(128, BIAS_KEYS) : biased ? ST_BWD_BOTH(128, BIAS_FULL) : ST_BWD_BOTH(128, BIAS_NONE);
   return keyb ? ST_BWD_BOTH(64, BIAS_KEYS) : biased ? ST_BWD_BOTH(64, BIAS_FULL) : ST_BWD_BOTH(64, BIAS_NONE);
 #undef ST_BWD_BOTH

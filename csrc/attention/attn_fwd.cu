@@ -1141,7 +1141,9 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
         ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         cfg[dev] = true;
       }
-      st::chained(kern, pgrid, PAIR_THREADS, smem_bytes, s)(tq, tk, tv, to, to32, p);
+      // with a key bias at head_dim 128 the L1 matters (PairSmem): a kernel that starts early finds what the one before it left
+      const bool own_l1 = keyb && a->D == 128;
+      (own_l1 ? st::in_order(kern, pgrid, PAIR_THREADS, smem_bytes, s) : st::chained(kern, pgrid, PAIR_THREADS, smem_bytes, s))(tq, tk, tv, to, to32, p);
       return ST_OK;
     };
     static bool pcfg[6][st::kMaxDevices] = {{false}};
@@ -1167,7 +1169,9 @@ int attn_fwd_run(const StAttnFwdArgs* a, float* out32, float* bias_ws, void* str
       ST_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
       cfg[st::current_device()] = true;
     }
-    st::chained(kern, grid, NUM_THREADS, smem_bytes, s)(tq, tk, tv, p);
+    // as above, for the bias per (query, key): us behind a product, early and in order, 25 contexts of 1048, 2 heads, 912 and 732
+    const bool own_l1 = biased && a->D == 64;
+    (own_l1 ? st::in_order(kern, grid, NUM_THREADS, smem_bytes, s) : st::chained(kern, grid, NUM_THREADS, smem_bytes, s))(tq, tk, tv, p);
     return ST_OK;
   };
   static bool cfg[4][st::kMaxDevices] = {{false}};

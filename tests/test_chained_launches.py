@@ -6,6 +6,7 @@ from pathlib import Path
 import pytest
 import torch
 
+from spiraltorch_b200.ops import attention as A
 from spiraltorch_b200.ops import conv as C
 from spiraltorch_b200.ops import gemm as G
 from spiraltorch_b200.ops import multi, native
@@ -108,6 +109,44 @@ def test_products_with_a_block_limit_wait_for_their_turn():
     if len(times) != 2:
         pytest.skip("kernels are not traced here")
     assert times[1][0] >= times[0][1]
+
+
+def _bias_per_pair(q, bias):
+    return A.attention_forward(q, q, q, False, attn_bias=bias)
+
+
+def _bias_per_pair_backward(q, bias):
+    o, lse = _bias_per_pair(q, bias)
+    return A.attention_backward(q, q, q, o, lse, q, False, attn_bias=bias)
+
+
+def _bias_per_key(q, bias):
+    return A.attention_forward(q, q, q, False, key_bias=bias[:, 0].contiguous())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,kernel,dim", [(_bias_per_pair, "attn_fwd_kernel", 64),
+                                           (_bias_per_pair_backward, "attn_bwd_kernel", 64), (_bias_per_key, "attn_fwd_pair_kernel", 128)])
+def test_kernels_that_start_in_order(op, kernel, dim):
+    """Attention that reads a bias through an L1 of its own size."""
+    a = torch.randn(8192, 4096, device="cuda").bfloat16()
+    args = torch.randn(24, 256, 8, dim, device="cuda").bfloat16(), torch.randn(24, 256, 256, device="cuda")
+
+    def both():
+        G.gemm(a, a)
+        op(*args)
+        torch.cuda.synchronize()
+
+    both()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as trace:
+        both()
+    times = sorted((e.time_range.start, e.time_range.end, e.name) for e in trace.events() if "kernel" in e.name)
+    if not any("gemm_bf16_kernel" in t[2] for t in times):
+        pytest.skip("kernels are not traced here")
+    found = [i for i, t in enumerate(times) if f"{kernel}<" in t[2] or t[2].endswith(kernel)]
+    assert found and found[0] > 0
+    for i in found:
+        assert times[i][0] >= max(t[1] for t in times[:i])
 
 
 def _chain(a, b, steps=6):
