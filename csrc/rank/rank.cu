@@ -284,6 +284,7 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
     // the share; k of the warp's 64 R parts hold a value at least as good as the k-th best of these, so the k-th best of
     // the row does too.  With 64 parts and k = 32 about 45 of 4096 elements then pass, instead of some 300 with a list
     // that starts empty, whose sorts were most of the time.  The second read of the share comes from L2.
+    bool infinities = true;                         // whether the share may hold the infinity on the better side
     if (BOUNDED && c_end - c_begin >= TOPK_BOUND_SHARE * R) {
       constexpr int PARTS = 2 * R;
       float ext[PARTS];
@@ -302,6 +303,10 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
                        : fminf(fminf(fminf(e, f[g].x), fminf(f[g].y, f[g].z)), f[g].w);
         }
       }
+      bool infinite = false;
+#pragma unroll
+      for (int g = 0; g < PARTS; ++g) infinite |= ext[g] == (TOP_MODE ? INFINITY : -INFINITY);
+      infinities = __any_sync(0xffffffffu, infinite);
       unsigned better[PARTS];                       // larger is better; 0 for a part whose extreme is not finite
 #pragma unroll
       for (int g = 0; g < PARTS; ++g) better[g] = !isfinite(ext[g]) ? 0u : (TOP_MODE ? orderable(ext[g]) : ~orderable(ext[g]));
@@ -352,14 +357,14 @@ rank_topk_kernel(const float* __restrict__ in, float* __restrict__ out_v, int* _
         unsigned marks = 0;
 #pragma unroll
         for (int j = 0; j < 16; ++j) marks |= near(v[j]) ? 1u << j : 0u;
-        for (int round = 0; __any_sync(0xffffffffu, marks != 0); ++round) {
-          // Many marks: the infinity on the better side passes every bound, and is left out before it takes a round.  us with seven of
-          // ten -inf, bottom k, with a round for each and so: 1257 x 26588, k = 4, 153 and 84; 1235 x 9029, k = 31, 73 and 56.
-          if (round == 2) {
+        // The infinity on the better side passes every bound, and every element that passes takes a round: 1257 x 26588, seven of ten -inf,
+        // bottom 4, 155 us so and 57 without their marks.  Only where there is one: 4096 x 4096, k = 32, 27 us with a comparison each.
+        if (infinities) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (!isfinite(v[i])) marks &= ~(1u << i);
-          }
+          for (int j = 0; j < 16; ++j)
+            if (isinf(v[j])) marks &= ~(1u << j);
+        }
+        while (__any_sync(0xffffffffu, marks != 0)) {
           const int j = marks ? __ffs(marks) - 1 : 0;
           float e8[8], e4[4], e2[2];                      // v[j]
 #pragma unroll
