@@ -22,9 +22,10 @@ __device__ __forceinline__ void chain_begin(P&... pointers) {
 // Between two kernels of a forward pass this saves the 1 to 2 us of launch latency and ramp-up.  A captured launch is an
 // ordinary one: a graph's edges to copies, fills and other streams' nodes only exist in that form.
 // in_order: the launch of such a kernel that starts when the one before it has completed.  For one that reads much through L1: an SM keeps
-// the split of its memory between L1 and shared memory while blocks follow one another, and a product leaves 28 KB of L1.  And for one
-// that leaves SMs to another stream: early blocks would hold SMs of that stream for as long as the kernel before them runs, beyond the
-// number left to this one (of two products of 40 blocks, 330 us each, the second's blocks were there 50 to 80 us after the first's).
+// the split of its memory between L1 and shared memory while blocks follow one another, and a product leaves 28 KB of L1.  For one of
+// a few heavy blocks per SM: early ones pile up on the SMs that fall free first.  And for one that leaves SMs to another stream: early
+// blocks would hold SMs of that stream for as long as the kernel before them runs, beyond the number left to this one (of two
+// products of 40 blocks, 330 us each, the second's blocks were there 50 to 80 us after the first's).
 template <typename... P>
 struct ChainedLaunch {
   void (*kernel)(P...);

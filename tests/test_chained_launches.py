@@ -10,6 +10,7 @@ from spiraltorch_b200.ops import attention as A
 from spiraltorch_b200.ops import conv as C
 from spiraltorch_b200.ops import gemm as G
 from spiraltorch_b200.ops import multi, native
+from spiraltorch_b200.ops import rank as R
 
 CSRC = Path(__file__).resolve().parents[1] / "csrc"
 
@@ -111,6 +112,10 @@ def test_products_with_a_block_limit_wait_for_their_turn():
     assert times[1][0] >= times[0][1]
 
 
+def _select(x):
+    return R.topk(x, 40)
+
+
 def _bias_per_pair(q, bias):
     return A.attention_forward(q, q, q, False, attn_bias=bias)
 
@@ -125,12 +130,13 @@ def _bias_per_key(q, bias):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("op,kernel,dim", [(_bias_per_pair, "attn_fwd_kernel", 64),
+@pytest.mark.parametrize("op,kernel,dim", [(_select, "rank_topk_kernel", 0), (_bias_per_pair, "attn_fwd_kernel", 64),
                                            (_bias_per_pair_backward, "attn_bwd_kernel", 64), (_bias_per_key, "attn_fwd_pair_kernel", 128)])
 def test_kernels_that_start_in_order(op, kernel, dim):
-    """Attention that reads a bias through an L1 of its own size."""
+    """Selection, whose blocks would pile up on a few SMs, and attention that reads a bias through an L1 of its own size."""
     a = torch.randn(8192, 4096, device="cuda").bfloat16()
-    args = torch.randn(24, 256, 8, dim, device="cuda").bfloat16(), torch.randn(24, 256, 256, device="cuda")
+    args = (torch.randn(500, 3000, device="cuda"),) if not dim else (torch.randn(24, 256, 8, dim, device="cuda").bfloat16(),
+                                                                     torch.randn(24, 256, 256, device="cuda"))
 
     def both():
         G.gemm(a, a)
